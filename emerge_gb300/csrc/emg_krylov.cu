@@ -31,6 +31,16 @@ __device__ __forceinline__ double2 cdiv(double2 a, double2 b) {
     const double d = b.x * b.x + b.y * b.y;
     return make_double2((a.x * b.x + a.y * b.y) / d, (a.y * b.x - a.x * b.y) / d);
 }
+// s += a b, s -= a b, s += conj(a) b in four FMAs each (cmul + cadd takes six operations of the
+// FP64 pipe, which bounds every FP64 kernel of this file: 1.18 TFLOP/s against 6.8 TB/s)
+__device__ __forceinline__ void cfma(double2& s, double2 a, double2 b) {
+    s.x = fma(a.x, b.x, s.x);
+    s.y = fma(a.x, b.y, s.y);
+    s.x = fma(-a.y, b.y, s.x);
+    s.y = fma(a.y, b.x, s.y);
+}
+__device__ __forceinline__ void cfms(double2& s, double2 a, double2 b) { cfma(s, make_double2(-a.x, -a.y), b); }
+__device__ __forceinline__ void cfmac(double2& s, double2 a, double2 b) { cfma(s, make_double2(a.x, -a.y), b); }
 __device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
 __device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 
@@ -68,19 +78,61 @@ __global__ void k_map(int64_t ns, const int64_t* __restrict__ sid, int32_t* map)
         map[sid[r]] = (int32_t)r;
 }
 
-// A[k][m] = E[s] - k2[m] B[s] + sum_p gam[p][m] P[p][s],  s = src[k]
-__global__ void k_form(int64_t nnz_r, int64_t Bm, const int64_t* __restrict__ src, const double2* __restrict__ E,
-                       const double2* __restrict__ B, const double* __restrict__ k2, int64_t n_ports,
-                       const double2* __restrict__ P, int64_t nnz_full, const double2* __restrict__ gam,
-                       double2* __restrict__ A) {
-    const int64_t total = nnz_r * Bm;
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t k = t / Bm, m = t % Bm;
-        const int64_t s = src[k];
-        const double2 e = E[s], b = B[s];
-        double2 v = make_double2(e.x - k2[m] * b.x, e.y - k2[m] * b.y);
-        for (int64_t p = 0; p < n_ports; ++p) v = cadd(v, cmul(gam[p * Bm + m], P[p * nnz_full + s]));
-        A[t] = v;
+// A[k][m] = E[s] - k2[m] B[s] + sum_p gam[p][m] P[p][s],  s = src[k].  A block stages the
+// values of kFormRows entries (one load per thread, all in flight) and stores their Bm
+// matrices.  A port matrix is zero off its own face, and a zero entry adds nothing for a
+// finite gamma: those products, 4/5 of the FP64 work, are skipped (a non-finite gamma takes
+// them all), which leaves the store of A as the bound.  Per-element gathers of E, B and P
+// and the port products took 1.86 ms for 45 frequencies of a 45k-DOF filter (1.2 GB of A);
+// form and product together 3.64 -> 1.42 ms.
+constexpr int kFormRows = 64, kFormPorts = 4;
+__global__ void __launch_bounds__(256) k_form(int64_t nnz_r, int64_t Bm, const int64_t* __restrict__ src,
+                                              const double2* __restrict__ E, const double2* __restrict__ B,
+                                              const double* __restrict__ k2, int64_t n_ports,
+                                              const double2* __restrict__ P, int64_t nnz_full,
+                                              const double2* __restrict__ gam, double2* __restrict__ A) {
+    __shared__ double2 val[2 + kFormPorts][kFormRows];
+    __shared__ int64_t pos[kFormRows];
+    __shared__ int on_port[kFormRows];
+    const int tid = threadIdx.x;
+    bool odd = false;
+    for (int64_t i = tid; i < n_ports * Bm; i += blockDim.x) odd |= !isfinite(gam[i].x) || !isfinite(gam[i].y);
+    const bool all = __syncthreads_or(odd);
+    const int np = (int)min(n_ports, (int64_t)kFormPorts);
+    const int64_t k0 = (int64_t)blockIdx.x * kFormRows;
+    const int nk = (int)min((int64_t)kFormRows, nnz_r - k0);
+    for (int i = tid; i < nk; i += blockDim.x) {
+        pos[i] = src[k0 + i];
+        on_port[i] = all;
+    }
+    __syncthreads();
+    for (int i = tid; i < (2 + np) * kFormRows; i += blockDim.x) {
+        const int a = i / kFormRows, kk = i % kFormRows;
+        if (kk >= nk) continue;
+        const double2 v = a == 0 ? E[pos[kk]] : a == 1 ? B[pos[kk]] : P[(int64_t)(a - 2) * nnz_full + pos[kk]];
+        val[a][kk] = v;
+        if (a >= 2 && !(v.x == 0.0 && v.y == 0.0)) on_port[kk] = 1;
+    }
+    for (int64_t p = np; p < n_ports; ++p)
+        for (int kk = tid; kk < nk; kk += blockDim.x) {
+            const double2 v = P[p * nnz_full + pos[kk]];
+            if (!(v.x == 0.0 && v.y == 0.0)) on_port[kk] = 1;
+        }
+    __syncthreads();
+    const int64_t cnt = nk * Bm, dk = blockDim.x / Bm, dm = blockDim.x % Bm;
+    int64_t kk = tid / Bm, m = tid % Bm;
+    double2* out = A + k0 * Bm;
+    for (int64_t t = tid; t < cnt; t += blockDim.x) {
+        const double2 e = val[0][kk], b = val[1][kk];
+        const double q = -k2[m];
+        double2 v = make_double2(fma(q, b.x, e.x), fma(q, b.y, e.y));
+        if (on_port[kk])
+            for (int64_t p = 0; p < n_ports; ++p)
+                cfma(v, gam[p * Bm + m], p < np ? val[2 + p][kk] : P[p * nnz_full + pos[kk]]);
+        out[t] = v;
+        kk += dk;
+        m += dm;
+        if (m >= Bm) { m -= Bm; ++kk; }
     }
 }
 
@@ -163,43 +215,61 @@ __global__ void k_trsv_level_w(int64_t nrows, const int32_t* __restrict__ rows, 
     }
 }
 
-__global__ void k_spmv_w(int64_t n, int64_t Bc, const int32_t* __restrict__ cmat, int64_t Bm,
+// Few columns (Bc <= CB): kSpmvLanes lanes per row.  Four lanes leave two shuffle levels of
+// FP64 adds for eight rows of a warp; a warp per row spends more of the FP64 pipe on its
+// five levels and on the idle lanes of a 41-entry row than on the products (2 columns on
+// 264k rows: 1451 -> 201 us).
+constexpr int kSpmvLanes = 4;
+template <int CB>
+__global__ void k_spmv_w(int64_t n, int Bc, const int32_t* __restrict__ cmat, int64_t Bm,
                          const int64_t* __restrict__ rptr, const int32_t* __restrict__ rind, const double2* __restrict__ A,
                          const double2* __restrict__ X, const double2* __restrict__ Bv, double2* __restrict__ Y) {
-    const int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (i >= n) return;
-    double2 acc[kSmallBc];
+    const int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / kSpmvLanes;
+    const int lane = threadIdx.x % kSpmvLanes;
+    if (blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31) >= n * kSpmvLanes) return;   // whole warps
+    double2 acc[CB];
+    int64_t cm[CB];
 #pragma unroll
-    for (int c = 0; c < kSmallBc; ++c) acc[c] = make_double2(0.0, 0.0);
-    for (int64_t k = rptr[i] + lane; k < rptr[i + 1]; k += 32) {
-        const int64_t col = rind[k];
+    for (int c = 0; c < CB; ++c) {
+        acc[c] = make_double2(0.0, 0.0);
+        cm[c] = c < Bc ? cmat[c] : 0;
+    }
+    if (i < n) {
+        const int64_t k1 = rptr[i + 1];
+        for (int64_t k = rptr[i] + lane; k < k1; k += kSpmvLanes) {
+            const double2* x = X + (int64_t)rind[k] * Bc;
+            const double2* a = A + k * Bm;
 #pragma unroll
-        for (int c = 0; c < kSmallBc; ++c)
-            if (c < Bc) acc[c] = cadd(acc[c], cmul(A[k * Bm + cmat[c]], X[col * Bc + c]));
+            for (int c = 0; c < CB; ++c)
+                if (c < Bc) cfma(acc[c], a[cm[c]], x[c]);
+        }
     }
 #pragma unroll
-    for (int c = 0; c < kSmallBc; ++c) {
+    for (int c = 0; c < CB; ++c) {
         if (c >= Bc) break;
         double2 v = acc[c];
-        for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+        for (int o = kSpmvLanes / 2; o > 0; o >>= 1) {
             v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
             v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
         }
-        if (lane == 0) Y[i * Bc + c] = Bv ? csub(Bv[i * Bc + c], v) : v;
+        if (i < n && lane == c % kSpmvLanes) Y[i * Bc + c] = Bv ? csub(Bv[i * Bc + c], v) : v;
     }
 }
 
-// Y = A X (batched, thread per (row, column)); alpha*A X + beta*Y when add.
+// Y = A X (batched, thread per (row, column)), or Bv - A X.
 __global__ void k_spmv(int64_t n, int64_t Bc, const int32_t* __restrict__ cmat, int64_t Bm,
                        const int64_t* __restrict__ rptr, const int32_t* __restrict__ rind, const double2* __restrict__ A,
                        const double2* __restrict__ X, const double2* __restrict__ Bv, double2* __restrict__ Y) {
     const int64_t total = n * Bc;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
         const int64_t i = t / Bc, c = t % Bc;
-        const int64_t m = cmat[c];
+        const double2* a = A + cmat[c];
+        const double2* x = X + c;
         double2 s = make_double2(0.0, 0.0);
-        for (int64_t k = rptr[i]; k < rptr[i + 1]; ++k) s = cadd(s, cmul(A[k * Bm + m], X[(int64_t)rind[k] * Bc + c]));
+        const int64_t k1 = rptr[i + 1];
+#pragma unroll 4
+        for (int64_t k = rptr[i]; k < k1; ++k) cfma(s, a[k * Bm], x[(int64_t)rind[k] * Bc]);
         // Bv != nullptr: Y = Bv - A X (residual)
         Y[t] = Bv ? csub(Bv[t], s) : s;
     }
@@ -222,54 +292,90 @@ __global__ void k_spmv_fam(int64_t n, int64_t nnz, int64_t Bc, int nfam, const d
             double2 v = make_double2(0.0, 0.0);
 #pragma unroll
             for (int a = 0; a < kMaxFamily; ++a)
-                if (a < nfam) v = cadd(v, cmul(cf[a], fam[a * nnz + k]));
-            s = cadd(s, cmul(v, X[(int64_t)rind[k] * Bc + c]));
+                if (a < nfam) cfma(v, cf[a], fam[a * nnz + k]);
+            cfma(s, v, X[(int64_t)rind[k] * Bc + c]);
         }
         Y[t] = Bv ? csub(Bv[t], s) : s;
     }
 }
 
 // Column-wise partial dots: part[blk][j][c] = sum_{rows in blk} conj(V_j[r,c]) W[r,c], j < nj.
-constexpr int kDotRows = 1024;
+// A block of 256 threads owns ``rows`` rows, a tile of cw columns and kDotJ vectors: the
+// threads lie over (row group, column), so a warp reads contiguous values for any column
+// count, each value of W serves kDotJ products, and the row groups are reduced in shared
+// memory in a fixed order.  Bound by the FP64 pipe (4 DFMA per product).  A thread per
+// column walking 1024 rows left 97 blocks with one load in flight each (48 columns, 98k
+// rows, 13 vectors on average: 3553 -> 276 us a call).
+constexpr int kDotThreads = 256, kDotJ = 4;
 constexpr int kMaxRestart = 256;
-__global__ void k_dots_partial(int64_t n, int64_t Bc, int nj, const double2* __restrict__ V, int64_t vstride,
-                               const double2* __restrict__ W, double2* __restrict__ part) {
-    const int64_t c = blockIdx.y * (int64_t)blockDim.x + threadIdx.x;
-    if (c >= Bc) return;
-    const int64_t r0 = (int64_t)blockIdx.x * kDotRows, r1 = min(n, r0 + kDotRows);
-    for (int j = 0; j < nj; ++j) {
-        double2 s = make_double2(0.0, 0.0);
-        const double2* Vj = V + j * vstride;
-        for (int64_t r = r0; r < r1; ++r) s = cadd(s, cmulc(Vj[r * Bc + c], W[r * Bc + c]));
-        part[((int64_t)blockIdx.x * nj + j) * Bc + c] = s;
-    }
+__device__ __forceinline__ void dot_acc(double2& s, double2 v, double2 w) { cfmac(s, v, w); }
+__device__ __forceinline__ void dot_acc(float2& s, float2 v, float2 w) {
+    s.x = fmaf(v.x, w.x, s.x);
+    s.y = fmaf(v.x, w.y, s.y);
+    s.x = fmaf(v.y, w.y, s.x);
+    s.y = fmaf(-v.y, w.x, s.y);
 }
-
-// Small batches (Bc < 32): warp per (vector j, column c) pair, lanes over rows.
-__global__ void k_dots_partial_small(int64_t n, int64_t Bc, int nj, const double2* __restrict__ V, int64_t vstride,
-                                     const double2* __restrict__ W, double2* __restrict__ part) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const int64_t r0 = (int64_t)blockIdx.x * kDotRows, r1 = min(n, r0 + kDotRows);
-    for (int64_t pr = warp; pr < (int64_t)nj * Bc; pr += nw) {
-        const int64_t j = pr / Bc, c = pr % Bc;
-        const double2* Vj = V + j * vstride;
-        double2 s = make_double2(0.0, 0.0);
-        for (int64_t r = r0 + lane; r < r1; r += 32) s = cadd(s, cmulc(Vj[r * Bc + c], W[r * Bc + c]));
-        for (int o = 16; o > 0; o >>= 1) {
-            s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
-            s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+template <typename T>
+__global__ void __launch_bounds__(kDotThreads) k_dots_partial(int64_t n, int Bc, int cw, int nj, int64_t rows,
+                                                              const T* __restrict__ V, int64_t vstride,
+                                                              const T* __restrict__ W, double2* __restrict__ part) {
+    __shared__ double2 red[kDotJ][kDotThreads];
+    const int tid = threadIdx.x, groups = kDotThreads / cw, g = tid / cw, cl = tid - g * cw;
+    const int c = (int)blockIdx.y * cw + cl, j0 = (int)blockIdx.z * kDotJ, jn = min(kDotJ, nj - j0);
+    const int64_t r0 = (int64_t)blockIdx.x * rows, r1 = min(n, r0 + rows);
+    T acc[kDotJ];
+#pragma unroll
+    for (int j = 0; j < kDotJ; ++j) acc[j].x = acc[j].y = 0;
+    if (g < groups && c < Bc) {
+        const T* Vb = V + j0 * vstride;
+        if (jn == kDotJ) {
+#pragma unroll 2
+            for (int64_t r = r0 + g; r < r1; r += groups) {
+                const int64_t t = r * Bc + c;
+                const T w = W[t];
+#pragma unroll
+                for (int j = 0; j < kDotJ; ++j) dot_acc(acc[j], Vb[j * vstride + t], w);
+            }
+        } else {
+            for (int64_t r = r0 + g; r < r1; r += groups) {
+                const int64_t t = r * Bc + c;
+                const T w = W[t];
+#pragma unroll
+                for (int j = 0; j < kDotJ - 1; ++j)
+                    if (j < jn) dot_acc(acc[j], Vb[j * vstride + t], w);
+            }
         }
-        if (lane == 0) part[((int64_t)blockIdx.x * nj + j) * Bc + c] = s;
     }
+#pragma unroll
+    for (int j = 0; j < kDotJ; ++j) red[j][tid] = make_double2(acc[j].x, acc[j].y);
+    for (int left = groups; left > 1;) {
+        const int half = (left + 1) / 2;
+        __syncthreads();
+        if (g < left - half) {
+#pragma unroll
+            for (int j = 0; j < kDotJ; ++j) red[j][tid] = cadd(red[j][tid], red[j][tid + half * cw]);
+        }
+        left = half;
+    }
+    __syncthreads();
+    if (g == 0 && c < Bc)
+        for (int j = 0; j < jn; ++j) part[((int64_t)blockIdx.x * nj + j0 + j) * Bc + c] = red[j][tid];
 }
 
+// out[j][c] = sum of the nblk partials: a warp per (j, c), lanes over the blocks
 __global__ void k_dots_final(int64_t nblk, int64_t Bc, int nj, const double2* __restrict__ part, double2* __restrict__ out) {
-    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (t >= (int64_t)nj * Bc) return;
-    const int64_t j = t / Bc, c = t % Bc;
+    const int64_t t = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    const int64_t cnt = (int64_t)nj * Bc;
+    if (t >= cnt) return;
     double2 s = make_double2(0.0, 0.0);
-    for (int64_t b = 0; b < nblk; ++b) s = cadd(s, part[(b * nj + j) * Bc + c]);
-    out[t] = s;
+    for (int64_t b = lane; b < nblk; b += 32) s = cadd(s, part[b * cnt + t]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+        s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+    }
+    if (lane == 0) out[t] = s;
 }
 
 // W[r,c] -= sum_j h[j][c] V_j[r,c]   (masked columns untouched)
@@ -280,7 +386,8 @@ __global__ void k_orth_update(int64_t n, int64_t Bc, int nj, const double2* __re
         const int64_t c = t % Bc;
         if (!active[c]) continue;
         double2 w = W[t];
-        for (int j = 0; j < nj; ++j) w = csub(w, cmul(h[(int64_t)j * Bc + c], V[j * vstride + t]));
+#pragma unroll 4
+        for (int j = 0; j < nj; ++j) cfms(w, h[(int64_t)j * Bc + c], V[j * vstride + t]);
         W[t] = w;
     }
 }
@@ -303,7 +410,7 @@ __global__ void k_combine_basis(int64_t n, int64_t Bc, int nj, const double2* __
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
         const int64_t c = t % Bc;
         double2 x = X[t];
-        for (int j = 0; j < nj; ++j) x = cadd(x, cmul(y[(int64_t)j * Bc + c], Z[j * zstride + t]));
+        for (int j = 0; j < nj; ++j) cfma(x, y[(int64_t)j * Bc + c], Z[j * zstride + t]);
         X[t] = x;
     }
 }
@@ -423,7 +530,6 @@ __global__ void k_sqrt_real(int64_t Bc, const double2* __restrict__ in, double* 
 }
 
 // ---- FP32-vector kernels for the inner solves of the mixed-precision refinement ----
-__device__ __forceinline__ float2 fmulc(float2 a, float2 b) { return make_float2(a.x * b.x + a.y * b.y, a.x * b.y - a.y * b.x); }
 __device__ __forceinline__ void ffma(float2& acc, float2 a, float2 b) {
     acc.x = fmaf(a.x, b.x, acc.x);
     acc.x = fmaf(-a.y, b.y, acc.x);
@@ -468,45 +574,6 @@ __global__ void k_spmv32_w(int64_t n, int64_t Bc, const int32_t* __restrict__ cm
             v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
         }
         if (lane == 0) Y[i * Bc + c] = Bv ? make_float2(Bv[i * Bc + c].x - v.x, Bv[i * Bc + c].y - v.y) : v;
-    }
-}
-
-// partial dots over kDotRows rows: FP32 products and running sums, FP64 block partials
-__global__ void k_dots32(int64_t n, int64_t Bc, int nj, const float2* __restrict__ V, int64_t vstride,
-                         const float2* __restrict__ W, double2* __restrict__ part) {
-    const int64_t c = blockIdx.y * (int64_t)blockDim.x + threadIdx.x;
-    if (c >= Bc) return;
-    const int64_t r0 = (int64_t)blockIdx.x * kDotRows, r1 = min(n, r0 + kDotRows);
-    for (int j = 0; j < nj; ++j) {
-        float2 s = make_float2(0.f, 0.f);
-        const float2* Vj = V + j * vstride;
-        for (int64_t r = r0; r < r1; ++r) {
-            const float2 p = fmulc(Vj[r * Bc + c], W[r * Bc + c]);
-            s.x += p.x;
-            s.y += p.y;
-        }
-        part[((int64_t)blockIdx.x * nj + j) * Bc + c] = make_double2(s.x, s.y);
-    }
-}
-
-__global__ void k_dots32_small(int64_t n, int64_t Bc, int nj, const float2* __restrict__ V, int64_t vstride,
-                               const float2* __restrict__ W, double2* __restrict__ part) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const int64_t r0 = (int64_t)blockIdx.x * kDotRows, r1 = min(n, r0 + kDotRows);
-    for (int64_t pr = warp; pr < (int64_t)nj * Bc; pr += nw) {
-        const int64_t j = pr / Bc, c = pr % Bc;
-        const float2* Vj = V + j * vstride;
-        float2 s = make_float2(0.f, 0.f);
-        for (int64_t r = r0 + lane; r < r1; r += 32) {
-            const float2 p = fmulc(Vj[r * Bc + c], W[r * Bc + c]);
-            s.x += p.x;
-            s.y += p.y;
-        }
-        for (int o = 16; o > 0; o >>= 1) {
-            s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
-            s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
-        }
-        if (lane == 0) part[((int64_t)blockIdx.x * nj + j) * Bc + c] = make_double2(s.x, s.y);
     }
 }
 
@@ -731,7 +798,7 @@ extern "C" int emg_rplan_form(const emg_rplan* p, int64_t Bm, const double* E, c
     EMG_CHECK_ARG(p && E && B && k2 && A && Bm > 0 && n_ports >= 0 && (n_ports == 0 || (P && gam)),
                   "emg_rplan_form: bad argument");
     if (p->nnz == 0) return EMG_OK;
-    kry::k_form<<<grid_for(p->nnz * Bm, 256), 256, 0, (cudaStream_t)stream>>>(
+    kry::k_form<<<(unsigned)((p->nnz + kry::kFormRows - 1) / kry::kFormRows), 256, 0, (cudaStream_t)stream>>>(
         p->nnz, Bm, p->rsrc, reinterpret_cast<const double2*>(E), reinterpret_cast<const double2*>(B), k2, n_ports,
         reinterpret_cast<const double2*>(P), p->nnz_full, reinterpret_cast<const double2*>(gam),
         reinterpret_cast<double2*>(A));
@@ -786,9 +853,12 @@ extern "C" int emg_spmv(const emg_rplan* p, int64_t Bc, const int32_t* cmat, int
     using namespace emg;
     EMG_CHECK_ARG(p && cmat && A && X && Y && Bc > 0 && Bm > 0, "emg_spmv: bad argument");
     if (p->ns == 0) return EMG_OK;
-    kry::k_spmv<<<grid_for(p->ns * Bc, 256), 256, 0, (cudaStream_t)stream>>>(
-        p->ns, Bc, cmat, Bm, p->rptr, p->rind, reinterpret_cast<const double2*>(A), reinterpret_cast<const double2*>(X),
-        reinterpret_cast<const double2*>(Bv), reinterpret_cast<double2*>(Y));
+    MatArg M;
+    M.A = reinterpret_cast<const double2*>(A);
+    M.Bm = Bm;
+    M.cmat = cmat;
+    spmv_op(p, Bc, M, reinterpret_cast<const double2*>(X), reinterpret_cast<const double2*>(Bv),
+            reinterpret_cast<double2*>(Y), (cudaStream_t)stream);
     EMG_CUDA(cudaGetLastError());
     return EMG_OK;
 }
@@ -841,20 +911,29 @@ namespace {
 void spmv(const emg_rplan* p, int64_t Bc, const int32_t* cmat, int64_t Bm, const double2* A, const double2* X,
           const double2* Bv, double2* Y, cudaStream_t s) {
     const int64_t n = p->ns;
-    if (Bc <= kry::kSmallBc)
-        kry::k_spmv_w<<<(unsigned)((n * 32 + 127) / 128), 128, 0, s>>>(n, Bc, cmat, Bm, p->rptr, p->rind, A, X, Bv, Y);
+    const unsigned g = (unsigned)((n * kry::kSpmvLanes + 127) / 128);
+    if (Bc <= 2)
+        kry::k_spmv_w<2><<<g, 128, 0, s>>>(n, (int)Bc, cmat, Bm, p->rptr, p->rind, A, X, Bv, Y);
+    else if (Bc <= 4)
+        kry::k_spmv_w<4><<<g, 128, 0, s>>>(n, (int)Bc, cmat, Bm, p->rptr, p->rind, A, X, Bv, Y);
+    else if (Bc <= kry::kSmallBc)
+        kry::k_spmv_w<kry::kSmallBc><<<g, 128, 0, s>>>(n, (int)Bc, cmat, Bm, p->rptr, p->rind, A, X, Bv, Y);
     else
         kry::k_spmv<<<grid_for(n * Bc, 256), 256, 0, s>>>(n, Bc, cmat, Bm, p->rptr, p->rind, A, X, Bv, Y);
 }
 
-void dots(int64_t n, int64_t Bc, int nj, const double2* V, int64_t vstride, const double2* W, double2* part,
-          int64_t nblk, cudaStream_t s) {
-    if (Bc < 32) {
-        kry::k_dots_partial_small<<<(unsigned)nblk, 256, 0, s>>>(n, Bc, nj, V, vstride, W, part);
-    } else {
-        const dim3 g((unsigned)nblk, (unsigned)((Bc + 127) / 128));
-        kry::k_dots_partial<<<g, 128, 0, s>>>(n, Bc, nj, V, vstride, W, part);
-    }
+// Rows of a block of the partial dots: two blocks per SM where there are at least 64 rows
+// for each (fewer spend more on the reduction than on the products).
+int64_t dot_rows(int64_t n) { return std::max<int64_t>(64, (n + 2 * 152 - 1) / (2 * 152)); }
+
+template <typename T>
+void dots(int64_t n, int64_t Bc, int nj, const T* V, int64_t vstride, const T* W, double2* part, double2* out,
+          cudaStream_t s) {
+    const int64_t rows = dot_rows(n), nblk = (n + rows - 1) / rows;
+    const int ct = (int)((Bc + 127) / 128), cw = (int)((Bc + ct - 1) / ct);
+    const dim3 g((unsigned)nblk, (unsigned)ct, (unsigned)((nj + kry::kDotJ - 1) / kry::kDotJ));
+    kry::k_dots_partial<T><<<g, kry::kDotThreads, 0, s>>>(n, (int)Bc, cw, nj, rows, V, vstride, W, part);
+    kry::k_dots_final<<<(unsigned)(((int64_t)nj * Bc * 32 + 127) / 128), 128, 0, s>>>(nblk, Bc, nj, part, out);
 }
 }  // namespace
 
@@ -883,7 +962,7 @@ int gmres_run(emg_rplan* p, int64_t Bc, const MatArg& A, const double2* rhs, dou
     cudaStream_t s = p->gs;
     const int m = restart;
     const int64_t vec = n * Bc;
-    const int64_t nblk = (n + kry::kDotRows - 1) / kry::kDotRows;
+    const int64_t nblk = (n + dot_rows(n) - 1) / dot_rows(n);
     // workspace layout
     size_t off = 0;
     auto take = [&](size_t bytes) { size_t o = off; off = (off + bytes + 255) & ~(size_t)255; return o; };
@@ -934,11 +1013,9 @@ int gmres_run(emg_rplan* p, int64_t Bc, const MatArg& A, const double2* rhs, dou
     auto* res = reinterpret_cast<double*>(base + oRes);
     auto* its = reinterpret_cast<int32_t*>(base + oIt);
     const int T = 256;
-    const dim3 dgrid((unsigned)nblk, (unsigned)((Bc + 127) / 128));
     const unsigned cgrid = (unsigned)((Bc + 127) / 128);
     auto norms2 = [&](const double2* Vv) {   // h1[c] = ||Vv[:,c]||^2 (real part)
-        dots(n, Bc, 1, Vv, vec, Vv, part, nblk, s);
-        kry::k_dots_final<<<cgrid, 128, 0, s>>>(nblk, Bc, 1, part, h1);
+        dots(n, Bc, 1, Vv, vec, Vv, part, h1, s);
         return h1;
     };
     kry::k_sqrt_real<<<cgrid, 128, 0, s>>>(Bc, norms2(rhs), bn);
@@ -952,15 +1029,11 @@ int gmres_run(emg_rplan* p, int64_t Bc, const MatArg& A, const double2* rhs, dou
         if (rc) return rc;
         spmv_op(p, Bc, A, Mv, nullptr, W, s);
         // CGS2: two passes of h = V^H w, w -= V h
-        const unsigned hgrid = (unsigned)(((int64_t)(j + 1) * Bc + 127) / 128);
-        dots(n, Bc, j + 1, V, vec, W, part, nblk, s);
-        kry::k_dots_final<<<hgrid, 128, 0, s>>>(nblk, Bc, j + 1, part, h1);
+        dots(n, Bc, j + 1, V, vec, W, part, h1, s);
         kry::k_orth_update<<<grid_for(vec, T), T, 0, s>>>(n, Bc, j + 1, V, vec, h1, act, W);
-        dots(n, Bc, j + 1, V, vec, W, part, nblk, s);
-        kry::k_dots_final<<<hgrid, 128, 0, s>>>(nblk, Bc, j + 1, part, h2);
+        dots(n, Bc, j + 1, V, vec, W, part, h2, s);
         kry::k_orth_update<<<grid_for(vec, T), T, 0, s>>>(n, Bc, j + 1, V, vec, h2, act, W);
-        dots(n, Bc, 1, W, vec, W, part, nblk, s);
-        kry::k_dots_final<<<cgrid, 128, 0, s>>>(nblk, Bc, 1, part, y);
+        dots(n, Bc, 1, W, vec, W, part, y, s);
         kry::k_real<<<cgrid, 128, 0, s>>>(Bc, y, wn);
         kry::k_arnoldi_col<<<cgrid, 128, 0, s>>>(Bc, j, m, h1, h2, wn, H, cs, sn, g, bn, tol, act, len, vs, res);
         kry::k_scale_cols<<<grid_for(vec, T), T, 0, s>>>(n, Bc, vs, W, V + (int64_t)(j + 1) * vec);
@@ -1064,21 +1137,11 @@ void spmv32(const emg_rplan* p, int64_t Bc, const int32_t* cmat, int64_t Bm, con
         kry::k_spmv32<<<grid_for(n * Bc, 256), 256, 0, s>>>(n, Bc, cmat, Bm, p->rptr, p->rind, A, X, Bv, Y);
 }
 
-void dots32(int64_t n, int64_t Bc, int nj, const float2* V, int64_t vstride, const float2* W, double2* part,
-            int64_t nblk, cudaStream_t s) {
-    if (Bc < 32) {
-        kry::k_dots32_small<<<(unsigned)nblk, 256, 0, s>>>(n, Bc, nj, V, vstride, W, part);
-    } else {
-        const dim3 g((unsigned)nblk, (unsigned)((Bc + 127) / 128));
-        kry::k_dots32<<<g, 128, 0, s>>>(n, Bc, nj, V, vstride, W, part);
-    }
-}
-
 // Workspace of the inner FP32 FGMRES (carved once per ir_run, reused by every step
 // so the captured Arnoldi-step graphs stay valid across refinement steps).
 struct Inner32 {
     int m = 0;
-    int64_t vec = 0, nblk = 0;
+    int64_t vec = 0;
     float2 *V = nullptr, *Z = nullptr, *W = nullptr;
     double2 *part = nullptr, *h1 = nullptr, *h2 = nullptr, *H = nullptr, *cs = nullptr, *sn = nullptr, *g = nullptr,
             *y = nullptr;
@@ -1096,12 +1159,11 @@ struct Inner32 {
 int gmres32(emg_rplan* p, int64_t Bc, const int32_t* cmat, int64_t Bm, const float2* A32, const float2* rhs,
             float2* x, int max_iter, double tol, Inner32& w, std::vector<int32_t>& hits, cudaStream_t s,
             Precond32& M) {
-    const int64_t n = p->ns, vec = w.vec, nblk = w.nblk;
+    const int64_t n = p->ns, vec = w.vec;
     const int m = w.m, T = 256;
     const unsigned cgrid = (unsigned)((Bc + 127) / 128);
     auto norms2 = [&](const float2* Vv) {
-        dots32(n, Bc, 1, Vv, vec, Vv, w.part, nblk, s);
-        kry::k_dots_final<<<cgrid, 128, 0, s>>>(nblk, Bc, 1, w.part, w.h1);
+        dots(n, Bc, 1, Vv, vec, Vv, w.part, w.h1, s);
         return w.h1;
     };
     kry::k_sqrt_real<<<cgrid, 128, 0, s>>>(Bc, norms2(rhs), w.bn);
@@ -1111,15 +1173,11 @@ int gmres32(emg_rplan* p, int64_t Bc, const int32_t* cmat, int64_t Bm, const flo
         int rc = M.apply(Vj, Zj, s);
         if (rc) return rc;
         spmv32(p, Bc, cmat, Bm, A32, Zj, nullptr, w.W, s);
-        const unsigned hgrid = (unsigned)(((int64_t)(j + 1) * Bc + 127) / 128);
-        dots32(n, Bc, j + 1, w.V, vec, w.W, w.part, nblk, s);
-        kry::k_dots_final<<<hgrid, 128, 0, s>>>(nblk, Bc, j + 1, w.part, w.h1);
+        dots(n, Bc, j + 1, w.V, vec, w.W, w.part, w.h1, s);
         kry::k_orth32<<<grid_for(vec, T), T, 0, s>>>(n, Bc, j + 1, w.V, vec, w.h1, w.act, w.W);
-        dots32(n, Bc, j + 1, w.V, vec, w.W, w.part, nblk, s);
-        kry::k_dots_final<<<hgrid, 128, 0, s>>>(nblk, Bc, j + 1, w.part, w.h2);
+        dots(n, Bc, j + 1, w.V, vec, w.W, w.part, w.h2, s);
         kry::k_orth32<<<grid_for(vec, T), T, 0, s>>>(n, Bc, j + 1, w.V, vec, w.h2, w.act, w.W);
-        dots32(n, Bc, 1, w.W, vec, w.W, w.part, nblk, s);
-        kry::k_dots_final<<<cgrid, 128, 0, s>>>(nblk, Bc, 1, w.part, w.y);
+        dots(n, Bc, 1, w.W, vec, w.W, w.part, w.y, s);
         kry::k_real<<<cgrid, 128, 0, s>>>(Bc, w.y, w.wn);
         kry::k_arnoldi_col<<<cgrid, 128, 0, s>>>(Bc, j, m, w.h1, w.h2, w.wn, w.H, w.cs, w.sn, w.g, w.bn, tol, w.act,
                                                  w.len, w.vs, w.res);
@@ -1194,7 +1252,7 @@ int ir_run(emg_rplan* p, int64_t Bc, const MatArg& A, const float2* A32, const d
     EMG_CUDA(cudaStreamWaitEvent(p->gs, p->ev_in, 0));
     cudaStream_t s = p->gs;
     const int m = restart, T = 256;
-    const int64_t vec = n * Bc, nblk = (n + kry::kDotRows - 1) / kry::kDotRows;
+    const int64_t vec = n * Bc, nblk = (n + dot_rows(n) - 1) / dot_rows(n);
     size_t off = 0;
     auto take = [&](size_t bytes) { size_t o = off; off = (off + bytes + 255) & ~(size_t)255; return o; };
     const size_t oR64 = take(sizeof(double2) * vec), oR32 = take(sizeof(float2) * vec), oD32 = take(sizeof(float2) * vec);
@@ -1222,7 +1280,6 @@ int ir_run(emg_rplan* p, int64_t Bc, const MatArg& A, const float2* A32, const d
     Inner32 w;
     w.m = m;
     w.vec = vec;
-    w.nblk = nblk;
     w.V = reinterpret_cast<float2*>(base + oV);
     w.Z = reinterpret_cast<float2*>(base + oZ);
     w.W = reinterpret_cast<float2*>(base + oW);
@@ -1246,8 +1303,7 @@ int ir_run(emg_rplan* p, int64_t Bc, const MatArg& A, const float2* A32, const d
     auto* sc = reinterpret_cast<double*>(base + oSc);
     const unsigned cgrid = (unsigned)((Bc + 127) / 128);
     // ||b|| in FP64
-    dots(n, Bc, 1, rhs, vec, rhs, w.part, nblk, s);
-    kry::k_dots_final<<<cgrid, 128, 0, s>>>(nblk, Bc, 1, w.part, w.h1);
+    dots(n, Bc, 1, rhs, vec, rhs, w.part, w.h1, s);
     kry::k_sqrt_real<<<cgrid, 128, 0, s>>>(Bc, w.h1, bn64);
     std::vector<double> hb(Bc), hr(Bc), hs(Bc), rel(Bc);
     EMG_CUDA(cudaMemcpyAsync(hb.data(), bn64, sizeof(double) * Bc, cudaMemcpyDeviceToHost, s));
@@ -1257,8 +1313,7 @@ int ir_run(emg_rplan* p, int64_t Bc, const MatArg& A, const float2* A32, const d
     for (;;) {
         // true residual in FP64
         spmv_op(p, Bc, A, x, rhs, r64, s);
-        dots(n, Bc, 1, r64, vec, r64, w.part, nblk, s);
-        kry::k_dots_final<<<cgrid, 128, 0, s>>>(nblk, Bc, 1, w.part, w.h1);
+        dots(n, Bc, 1, r64, vec, r64, w.part, w.h1, s);
         kry::k_sqrt_real<<<cgrid, 128, 0, s>>>(Bc, w.h1, rn);
         EMG_CUDA(cudaGetLastError());
         EMG_CUDA(cudaMemcpyAsync(hr.data(), rn, sizeof(double) * Bc, cudaMemcpyDeviceToHost, s));
