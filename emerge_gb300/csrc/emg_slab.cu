@@ -34,6 +34,7 @@
 #include <cmath>
 #include <vector>
 
+#include "emg_gj.cuh"
 #include "emg_krylov.cuh"
 
 namespace emg {
@@ -414,6 +415,24 @@ __global__ void __launch_bounds__(kDiagThreads, 1) k_gj_diag(int64_t w, int k, t
         }
 }
 
+// The FP32 pivot tile k by itself (emg_gj.cuh): M[k, k] and pinv receive its inverse.  Grid 1 x 1 x F.
+__global__ void __launch_bounds__(gj::kThreads, 1) k_gj_tile32(int64_t w, int k, float2* __restrict__ Sinv, int64_t totD,
+                                                               int64_t offD, float2* __restrict__ pinv, float rel_thr,
+                                                               int32_t* __restrict__ perturbed) {
+    __shared__ float2 Ts[kTile * gj::kLd];
+    __shared__ gj::PivotShared sh;
+    const int64_t f = blockIdx.z, k0 = (int64_t)k * kTile;
+    float2* M = Sinv + f * totD + offD + k0 * w + k0;
+    const int tb = (int)min((int64_t)kTile, w - k0);
+#pragma unroll
+    for (int q = 0; q < kTile * kTile / gj::kThreads; ++q) {
+        const int r = (threadIdx.x + q * gj::kThreads) / kTile, c = threadIdx.x % kTile;
+        Ts[r * gj::kLd + c] = (r < tb && c < tb) ? M[r * w + c] : make_float2(r == c ? 1.f : 0.f, 0.f);
+    }
+    __syncthreads();
+    gj::invert_tile(Ts, tb, rel_thr, sh, perturbed + f, M, w, pinv + f * kTile * kTile);
+}
+
 // mode 0: row panel  M[k, c] = Pinv M[k, c]       (grid: column tiles x 1 x F, c != k)
 // mode 1: col panel  M[r, k] = -M[r, k] Pinv      (grid: row tiles x 1 x F, r != k)
 // mode 2: update     M[r, c] -= M[r, k] M[k, c]   (grid: column tiles x row tiles x F, r, c != k),
@@ -474,6 +493,50 @@ __global__ void __launch_bounds__(kThreads) k_gj_panel(int mode, int64_t w, int 
                 else if (mode == 1) o = mk(-acc[i][j].x, -acc[i][j].y);
                 else { o.x -= acc[i][j].x; o.y -= acc[i][j].y; }
             }
+        }
+}
+
+// First half of step k for the tensor-core update: CTAs x < nt form the row panel M[k, c] = Pinv
+// M[k, c] (c != k), CTAs nt + r keep the column tiles M[r, k] in colbuf (rows of 64, zero
+// beyond the tile), so that the second half may overwrite them.  Grid: 2 nt x 1 x F.
+template <typename R>
+__global__ void __launch_bounds__(kThreads) k_gj_row(int64_t w, int k, int nt, typename C2<R>::T* __restrict__ Sinv,
+                                                     int64_t totD, int64_t offD, const typename C2<R>::T* __restrict__ pinv,
+                                                     typename C2<R>::T* __restrict__ colbuf, int64_t scol) {
+    using T = typename C2<R>::T;
+    __shared__ Tile<R> sm;
+    const int64_t f = blockIdx.z, k0 = (int64_t)k * kTile;
+    T* M = Sinv + f * totD + offD;
+    const int tb = (int)min((int64_t)kTile, w - k0);
+    const int tid = threadIdx.x;
+    const int bx = (int)blockIdx.x;
+    if (bx >= nt) {
+        const int64_t r0 = (int64_t)(bx - nt) * kTile;
+        T* out = colbuf + f * scol + r0 * kTile;
+#pragma unroll
+        for (int q = 0; q < kTile * kTile / kThreads; ++q) {
+            const int i = tid + q * kThreads, r = i / kTile, c = i % kTile;
+            if (r0 + r < w) out[i] = c < tb ? M[(r0 + r) * w + k0 + c] : czero<T>();
+        }
+        return;
+    }
+    if (bx == k) return;
+    const int ty = tid >> 4, tx = tid & 15;
+    const int64_t c0 = (int64_t)bx * kTile;
+    const int nc = (int)min((int64_t)kTile, w - c0);
+    T* out = M + k0 * w + c0;
+    T acc[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = czero<T>();
+    tile_mac<R>(acc, pinv + f * kTile * kTile, kTile, out, w, tb, nc, tb, sm);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int r = ty + 16 * i, c = tx + 16 * j;
+            if (r < tb && c < nc) out[(int64_t)r * w + c] = acc[i][j];
         }
 }
 
@@ -1159,6 +1222,13 @@ int slab_factor_t(emg_slab* s, int64_t F, const int32_t* amat_h, int64_t Bm, con
     rc = dalloc(&amat, F, "slab amat");
     if (rc) { slab_free_factors(s); return rc; }
     struct Tmp { int32_t* p; ~Tmp() { if (p) cudaFree(p); } } tmp{amat};
+    const bool tc_update = sizeof(R) == 4 && s->tc_factor;
+    T* colbuf = nullptr;   // old column panel of a tensor-core step
+    if (tc_update) {
+        rc = dalloc(&colbuf, F * s->maxw * kTile, "slab column panel");
+        if (rc) { slab_free_factors(s); return rc; }
+    }
+    struct TmpC { T* p; ~TmpC() { if (p) cudaFree(p); } } tmpc{colbuf};
     // Newton-Schulz scratch: a copy of S_i and the factor 2I - S_i X (F blocks of maxw^2)
     T *Scopy = nullptr, *Rbuf = nullptr;
     double* npart = nullptr;
@@ -1201,7 +1271,6 @@ int slab_factor_t(emg_slab* s, int64_t F, const int32_t* amat_h, int64_t Bm, con
     int prio_lo = 0, prio_hi = 0;
     EMG_CUDA(cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi));
     EMG_CUDA(cudaStreamCreateWithPriority(&side.st, cudaStreamNonBlocking, prio_hi));
-    const bool tc_update = sizeof(R) == 4 && s->tc_factor;
     if (tc_update && !s->tc_status) {
         rc = dalloc(&s->tc_status, 1, "slab tensor-core status");
         if (rc) return rc;
@@ -1227,34 +1296,48 @@ int slab_factor_t(emg_slab* s, int64_t F, const int32_t* amat_h, int64_t Bm, con
             EMG_CUDA(cudaMemcpy2DAsync(Scopy, sizeof(T) * sq, Sinv + s->offD[i], sizeof(T) * s->totD, sizeof(T) * w * w,
                                        (size_t)F, cudaMemcpyDeviceToDevice, st));
         // Block Gauss-Jordan over the tile steps with a one-step lookahead: the pivot tile
-        // of step k + 1 is updated first and inverted on the side stream while the rest
-        // of step k's update and its column panel run on st.  Step k + 1 waits for it.
+        // of step k + 1 is updated first and inverted while the rest of step k's update runs.
         T* const P0 = static_cast<T*>(s->pinv);
         auto pset = [&](int k) { return P0 + (int64_t)(k & 1) * F * kTile * kTile; };
-        k_gj_diag<R><<<dim3(1, 1, (unsigned)F), kDiagThreads, 0, st>>>(w, 0, Sinv, s->totD, s->offD[i], pset(0),
-                                                                  rel_thr, s->perturbed);
-        for (int k = 0; k < nt; ++k) {
-            if (k > 0) EMG_CUDA(cudaStreamWaitEvent(st, side.diag_done, 0));
-            if (nt == 1) break;
-            const T* P = pset(k);
-            const int la = k + 1 < nt ? k + 1 : -1;
-            k_gj_panel<R><<<dim3(nt, 1, (unsigned)F), kThreads, 0, st>>>(0, w, k, Sinv, s->totD, s->offD[i], P, -1);
-            if (la >= 0) {
-                k_gj_panel<R><<<dim3(1, 1, (unsigned)F), kThreads, 0, st>>>(3, w, k, Sinv, s->totD, s->offD[i], P, la);
-                EMG_CUDA(cudaEventRecord(side.tile_ready, st));
-                EMG_CUDA(cudaStreamWaitEvent(side.st, side.tile_ready, 0));
-                k_gj_diag<R><<<dim3(1, 1, (unsigned)F), kDiagThreads, 0, side.st>>>(w, la, Sinv, s->totD, s->offD[i],
-                                                                               pset(la), rel_thr, s->perturbed);
-                EMG_CUDA(cudaEventRecord(side.diag_done, side.st));
-            }
-            if (tc_update)
-                rc = emg::tc_gj_update(w, k, la, F, reinterpret_cast<float2*>(Sinv), s->totD, s->offD[i],
-                                       s->tc_status, st);
+        auto tile = [&](int k, cudaStream_t ts) {   // inverse of tile (k, k) by itself
+            if constexpr (sizeof(R) == 4)
+                k_gj_tile32<<<dim3(1, 1, (unsigned)F), gj::kThreads, 0, ts>>>(w, k, Sinv, s->totD, s->offD[i], pset(k),
+                                                                             rel_thr, s->perturbed);
             else
-                k_gj_panel<R><<<dim3(nt, nt, (unsigned)F), kThreads, 0, st>>>(2, w, k, Sinv, s->totD, s->offD[i], P,
-                                                                               la);
-            if (rc) return rc;
-            k_gj_panel<R><<<dim3(nt, 1, (unsigned)F), kThreads, 0, st>>>(1, w, k, Sinv, s->totD, s->offD[i], P, -1);
+                k_gj_diag<R><<<dim3(1, 1, (unsigned)F), kDiagThreads, 0, ts>>>(w, k, Sinv, s->totD, s->offD[i], pset(k),
+                                                                              rel_thr, s->perturbed);
+        };
+        tile(0, st);
+        if (tc_update) {
+            // FP32: two launches a step on one stream; the second one's first CTA is the lookahead
+            for (int k = 0; k < nt && nt > 1; ++k) {
+                if constexpr (sizeof(R) == 4) {
+                    k_gj_row<R><<<dim3(2 * nt, 1, (unsigned)F), kThreads, 0, st>>>(w, k, nt, Sinv, s->totD, s->offD[i],
+                                                                                   pset(k), colbuf, s->maxw * kTile);
+                    rc = emg::tc_gj_update(w, k, k + 1 < nt ? k + 1 : -1, F, Sinv, s->totD, s->offD[i], colbuf,
+                                           s->maxw * kTile, pset(k), pset(k + 1), rel_thr, s->perturbed, s->tc_status,
+                                           st);
+                    if (rc) return rc;
+                }
+            }
+        } else {
+            // the lookahead tile on the side stream; step k + 1 waits for it
+            for (int k = 0; k < nt; ++k) {
+                if (k > 0) EMG_CUDA(cudaStreamWaitEvent(st, side.diag_done, 0));
+                if (nt == 1) break;
+                const T* P = pset(k);
+                const int la = k + 1 < nt ? k + 1 : -1;
+                k_gj_panel<R><<<dim3(nt, 1, (unsigned)F), kThreads, 0, st>>>(0, w, k, Sinv, s->totD, s->offD[i], P, -1);
+                if (la >= 0) {
+                    k_gj_panel<R><<<dim3(1, 1, (unsigned)F), kThreads, 0, st>>>(3, w, k, Sinv, s->totD, s->offD[i], P, la);
+                    EMG_CUDA(cudaEventRecord(side.tile_ready, st));
+                    EMG_CUDA(cudaStreamWaitEvent(side.st, side.tile_ready, 0));
+                    tile(la, side.st);
+                    EMG_CUDA(cudaEventRecord(side.diag_done, side.st));
+                }
+                k_gj_panel<R><<<dim3(nt, nt, (unsigned)F), kThreads, 0, st>>>(2, w, k, Sinv, s->totD, s->offD[i], P, la);
+                k_gj_panel<R><<<dim3(nt, 1, (unsigned)F), kThreads, 0, st>>>(1, w, k, Sinv, s->totD, s->offD[i], P, -1);
+            }
         }
         // X <- X (2I - S X): squares the residual I - S X of the inverse.  S_i's copy
         // is free once 2I - S X is formed and receives the new X.

@@ -18,6 +18,7 @@
 // not relaunch on the same data.
 #include <cuda_bf16.h>
 
+#include "emg_gj.cuh"
 #include "emg_krylov.cuh"
 
 namespace emg {
@@ -504,26 +505,32 @@ __global__ void __launch_bounds__(kThreads) k_gemm_bf16_tc(int M, int N, int K, 
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(kTmemCols) : "memory");
 }
 
-// Rank-64 update of the block Gauss-Jordan inversion on the tensor cores, in
-// FP32-equivalent precision: M[r, c] -= M[r, K] M[K, c] over a 128-row x 64-column
-// block of the w x w complex64 matrix M (row-major, interleaved), K = the 64 columns /
-// rows of pivot tile k.  Each operand x is split as hi = tf32(x) and lo = x - hi, and
-// the product is accumulated from hi*hi + hi*lo + lo*hi (the lo*lo term is below FP32
-// rounding), i.e. 12 MMAs (M = 128, N = 64, K = 8) per K step of 8 for the four real
-// products of the complex one: the real accumulator (TMEM columns 0-63) takes
-// Re*Re - Im*Im (negation in the instruction descriptor), the imaginary one (columns
-// 64-127) Re*Im + Im*Re.
+// Second half of a step of the block Gauss-Jordan inversion on the tensor cores, in
+// FP32-equivalent precision, on the w x w complex64 matrix M (row-major, interleaved):
+// M[r, c] -= C[r, :] M[k, c] over 128-row x 64-column blocks, C the old column panel (its
+// 64 columns kept in colbuf) and M[k, c] the row panel; the blocks of column tile k become
+// -C[r, :] pinv.  Each operand x is split as hi = tf32(x) and lo = x - hi, and
+// the product is accumulated from all four terms (lo is rounded to TF32 too, where the MMA would
+// cut it), i.e. 16 MMAs (M = 128, N = 64, K = 8) per K step of 8 for the four real products of
+// the complex one: the real accumulator takes Re*Re - Im*Im (negation in the instruction
+// descriptor), the imaginary one Re*Im + Im*Re; every 16 of K have their own pair (512 TMEM
+// columns), summed in FP32.  One application of a factor is then as close to the solution as
+// with FP32 FMAs (geometric mean over 24 frequencies of a 7.9k-DOF guide: 2.1e-4, FMAs 2.8e-4;
+// three terms in one pair of accumulators 3.8e-4), and the tensor pipe is not what bounds it.
 // One CTA of 256 threads per SM:
 //   1. every thread loads its share of both operands (all 64 K) into registers, so
 //      the whole block's loads are in flight at once;
 //   2. they are split and stored as two 32-wide K chunks (192 KB of shared memory in
 //      the canonical K-major layout; a half-warp stores one 8 x 4 core matrix);
-//   3. one thread issues the 96 MMAs; meanwhile every thread loads its part of the
+//   3. one thread issues the 128 MMAs; meanwhile every thread loads its part of the
 //      output block (coalesced rows);
 //   4. the accumulators go TMEM -> shared memory, and the output block is written
 //      back minus the product.
-// Rows of tile k, and tile (la, la) when la >= 0, keep their values.  Grid: column
-// tiles x row blocks of 128 x F (column tile k returns at once).
+// Rows of tile k, and tile (la, la) when la >= 0, keep their values.  The first CTA of each
+// factor (la >= 0) is the lookahead: it forms tile (la, la) in FP32 and inverts it, so the
+// serial pivot chain runs under the update and a step is two launches on one stream (with
+// the lookahead on a side stream, its events and three more launches a step took 113 us on
+// average at widths up to 2768 and 61 + 15 at up to 1358; this takes 72 and 55).  Grid: 1 + column tiles x row blocks of 128, x F.
 constexpr int kUpdM = 128, kUpdN = 64, kUpdTile = 64, kUpdThreads = 256;
 constexpr int kUpdATile = kUpdM * kK * 4;                  // one 128 x 32 FP32 tile: 16 KB
 constexpr int kUpdBTile = kUpdN * kK * 4;                  // one 64 x 32 FP32 tile: 8 KB
@@ -537,21 +544,81 @@ __device__ __forceinline__ float tf32_hi(float x) {
     return __uint_as_float(r);
 }
 
-__global__ void __launch_bounds__(kUpdThreads, 1) k_gj_update_tc(int64_t w, int k, int la, float2* __restrict__ Sinv,
-                                                                  int64_t totD, int64_t offD,
-                                                                  int32_t* __restrict__ status) {
+// The lookahead CTA: T = M[la, la] - C[la] M[k, la] in FP32, inverted into M[la, la] and pout.
+// buf: 3 x 64 x 65 complex in shared memory.
+__device__ __forceinline__ void gj_lookahead(int64_t w, int k, int la, int tb, float2* __restrict__ M,
+                                             const float2* __restrict__ C, float2* __restrict__ pout, float rel_thr,
+                                             int32_t* __restrict__ pert, float2* buf) {
+    __shared__ gj::PivotShared sh;
+    constexpr int kLd = gj::kLd;
+    float2 *Ts = buf, *As = buf + kUpdTile * kLd, *Bs = As + kUpdTile * kLd;
+    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+    const int64_t l0 = (int64_t)la * kUpdTile, k0 = (int64_t)k * kUpdTile;
+    const int lt = (int)min((int64_t)kUpdTile, w - l0);
+#pragma unroll
+    for (int q = 0; q < kUpdTile * kUpdTile / kUpdThreads; ++q) {
+        const int r = (tid + q * kUpdThreads) / kUpdTile, c = tid % kUpdTile;
+        As[r * kLd + c] = r < lt ? C[(l0 + r) * kUpdTile + c] : make_float2(0.f, 0.f);
+        Bs[r * kLd + c] = (r < tb && c < lt) ? M[(k0 + r) * w + l0 + c] : make_float2(0.f, 0.f);
+    }
+    float2 acc[4][4], m[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int r = ty + 16 * i, c = tx + 16 * j;
+            m[i][j] = (r < lt && c < lt) ? M[(l0 + r) * w + l0 + c] : make_float2(r == c ? 1.f : 0.f, 0.f);
+            acc[i][j] = make_float2(0.f, 0.f);
+        }
+    __syncthreads();
+#pragma unroll 8
+    for (int kk = 0; kk < kUpdTile; ++kk) {
+        float2 av[4], bv[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) av[i] = As[(ty + 16 * i) * kLd + kk];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) bv[j] = Bs[kk * kLd + tx + 16 * j];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) gj::cmadd(acc[i][j], av[i], bv[j]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            Ts[(ty + 16 * i) * kLd + tx + 16 * j] = make_float2(m[i][j].x - acc[i][j].x, m[i][j].y - acc[i][j].y);
+    __syncthreads();
+    gj::invert_tile(Ts, lt, rel_thr, sh, pert, M + l0 * w + l0, w, pout);
+}
+
+__global__ void __launch_bounds__(kUpdThreads, 1) k_gj_update_tc(
+    int64_t w, int k, int la, float2* __restrict__ Sinv, int64_t totD, int64_t offD, const float2* __restrict__ colbuf,
+    int64_t scol, const float2* __restrict__ pinv, float2* __restrict__ pinv_next, float rel_thr,
+    int32_t* __restrict__ perturbed, int32_t* __restrict__ status) {
     extern __shared__ __align__(1024) unsigned char dsm[];
     char* base = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(dsm) + 1023) & ~(uintptr_t)1023);
     __shared__ __align__(8) uint64_t mbar;
     __shared__ uint32_t tmem_base;
     __shared__ int s_fail;
-    const int cx = (int)blockIdx.x;
-    if (cx == k) return;               // uniform per CTA, before any TMEM allocation
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     float2* M = Sinv + (int64_t)blockIdx.z * totD + offD;
-    const int64_t r0 = (int64_t)blockIdx.y * kUpdM, c0 = (int64_t)cx * kUpdN, k0 = (int64_t)k * kUpdTile;
+    const float2* C = colbuf + (int64_t)blockIdx.z * scol;
+    const float2* P = pinv + (int64_t)blockIdx.z * kUpdTile * kUpdTile;
+    const int64_t k0 = (int64_t)k * kUpdTile;
     const int tb = (int)min((int64_t)kUpdTile, w - k0);
     const float2 z2 = make_float2(0.f, 0.f);
+    if (blockIdx.x == 0) {             // uniform per CTA, before any TMEM allocation
+        if (la >= 0) gj_lookahead(w, k, la, tb, M, C, pinv_next + (int64_t)blockIdx.z * kUpdTile * kUpdTile, rel_thr,
+                                  perturbed + blockIdx.z, reinterpret_cast<float2*>(base));
+        return;
+    }
+    const int nct = (int)((w + kUpdN - 1) / kUpdN);
+    const int cx = ((int)blockIdx.x - 1) % nct;
+    const int64_t r0 = (int64_t)(((int)blockIdx.x - 1) / nct) * kUpdM, c0 = (int64_t)cx * kUpdN;
+    // row kk of the B operand: the row panel, or the pivot inverse for column tile k
+    const float2* Bp = cx == k ? P : M + k0 * w + c0;
+    const int64_t ldb = cx == k ? kUpdTile : w, bn = cx == k ? tb : min((int64_t)kUpdN, w - c0);
     if (tid == 0) {
         s_fail = 0;
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&mbar)) : "memory");
@@ -559,7 +626,7 @@ __global__ void __launch_bounds__(kUpdThreads, 1) k_gj_update_tc(int64_t w, int 
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
-                     "r"(2 * kTmemCols)
+                     "r"(8 * kTmemCols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -575,18 +642,18 @@ __global__ void __launch_bounds__(kUpdThreads, 1) k_gj_update_tc(int64_t w, int 
         const int wi = warp + 8 * it;
         const int64_t gr = r0 + (wi >> 3) * 8 + ar;
         const int kk = (wi & 7) * 8 + aq;
-        const float2* src = M + gr * w + k0 + kk;
-        va[it][0] = (gr < w && kk < tb) ? src[0] : z2;
-        va[it][1] = (gr < w && kk + 1 < tb) ? src[1] : z2;
+        const float4 v = gr < w ? *reinterpret_cast<const float4*>(C + gr * kUpdTile + kk) : make_float4(0.f, 0.f, 0.f, 0.f);
+        va[it][0] = make_float2(v.x, v.y);
+        va[it][1] = make_float2(v.z, v.w);
     }
 #pragma unroll
     for (int it = 0; it < 8; ++it) {
         const int wi = warp + 8 * it;
         const int kk = (wi & 15) * 4 + bk;
-        const int64_t gc = c0 + (wi >> 4) * 16 + bp;
-        const float2* src = M + (k0 + kk) * w + gc;
-        vb[it][0] = (kk < tb && gc < w) ? src[0] : z2;
-        vb[it][1] = (kk < tb && gc + 1 < w) ? src[1] : z2;
+        const int nc = (wi >> 4) * 16 + bp;
+        const float2* src = Bp + kk * ldb + nc;
+        vb[it][0] = (kk < tb && nc < bn) ? src[0] : z2;
+        vb[it][1] = (kk < tb && nc + 1 < bn) ? src[1] : z2;
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -603,9 +670,9 @@ __global__ void __launch_bounds__(kUpdThreads, 1) k_gj_update_tc(int64_t w, int 
         const float2 x0 = va[it][0], x1 = va[it][1];
         const float r0h = tf32_hi(x0.x), r1h = tf32_hi(x1.x), i0h = tf32_hi(x0.y), i1h = tf32_hi(x1.y);
         *reinterpret_cast<float2*>(cb + 0 * kUpdATile + o) = make_float2(r0h, r1h);
-        *reinterpret_cast<float2*>(cb + 1 * kUpdATile + o) = make_float2(x0.x - r0h, x1.x - r1h);
+        *reinterpret_cast<float2*>(cb + 1 * kUpdATile + o) = make_float2(tf32_hi(x0.x - r0h), tf32_hi(x1.x - r1h));
         *reinterpret_cast<float2*>(cb + 2 * kUpdATile + o) = make_float2(i0h, i1h);
-        *reinterpret_cast<float2*>(cb + 3 * kUpdATile + o) = make_float2(x0.y - i0h, x1.y - i1h);
+        *reinterpret_cast<float2*>(cb + 3 * kUpdATile + o) = make_float2(tf32_hi(x0.y - i0h), tf32_hi(x1.y - i1h));
     }
 #pragma unroll
     for (int it = 0; it < 8; ++it) {
@@ -620,9 +687,9 @@ __global__ void __launch_bounds__(kUpdThreads, 1) k_gj_update_tc(int64_t w, int 
             const float2 x = vb[it][e];
             const float rh = tf32_hi(x.x), ih = tf32_hi(x.y);
             *reinterpret_cast<float*>(cb + 0 * kUpdBTile + o) = rh;
-            *reinterpret_cast<float*>(cb + 1 * kUpdBTile + o) = x.x - rh;
+            *reinterpret_cast<float*>(cb + 1 * kUpdBTile + o) = tf32_hi(x.x - rh);
             *reinterpret_cast<float*>(cb + 2 * kUpdBTile + o) = ih;
-            *reinterpret_cast<float*>(cb + 3 * kUpdBTile + o) = x.y - ih;
+            *reinterpret_cast<float*>(cb + 3 * kUpdBTile + o) = tf32_hi(x.y - ih);
         }
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -633,43 +700,55 @@ __global__ void __launch_bounds__(kUpdThreads, 1) k_gj_update_tc(int64_t w, int 
     //    element (idx / 64, idx % 64), idx = tid + 256 q
     if (tid == 0) {
         const uint32_t id = idesc_tf32(kUpdM, kUpdN), idneg = id | (1u << 13);
-        const uint32_t dre = taddr, dim = taddr + kTmemCols;
-#pragma unroll
-        for (int ch = 0; ch < 2; ++ch) {
-            const uint32_t a0 = smem_u32(base + ch * kUpdChunk), b0 = a0 + 4 * kUpdATile;
-#pragma unroll
-            for (int ks = 0; ks < kK / 8; ++ks) {
-                const uint32_t off = ks * 256;
-                const uint64_t arh = make_desc(a0 + 0 * kUpdATile + off, 128, 1024);
-                const uint64_t arl = make_desc(a0 + 1 * kUpdATile + off, 128, 1024);
-                const uint64_t aih = make_desc(a0 + 2 * kUpdATile + off, 128, 1024);
-                const uint64_t ail = make_desc(a0 + 3 * kUpdATile + off, 128, 1024);
-                const uint64_t brh = make_desc(b0 + 0 * kUpdBTile + off, 128, 1024);
-                const uint64_t brl = make_desc(b0 + 1 * kUpdBTile + off, 128, 1024);
-                const uint64_t bih = make_desc(b0 + 2 * kUpdBTile + off, 128, 1024);
-                const uint64_t bil = make_desc(b0 + 3 * kUpdBTile + off, 128, 1024);
-                const uint32_t first = (ch == 0 && ks == 0) ? 0u : 1u;
 #define EMG_UMMA(D, A, B, ID, ACC)                                                              \
     asm volatile(                                                                               \
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"                                       \
         "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(D), "l"(A), "l"(B), \
         "r"(ID), "r"(ACC)                                                                       \
         : "memory")
-                EMG_UMMA(dre, arh, brh, id, first);
-                EMG_UMMA(dre, arh, brl, id, 1u);
-                EMG_UMMA(dre, arl, brh, id, 1u);
-                EMG_UMMA(dre, aih, bih, idneg, 1u);
-                EMG_UMMA(dre, aih, bil, idneg, 1u);
-                EMG_UMMA(dre, ail, bih, idneg, 1u);
-                EMG_UMMA(dim, arh, bih, id, first);
-                EMG_UMMA(dim, arh, bil, id, 1u);
-                EMG_UMMA(dim, arl, bih, id, 1u);
-                EMG_UMMA(dim, aih, brh, id, 1u);
-                EMG_UMMA(dim, aih, brl, id, 1u);
-                EMG_UMMA(dim, ail, brh, id, 1u);
-#undef EMG_UMMA
+        // an accumulator rounds toward zero at every MMA: each 16 of K have their own pair, summed
+        // in FP32 afterwards, which takes the small terms first
+#pragma unroll
+        for (int term = 0; term < 3; ++term)
+#pragma unroll
+            for (int ch = 0; ch < 2; ++ch) {
+                const uint32_t a0 = smem_u32(base + ch * kUpdChunk), b0 = a0 + 4 * kUpdATile;
+#pragma unroll
+                for (int ks = 0; ks < kK / 8; ++ks) {
+                    const uint32_t off = ks * 256;
+                    const uint64_t arh = make_desc(a0 + 0 * kUpdATile + off, 128, 1024);
+                    const uint64_t arl = make_desc(a0 + 1 * kUpdATile + off, 128, 1024);
+                    const uint64_t aih = make_desc(a0 + 2 * kUpdATile + off, 128, 1024);
+                    const uint64_t ail = make_desc(a0 + 3 * kUpdATile + off, 128, 1024);
+                    const uint64_t brh = make_desc(b0 + 0 * kUpdBTile + off, 128, 1024);
+                    const uint64_t brl = make_desc(b0 + 1 * kUpdBTile + off, 128, 1024);
+                    const uint64_t bih = make_desc(b0 + 2 * kUpdBTile + off, 128, 1024);
+                    const uint64_t bil = make_desc(b0 + 3 * kUpdBTile + off, 128, 1024);
+                    const uint32_t dre = taddr + 2 * (2 * ch + ks / 2) * kTmemCols, dim = dre + kTmemCols;
+                    const uint32_t first = (ks & 1) ? 1u : 0u;
+                    if (term == 0) {
+                        EMG_UMMA(dre, arl, brl, id, first);
+                        EMG_UMMA(dre, ail, bil, idneg, 1u);
+                        EMG_UMMA(dim, arl, bil, id, first);
+                        EMG_UMMA(dim, ail, brl, id, 1u);
+                    } else if (term == 1) {
+                        EMG_UMMA(dre, arh, brl, id, 1u);
+                        EMG_UMMA(dre, arl, brh, id, 1u);
+                        EMG_UMMA(dre, aih, bil, idneg, 1u);
+                        EMG_UMMA(dre, ail, bih, idneg, 1u);
+                        EMG_UMMA(dim, arh, bil, id, 1u);
+                        EMG_UMMA(dim, arl, bih, id, 1u);
+                        EMG_UMMA(dim, aih, brl, id, 1u);
+                        EMG_UMMA(dim, ail, brh, id, 1u);
+                    } else {
+                        EMG_UMMA(dre, arh, brh, id, 1u);
+                        EMG_UMMA(dre, aih, bih, idneg, 1u);
+                        EMG_UMMA(dim, arh, bih, id, 1u);
+                        EMG_UMMA(dim, aih, brh, id, 1u);
+                    }
+                }
             }
-        }
+#undef EMG_UMMA
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mb)
                      : "memory");
     }
@@ -679,44 +758,48 @@ __global__ void __launch_bounds__(kUpdThreads, 1) k_gj_update_tc(int64_t w, int 
     for (int q = 0; q < kQ; ++q) {
         const int idx = tid + kUpdThreads * q;
         const int64_t gr = r0 + idx / kUpdN, gc = c0 + idx % kUpdN;
-        vc[q] = (gr < w && gc < w) ? M[gr * w + gc] : z2;
+        vc[q] = (gr < w && gc < w && cx != k) ? M[gr * w + gc] : z2;
     }
     if (!mbar_wait(mb, 0u)) s_fail = 1;
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     // 4. warp w reads TMEM lanes 32 (w % 4) .. + 31 (rows), columns 32 (w / 4) .. + 31
     if (!s_fail) {
-        float2* P = reinterpret_cast<float2*>(base);
+        float2* Q = reinterpret_cast<float2*>(base);
         const int row = (warp & 3) * 32 + lane, ch0 = (warp >> 2) * 32;
         const uint32_t lane_addr = taddr + ((uint32_t)((warp & 3) * 32) << 16);
 #pragma unroll
         for (int cb = 0; cb < 32; cb += 16) {
-            uint32_t vr[16], vi[16];
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
-                "%14, %15}, [%16];"
-                : "=r"(vr[0]), "=r"(vr[1]), "=r"(vr[2]), "=r"(vr[3]), "=r"(vr[4]), "=r"(vr[5]), "=r"(vr[6]),
-                  "=r"(vr[7]), "=r"(vr[8]), "=r"(vr[9]), "=r"(vr[10]), "=r"(vr[11]), "=r"(vr[12]), "=r"(vr[13]),
-                  "=r"(vr[14]), "=r"(vr[15])
-                : "r"(lane_addr + (uint32_t)(ch0 + cb))
-                : "memory");
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
-                "%14, %15}, [%16];"
-                : "=r"(vi[0]), "=r"(vi[1]), "=r"(vi[2]), "=r"(vi[3]), "=r"(vi[4]), "=r"(vi[5]), "=r"(vi[6]),
-                  "=r"(vi[7]), "=r"(vi[8]), "=r"(vi[9]), "=r"(vi[10]), "=r"(vi[11]), "=r"(vi[12]), "=r"(vi[13]),
-                  "=r"(vi[14]), "=r"(vi[15])
-                : "r"(lane_addr + kTmemCols + (uint32_t)(ch0 + cb))
-                : "memory");
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            float2 sum[16];
 #pragma unroll
-            for (int c = 0; c < 16; ++c)
-                P[row * kUpdLd + ch0 + cb + c] = make_float2(__uint_as_float(vr[c]), __uint_as_float(vi[c]));
+            for (int g = 0; g < 4; ++g) {
+                uint32_t vr[16], vi[16];
+                asm volatile(
+                    "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, "
+                    "%13, %14, %15}, [%16];"
+                    : "=r"(vr[0]), "=r"(vr[1]), "=r"(vr[2]), "=r"(vr[3]), "=r"(vr[4]), "=r"(vr[5]), "=r"(vr[6]), "=r"(vr[7]), "=r"(vr[8]), "=r"(vr[9]), "=r"(vr[10]), "=r"(vr[11]), "=r"(vr[12]), "=r"(vr[13]), "=r"(vr[14]), "=r"(vr[15])
+                    : "r"(lane_addr + (uint32_t)(2 * g * kTmemCols + ch0 + cb))
+                    : "memory");
+                asm volatile(
+                    "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, "
+                    "%13, %14, %15}, [%16];"
+                    : "=r"(vi[0]), "=r"(vi[1]), "=r"(vi[2]), "=r"(vi[3]), "=r"(vi[4]), "=r"(vi[5]), "=r"(vi[6]), "=r"(vi[7]), "=r"(vi[8]), "=r"(vi[9]), "=r"(vi[10]), "=r"(vi[11]), "=r"(vi[12]), "=r"(vi[13]), "=r"(vi[14]), "=r"(vi[15])
+                    : "r"(lane_addr + (uint32_t)((2 * g + 1) * kTmemCols + ch0 + cb))
+                    : "memory");
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                for (int c = 0; c < 16; ++c) {
+                    const float2 v = make_float2(__uint_as_float(vr[c]), __uint_as_float(vi[c]));
+                    sum[c] = g == 0 ? v : make_float2(sum[c].x + v.x, sum[c].y + v.y);
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < 16; ++c) Q[row * kUpdLd + ch0 + cb + c] = sum[c];
         }
     }
     __syncthreads();
     if (!s_fail) {
-        const float2* P = reinterpret_cast<const float2*>(base);
+        const float2* Q = reinterpret_cast<const float2*>(base);
         const int64_t lr0 = (int64_t)la * kUpdTile;                   // rows of tile la
         const bool lacol = la >= 0 && cx == la;
 #pragma unroll
@@ -726,7 +809,7 @@ __global__ void __launch_bounds__(kUpdThreads, 1) k_gj_update_tc(int64_t w, int 
             const int64_t gr = r0 + r, gc = c0 + c;
             if (gr >= w || gc >= w || (gr >= k0 && gr < k0 + kUpdTile) || (lacol && gr >= lr0 && gr < lr0 + kUpdTile))
                 continue;
-            const float2 d = P[r * kUpdLd + c];
+            const float2 d = Q[r * kUpdLd + c];
             M[gr * w + gc] = make_float2(vc[q].x - d.x, vc[q].y - d.y);
         }
     } else if (tid == 0) {
@@ -736,7 +819,7 @@ __global__ void __launch_bounds__(kUpdThreads, 1) k_gj_update_tc(int64_t w, int 
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(2 * kTmemCols)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(8 * kTmemCols)
                      : "memory");
 }
 
@@ -772,19 +855,20 @@ int tc_gemm_bf16(int M, int N, int K, const __nv_bfloat16* a, int sam, int sak, 
 }
 }  // namespace emg
 
-// Rank-64 Gauss-Jordan update of step k on the tensor cores (declared in emg_krylov.cuh).
+// Second half of Gauss-Jordan step k on the tensor cores (declared in emg_krylov.cuh).
 namespace emg {
-int tc_gj_update(int64_t w, int k, int la, int64_t F, float2* Sinv, int64_t totD, int64_t offD, int32_t* status,
-                 cudaStream_t st) {
+int tc_gj_update(int64_t w, int k, int la, int64_t F, float2* Sinv, int64_t totD, int64_t offD, const float2* colbuf,
+                 int64_t scol, const float2* pinv, float2* pinv_next, float rel_thr, int32_t* perturbed,
+                 int32_t* status, cudaStream_t st) {
     static bool attr = false;
     if (!attr) {
         EMG_CUDA(cudaFuncSetAttribute(tc::k_gj_update_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       tc::kUpdSmem + 1024));
         attr = true;
     }
-    const dim3 grid((unsigned)((w + tc::kUpdN - 1) / tc::kUpdN), (unsigned)((w + tc::kUpdM - 1) / tc::kUpdM),
-                    (unsigned)F);
-    tc::k_gj_update_tc<<<grid, tc::kUpdThreads, tc::kUpdSmem + 1024, st>>>(w, k, la, Sinv, totD, offD, status);
+    const int64_t tiles = ((w + tc::kUpdN - 1) / tc::kUpdN) * ((w + tc::kUpdM - 1) / tc::kUpdM);
+    tc::k_gj_update_tc<<<dim3((unsigned)(1 + tiles), 1, (unsigned)F), tc::kUpdThreads, tc::kUpdSmem + 1024, st>>>(
+        w, k, la, Sinv, totD, offD, colbuf, scol, pinv, pinv_next, rel_thr, perturbed, status);
     EMG_CUDA(cudaGetLastError());
     return EMG_OK;
 }
