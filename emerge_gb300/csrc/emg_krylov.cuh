@@ -71,6 +71,12 @@ int tc_slab_product(int64_t w, int64_t row0, int64_t Bc, const void* groups, int
                     int64_t totD, int64_t offD, const float2* Y, float alpha, int beta, float2* Out, int32_t* status,
                     cudaStream_t st);
 
+// The same product in FP32-equivalent precision (split-TF32 operands), K split over clusters of
+// up to max_splits CTAs.
+int tc_slab_split(int64_t w, int64_t row0, int64_t Bc, const void* groups, int G, int maxcol, int max_splits,
+                  const float2* Sinv, int64_t totD, int64_t offD, const float2* Y, float alpha, int beta, float2* Out,
+                  int32_t* status, cudaStream_t st);
+
 // Second half of Gauss-Jordan step k on the tcgen05 tensor cores in FP32-equivalent
 // precision (split-TF32 products, FP32 accumulation; emg_tc.cu), for the F complex64 w x w
 // blocks Sinv + f totD + offD: M[r, c] -= C[r] M[k, c] and M[r, k] = -C[r] pinv with the old

@@ -641,6 +641,7 @@ __global__ void k_scatter(int64_t n, int64_t Bc, const int32_t* __restrict__ per
 
 // mode 0: Y[row] -= sum C[row,k] Z[prev0 + cidx[k]]    (forward coupling)
 // mode 1: Y[row]  = sum U[row,k] Z[next0 + uidx[k]]    (backward coupling)
+// A row has some 20 entries: four of them in flight per thread, two of its columns apart.
 template <typename R>
 __global__ void k_couple(int mode, int64_t w, int64_t row0, int64_t nb0, int64_t Bc, const int32_t* __restrict__ colfac,
                          const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx,
@@ -651,9 +652,22 @@ __global__ void k_couple(int mode, int64_t w, int64_t row0, int64_t nb0, int64_t
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
         const int64_t row = row0 + t / Bc, c = t % Bc;
         const T* v = val + (int64_t)colfac[c] * nval;
-        T s = czero<T>();
-        for (int64_t k = ptr[row]; k < ptr[row + 1]; ++k) cfma(s, v[k], Z[(nb0 + idx[k]) * Bc + c]);
+        const T* z = Z + nb0 * Bc + c;
+        const int64_t k1 = ptr[row + 1];
+        int64_t k = ptr[row];
+        T s0 = czero<T>(), s1 = czero<T>();
+        for (; k + 4 <= k1; k += 4) {
+            const int32_t i0 = idx[k], i1 = idx[k + 1], i2 = idx[k + 2], i3 = idx[k + 3];
+            const T a0 = v[k], a1 = v[k + 1], a2 = v[k + 2], a3 = v[k + 3];
+            const T z0 = z[i0 * Bc], z1 = z[i1 * Bc], z2 = z[i2 * Bc], z3 = z[i3 * Bc];
+            cfma(s0, a0, z0);
+            cfma(s1, a1, z1);
+            cfma(s0, a2, z2);
+            cfma(s1, a3, z3);
+        }
+        for (; k < k1; ++k) cfma(s0, v[k], z[idx[k] * Bc]);
         T& y = Y[row * Bc + c];
+        const T s = mk(s0.x + s1.x, s0.y + s1.y);
         if (mode == 0) { y.x -= s.x; y.y -= s.y; }
         else y = s;
     }
@@ -668,52 +682,98 @@ __global__ void k_narrow(int64_t nv, const double2* __restrict__ in, float2* __r
         out[t] = make_float2((float)in[t].x, (float)in[t].y);
 }
 
-// Out[r, cols of group g] = beta Out + alpha S_i^-1[r, :] Y[:, cols]: warp per row,
-// lanes over the row of S_i^-1 (coalesced), 16 columns per pass.  Grid: row blocks x groups.
-constexpr int kRowCols = 16;
-template <typename R>
+// Out[r, cols of group g] = beta Out + alpha S_i^-1[r, :] Y[:, cols] for few columns (NC at a
+// time): a CTA takes kRowRows rows, kRowWarps warps each, lanes over the row of S_i^-1
+// (coalesced, four loads in flight per lane).  The column count is a template argument and the
+// lane sums are folded so that each shuffle halves the values a lane carries (9 adds for four
+// complex columns, 40 one by one): in FP64 the pipe bounds the kernel, and the run-time column
+// count of up to 16 issued its unused products too (4 columns, 1250 wide: 268 -> 45
+// us); in FP32 it is bound by reading S_i^-1 (2 columns, 1812 wide: 37.7 -> 12 us).
+// Grid: row blocks x groups.
+constexpr int kRowRows = 2, kRowWarps = kThreads / 32 / kRowRows;
+template <int NV, typename R>
+__device__ __forceinline__ R lane_sum(R (&v)[NV]) {   // lane l: the sum of value l >> (5 - log2 NV)
+    const int lane = threadIdx.x & 31;
+    int n = NV;
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        if (n > 1) {
+            n >>= 1;
+            const bool up = lane & o;
+#pragma unroll
+            for (int i = 0; i < NV / 2; ++i)
+                if (i < n) {
+                    const R send = up ? v[i] : v[i + n], keep = up ? v[i + n] : v[i];
+                    v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                }
+        } else {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+        }
+    }
+    return v[0];
+}
+template <typename R, int NC>
 __global__ void __launch_bounds__(kThreads) k_rowmv(int64_t w, int64_t row0, int64_t Bc, const Group* __restrict__ groups,
                                                     const typename C2<R>::T* __restrict__ Sinv, int64_t totD, int64_t offD,
                                                     const typename C2<R>::T* __restrict__ Y, R alpha, int beta,
                                                     typename C2<R>::T* __restrict__ Out) {
     using T = typename C2<R>::T;
-    const int64_t r = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (r >= w) return;
+    constexpr int NV = 2 * NC;                     // values of a lane: re and im of NC columns
+    __shared__ R part[kRowRows][kRowWarps][NV];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, rr = warp / kRowWarps, kw = warp % kRowWarps;
+    const int64_t r = (int64_t)blockIdx.x * kRowRows + rr;
     const Group g = groups[blockIdx.y];
     const T* S = Sinv + (int64_t)g.fac * totD + offD + r * w;
-    const T* Yb = Y + row0 * Bc;
-    for (int c0 = 0; c0 < g.ncol; c0 += kRowCols) {
-        const int nc = min(kRowCols, g.ncol - c0);
-        const int64_t cb = g.col0 + c0;
-        T acc[kRowCols];
+    const T* Yb = Y + row0 * Bc + g.col0;
+    for (int c0 = 0; c0 < g.ncol; c0 += NC) {
+        const int nc = min(NC, g.ncol - c0);
+        R v[NV];
 #pragma unroll
-        for (int j = 0; j < kRowCols; ++j) acc[j] = czero<T>();
-        for (int64_t k = lane; k < w; k += 32) {
-            const T s = S[k];
-            const T* yr = Yb + k * Bc + cb;
+        for (int j = 0; j < NV; ++j) v[j] = 0;
+        if (r < w) {
+            auto mac = [&](T s, int64_t k) {
+                const T* y = Yb + k * Bc + c0;
 #pragma unroll
-            for (int j = 0; j < kRowCols; ++j)
-                if (j < nc) cfma(acc[j], s, yr[j]);
+                for (int j = 0; j < NC; ++j) {
+                    if (NC > 1 && j >= nc) break;   // uniform
+                    const T x = y[j];
+                    v[2 * j] = fma(s.x, x.x, v[2 * j]);
+                    v[2 * j] = fma(-s.y, x.y, v[2 * j]);
+                    v[2 * j + 1] = fma(s.x, x.y, v[2 * j + 1]);
+                    v[2 * j + 1] = fma(s.y, x.x, v[2 * j + 1]);
+                }
+            };
+            int64_t k = kw * 32 + lane;
+            constexpr int kStep = kRowWarps * 32;
+            for (; k + 3 * kStep < w; k += 4 * kStep) {
+                const T s0 = S[k], s1 = S[k + kStep], s2 = S[k + 2 * kStep], s3 = S[k + 3 * kStep];
+                mac(s0, k);
+                mac(s1, k + kStep);
+                mac(s2, k + 2 * kStep);
+                mac(s3, k + 3 * kStep);
+            }
+            for (; k < w; k += kStep) mac(S[k], k);
         }
+        const R sum = lane_sum<NV>(v);
+        constexpr int kPer = 32 / NV;              // lanes holding the same value
+        if (lane % kPer == 0) part[rr][kw][lane / kPer] = sum;
+        __syncthreads();
+        if (threadIdx.x < kRowRows * NC) {
+            const int ro = threadIdx.x / NC, j = threadIdx.x % NC;
+            const int64_t row = (int64_t)blockIdx.x * kRowRows + ro;
+            if (row < w && j < nc) {
+                R x = 0, y = 0;
 #pragma unroll
-        for (int j = 0; j < kRowCols; ++j) {
-#pragma unroll
-            for (int o = 16; o; o >>= 1) {
-                acc[j].x += __shfl_xor_sync(0xffffffffu, acc[j].x, o);
-                acc[j].y += __shfl_xor_sync(0xffffffffu, acc[j].y, o);
+                for (int q = 0; q < kRowWarps; ++q) {
+                    x += part[ro][q][2 * j];
+                    y += part[ro][q][2 * j + 1];
+                }
+                T& o = Out[(row0 + row) * Bc + g.col0 + c0 + j];
+                if (beta) { o.x += alpha * x; o.y += alpha * y; }
+                else o = mk(alpha * x, alpha * y);
             }
         }
-        if (lane < nc) {
-            T v = acc[0];
-#pragma unroll
-            for (int j = 1; j < kRowCols; ++j)
-                if (j == lane) v = acc[j];
-            T& o = Out[(row0 + r) * Bc + cb + lane];
-            const T res = mk(alpha * v.x, alpha * v.y);
-            if (beta) { o.x += res.x; o.y += res.y; }
-            else o = res;
-        }
+        __syncthreads();
     }
 }
 
@@ -1388,7 +1448,7 @@ extern "C" int emg_slab_factor(emg_slab* s, int precision, int64_t F, const int3
 namespace {
 // EMG_ERR_CUDA if a tensor-core tile of the last solve gave up waiting (and reset).
 int tc_check(emg_slab* s, cudaStream_t st) {
-    if (!s->tc_status || !s->use_tc) return EMG_OK;
+    if (!s->tc_status || s->prec != 1) return EMG_OK;
     int32_t h = 0;
     EMG_CUDA(cudaMemcpyAsync(&h, s->tc_status, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
     EMG_CUDA(cudaStreamSynchronize(st));
@@ -1431,7 +1491,7 @@ struct SlabPrecond : emg::Precond {
         // split-K scratch for the wide-group products (largest need over the slabs)
         int maxcol = 0;
         for (const auto& g : groups) maxcol = std::max(maxcol, (int)g.ncol);
-        if (maxcol >= s->wide) {
+        if (s->prec == 2 && maxcol >= s->wide) {
             const int64_t ct = (maxcol + emg::slab::kTile - 1) / emg::slab::kTile, G = (int64_t)groups.size();
             size_t need = 0;
             int64_t tiles_max = 0;
@@ -1445,8 +1505,7 @@ struct SlabPrecond : emg::Precond {
                 const int sp = emg::slab::gemm_splits(tiles, w, s->max_splits);
                 tiles_max = std::max(tiles_max, tiles);
                 if (sp > 1)
-                    need = std::max(need, (size_t)tiles * sp * (size_t)slot *
-                                              (s->prec == 1 ? sizeof(float2) : sizeof(double2)));
+                    need = std::max(need, (size_t)tiles * sp * (size_t)slot * sizeof(double2));
             }
             if (need > s->kpart_bytes) {
                 if (s->kpart) cudaFree(s->kpart);
@@ -1491,39 +1550,55 @@ struct SlabPrecond : emg::Precond {
         const unsigned G = (unsigned)groups.size();
         int maxcol = 0;
         for (const auto& g : groups) maxcol = std::max(maxcol, (int)g.ncol);
-        static bool narrow_attr = false;   // per instantiation: the 128 x 16 tiles need 74 KB
-        if (!narrow_attr) {
-            EMG_CUDA(cudaFuncSetAttribute(k_slab_gemm16<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)sizeof(NarrowTile<R>)));
-            narrow_attr = true;
+        if constexpr (sizeof(R) == 8) {
+            static bool narrow_attr = false;   // the 128 x 16 tiles need 74 KB
+            if (!narrow_attr) {
+                EMG_CUDA(cudaFuncSetAttribute(k_slab_gemm16<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              (int)sizeof(NarrowTile<R>)));
+                narrow_attr = true;
+            }
         }
-        // dense slab product: warp-per-row for groups narrower than s->wide, 128 x 16
-        // tiles up to 16 columns, 64 x 64 tiles for wider ones
+        // dense slab product: rows of few columns for groups narrower than s->wide; wider FP32
+        // groups on the tensor cores (TF32 products if asked for, else split ones), FP64 groups
+        // as 128 x 16 tiles up to 16 columns and 64 x 64 tiles above
+        int rc = EMG_OK;
         auto dense = [&](int64_t w, int64_t i, R alpha, int beta) {
             if constexpr (sizeof(R) == 4) {
-                if (s->use_tc && maxcol >= s->wide) {
-                    emg::tc_slab_product(w, s->off[i], Bc, s->groups, (int)G, maxcol,
-                                         reinterpret_cast<const float2*>(Sinv), s->totD, s->offD[i],
-                                         reinterpret_cast<const float2*>(Y), (float)alpha, beta,
-                                         reinterpret_cast<float2*>(Z), s->tc_status, st);
+                if (maxcol >= s->wide) {
+                    const auto* Sf = reinterpret_cast<const float2*>(Sinv);
+                    const auto* Yf = reinterpret_cast<const float2*>(Y);
+                    const int e = s->use_tc ? emg::tc_slab_product(w, s->off[i], Bc, s->groups, (int)G, maxcol, Sf, s->totD,
+                                                                   s->offD[i], Yf, (float)alpha, beta,
+                                                                   reinterpret_cast<float2*>(Z), s->tc_status, st)
+                                            : emg::tc_slab_split(w, s->off[i], Bc, s->groups, (int)G, maxcol,
+                                                                 s->max_splits, Sf, s->totD, s->offD[i], Yf, (float)alpha,
+                                                                 beta, reinterpret_cast<float2*>(Z), s->tc_status, st);
+                    if (e && !rc) rc = e;
                     return;
                 }
             }
-            if (maxcol >= s->wide && maxcol <= kNarrowN) {
-                const int64_t rt = (w + kNarrowM - 1) / kNarrowM;
-                const int sp = gemm_splits(rt * G, w, s->max_splits);
-                k_slab_gemm16<R><<<dim3(1u, (unsigned)(rt * sp), G), kThreads, sizeof(NarrowTile<R>), st>>>(
-                    w, s->off[i], Bc, s->groups, Sinv, s->totD, s->offD[i], Y, alpha, beta, Z, sp,
-                    static_cast<T*>(s->kpart), s->kcnt);
-            } else if (maxcol >= s->wide) {
-                const int64_t ct = (maxcol + kTile - 1) / kTile, rt = (w + kTile - 1) / kTile;
-                const int sp = gemm_splits(ct * rt * G, w, s->max_splits);
-                k_slab_gemm<R><<<dim3((unsigned)ct, (unsigned)(rt * sp), G), kThreads, 0, st>>>(
-                    w, s->off[i], Bc, s->groups, Sinv, s->totD, s->offD[i], Y, alpha, beta, Z, sp,
-                    static_cast<T*>(s->kpart), s->kcnt);
-            } else
-                k_rowmv<R><<<dim3((unsigned)((w * 32 + kThreads - 1) / kThreads), G), kThreads, 0, st>>>(
-                    w, s->off[i], Bc, s->groups, Sinv, s->totD, s->offD[i], Y, alpha, beta, Z);
+            if constexpr (sizeof(R) == 8) {
+                if (maxcol >= s->wide && maxcol <= kNarrowN) {
+                    const int64_t rt = (w + kNarrowM - 1) / kNarrowM;
+                    const int sp = gemm_splits(rt * G, w, s->max_splits);
+                    k_slab_gemm16<R><<<dim3(1u, (unsigned)(rt * sp), G), kThreads, sizeof(NarrowTile<R>), st>>>(
+                        w, s->off[i], Bc, s->groups, Sinv, s->totD, s->offD[i], Y, alpha, beta, Z, sp,
+                        static_cast<T*>(s->kpart), s->kcnt);
+                    return;
+                }
+                if (maxcol >= s->wide) {
+                    const int64_t ct = (maxcol + kTile - 1) / kTile, rt = (w + kTile - 1) / kTile;
+                    const int sp = gemm_splits(ct * rt * G, w, s->max_splits);
+                    k_slab_gemm<R><<<dim3((unsigned)ct, (unsigned)(rt * sp), G), kThreads, 0, st>>>(
+                        w, s->off[i], Bc, s->groups, Sinv, s->totD, s->offD[i], Y, alpha, beta, Z, sp,
+                        static_cast<T*>(s->kpart), s->kcnt);
+                    return;
+                }
+            }
+            const dim3 g((unsigned)((w + kRowRows - 1) / kRowRows), G);
+            auto rowmv = maxcol <= 1 ? k_rowmv<R, 1> : maxcol <= 2 ? k_rowmv<R, 2> : maxcol <= 4 ? k_rowmv<R, 4>
+                                                                                              : k_rowmv<R, 8>;
+            rowmv<<<g, kThreads, 0, st>>>(w, s->off[i], Bc, s->groups, Sinv, s->totD, s->offD[i], Y, alpha, beta, Z);
         };
         k_gather<R, TI><<<grid_for(s->n * Bc, 256), 256, 0, st>>>(s->n, Bc, s->perm, in, Y);
         for (int i = 0; i < s->m; ++i) {
@@ -1541,7 +1616,7 @@ struct SlabPrecond : emg::Precond {
         }
         k_scatter<R, TI><<<grid_for(s->n * Bc, 256), 256, 0, st>>>(s->n, Bc, s->perm, Z, out);
         EMG_CUDA(cudaGetLastError());
-        return EMG_OK;
+        return rc;
     }
     int apply(const double2* in, double2* out, cudaStream_t st) override {
         return s->prec == 1 ? run<float, double2>(in, out, st) : run<double, double2>(in, out, st);
@@ -1636,8 +1711,9 @@ extern "C" int emg_gmres_slab_family(const emg_rplan* pc, emg_slab* s, int64_t B
     Am.nfam = nfam;
     Am.fam = reinterpret_cast<const double2*>(fam);
     Am.coef = reinterpret_cast<const double2*>(coef);
-    return gmres_run(p, Bc, Am, reinterpret_cast<const double2*>(rhs), reinterpret_cast<double2*>(x), restart, max_iter,
-                     tol, iters_out, resid_out, (cudaStream_t)stream, M, true);
+    const int rc = gmres_run(p, Bc, Am, reinterpret_cast<const double2*>(rhs), reinterpret_cast<double2*>(x), restart,
+                             max_iter, tol, iters_out, resid_out, (cudaStream_t)stream, M, true);
+    return rc ? rc : tc_check(s, (cudaStream_t)stream);
 }
 
 extern "C" int emg_gmres_slab_mixed(const emg_rplan* pc, emg_slab* s, int64_t Bc, const int32_t* cmat, int64_t Bm,
@@ -1670,5 +1746,5 @@ extern "C" int emg_gmres_slab_mixed(const emg_rplan* pc, emg_slab* s, int64_t Bc
     rc = ir_run(p, Bc, Am, A32, reinterpret_cast<const double2*>(rhs), reinterpret_cast<double2*>(x), restart, max_iter,
                 tol, inner_tol, iters_out, resid_out, steps_out, st, M);
     EMG_CUDA(cudaStreamSynchronize(st));   // A32 is freed on return
-    return rc;
+    return rc ? rc : tc_check(s, st);
 }

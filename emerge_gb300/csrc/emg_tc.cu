@@ -355,6 +355,253 @@ __global__ void __launch_bounds__(kThreads) k_cgemm_tf32(int64_t w, int64_t row0
                      : "memory");
 }
 
+// The complex slab product in FP32-equivalent precision: Out[r0.., cols] = alpha S[128 rows x K]
+// Y[K x up to 64 cols] + beta Out, every operand split as hi + lo TF32 (lo rounded), hi hi + hi lo
+// + lo hi accumulated in FP32.  A cluster of CTAs shares one 128-row tile and splits K: a
+// slab is a few hundred to a few thousand wide, so the row tiles alone leave most SMs idle and
+// the product is bound by latency.  Per CTA, 32-wide K chunks through two shared buffers: the
+// loads of the next chunk (registers) and the split run under the MMAs of the last.  An accumulator
+// rounds toward zero at every MMA, so chunk ch goes to accumulator pair ch % 4 (512 TMEM columns,
+// small terms first), summed in FP32.  The partial tiles meet in distributed shared memory,
+// each CTA adding the ranks of its share of the rows in rank order.
+// The 64 x 64 CUDA-core tiles with a K split through global partials took 53 us for 48
+// columns of a 950-wide slab on average (45 CTAs) and 29 us for 16 columns, this 19 and 12 to 22
+// (at 150 to 1380 wide).
+// Grid: cluster x row tiles x (groups * column tiles).
+constexpr int kSpThreads = 256;
+constexpr int kSpATile = kM * kK * 4, kSpBTile = kN * kK * 4;           // one 128 x 32 / 64 x 32 FP32 tile
+constexpr int kSpChunk = 4 * kSpATile + 4 * kSpBTile;                   // re hi, re lo, im hi, im lo of both: 96 KB
+constexpr int kSpSmem = 2 * kSpChunk;
+constexpr int kSpLd = kN + 1;
+
+__device__ __forceinline__ float tf32_rn(float x) {
+    uint32_t r;
+    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
+    return __uint_as_float(r);
+}
+
+__global__ void __launch_bounds__(kSpThreads, 1) k_slab_split(int64_t w, int64_t row0, int64_t Bc,
+                                                              const TcGroup* __restrict__ groups, int G,
+                                                              const float2* __restrict__ Sinv, int64_t totD, int64_t offD,
+                                                              const float2* __restrict__ Y, float alpha, int beta,
+                                                              float2* __restrict__ Out, int32_t* __restrict__ status) {
+    extern __shared__ __align__(1024) unsigned char dsm[];
+    char* base = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(dsm) + 1023) & ~(uintptr_t)1023);
+    __shared__ __align__(8) uint64_t mbar[2];
+    __shared__ uint32_t tmem_base;
+    const TcGroup g = groups[blockIdx.z % G];
+    const int64_t c0 = (int64_t)(blockIdx.z / G) * kN, r0 = (int64_t)blockIdx.y * kM;
+    if (c0 >= g.ncol) return;          // uniform per cluster, before any TMEM allocation or cluster barrier
+    const int rank = (int)blockIdx.x, ranks = (int)gridDim.x;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const float2* S = Sinv + (int64_t)g.fac * totD + offD;
+    const float2* Yb = Y + row0 * Bc + g.col0 + c0;
+    const int ncl = (int)min((int64_t)kN, (int64_t)g.ncol - c0), n16 = (ncl + 15) >> 4;
+    const int64_t kper = ((w + ranks - 1) / ranks + 7) & ~(int64_t)7;
+    const int64_t ks0 = min(w, rank * kper), ks1 = min(w, ks0 + kper);
+    const int nk = (int)((ks1 - ks0 + kK - 1) / kK);
+    if (tid == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&mbar[0])) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&mbar[1])) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
+                     "r"(8 * kTmemCols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    // loads of a chunk.  A: item wi = warp + 8 it is row block wi / 4 and 8-wide K block wi % 4, lane ->
+    // row (lane & 15) / 2 and K pair 2 (lane & 1) + 4 (lane >> 4).  B: item it is column block it and
+    // 4-deep K block ``warp``, lane -> column pair 2 (lane & 3) + 8 (lane >> 4), K (lane >> 2) & 3.
+    const int ar = (lane & 15) >> 1, aq = ((lane & 1) << 1) + ((lane >> 4) << 2);
+    const int bp = ((lane & 3) << 1) + ((lane >> 4) << 3), bk = (lane >> 2) & 3;
+    const float2 z2 = make_float2(0.f, 0.f);
+    float2 va[8][2], vb[4][2];
+    auto load = [&](int ch) {
+        const int64_t k0 = ks0 + (int64_t)ch * kK;
+#pragma unroll
+        for (int it = 0; it < 8; ++it) {
+            const int wi = warp + 8 * it;
+            const int64_t gr = r0 + (wi >> 2) * 8 + ar, gk = k0 + (wi & 3) * 8 + aq;
+            const float2* src = S + gr * w + gk;
+            va[it][0] = (gr < w && gk < ks1) ? src[0] : z2;
+            va[it][1] = (gr < w && gk + 1 < ks1) ? src[1] : z2;
+        }
+#pragma unroll
+        for (int it = 0; it < 4; ++it) {
+            if (it >= n16) break;
+            const int64_t gk = k0 + warp * 4 + bk;
+            const int n = it * 16 + bp;
+            const float2* src = Yb + gk * Bc + n;
+            vb[it][0] = (gk < ks1 && n < ncl) ? src[0] : z2;
+            vb[it][1] = (gk < ks1 && n + 1 < ncl) ? src[1] : z2;
+        }
+    };
+    auto split = [&](char* cb) {
+#pragma unroll
+        for (int it = 0; it < 8; ++it) {
+            const int wi = warp + 8 * it, kk = (wi & 3) * 8 + aq;
+            const uint32_t o = (uint32_t)((((wi >> 2) * (kK / 4) + (kk >> 2)) * 128) + ar * 16 + (kk & 3) * 4);
+            const float2 x0 = va[it][0], x1 = va[it][1];
+            const float r0h = tf32_rn(x0.x), r1h = tf32_rn(x1.x), i0h = tf32_rn(x0.y), i1h = tf32_rn(x1.y);
+            *reinterpret_cast<float2*>(cb + 0 * kSpATile + o) = make_float2(r0h, r1h);
+            *reinterpret_cast<float2*>(cb + 1 * kSpATile + o) = make_float2(tf32_rn(x0.x - r0h), tf32_rn(x1.x - r1h));
+            *reinterpret_cast<float2*>(cb + 2 * kSpATile + o) = make_float2(i0h, i1h);
+            *reinterpret_cast<float2*>(cb + 3 * kSpATile + o) = make_float2(tf32_rn(x0.y - i0h), tf32_rn(x1.y - i1h));
+        }
+        cb += 4 * kSpATile;
+#pragma unroll
+        for (int it = 0; it < 4; ++it) {
+            if (it >= n16) break;
+            const int kc = warp * 4 + bk;
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int n = it * 16 + bp + e;
+                const uint32_t o = (uint32_t)((((n >> 3) * (kK / 4) + (kc >> 2)) * 128) + (n & 7) * 16 + (kc & 3) * 4);
+                const float2 x = vb[it][e];
+                const float rh = tf32_rn(x.x), ih = tf32_rn(x.y);
+                *reinterpret_cast<float*>(cb + 0 * kSpBTile + o) = rh;
+                *reinterpret_cast<float*>(cb + 1 * kSpBTile + o) = tf32_rn(x.x - rh);
+                *reinterpret_cast<float*>(cb + 2 * kSpBTile + o) = ih;
+                *reinterpret_cast<float*>(cb + 3 * kSpBTile + o) = tf32_rn(x.y - ih);
+            }
+        }
+    };
+    if (nk > 0) load(0);
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t taddr = tmem_base;
+    const uint32_t id = idesc_tf32(kM, 16 * n16), idneg = id | (1u << 13);
+    bool ok = true;
+    for (int ch = 0; ch < nk; ++ch) {
+        const int buf = ch & 1;
+        char* cb = base + buf * kSpChunk;
+        // the MMAs that read this buffer two chunks ago are done
+        if (ch >= 2 && ok && !mbar_wait(smem_u32(&mbar[buf]), (uint32_t)(((ch >> 1) - 1) & 1))) ok = false;
+        if (ok) split(cb);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        ok = !__syncthreads_or(!ok);   // uniform
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (!ok) break;
+        if (tid == 0) {
+            const uint32_t a0 = smem_u32(cb), b0 = a0 + 4 * kSpATile;
+            const uint32_t dre = taddr + 2 * (ch & 3) * kTmemCols, dim = dre + kTmemCols;
+#define EMG_UMMA(D, A, B, ID, ACC)                                                              \
+    asm volatile(                                                                               \
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"                                       \
+        "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(D), "l"(A), "l"(B), \
+        "r"(ID), "r"(ACC)                                                                       \
+        : "memory")
+#pragma unroll
+            for (int term = 0; term < 2; ++term)
+#pragma unroll
+                for (int ks = 0; ks < kK / 8; ++ks) {
+                    const uint32_t off = ks * 256;
+                    const uint64_t arh = make_desc(a0 + 0 * kSpATile + off, 128, 1024);
+                    const uint64_t arl = make_desc(a0 + 1 * kSpATile + off, 128, 1024);
+                    const uint64_t aih = make_desc(a0 + 2 * kSpATile + off, 128, 1024);
+                    const uint64_t ail = make_desc(a0 + 3 * kSpATile + off, 128, 1024);
+                    const uint64_t brh = make_desc(b0 + 0 * kSpBTile + off, 128, 1024);
+                    const uint64_t brl = make_desc(b0 + 1 * kSpBTile + off, 128, 1024);
+                    const uint64_t bih = make_desc(b0 + 2 * kSpBTile + off, 128, 1024);
+                    const uint64_t bil = make_desc(b0 + 3 * kSpBTile + off, 128, 1024);
+                    const uint32_t first = (ch < 4 && ks == 0) ? 0u : 1u;
+                    if (term == 0) {
+                        EMG_UMMA(dre, arh, brl, id, first);
+                        EMG_UMMA(dre, arl, brh, id, 1u);
+                        EMG_UMMA(dre, aih, bil, idneg, 1u);
+                        EMG_UMMA(dre, ail, bih, idneg, 1u);
+                        EMG_UMMA(dim, arh, bil, id, first);
+                        EMG_UMMA(dim, arl, bih, id, 1u);
+                        EMG_UMMA(dim, aih, brl, id, 1u);
+                        EMG_UMMA(dim, ail, brh, id, 1u);
+                    } else {
+                        EMG_UMMA(dre, arh, brh, id, 1u);
+                        EMG_UMMA(dre, aih, bih, idneg, 1u);
+                        EMG_UMMA(dim, arh, bih, id, 1u);
+                        EMG_UMMA(dim, aih, brh, id, 1u);
+                    }
+                }
+#undef EMG_UMMA
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                             smem_u32(&mbar[buf]))
+                         : "memory");
+        }
+        if (ch + 1 < nk) load(ch + 1);
+    }
+    // the last two chunks' MMAs (one more bounded wait each after a time-out, before the TMEM goes)
+    for (int ch = max(0, nk - 2); ch < nk; ++ch)
+        if (!mbar_wait(smem_u32(&mbar[ch & 1]), (uint32_t)((ch >> 1) & 1))) ok = false;
+    if (!ok) atomicExch(status, 1);
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    float2* P = reinterpret_cast<float2*>(base);
+    {
+        // warp w reads TMEM lanes 32 (w % 4) .. + 31 (rows), column blocks w / 4, w / 4 + 2
+        const int row = (warp & 3) * 32 + lane, sets = min(nk, 4);
+        const uint32_t lane_addr = taddr + ((uint32_t)((warp & 3) * 32) << 16);
+        for (int b = warp >> 2; b < n16; b += 2) {
+            float2 sum[16];
+#pragma unroll
+            for (int c = 0; c < 16; ++c) sum[c] = z2;
+            for (int q = 0; q < sets; ++q) {
+                uint32_t vr[16], vi[16];
+                asm volatile(
+                    "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
+                    "%14, %15}, [%16];"
+                    : "=r"(vr[0]), "=r"(vr[1]), "=r"(vr[2]), "=r"(vr[3]), "=r"(vr[4]), "=r"(vr[5]), "=r"(vr[6]), "=r"(vr[7]), "=r"(vr[8]), "=r"(vr[9]), "=r"(vr[10]), "=r"(vr[11]), "=r"(vr[12]), "=r"(vr[13]), "=r"(vr[14]), "=r"(vr[15])
+                    : "r"(lane_addr + (uint32_t)(2 * q * kTmemCols + 16 * b))
+                    : "memory");
+                asm volatile(
+                    "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
+                    "%14, %15}, [%16];"
+                    : "=r"(vi[0]), "=r"(vi[1]), "=r"(vi[2]), "=r"(vi[3]), "=r"(vi[4]), "=r"(vi[5]), "=r"(vi[6]), "=r"(vi[7]), "=r"(vi[8]), "=r"(vi[9]), "=r"(vi[10]), "=r"(vi[11]), "=r"(vi[12]), "=r"(vi[13]), "=r"(vi[14]), "=r"(vi[15])
+                    : "r"(lane_addr + (uint32_t)((2 * q + 1) * kTmemCols + 16 * b))
+                    : "memory");
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                for (int c = 0; c < 16; ++c) {
+                    sum[c].x += __uint_as_float(vr[c]);
+                    sum[c].y += __uint_as_float(vi[c]);
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < 16; ++c) P[row * kSpLd + 16 * b + c] = sum[c];
+        }
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    {
+        const int rows = kM / ranks, rb = rank * rows;   // ranks: 1, 2, 4 or 8
+        const uint32_t pl = smem_u32(P);
+        for (int e = tid; e < rows * ncl; e += kSpThreads) {
+            const int r = rb + e / ncl, c = e % ncl;
+            if (r0 + r >= w) continue;
+            float2 v = z2;
+            for (int q = 0; q < ranks; ++q) {
+                uint32_t addr;
+                float2 x;
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(pl + (uint32_t)((r * kSpLd + c) * 8)), "r"(q));
+                asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(x.x), "=f"(x.y) : "r"(addr) : "memory");
+                v.x += x.x;
+                v.y += x.y;
+            }
+            float2& o = Out[(row0 + r0 + r) * Bc + g.col0 + c0 + c];
+            if (beta) { o.x += alpha * v.x; o.y += alpha * v.y; }
+            else o = make_float2(alpha * v.x, alpha * v.y);
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // no CTA leaves while its tile is read
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(8 * kTmemCols)
+                     : "memory");
+}
+
 // BF16 GEMM of the warm-start network (tcgen05 kind::f16, FP32 accumulation in TMEM):
 // C[m][n] = sum_k A(m,k) B(k,n) (+ bias[n]) with A(m,k) = a[m sam + k sak] and
 // B(k,n) = b[k sbk + n sbn], so one kernel serves the forward product and both
@@ -538,12 +785,6 @@ constexpr int kUpdChunk = 4 * kUpdATile + 4 * kUpdBTile;   // one K chunk: 96 KB
 constexpr int kUpdSmem = 2 * kUpdChunk;                    // the epilogue reuses 66.5 KB of it
 constexpr int kUpdLd = kUpdN + 1;                          // row stride of the staged product (float2)
 
-__device__ __forceinline__ float tf32_hi(float x) {
-    uint32_t r;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-    return __uint_as_float(r);
-}
-
 // The lookahead CTA: T = M[la, la] - C[la] M[k, la] in FP32, inverted into M[la, la] and pout.
 // buf: 3 x 64 x 65 complex in shared memory.
 __device__ __forceinline__ void gj_lookahead(int64_t w, int k, int la, int tb, float2* __restrict__ M,
@@ -668,11 +909,11 @@ __global__ void __launch_bounds__(kUpdThreads, 1) k_gj_update_tc(
         char* cb = base + (kk >> 5) * kUpdChunk;
         const uint32_t o = (uint32_t)((((wi >> 3) * (kK / 4) + (kc >> 2)) * 128) + ar * 16 + (kc & 3) * 4);
         const float2 x0 = va[it][0], x1 = va[it][1];
-        const float r0h = tf32_hi(x0.x), r1h = tf32_hi(x1.x), i0h = tf32_hi(x0.y), i1h = tf32_hi(x1.y);
+        const float r0h = tf32_rn(x0.x), r1h = tf32_rn(x1.x), i0h = tf32_rn(x0.y), i1h = tf32_rn(x1.y);
         *reinterpret_cast<float2*>(cb + 0 * kUpdATile + o) = make_float2(r0h, r1h);
-        *reinterpret_cast<float2*>(cb + 1 * kUpdATile + o) = make_float2(tf32_hi(x0.x - r0h), tf32_hi(x1.x - r1h));
+        *reinterpret_cast<float2*>(cb + 1 * kUpdATile + o) = make_float2(tf32_rn(x0.x - r0h), tf32_rn(x1.x - r1h));
         *reinterpret_cast<float2*>(cb + 2 * kUpdATile + o) = make_float2(i0h, i1h);
-        *reinterpret_cast<float2*>(cb + 3 * kUpdATile + o) = make_float2(tf32_hi(x0.y - i0h), tf32_hi(x1.y - i1h));
+        *reinterpret_cast<float2*>(cb + 3 * kUpdATile + o) = make_float2(tf32_rn(x0.y - i0h), tf32_rn(x1.y - i1h));
     }
 #pragma unroll
     for (int it = 0; it < 8; ++it) {
@@ -685,11 +926,11 @@ __global__ void __launch_bounds__(kUpdThreads, 1) k_gj_update_tc(
             const int ne = n + e;
             const uint32_t o = (uint32_t)((((ne >> 3) * (kK / 4) + (kc >> 2)) * 128) + (ne & 7) * 16 + (kc & 3) * 4);
             const float2 x = vb[it][e];
-            const float rh = tf32_hi(x.x), ih = tf32_hi(x.y);
+            const float rh = tf32_rn(x.x), ih = tf32_rn(x.y);
             *reinterpret_cast<float*>(cb + 0 * kUpdBTile + o) = rh;
-            *reinterpret_cast<float*>(cb + 1 * kUpdBTile + o) = tf32_hi(x.x - rh);
+            *reinterpret_cast<float*>(cb + 1 * kUpdBTile + o) = tf32_rn(x.x - rh);
             *reinterpret_cast<float*>(cb + 2 * kUpdBTile + o) = ih;
-            *reinterpret_cast<float*>(cb + 3 * kUpdBTile + o) = tf32_hi(x.y - ih);
+            *reinterpret_cast<float*>(cb + 3 * kUpdBTile + o) = tf32_rn(x.y - ih);
         }
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -840,6 +1081,39 @@ int tc_slab_product(int64_t w, int64_t row0, int64_t Bc, const void* groups, int
     tc::k_cgemm_tf32<<<grid, tc::kThreads, tc::kCxSmem + 1024, st>>>(
         w, row0, Bc, static_cast<const tc::TcGroup*>(groups), Sinv, totD, offD, Y, alpha, beta, Out, status);
     EMG_CUDA(cudaGetLastError());
+    return EMG_OK;
+}
+}  // namespace emg
+
+// Split-TF32 slab product (declared in emg_krylov.cuh).
+namespace emg {
+int tc_slab_split(int64_t w, int64_t row0, int64_t Bc, const void* groups, int G, int maxcol, int max_splits,
+                  const float2* Sinv, int64_t totD, int64_t offD, const float2* Y, float alpha, int beta, float2* Out,
+                  int32_t* status, cudaStream_t st) {
+    static bool attr = false;
+    if (!attr) {
+        EMG_CUDA(cudaFuncSetAttribute(tc::k_slab_split, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::kSpSmem + 1024));
+        attr = true;
+    }
+    const int ct = (maxcol + tc::kN - 1) / tc::kN, rt = (int)((w + tc::kM - 1) / tc::kM);
+    // K split: double it while the CTAs fit one wave and each keeps two chunks
+    int ranks = 1;
+    while (ranks < 8 && 2 * ranks <= max_splits && (int64_t)ct * rt * G * 2 * ranks <= 152 && w >= 2 * ranks * 2 * tc::kK)
+        ranks *= 2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)ranks, (unsigned)rt, (unsigned)(G * ct));
+    cfg.blockDim = dim3(tc::kSpThreads);
+    cfg.dynamicSmemBytes = tc::kSpSmem + 1024;
+    cfg.stream = st;
+    cudaLaunchAttribute la[1];
+    la[0].id = cudaLaunchAttributeClusterDimension;
+    la[0].val.clusterDim.x = (unsigned)ranks;
+    la[0].val.clusterDim.y = 1;
+    la[0].val.clusterDim.z = 1;
+    cfg.attrs = la;
+    cfg.numAttrs = 1;
+    EMG_CUDA(cudaLaunchKernelEx(&cfg, tc::k_slab_split, w, row0, Bc, static_cast<const tc::TcGroup*>(groups), G, Sinv, totD,
+                                offD, Y, alpha, beta, Out, status));
     return EMG_OK;
 }
 }  // namespace emg

@@ -1,0 +1,73 @@
+"""Slab solves of every column count at which the dense product changes (rows of few columns,
+tensor-core tiles, column tiles of 64), one and two factors, odd slab widths.
+
+The products work on the same factors, so the error of a solve is the factor's: each column
+count must be within twice the error of single columns (FP32), or within 1e-9 (FP64).
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def system():
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from emerge_gb300 import _build
+    _build.build()
+    from emerge_gb300.freq import Assembler
+    from emerge_gb300.geometry import straight_waveguide
+    from emerge_gb300.solver import FrequencySweep, RestrictedSystem, SlabFactor, locality_key
+    p = straight_waveguide(5e-3)
+    sw = FrequencySweep(Assembler(), p.field, p.er, p.ur, p.bcs)
+    k0, gam, _ = sw._coeffs([9.1e9, 10.7e9])
+    # without every 29th unknown some slabs are odd: their rows are not 16-byte aligned
+    ids = np.delete(sw.solve_ids, np.arange(0, len(sw.solve_ids), 29))
+    sysr = RestrictedSystem(sw.plan.indptr, sw.plan.indices[: sw.plan.nnz], sw.plan.nnz, ids)
+    A = sysr.form(sw.E, sw.B, k0 ** 2, sw.P, gam)
+    return torch, sysr, A, SlabFactor(sysr, None, locality_key(p.field, ids))
+
+
+COLUMNS = [1, 2, 3, 4, 5, 7, 8, 9, 15, 16, 17, 31, 33, 48, 63, 64, 65, 130]
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_column_counts(system, precision):
+    torch, sysr, A, slab = system
+    off, _ = slab.levels()
+    assert np.any(np.diff(off) % 2 == 1)
+    slab.factor(A, [0, 1], precision)
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    n = sysr.n
+    x = torch.view_as_complex(torch.randn((n, 2 * max(COLUMNS), 2), generator=gen, device="cuda", dtype=torch.float64))
+    cm = torch.zeros(x.shape[1], dtype=torch.int32, device="cuda")
+    cm[1::2] = 1                                   # column c belongs to matrix c % 2
+    b = sysr.spmv(A, x, cm)
+    err = lambda y, ref: (torch.linalg.norm(y - ref, dim=0) / torch.linalg.norm(ref, dim=0)).cpu().numpy()  # noqa: E731
+    single = max(err(slab.apply(b[:, c:c + 1], [c % 2]), x[:, c:c + 1])[0] for c in range(12))
+    limit = 2 * single if precision == "fp32" else 1e-9
+    for cols in COLUMNS:
+        one = torch.arange(0, 2 * cols, 2, device="cuda")            # one group
+        two = torch.cat([one, one + 1])                                # two groups, one per factor
+        for pick, fac in ((one, [0] * cols), (two, [0] * cols + [1] * cols)):
+            e = err(slab.apply(b[:, pick], fac), x[:, pick])
+            assert e.max() <= limit, (cols, len(fac), e.max(), limit)
+
+
+def test_split_settings_agree(system):
+    """The K split changes the order of the sum only."""
+    torch, sysr, A, slab = system
+    slab.factor(A, [0], "fp32")
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    x = torch.view_as_complex(torch.randn((sysr.n, 20, 2), generator=gen, device="cuda", dtype=torch.float64))
+    b = sysr.spmv(A, x, torch.zeros(20, dtype=torch.int32, device="cuda"))
+    errs = []
+    for splits in (1, 2, 4, 8, 16):
+        slab.set_max_splits(splits)
+        y = slab.apply(b, [0] * 20)
+        assert torch.equal(torch.view_as_real(y), torch.view_as_real(slab.apply(b, [0] * 20)))
+        errs.append(float(torch.linalg.norm(y - x) / torch.linalg.norm(x)))
+    slab.set_max_splits(8)
+    assert max(errs) <= 2 * min(errs)
