@@ -87,6 +87,16 @@ int tc_gj_update(int64_t w, int k, int la, int64_t F, float2* Sinv, int64_t totD
                  int64_t scol, const float2* pinv, float2* pinv_next, float rel_thr, int32_t* perturbed,
                  int32_t* status, cudaStream_t st);
 
+// FP64 block Gauss-Jordan on the tensor cores (emg_fp64.cu).  fp64_tile: inverse of pivot tile
+// (k, k) of the F complex128 w x w blocks Sinv + f totD + offD, into M and pinv (64 x 64 per
+// factor).  fp64_step: stage 0 forms the row panel (``rows``, 64 x w) and keeps the column panel
+// (``cols``, w x 64), stage 1 updates tile (la, la), stage 2 everything else; rows and cols
+// have sbuf entries per factor.  status (device) is set to 1 if a bounded wait ran out.
+int fp64_tile(int64_t w, int k, int64_t F, double2* Sinv, int64_t totD, int64_t offD, double2* pinv, double rel_thr,
+              int32_t* perturbed, cudaStream_t st);
+int fp64_step(int stage, int64_t w, int k, int la, int64_t F, double2* Sinv, int64_t totD, int64_t offD, const double2* pinv,
+              double2* rows, double2* cols, int64_t sbuf, int32_t* status, cudaStream_t st);
+
 // Preconditioner on FP32 vectors (the inner solves of the mixed-precision refinement).
 struct Precond32 {
     virtual ~Precond32() = default;

@@ -62,7 +62,6 @@ __device__ __forceinline__ double2 to_d(double2 v) { return v; }
 
 constexpr int kTile = 64;          // Gauss-Jordan tile and GEMM output tile
 constexpr int kThreads = 256;
-constexpr int kDiagThreads = 256;   // pivot-tile inversion: a 4 x 4 block per thread
 constexpr int kMaxRows = 16;       // rows per CTA in the Schur-complement kernel
 constexpr int kSchurSmem = 200 * 1024;
 constexpr int64_t kMaxWidth = 12288;
@@ -203,216 +202,6 @@ __global__ void __launch_bounds__(kThreads) k_schur(int64_t wp, int64_t w, int64
                 s.y -= acc[a].y;
             }
     }
-}
-
-// In-place inverse of pivot tile k (tb x tb, padded with the identity when tb < 64)
-// with partial pivoting inside the tile; the inverse also goes to pinv (ld 64).
-// Grid 1 x 1 x F.  Gauss-Jordan: pivot = largest |a_rc| on or below the diagonal, the
-// lower row on ties (magnitudes compared in FP32); pivots with |a|^2 at or below
-// rel_thr^2 max|a|^2 are replaced by that threshold and counted; the row swaps are
-// applied as one column permutation at the end.
-//
-// 256 threads as a 16 x 16 grid: thread (ty, tx) holds rows ty + 16 i and columns
-// tx + 16 j (i, j < 4) of the tile in registers.  The pivot loop runs over four
-// column blocks of 16 with the block index a compile-time constant, so the pivot
-// column and row sit at fixed register positions.  Step c:
-//   (S) the owners of row p and row c leave them in shared memory, the owners of
-//       column c leave it with rows c and p exchanged, the owner of a_pc forms the
-//       reciprocal of the pivot;
-//   (U) the owners of row p take the old row c; column c becomes the identity column
-//       and row c of the multiplier row the reciprocal, so one rank-1 update forms
-//       both the eliminated entries and the new column c; row c takes the scaled
-//       pivot row; the owners of column c + 1 (two lanes per warp) reduce their rows
-//       to one packed (|a|^2, row) key per warp.
-// Two barriers per pivot, no tile in shared memory.
-template <typename T> __device__ __forceinline__ T crecip(T v);
-template <> __device__ __forceinline__ float2 crecip<float2>(float2 v) {
-    const float s = __frcp_rn(v.x * v.x + v.y * v.y);
-    return make_float2(v.x * s, -v.y * s);
-}
-template <> __device__ __forceinline__ double2 crecip<double2>(double2 v) {
-    const double s = __drcp_rn(v.x * v.x + v.y * v.y);
-    return make_double2(v.x * s, -v.y * s);
-}
-
-// (|a|^2 as FP32 bits, 63 - row): the unsigned maximum is the largest magnitude, then the lowest row
-template <typename R> __device__ __forceinline__ unsigned long long pivot_key(R m2, int r) {
-    return ((unsigned long long)__float_as_uint((float)m2) << 32) | (unsigned)(63 - r);
-}
-
-template <typename R> struct DiagShared {
-    using T = typename C2<R>::T;
-    T prow[kTile], orow[kTile], colc[kTile];
-    unsigned long long cand[kDiagThreads / 32];
-    int piv[kTile], perm[kTile], iperm[kTile];
-    R red[kDiagThreads / 32];
-    T inv;
-};
-
-// the key of the best row r > rmin (r < tb) of column 16 JN + tx among this thread's
-// rows, combined over lanes tx and tx + 16; lane tx (== column % 16) stores it
-template <int JN, typename R>
-__device__ __forceinline__ void diag_candidates(const typename C2<R>::T (&a)[4][4], int cn, int rmin, int tb,
-                                                DiagShared<R>& sh) {
-    const int tid = threadIdx.x, lane = tid & 31, ty = tid >> 4, tx = tid & 15;
-    unsigned long long key = 0;
-    if (tx == (cn & 15)) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int r = ty + 16 * i;
-            const R m2 = a[i][JN].x * a[i][JN].x + a[i][JN].y * a[i][JN].y;
-            const unsigned long long kk = (r > rmin && r < tb) ? pivot_key<R>(m2, r) : 0ull;
-            key = kk > key ? kk : key;
-        }
-    }
-    const unsigned long long o = __shfl_xor_sync(0xffffffffu, key, 16);
-    key = o > key ? o : key;
-    if (lane == (cn & 15)) sh.cand[tid >> 5] = key;
-}
-
-template <int JC, typename R>
-__device__ __forceinline__ void diag_block(typename C2<R>::T (&a)[4][4], int tb, R thr2, typename C2<R>::T thr_pivot,
-                                           DiagShared<R>& sh, int32_t* __restrict__ pert) {
-    using T = typename C2<R>::T;
-    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-    for (int cl = 0; cl < 16; ++cl) {
-        const int c = 16 * JC + cl;
-        if (c >= tb) return;   // uniform
-        unsigned long long best = 0;
-#pragma unroll
-        for (int q = 0; q < kDiagThreads / 32; ++q) best = sh.cand[q] > best ? sh.cand[q] : best;
-        const int p = 63 - (int)(best & 0xffffffffu);
-        // (S)
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-            if (ty + 16 * i == p) {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) sh.prow[tx + 16 * j] = a[i][j];
-                if (tx == cl) {
-                    const T v = a[i][JC];
-                    const bool small = !(v.x * v.x + v.y * v.y > thr2);   // also catches a zero pivot
-                    sh.inv = crecip(small ? thr_pivot : v);
-                    if (small) atomicAdd(pert, 1);
-                }
-            }
-        if (ty == cl && p != c) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) sh.orow[tx + 16 * j] = a[JC][j];
-        }
-        if (tx == cl) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int r = ty + 16 * i;
-                sh.colc[(r == p || r == c) ? (r ^ p ^ c) : r] = a[i][JC];
-            }
-        }
-        if (tid == 0) sh.piv[c] = p;
-        __syncthreads();
-        // (U)
-        const T inv = sh.inv;
-        T rj[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) rj[j] = cmul(sh.prow[tx + 16 * j], inv);
-        if (p != c) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-                if (ty + 16 * i == p) {
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) a[i][j] = sh.orow[tx + 16 * j];
-                }
-        }
-        if (tx == cl) {   // after the swap: column c -> 0, its multiplier -> 1 / pivot
-            rj[JC] = inv;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) a[i][JC] = mk((R)0, (R)0);
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const T cr = sh.colc[ty + 16 * i];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const T t = cmul(cr, rj[j]);
-                a[i][j].x -= t.x;
-                a[i][j].y -= t.y;
-            }
-        }
-        if (ty == cl) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) a[JC][j] = rj[j];
-        }
-        if (c + 1 < tb) {
-            if (cl < 15) diag_candidates<JC, R>(a, c + 1, c, tb, sh);
-            else if (JC < 3) diag_candidates<(JC < 3 ? JC + 1 : 3), R>(a, c + 1, c, tb, sh);
-        }
-        __syncthreads();
-    }
-}
-
-template <typename R>
-__global__ void __launch_bounds__(kDiagThreads, 1) k_gj_diag(int64_t w, int k, typename C2<R>::T* __restrict__ Sinv,
-                                                         int64_t totD, int64_t offD, typename C2<R>::T* __restrict__ pinv,
-                                                         R rel_thr, int32_t* __restrict__ perturbed) {
-    using T = typename C2<R>::T;
-    __shared__ DiagShared<R> sh;
-    const int64_t f = blockIdx.z;
-    T* M = Sinv + f * totD + offD;
-    const int64_t k0 = (int64_t)k * kTile;
-    const int tb = (int)min((int64_t)kTile, w - k0);
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const int ty = tid >> 4, tx = tid & 15;
-    T a[4][4];
-    R mx = 0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int r = ty + 16 * i, cc = tx + 16 * j;
-            T v;
-            if (r < tb && cc < tb) {
-                v = M[(k0 + r) * w + k0 + cc];
-                mx = max(mx, v.x * v.x + v.y * v.y);
-            } else {
-                v = mk((R)(r == cc ? 1 : 0), (R)0);
-            }
-            a[i][j] = v;
-        }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if (lane == 0) sh.red[wid] = mx;
-    diag_candidates<0, R>(a, 0, -1, tb, sh);
-    __syncthreads();
-    R thr2 = 0;
-#pragma unroll
-    for (int i = 0; i < kDiagThreads / 32; ++i) thr2 = max(thr2, sh.red[i]);
-    thr2 *= rel_thr * rel_thr;   // |pivot|^2 at or below this is replaced
-    const T thr_pivot = mk(thr2 > 0 ? (R)sqrt(thr2) : (R)1, (R)0);
-    int32_t* pert = perturbed + f;
-    diag_block<0, R>(a, tb, thr2, thr_pivot, sh, pert);
-    diag_block<1, R>(a, tb, thr2, thr_pivot, sh, pert);
-    diag_block<2, R>(a, tb, thr2, thr_pivot, sh, pert);
-    diag_block<3, R>(a, tb, thr2, thr_pivot, sh, pert);
-    if (tid == 0) {   // the swaps in reverse give the column permutation; iperm is its inverse
-        for (int c = 0; c < kTile; ++c) sh.perm[c] = c;
-        for (int c = tb - 1; c >= 0; --c) {
-            const int q = sh.piv[c];
-            if (q != c) { const int t = sh.perm[c]; sh.perm[c] = sh.perm[q]; sh.perm[q] = t; }
-        }
-        for (int c = 0; c < kTile; ++c) sh.iperm[sh.perm[c]] = c;
-    }
-    __syncthreads();
-    // column cc of the unpermuted inverse is column iperm[cc] of the result
-    T* P = pinv + f * kTile * kTile;
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int r = ty + 16 * i, cc = tx + 16 * j;
-            if (r < tb && cc < tb) {
-                const int cd = sh.iperm[cc];
-                M[(k0 + r) * w + k0 + cd] = a[i][j];
-                P[r * kTile + cd] = a[i][j];
-            }
-        }
 }
 
 // The FP32 pivot tile k by itself (emg_gj.cuh): M[k, k] and pinv receive its inverse.  Grid 1 x 1 x F.
@@ -1282,13 +1071,14 @@ int slab_factor_t(emg_slab* s, int64_t F, const int32_t* amat_h, int64_t Bm, con
     rc = dalloc(&amat, F, "slab amat");
     if (rc) { slab_free_factors(s); return rc; }
     struct Tmp { int32_t* p; ~Tmp() { if (p) cudaFree(p); } } tmp{amat};
-    const bool tc_update = sizeof(R) == 4 && s->tc_factor;
-    T* colbuf = nullptr;   // old column panel of a tensor-core step
+    const bool tc_update = s->tc_factor != 0;
+    T *colbuf = nullptr, *rowbuf = nullptr;   // column panel of a tensor-core step; row panel (FP64)
     if (tc_update) {
         rc = dalloc(&colbuf, F * s->maxw * kTile, "slab column panel");
-        if (rc) { slab_free_factors(s); return rc; }
+        if (!rc && sizeof(R) == 8) rc = dalloc(&rowbuf, F * s->maxw * kTile, "slab row panel");
+        if (rc) { dfree(colbuf); slab_free_factors(s); return rc; }
     }
-    struct TmpC { T* p; ~TmpC() { if (p) cudaFree(p); } } tmpc{colbuf};
+    struct TmpC { T *a, *b; ~TmpC() { if (a) cudaFree(a); if (b) cudaFree(b); } } tmpc{colbuf, rowbuf};
     // Newton-Schulz scratch: a copy of S_i and the factor 2I - S_i X (F blocks of maxw^2)
     T *Scopy = nullptr, *Rbuf = nullptr;
     double* npart = nullptr;
@@ -1359,16 +1149,17 @@ int slab_factor_t(emg_slab* s, int64_t F, const int32_t* amat_h, int64_t Bm, con
         // of step k + 1 is updated first and inverted while the rest of step k's update runs.
         T* const P0 = static_cast<T*>(s->pinv);
         auto pset = [&](int k) { return P0 + (int64_t)(k & 1) * F * kTile * kTile; };
-        auto tile = [&](int k, cudaStream_t ts) {   // inverse of tile (k, k) by itself
+        auto tile = [&](int k, cudaStream_t ts) -> int {   // inverse of tile (k, k) by itself
             if constexpr (sizeof(R) == 4)
                 k_gj_tile32<<<dim3(1, 1, (unsigned)F), gj::kThreads, 0, ts>>>(w, k, Sinv, s->totD, s->offD[i], pset(k),
                                                                              rel_thr, s->perturbed);
             else
-                k_gj_diag<R><<<dim3(1, 1, (unsigned)F), kDiagThreads, 0, ts>>>(w, k, Sinv, s->totD, s->offD[i], pset(k),
-                                                                              rel_thr, s->perturbed);
+                return emg::fp64_tile(w, k, F, Sinv, s->totD, s->offD[i], pset(k), rel_thr, s->perturbed, ts);
+            return EMG_OK;
         };
-        tile(0, st);
-        if (tc_update) {
+        rc = tile(0, st);
+        if (rc) return rc;
+        if (tc_update && sizeof(R) == 4) {
             // FP32: two launches a step on one stream; the second one's first CTA is the lookahead
             for (int k = 0; k < nt && nt > 1; ++k) {
                 if constexpr (sizeof(R) == 4) {
@@ -1387,16 +1178,40 @@ int slab_factor_t(emg_slab* s, int64_t F, const int32_t* amat_h, int64_t Bm, con
                 if (nt == 1) break;
                 const T* P = pset(k);
                 const int la = k + 1 < nt ? k + 1 : -1;
-                k_gj_panel<R><<<dim3(nt, 1, (unsigned)F), kThreads, 0, st>>>(0, w, k, Sinv, s->totD, s->offD[i], P, -1);
-                if (la >= 0) {
-                    k_gj_panel<R><<<dim3(1, 1, (unsigned)F), kThreads, 0, st>>>(3, w, k, Sinv, s->totD, s->offD[i], P, la);
+                // stage 0: row panel, 1: tile (la, la), 2: the rest
+                auto stage = [&](int q) -> int {
+                    if constexpr (sizeof(R) == 8) {
+                        if (tc_update)
+                            return emg::fp64_step(q, w, k, la, F, Sinv, s->totD, s->offD[i], P, rowbuf, colbuf,
+                                                  s->maxw * kTile, s->tc_status, st);
+                    }
+                    if (q == 0)
+                        k_gj_panel<R><<<dim3(nt, 1, (unsigned)F), kThreads, 0, st>>>(0, w, k, Sinv, s->totD, s->offD[i], P,
+                                                                                     -1);
+                    else if (q == 1)
+                        k_gj_panel<R><<<dim3(1, 1, (unsigned)F), kThreads, 0, st>>>(3, w, k, Sinv, s->totD, s->offD[i], P,
+                                                                                    la);
+                    else {
+                        k_gj_panel<R><<<dim3(nt, nt, (unsigned)F), kThreads, 0, st>>>(2, w, k, Sinv, s->totD, s->offD[i],
+                                                                                      P, la);
+                        k_gj_panel<R><<<dim3(nt, 1, (unsigned)F), kThreads, 0, st>>>(1, w, k, Sinv, s->totD, s->offD[i], P,
+                                                                                     -1);
+                    }
+                    return EMG_OK;
+                };
+                rc = stage(0);
+                if (!rc && la >= 0) {
+                    rc = stage(1);
                     EMG_CUDA(cudaEventRecord(side.tile_ready, st));
                     EMG_CUDA(cudaStreamWaitEvent(side.st, side.tile_ready, 0));
-                    tile(la, side.st);
+                    if (!rc) rc = tile(la, side.st);
                     EMG_CUDA(cudaEventRecord(side.diag_done, side.st));
                 }
-                k_gj_panel<R><<<dim3(nt, nt, (unsigned)F), kThreads, 0, st>>>(2, w, k, Sinv, s->totD, s->offD[i], P, la);
-                k_gj_panel<R><<<dim3(nt, 1, (unsigned)F), kThreads, 0, st>>>(1, w, k, Sinv, s->totD, s->offD[i], P, -1);
+                if (!rc) rc = stage(2);
+                if (rc) {
+                    cudaDeviceSynchronize();   // the side stream and the buffers go away
+                    return rc;
+                }
             }
         }
         // X <- X (2I - S X): squares the residual I - S X of the inverse.  S_i's copy

@@ -1,0 +1,91 @@
+"""FP64 slab factors from FP16 digits on the tensor cores: one dense block at the tile edges, rows
+and columns scaled over many orders of magnitude, and non-finite entries.
+
+The inverse of a well-conditioned n x n block (condition below 100 after scaling) has a relative
+error of a few n eps; scaling rows and columns by powers of two changes no digit of it.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+EPS = 2.0 ** -52
+
+
+@pytest.fixture(scope="module")
+def torch_cuda():
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from emerge_gb300 import _build
+    _build.build()
+    return torch
+
+
+def _dense_system(torch, n):
+    from emerge_gb300.solver import RestrictedSystem, SlabFactor
+    ip = torch.arange(0, n * n + 1, n, dtype=torch.int64, device="cuda")
+    ix = torch.arange(n, dtype=torch.int32, device="cuda").repeat(n)
+    sysr = RestrictedSystem(ip, ix, n * n, np.arange(n))
+    slab = SlabFactor(sysr, np.arange(n))          # all unknowns are seeds: one slab
+    assert slab.info()["slabs"] == 1
+    return sysr, slab
+
+
+def _matrix(torch, n, seed):
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    A = torch.view_as_complex(torch.randn((n, n, 2), generator=gen, device="cuda", dtype=torch.float64)) / (2 * n) ** 0.5
+    return A + 3.0 * torch.eye(n, device="cuda")
+
+
+@pytest.mark.parametrize("n", [1, 2, 63, 64, 65, 96, 127, 128, 129, 191, 193, 320])
+@pytest.mark.parametrize("tensor_cores", [True, False])
+def test_dense_inverse(torch_cuda, n, tensor_cores):
+    torch = torch_cuda
+    sysr, slab = _dense_system(torch, n)
+    A = _matrix(torch, n, n)
+    slab.set_factor_tensor_cores(tensor_cores)
+    slab.factor(A.reshape(-1, 1).contiguous(), [0], "fp64")
+    X = slab.apply(torch.eye(n, dtype=torch.complex128, device="cuda"), [0] * n)
+    R = A @ X - torch.eye(n, device="cuda")
+    assert float(torch.linalg.norm(R, ord=2)) <= 100 * n * EPS
+    assert slab.info()["perturbed_pivots"] == 0
+
+
+def test_scaled_rows_and_columns(torch_cuda):
+    torch = torch_cuda
+    n = 200
+    sysr, slab = _dense_system(torch, n)
+    A = _matrix(torch, n, 5)
+    rng = np.random.default_rng(2)
+    # the largest spread that keeps every pivot above the 1e-13 of the tile maximum where it is replaced
+    dr = torch.as_tensor(2.0 ** rng.integers(-8, 9, n), device="cuda")
+    dc = torch.as_tensor(2.0 ** rng.integers(-8, 9, n), device="cuda")
+    S = dr[:, None] * A * dc[None, :]
+    slab.factor(S.reshape(-1, 1).contiguous(), [0], "fp64")
+    X = slab.apply(torch.eye(n, dtype=torch.complex128, device="cuda"), [0] * n)
+    assert slab.info()["perturbed_pivots"] == 0
+    R = A @ (dc[:, None] * X * dr[None, :]) - torch.eye(n, device="cuda")
+    assert float(torch.linalg.norm(R, ord=2)) <= 1e5 * n * EPS    # row scaling changes the pivots of a tile
+
+
+def test_two_factors_of_one_launch(torch_cuda):
+    torch = torch_cuda
+    n = 130
+    sysr, slab = _dense_system(torch, n)
+    A, B = _matrix(torch, n, 8), _matrix(torch, n, 9)
+    slab.factor(torch.stack([A.reshape(-1), B.reshape(-1)], dim=1).contiguous(), [1, 0], "fp64")
+    eye = torch.eye(n, dtype=torch.complex128, device="cuda")
+    for f, M in ((0, B), (1, A)):
+        assert float(torch.linalg.norm(M @ slab.apply(eye, [f] * n) - eye, ord=2)) <= 100 * n * EPS
+
+
+def test_non_finite_entries_stay_visible(torch_cuda):
+    """A non-finite entry outside the first pivot tile gives non-finite results, not finite wrong ones."""
+    torch = torch_cuda
+    n = 150
+    sysr, slab = _dense_system(torch, n)
+    A = _matrix(torch, n, 11)
+    A[100, 20] = complex(float("inf"), 0.0)
+    slab.factor(A.reshape(-1, 1).contiguous(), [0], "fp64")
+    X = slab.apply(torch.ones((n, 1), dtype=torch.complex128, device="cuda"), [0])
+    assert not bool(torch.isfinite(torch.view_as_real(X)).all())
