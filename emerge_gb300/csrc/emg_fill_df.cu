@@ -545,7 +545,9 @@ __global__ void __launch_bounds__(32 * kWarps) k_fill_df(const Rec2* __restrict_
 //              columns in the entity's row.
 //   k_elem     (per fill, thread per tet): the element blocks of D and F into a staging
 //              buffer laid out (tet, row pair, column)-major.
-//   k_fill_st  (per fill, warp per entity group): the owner pass over the staging buffer.
+//   k_pos_desc (plan, warp per entity): per CSR position, the one or two staged units it sums.
+//   k_fill_st, k_fill_own (per fill, thread per CSR position): the owner pass over the
+//              staging buffer.
 constexpr int kInv = 43;                 // 10 Gram + 21 cross-product Gram + 6 distances + 6 edge lengths
 constexpr int kInvDs = 31, kInvLen = 37;
 constexpr int kElemThreads = 128;
@@ -741,8 +743,9 @@ __global__ void k_inc_pos(const int32_t* __restrict__ ent_list, int64_t n_ent, c
 }
 
 // Staging layout: for tet t, entity slot s (the row pair) and column c = j + 10 b
-// (column slot j, mode b), one 32-byte unit of two float4: (D[0][c], D[1][c]) and
-// (F[0][c], F[1][c]), float-float, rows 0 and 1 of the pair.  Units are interleaved over
+// (column slot j, mode b), one 32-byte unit of two float4: D[0][c], D[1][c] and F[0][c],
+// F[1][c] in float-float, rows 0 and 1 of the pair, as (high, high, low, low): the owner pass
+// handles both rows with packed FP32 instructions.  Units are interleaved over
 // blocks of kStBlk consecutive tets, unit index ((t / kStBlk * 10 + s) * 20 + c) * kStBlk
 // + t % kStBlk: the element kernel's warp (one tet per lane) stores whole lines, and the
 // owner pass reads the 20 columns of a (tet, row pair) as 20 full sectors.
@@ -752,8 +755,8 @@ __host__ __device__ __forceinline__ int64_t st_unit(int64_t t, int s, int c) {
 }
 __device__ __forceinline__ void st_col(float4* st, int64_t t, int s, int c, df d0, df d1, df f0, df f1) {
     float4* o = st + st_unit(t, s, c) * 2;
-    o[0] = make_float4(d0.h, d0.l, d1.h, d1.l);
-    o[1] = make_float4(f0.h, f0.l, f1.h, f1.l);
+    o[0] = make_float4(d0.h, d1.h, d0.l, d1.l);
+    o[1] = make_float4(f0.h, f1.h, f0.l, f1.l);
 }
 
 // block (s, j) into the rows of s, and (when s != j) its transpose into the rows of j;
@@ -771,12 +774,15 @@ __device__ __forceinline__ void st_pair(float4* st, int64_t t, int s, int j, con
 }
 
 // Per fill, thread per tet: the 20 x 20 element blocks of D and F, each symmetric block
-// evaluated once and staged on both sides.
+// evaluated once and staged on both sides.  Grid y: the row slots s = y, y + gridDim.y, ...
+// of every tet, for meshes whose tets alone do not fill the GPU (a thread takes 45 us for its
+// 61 blocks: 360 tets 49 -> 17 us; from 30k tets on one slice is the fastest).
 __global__ void __launch_bounds__(kElemThreads) k_elem(const float2* __restrict__ inv, int64_t nT,
-                                                       float4* __restrict__ st) {
+                                                       float4* __restrict__ st, int* __restrict__ complex_mu) {
     __shared__ float2 sinv[kInv * kElemThreads];
     __shared__ float vt[625];
     const int tid = threadIdx.x;
+    if (blockIdx.x == 0 && blockIdx.y == 0 && tid == 0) *complex_mu = 0;   // k_scales, launched after this, sets it
     for (int i = tid; i < 625; i += kElemThreads) vt[i] = c_vint[i];
     for (int64_t t0 = (int64_t)blockIdx.x * kElemThreads; t0 < nT; t0 += (int64_t)gridDim.x * kElemThreads) {
         const int64_t t = t0 + tid;
@@ -789,7 +795,7 @@ __global__ void __launch_bounds__(kElemThreads) k_elem(const float2* __restrict_
         const SmTet T{sinv, tid};
         df D[2][2], F[2][2], Fl[2][2];
 #pragma unroll 1
-        for (int s = 0; s < 6; ++s) {
+        for (int s = (int)blockIdx.y; s < 6; s += (int)gridDim.y) {
 #pragma unroll 1
             for (int j = s; j < 6; ++j) {
                 blk_ee(T, vt, c_cedge[s][0], c_cedge[s][1], s, c_cedge[j][0], c_cedge[j][1], j, D, F);
@@ -803,6 +809,7 @@ __global__ void __launch_bounds__(kElemThreads) k_elem(const float2* __restrict_
         }
 #pragma unroll 1
         for (int fi = 0; fi < 4; ++fi) {
+            if ((6 + fi) % gridDim.y != blockIdx.y) continue;
 #pragma unroll 1
             for (int fj = fi; fj < 4; ++fj) {
                 blk_ff(T, vt, c_cface[fi][0], c_cface[fi][1], c_cface[fi][2], c_cface[fj][0], c_cface[fj][1],
@@ -816,201 +823,317 @@ __global__ void __launch_bounds__(kElemThreads) k_elem(const float2* __restrict_
     }
 }
 
-// One fast-fill entity in group order: its two CSR row offsets, first incidence, row
-// length and incidence count (built at plan time, read with one load per entity).
-struct __align__(16) EntDesc {
-    int64_t b1, b2, i0;
-    int32_t n, k;
-};
-
-__global__ void k_ent_desc(const int32_t* __restrict__ gents, int64_t n, const int32_t* __restrict__ partner,
-                           const int64_t* __restrict__ inc_ptr, const int64_t* __restrict__ indptr,
-                           EntDesc* __restrict__ d) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t r = gents[i];
-        EntDesc e;
-        e.b1 = indptr[r];
-        e.b2 = indptr[partner[r]];
-        e.i0 = inc_ptr[r];
-        e.n = (int32_t)(indptr[r + 1] - e.b1);
-        e.k = (int32_t)(inc_ptr[r + 1] - e.i0);
-        d[i] = e;
-    }
-}
-
-// Owner pass, warp per entity group.  At the start of a group its entity descriptors and
-// incidences go to shared memory; the group's incident tets then run as one sequence,
-// entity after entity, each entity's tets in ascending order.  For each tet, lane c < 20
-// takes column c (slot c % 10, mode c / 10) of the tet's staged row pair, i.e. one CSR
-// position of the entity's rows, and adds the scaled D and F entries of both rows into
-// the entity's accumulators in shared memory.  A tet's 20 columns are 20 different
-// positions, so the lanes never collide, and every position sums its contributions in
-// tet order (deterministic, bitwise repeatable).  The next tet's run is loaded while the
-// current one is added, across entity boundaries too; an entity's rows are converted and
-// stored after its last tet.  The kernel runs in two modes: IM = false accumulates Re E,
-// Re B and Im B and writes E and B (Im E = 0); IM = true, launched after it, returns at
-// once unless some tet's mu^-1 is complex, and then accumulates Im E and writes it.
-constexpr int kAcc = 3;                 // accumulators per (row, position)
-constexpr int kRing = 4;                // tets in flight per warp (prefetch distance kRing - 1)
-struct __align__(16) RingSlot {
-    float4 col[20][2];                  // the staged unit of each column: (D0, D1), (F0, F1)
-    float4 sc[2];                       // the tet's material scales
-    uint32_t pos[8];                    // the 20 CSR positions (bytes), padded
-};
-struct __align__(16) OwnSm {
-    float2 acc[2 * kNmax * kAcc];       // [row][position][component] compensated (s, e)
-    RingSlot ring[kRing];
-    EntDesc ed[kGmax];
-    int64_t iidx[kKmax];                // incidence index of each step
-    int32_t tet[kKmax];
-    int8_t slot[kKmax];
-    int8_t ent[kKmax];                  // entity (within the group) of each step
-    int32_t kofs[kGmax + 1];
-};
-constexpr int kOwnWarps = 4;
-constexpr size_t kStSmem = sizeof(OwnSm) * kOwnWarps;
-
-__device__ __forceinline__ void acc_sm(float2& c, df x, df y) {   // c += x * y
-    const float p = __fmul_rn(x.h, y.h);
-    float pe = __fmaf_rn(x.h, y.h, -p);
-    pe = __fmaf_rn(x.h, y.l, pe);
-    pe = __fmaf_rn(x.l, y.h, pe);
-    const float t = __fadd_rn(c.x, p);
-    const float bb = __fsub_rn(t, c.x);
-    const float err = __fadd_rn(__fsub_rn(c.x, __fsub_rn(t, bb)), __fsub_rn(p, bb));
-    c.y = __fadd_rn(c.y, __fadd_rn(err, pe));
-    c.x = t;
-}
-
-__device__ __forceinline__ void cp16(void* smem, const void* gmem) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)),
-                 "l"(gmem)
-                 : "memory");
-}
-__device__ __forceinline__ void cp4(void* smem, const void* gmem) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)),
-                 "l"(gmem)
-                 : "memory");
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-// Asynchronous copies of step i's data into ring slot i % kRing: lane c < 20 its staged
-// column unit, lanes 20-21 the tet's scales, lanes 22-26 the 20 position bytes.  Every
-// lane commits one group per step (empty for idle lanes), so group counts stay aligned.
-__device__ __forceinline__ void ring_issue(RingSlot& r, const float4* __restrict__ st, const float4* __restrict__ tscale,
-                                           const uint8_t* __restrict__ ipos, int64_t t, int slot, int64_t iidx,
-                                           int lane, bool im) {
-    if (lane < 20) {
-        const float4* u = st + st_unit(t, slot, lane) * 2;
-        cp16(&r.col[lane][0], u);
-        if (!im) cp16(&r.col[lane][1], u + 1);
-    } else if (lane < 22) {
-        cp16(&r.sc[lane - 20], tscale + 2 * t + (lane - 20));
-    } else if (lane < 27) {
-        cp4(&r.pos[lane - 22], ipos + iidx * 20 + 4 * (lane - 22));
-    }
-    cp_commit();
-}
-
-template <bool IM>
-__global__ void __launch_bounds__(32 * kOwnWarps) k_fill_st(const float4* __restrict__ st, const uint8_t* __restrict__ ipos,
-                                                            const int2* __restrict__ groups, int64_t n_groups,
-                                                            const EntDesc* __restrict__ edesc,
-                                                            const int64_t* __restrict__ inc_c,
-                                                            const float4* __restrict__ tscale,
-                                                            const int* __restrict__ complex_mu,
-                                                            double2* __restrict__ E, double2* __restrict__ B) {
-    if (IM && *complex_mu == 0) return;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    OwnSm* sm_all = reinterpret_cast<OwnSm*>(smem_raw);
+// Two tets share at most a face, so an entity's column gets contributions from at most two
+// of its tets, but for an edge's own two columns (all of them).  Plan time, warp per entity:
+// over[e] = 1 if some other column has more (no such mesh has been seen; the entity then goes
+// to the FP64 fill).
+__global__ void k_pos_check(const int32_t* __restrict__ ent_list, int64_t n_ent, const int64_t* __restrict__ inc_ptr,
+                            const int64_t* __restrict__ inc_c, const int64_t* __restrict__ indptr,
+                            const uint8_t* __restrict__ ipos, uint8_t* __restrict__ over) {
+    __shared__ int cnt[8][256];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    OwnSm& sm = sm_all[w];
-    constexpr int nc = IM ? 1 : kAcc;
-    for (int64_t g = blockIdx.x * (int64_t)kOwnWarps + w; g < n_groups; g += (int64_t)gridDim.x * kOwnWarps) {
-        const int2 gr = groups[g];
-        const int nsub = gr.y;
-        if (lane < nsub) sm.ed[lane] = edesc[gr.x + lane];
-        __syncwarp();
-        if (lane == 0) {
-            int ko = 0;
-            for (int u = 0; u < nsub; ++u) {
-                sm.kofs[u] = ko;
-                ko += sm.ed[u].k;
-            }
-            sm.kofs[nsub] = ko;
-        }
-        __syncwarp();
-        const int ktot = sm.kofs[nsub];
-        int nmax = 0;
-        for (int u = 0; u < nsub; ++u) nmax = max(nmax, sm.ed[u].n);
-        if (lane < ktot) {
-            int u = 0;
-            while (lane >= sm.kofs[u + 1]) ++u;
-            const int64_t ii = sm.ed[u].i0 + (lane - sm.kofs[u]);
-            const int64_t code = inc_c[ii];
-            sm.iidx[lane] = ii;
-            sm.tet[lane] = (int32_t)(code >> 4);
-            sm.slot[lane] = (int8_t)(code & 15);
-            sm.ent[lane] = (int8_t)u;
-        }
-        for (int i = lane; i < 2 * nmax * nc; i += 32) sm.acc[i] = make_float2(0.f, 0.f);
-        __syncwarp();
-        for (int i = 0; i < kRing - 1; ++i) {
-            if (i < ktot) ring_issue(sm.ring[i], st, tscale, ipos, sm.tet[i], sm.slot[i], sm.iidx[i], lane, IM);
-            else cp_commit();
-        }
-        for (int i = 0; i < ktot; ++i) {
-            const int u = sm.ent[i];
-            const int n = sm.ed[u].n;
-            const int ip = i + kRing - 1;
-            if (ip < ktot) ring_issue(sm.ring[ip % kRing], st, tscale, ipos, sm.tet[ip], sm.slot[ip], sm.iidx[ip], lane, IM);
-            else cp_commit();
-            cp_wait<kRing - 1>();
+    for (int64_t e = blockIdx.x * 8ll + w; e < n_ent; e += gridDim.x * 8ll) {
+        const int32_t r = ent_list[e];
+        const int64_t i0 = inc_ptr[r], k = inc_ptr[r + 1] - i0, n = indptr[r + 1] - indptr[r];
+        bool bad = false;
+        if (n <= 255) {
+            for (int i = lane; i < 256; i += 32) cnt[w][i] = 0;
             __syncwarp();
-            const RingSlot& r = sm.ring[i % kRing];
-            if (lane < 20) {
-                const int cp = reinterpret_cast<const uint8_t*>(r.pos)[lane];
-                const float4 cd = r.col[lane][0];
-                const float4 cse = r.sc[0];
-                float2* c0 = sm.acc + cp * nc;
-                float2* c1 = sm.acc + (n + cp) * nc;
-                const df D0 = mk(cd.x, cd.y), D1 = mk(cd.z, cd.w);
-                if (IM) {
-                    acc_sm(c0[0], mk(cse.z, cse.w), D0);
-                    acc_sm(c1[0], mk(cse.z, cse.w), D1);
-                } else {
-                    const float4 cf = r.col[lane][1];
-                    const float4 csb = r.sc[1];
-                    const df F0 = mk(cf.x, cf.y), F1 = mk(cf.z, cf.w);
-                    acc_sm(c0[0], mk(cse.x, cse.y), D0);
-                    acc_sm(c1[0], mk(cse.x, cse.y), D1);
-                    acc_sm(c0[1], mk(csb.x, csb.y), F0);
-                    acc_sm(c1[1], mk(csb.x, csb.y), F1);
-                    acc_sm(c0[2], mk(csb.z, csb.w), F0);
-                    acc_sm(c1[2], mk(csb.z, csb.w), F1);
-                }
-            }
-            __syncwarp();
-            if (i + 1 == ktot || sm.ent[i + 1] != u) {
-                const EntDesc& ed = sm.ed[u];
-                for (int x = lane; x < 2 * n; x += 32) {
-                    const int a = x >= n ? 1 : 0, p = x - a * n;
-                    float2* c = sm.acc + (a * n + p) * nc;
-                    const int64_t o = (a == 0 ? ed.b1 : ed.b2) + p;
-                    if (IM) {
-                        reinterpret_cast<double*>(E + o)[1] = to_double(fts(c[0].x, c[0].y));
-                    } else {
-                        E[o] = make_double2(to_double(fts(c[0].x, c[0].y)), 0.0);
-                        B[o] = make_double2(to_double(fts(c[1].x, c[1].y)), to_double(fts(c[2].x, c[2].y)));
-                    }
-#pragma unroll
-                    for (int cc = 0; cc < nc; ++cc) c[cc] = make_float2(0.f, 0.f);
+            for (int64_t q = 0; q < k; ++q) {
+                const int slot = (int)(inc_c[i0 + q] & 15);
+                if (lane < 20) {
+                    const int p = ipos[(i0 + q) * 20 + lane];
+                    if (++cnt[w][p] > 2 && (lane % 10 != slot || slot >= 6)) bad = true;
                 }
                 __syncwarp();
             }
         }
+        bad = __any_sync(0xffffffffu, bad);
+        if (lane == 0) over[e] = bad;
+        __syncwarp();
+    }
+}
+
+__global__ void k_ent_sizes(const int32_t* __restrict__ gents, int64_t n, const int64_t* __restrict__ indptr,
+                            int64_t* __restrict__ cnt) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        cnt[i] = indptr[gents[i] + 1] - indptr[gents[i]];
+}
+
+// *ragged becomes 1 unless entity i owns rows i and i + n_ent (in the fill's order), i.e. CSR
+// position o of a first row belongs to position o + nnz / 2 of the second.
+__global__ void k_pair_check(const int32_t* __restrict__ ent_list, int64_t n_ent, const int32_t* __restrict__ partner,
+                             const uint8_t* __restrict__ over, int* __restrict__ ragged) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n_ent; i += (int64_t)gridDim.x * blockDim.x)
+        if (ent_list[i] != i || partner[i] != i + n_ent || over[i]) atomicOr(ragged, 1);
+}
+
+// Plan time, warp per fast-fill entity: per CSR position of its first row the one or two staged
+// units summed there, in tet order (kNoUnit: none), and (rows given) the position in both rows.  An
+// own column of an edge with more than two tets has (kNoUnit, i) instead, and its units in
+// column i of ``own_u``: kKmax arrays of 2 n_e, kNoUnit beyond the edge's tets.
+constexpr uint32_t kNoUnit = 0xffffffffu;
+__global__ void k_pos_desc(const int32_t* __restrict__ ents, int64_t n_e, const int32_t* __restrict__ partner,
+                           const int64_t* __restrict__ inc_ptr, const int64_t* __restrict__ inc_c,
+                           const int64_t* __restrict__ indptr, const uint8_t* __restrict__ ipos,
+                           const int64_t* __restrict__ pofs, uint2* __restrict__ pdesc, longlong2* __restrict__ rows,
+                           uint32_t* __restrict__ own_u,
+                           unsigned long long* __restrict__ n_own) {
+    __shared__ uint2 con[8][kNmax];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int64_t i = blockIdx.x * 8ll + w; i < n_e; i += gridDim.x * 8ll) {
+        const int32_t r = ents[i];
+        const int64_t b1 = indptr[r], b2 = indptr[partner[r]], i0 = inc_ptr[r], k = inc_ptr[r + 1] - i0;
+        const int n = (int)(indptr[r + 1] - b1);
+        for (int x = lane; x < n; x += 32) con[w][x] = make_uint2(kNoUnit, kNoUnit);
+        __syncwarp();
+        int own_p = -1;
+        for (int64_t q = 0; q < k; ++q) {
+            const int64_t code = inc_c[i0 + q];
+            const int slot = (int)(code & 15);
+            if (lane < 20) {
+                const int p = ipos[(i0 + q) * 20 + lane];
+                if (k > 2 && slot < 6 && lane % 10 == slot) {
+                    if (q == 0) own_p = p;
+                } else {
+                    const uint32_t u = (uint32_t)st_unit(code >> 4, slot, lane);
+                    if (con[w][p].x == kNoUnit) con[w][p].x = u;
+                    else con[w][p].y = u;
+                }
+            }
+            __syncwarp();
+        }
+        if (own_p >= 0) {
+            const unsigned long long at = atomicAdd(n_own, 1ull);
+            con[w][own_p] = make_uint2(kNoUnit, (uint32_t)at);
+            for (int64_t q = 0; q < kKmax; ++q) {
+                const int64_t code = q < k ? inc_c[i0 + q] : 0;
+                const int slot = (int)(code & 15);
+                own_u[q * 2 * n_e + (int64_t)at] =
+                    q < k ? (uint32_t)st_unit(code >> 4, slot, slot + (lane < 10 ? 0 : 10)) : kNoUnit;
+            }
+        }
+        __syncwarp();
+        for (int x = lane; x < n; x += 32) {
+            pdesc[pofs[i] + x] = con[w][x];
+            if (rows) rows[pofs[i] + x] = make_longlong2(b1 + x, b2 + x);
+        }
+        __syncwarp();
+    }
+}
+
+// Owner pass, thread per CSR position of an entity's first row: the one or two staged units that
+// land there (both rows of the pair) are read, scaled and added in tet order in registers, and
+// both rows' E and B stored once.  The threads of a warp lie along a row: coalesced
+// descriptors and stores, whole 32-byte units, and no more dependent loads than descriptor
+// -> units.  The own columns of an edge, to which all its tets add, are summed by k_fill_own
+// before and only copied here, so that every line of E and B is written whole.  Every entry's
+// order is fixed: deterministic, bitwise repeatable.  Rows 0 and 1 share every scale and go
+// through packed FP32 instructions.  IM: some tet's mu^-1 is complex (the flag of
+// k_scales, read here so that the launch need not wait for it), Im E is accumulated too.
+// Scattering a tet's 20 columns into accumulators in shared memory (20 of 32 lanes, six loads
+// and six stores per tet and column, a second launch for Im E) took 13.4 ms at 80^3 cells and
+// 395 + 257 us for 85k tets of complex mu; a warp per entity with its descriptors, tets and
+// positions read one after the other 12.4 ms and 461 us; this 9.2 ms (5.2 TB/s) and 300 us with
+// k_fill_own.
+constexpr unsigned long long kNeg2 = 0x8000000080000000ull;
+__device__ __forceinline__ unsigned long long pk(float a, float b) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 unpk(unsigned long long v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long sub2(unsigned long long a, unsigned long long b) { return add2(a, b ^ kNeg2); }
+
+struct acc2 {                           // compensated sums of two rows
+    unsigned long long s, e;
+};
+// x * (yh + yl) of both rows as a value and its error
+__device__ __forceinline__ acc2 prod2(float xh, float xl, unsigned long long yh, unsigned long long yl) {
+    const unsigned long long h = pk(xh, xh), l = pk(xl, xl), p = mul2(h, yh);
+    return {p, fma2(l, yh, fma2(h, yl, fma2(h, yh, p ^ kNeg2)))};
+}
+__device__ __forceinline__ void add_to(acc2& a, const acc2& b) {
+    const unsigned long long t = add2(a.s, b.s), bb = sub2(t, a.s);
+    const unsigned long long err = add2(sub2(a.s, sub2(t, bb)), sub2(b.s, bb));
+    a.e = add2(a.e, add2(err, b.e));
+    a.s = t;
+}
+
+// (s + e) in FP64: the FP64 bits of the renormalised high part plus the low part in its
+// FP64 ulps as an integer.  High parts below 2^-66, zeros and non-finite values take to_double.
+__device__ __forceinline__ double sum_double(float s, float e) {
+    const df x = fts(s, e);
+    const unsigned hb = __float_as_uint(x.h), eh = (hb >> 23) & 0xffu;
+    if (eh - 61u > 193u) return to_double(x);
+    int t = __float2int_rn(x.l * __uint_as_float((hb & 0x80000000u) | ((306u - eh) << 23)));   // |t| <= 2^28
+    if ((hb & 0x7fffffu) == 0u && t < 0) t *= 2;   // below a power of two the ulp halves
+    const unsigned long long v = ((unsigned long long)(((hb & 0x7fffffffu) >> 3) + 0x38000000u) << 32) | (unsigned)(hb << 29);
+    return __longlong_as_double((long long)((v + (unsigned long long)(long long)t) | ((unsigned long long)(hb & 0x80000000u) << 32)));
+}
+
+// the products of staged unit u with its tet's scales: Re B, Im B, Re E and (IM) Im E of both rows
+template <int NC>
+__device__ __forceinline__ void unit_products(const float4* __restrict__ st, const float4* __restrict__ tscale, uint32_t u,
+                                              acc2 (&r)[NC]) {
+    const int64_t t = (int64_t)(u / (200u * kStBlk)) * kStBlk + u % kStBlk;
+    const float4 d = __ldg(st + 2 * (int64_t)u), f = __ldg(st + 2 * (int64_t)u + 1);
+    const float4 ce = __ldg(tscale + 2 * t), cb = __ldg(tscale + 2 * t + 1);
+    const unsigned long long dh = pk(d.x, d.y), dl = pk(d.z, d.w), fh = pk(f.x, f.y), fl = pk(f.z, f.w);
+    r[0] = prod2(cb.x, cb.y, fh, fl);
+    r[1] = prod2(cb.z, cb.w, fh, fl);
+    r[2] = prod2(ce.x, ce.y, dh, dl);
+    if (NC == 4) r[NC - 1] = prod2(ce.z, ce.w, dh, dl);
+}
+template <int NC>
+__device__ __forceinline__ void to_rows(const acc2 (&a)[NC], double2 (&r)[4]) {   // B, E of row 0, B, E of row 1
+    float2 s[NC], e[NC];
+#pragma unroll
+    for (int i = 0; i < NC; ++i) {
+        s[i] = unpk(a[i].s);
+        e[i] = unpk(a[i].e);
+    }
+    r[0] = make_double2(sum_double(s[0].x, e[0].x), sum_double(s[1].x, e[1].x));
+    r[2] = make_double2(sum_double(s[0].y, e[0].y), sum_double(s[1].y, e[1].y));
+    r[1] = make_double2(sum_double(s[2].x, e[2].x), NC == 4 ? sum_double(s[NC - 1].x, e[NC - 1].x) : 0.0);
+    r[3] = make_double2(sum_double(s[2].y, e[2].y), NC == 4 ? sum_double(s[NC - 1].y, e[NC - 1].y) : 0.0);
+}
+
+constexpr int kFillThreads = 256;
+// both rows of position i: its one or two units, or (own column) the sum of k_fill_own
+template <int NC, bool INLINE>
+__device__ __forceinline__ void fill_position(const float4* __restrict__ st, const float4* __restrict__ tscale, uint2 u,
+                                              const uint32_t* __restrict__ own_u, int64_t stride,
+                                              const double2* __restrict__ own_r, double2 (&r)[4]) {
+    acc2 a[NC], b[NC];
+    if (u.x != kNoUnit) {
+        unit_products<NC>(st, tscale, u.x, a);
+        if (u.y != kNoUnit) {
+            unit_products<NC>(st, tscale, u.y, b);
+#pragma unroll
+            for (int c = 0; c < NC; ++c) add_to(a[c], b[c]);
+        }
+        to_rows<NC>(a, r);
+    } else if (INLINE) {
+        unit_products<NC>(st, tscale, own_u[u.y], a);
+        for (int q = 1; q < kKmax; ++q) {
+            const uint32_t v = own_u[q * stride + u.y];
+            if (v == kNoUnit) break;
+            unit_products<NC>(st, tscale, v, b);
+#pragma unroll
+            for (int c = 0; c < NC; ++c) add_to(a[c], b[c]);
+        }
+        to_rows<NC>(a, r);
+    } else {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) r[c] = own_r[4 * (int64_t)u.y + c];
+    }
+}
+
+template <bool IM>
+__global__ void __launch_bounds__(kFillThreads) k_fill_st(const float4* __restrict__ st, int64_t n_pos,
+                                                          const uint2* __restrict__ pdesc,
+                                                          const longlong2* __restrict__ rows, int64_t half,
+                                                          const double2* __restrict__ own_r,
+                                                          const float4* __restrict__ tscale,
+                                                          const int* __restrict__ complex_mu, double2* __restrict__ E,
+                                                          double2* __restrict__ B) {
+    if ((*complex_mu != 0) != IM) return;
+    const int64_t step = (int64_t)gridDim.x * kFillThreads;
+    int64_t i = blockIdx.x * (int64_t)kFillThreads + threadIdx.x;
+    uint2 next = i < n_pos ? pdesc[i] : make_uint2(kNoUnit, kNoUnit);
+    for (; i < n_pos; i += step) {
+        const uint2 u = next;
+        if (i + step < n_pos) next = pdesc[i + step];
+        double2 r[4];
+        fill_position<IM ? 4 : 3, false>(st, tscale, u, nullptr, 0, own_r, r);
+        int64_t o1 = i, o2 = i + half;
+        if (rows) {
+            const longlong2 o = rows[i];
+            o1 = o.x;
+            o2 = o.y;
+        }
+        B[o1] = r[0];
+        B[o2] = r[2];
+        E[o1] = r[1];
+        E[o2] = r[3];
+    }
+}
+
+// The whole owner pass of a small mesh in one launch, thread per position: up to kSmallPos positions a
+// launch costs as much as its work (360 tets: five launches 74 us a fill, three and sliced
+// element blocks 31).
+constexpr int64_t kSmallPos = 152 * 4 * kFillThreads;
+__global__ void __launch_bounds__(kFillThreads) k_fill_small(const float4* __restrict__ st, int64_t n_pos,
+                                                             const uint2* __restrict__ pdesc,
+                                                             const longlong2* __restrict__ rows, int64_t half,
+                                                             const uint32_t* __restrict__ own_u, int64_t stride,
+                                                             const float4* __restrict__ tscale,
+                                                             const int* __restrict__ complex_mu, double2* __restrict__ E,
+                                                             double2* __restrict__ B) {
+    const int64_t i = blockIdx.x * (int64_t)kFillThreads + threadIdx.x;
+    if (i >= n_pos) return;
+    double2 r[4];
+    if (*complex_mu) fill_position<4, true>(st, tscale, pdesc[i], own_u, stride, nullptr, r);
+    else fill_position<3, true>(st, tscale, pdesc[i], own_u, stride, nullptr, r);
+    int64_t o1 = i, o2 = i + half;
+    if (rows) {
+        const longlong2 o = rows[i];
+        o1 = o.x;
+        o2 = o.y;
+    }
+    B[o1] = r[0];
+    B[o2] = r[2];
+    E[o1] = r[1];
+    E[o2] = r[3];
+}
+
+// The own columns of edges with more than two tets, thread per (edge, column), tets in order.
+template <bool IM>
+__global__ void __launch_bounds__(kFillThreads) k_fill_own(const float4* __restrict__ st, int64_t n_own, int64_t stride,
+                                                           const uint32_t* __restrict__ own_u,
+                                                           const float4* __restrict__ tscale,
+                                                           const int* __restrict__ complex_mu,
+                                                           double2* __restrict__ own_r) {
+    if ((*complex_mu != 0) != IM) return;
+    constexpr int NC = IM ? 4 : 3;
+    for (int64_t i = blockIdx.x * (int64_t)kFillThreads + threadIdx.x; i < n_own; i += (int64_t)gridDim.x * kFillThreads) {
+        uint32_t u[kKmax];
+#pragma unroll
+        for (int q = 0; q < kKmax; ++q) u[q] = own_u[q * stride + i];
+        acc2 a[NC];
+        unit_products<NC>(st, tscale, u[0], a);
+#pragma unroll
+        for (int q = 1; q < kKmax; ++q) {
+            if (u[q] == kNoUnit) break;
+            acc2 b[NC];
+            unit_products<NC>(st, tscale, u[q], b);
+#pragma unroll
+            for (int c = 0; c < NC; ++c) add_to(a[c], b[c]);
+        }
+        double2 r[4];
+        to_rows<NC>(a, r);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) own_r[4 * i + c] = r[c];
     }
 }
 
@@ -1018,7 +1141,8 @@ __global__ void __launch_bounds__(32 * kOwnWarps) k_fill_st(const float4* __rest
 // Entity classes: 0 edge with k <= kKmax/2 (two per group), 1 edge with
 // kKmax/2 < k <= kKmax (one per group), 2 face (kGmax per group), 3 FP64 fallback.
 __global__ void k_classify(const int32_t* __restrict__ ent_list, int64_t n_ent, const int64_t* __restrict__ inc_ptr,
-                           const int64_t* __restrict__ inc, const int64_t* __restrict__ indptr, int64_t* flags) {
+                           const int64_t* __restrict__ inc, const int64_t* __restrict__ indptr,
+                           const uint8_t* __restrict__ over, int64_t* flags) {
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n_ent; e += (int64_t)gridDim.x * blockDim.x) {
         const int32_t r = ent_list[e];
         const int64_t k = inc_ptr[r + 1] - inc_ptr[r];
@@ -1031,6 +1155,7 @@ __global__ void k_classify(const int32_t* __restrict__ ent_list, int64_t n_ent, 
             uniform &= (kk == kind);
         }
         int cls = 3;
+        if (over && over[e]) uniform = false;
         if (uniform && kind == 0 && n <= kNmax && k <= kKmax / 2) cls = 0;
         else if (uniform && kind == 0 && n <= kNmax && k <= kKmax) cls = 1;
         else if (uniform && kind == 1 && n <= kColPool / kGmax && k <= kKmax / kGmax) cls = 2;
@@ -1096,8 +1221,10 @@ void df_plan_free(DfPlan* p) {
     dfree(p->inv);
     dfree(p->dofc);
     dfree(p->inc_c);
-    dfree(p->ipos);
-    dfree(p->edesc);
+    dfree(p->pdesc);
+    dfree(p->prows);
+    dfree(p->own_u);
+    dfree(p->own_r);
     dfree(p->st);
     dfree(p->mu_flag);
     p->canon = false;
@@ -1120,7 +1247,10 @@ int df_plan_build(const double* nodes, int64_t nN, const int32_t* tets, int64_t 
     int* d_err = nullptr;
     int64_t *flags = nullptr, *scans = nullptr, *tmp = nullptr;
     uint64_t* cslot = nullptr;
-    auto cleanup = [&]() { dfree(d_err); dfree(flags); dfree(scans); dfree(tmp); dfree(cslot); };
+    uint8_t *ipos = nullptr, *over = nullptr;   // CSR positions of the incidences' 20 columns; see k_pos_check
+    auto cleanup = [&]() {
+        dfree(d_err); dfree(flags); dfree(scans); dfree(tmp); dfree(cslot); dfree(ipos); dfree(over);
+    };
 #define TRY(x) do { int _r = (x); if (_r) { cleanup(); df_plan_free(p); return _r; } } while (0)
 #define TRYC(x) do { cudaError_t _e = (x); if (_e != cudaSuccess) { cleanup(); df_plan_free(p); return cuda_status(_e, #x); } } while (0)
     TRY(dalloc(&d_err, 2, "df err"));
@@ -1148,10 +1278,13 @@ int df_plan_build(const double* nodes, int64_t nN, const int32_t* tets, int64_t 
             dfk::k_inc_canon<<<grid_for(n_inc, T), T, 0, s>>>(inc, n_inc, cslot, p->inc_c);
             TRYC(cudaGetLastError());
         }
-        TRY(dalloc(&p->ipos, 20 * n_inc, "df CSR positions of the incidences"));
+        TRY(dalloc(&ipos, 20 * n_inc, "df CSR positions of the incidences"));
+        TRY(dalloc(&over, n_ent, "df position check"));
         if (n_ent > 0) {
             dfk::k_inc_pos<<<grid_for(n_ent * 32, T, 152u * 64u), T, 0, s>>>(ent_list, n_ent, inc_ptr, p->inc_c, p->dofc,
-                                                                            indptr, indices, p->ipos);
+                                                                            indptr, indices, ipos);
+            dfk::k_pos_check<<<grid_for(n_ent * 32, T, 152u * 64u), T, 0, s>>>(ent_list, n_ent, inc_ptr, p->inc_c, indptr,
+                                                                              ipos, over);
             TRYC(cudaGetLastError());
         }
         TRY(dalloc(&p->st, (nT + dfk::kStBlk - 1) / dfk::kStBlk * dfk::kStBlk * 10 * 20 * 2,
@@ -1173,7 +1306,7 @@ int df_plan_build(const double* nodes, int64_t nN, const int32_t* tets, int64_t 
     TRY(dalloc(&scans, 4 * L, "df class scans"));
     TRY(dalloc(&tmp, scan_scratch_elems(L) + 1, "df scan scratch"));
     if (n_ent > 0) {
-        dfk::k_classify<<<grid_for(n_ent, T), T, 0, s>>>(ent_list, n_ent, inc_ptr, inc, indptr, flags);
+        dfk::k_classify<<<grid_for(n_ent, T), T, 0, s>>>(ent_list, n_ent, inc_ptr, inc, indptr, over, flags);
         TRYC(cudaGetLastError());
     }
     for (int c = 0; c < 4; ++c) TRY(scan_exclusive_i64(flags + c * L, scans + c * L, n_ent, tmp, s));
@@ -1199,11 +1332,37 @@ int df_plan_build(const double* nodes, int64_t nN, const int32_t* tets, int64_t 
     }
     if (p->canon) {
         const int64_t ng = cnt[0] + cnt[1] + cnt[2];
-        TRY(dalloc(reinterpret_cast<dfk::EntDesc**>(&p->edesc), ng, "df entity descriptors"));
         if (ng > 0) {
-            dfk::k_ent_desc<<<grid_for(ng, T), T, 0, s>>>(p->gents, ng, partner, inc_ptr, indptr,
-                                                          reinterpret_cast<dfk::EntDesc*>(p->edesc));
+            // the usual numbering needs no row table: entity i owns rows i and i + n_ent, none is slow
+            int ragged = 1;
+            if (cnt[3] == 0) {
+                TRYC(cudaMemsetAsync(d_err, 0, sizeof(int), s));
+                dfk::k_pair_check<<<grid_for(n_ent, T), T, 0, s>>>(ent_list, n_ent, partner, over, d_err);
+                TRYC(cudaMemcpyAsync(&ragged, d_err, sizeof(int), cudaMemcpyDeviceToHost, s));
+            }
+            // flags and scans are free again: row lengths and their offsets
+            const int32_t* ents = cnt[3] == 0 ? ent_list : p->gents;
+            dfk::k_ent_sizes<<<grid_for(ng, T), T, 0, s>>>(ents, ng, indptr, flags);
             TRYC(cudaGetLastError());
+            TRY(scan_exclusive_i64(flags, scans, ng, tmp, s));
+            TRYC(cudaMemcpyAsync(&p->n_pos, scans + ng, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+            TRYC(cudaStreamSynchronize(s));
+            if (nT >= (int64_t)(0xffffffffu / 200u) - dfk::kStBlk) {   // (its matrices alone exceed the memory)
+                set_error("mesh too large: staged units beyond 32-bit indices");
+                TRY(EMG_ERR_LIMIT);
+            }
+            TRY(dalloc(&p->pdesc, p->n_pos, "df position descriptors"));
+            if (ragged) TRY(dalloc(&p->prows, p->n_pos, "df position rows"));
+            TRY(dalloc(&p->own_u, 2 * ng * dfk::kKmax, "df own column units"));
+            p->own_stride = 2 * ng;
+            unsigned long long* n_own = reinterpret_cast<unsigned long long*>(flags);
+            TRYC(cudaMemsetAsync(n_own, 0, sizeof(unsigned long long), s));
+            dfk::k_pos_desc<<<grid_for(ng * 32, T, 152u * 64u), T, 0, s>>>(
+                ents, ng, partner, inc_ptr, p->inc_c, indptr, ipos, scans, p->pdesc, p->prows, p->own_u, n_own);
+            TRYC(cudaGetLastError());
+            TRYC(cudaMemcpyAsync(&p->n_own, n_own, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+            TRYC(cudaStreamSynchronize(s));
+            TRY(dalloc(&p->own_r, 4 * p->n_own, "df own column sums"));
         }
     }
     TRYC(cudaStreamSynchronize(s));
@@ -1222,32 +1381,40 @@ int df_fill(const DfPlan& p, int64_t nT, const int32_t* partner, const int64_t* 
     if (dev >= 0 && dev < 64 && !attr_set[dev]) {
         EMG_CUDA(cudaFuncSetAttribute(dfk::k_fill_df, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)dfk::kFillSmem));
-        EMG_CUDA(cudaFuncSetAttribute(dfk::k_fill_st<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)dfk::kStSmem));
-        EMG_CUDA(cudaFuncSetAttribute(dfk::k_fill_st<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)dfk::kStSmem));
         attr_set[dev] = true;
     }
-    if (p.mu_flag) EMG_CUDA(cudaMemsetAsync(p.mu_flag, 0, sizeof(int), s));
+    if (p.n_groups > 0 && p.canon) {
+        const unsigned ge = grid_for(nT, dfk::kElemThreads, 152u * 64u);
+        // (measured at 10, 12, 16 and 20 cells a side; more slices restage the invariants for less work each)
+        const unsigned gy = ge <= 48u ? 10u : ge <= 120u ? 5u : ge <= 240u ? 3u : 1u;
+        dfk::k_elem<<<dim3(ge, gy), dfk::kElemThreads, 0, s>>>(p.inv, nT, p.st, p.mu_flag);
+    }
     if (nT > 0) {
         dfk::k_scales<<<grid_for(nT, 256), 256, 0, s>>>(p.gscale, reinterpret_cast<const double2*>(eps),
                                                          reinterpret_cast<const double2*>(mu_inv), nT, p.tscale,
                                                          p.mu_flag);
         EMG_CUDA(cudaGetLastError());
     }
-    if (p.n_groups > 0 && p.canon) {
-        dfk::k_elem<<<grid_for(nT, dfk::kElemThreads, 152u * 64u), dfk::kElemThreads, 0, s>>>(p.inv, nT, p.st);
-        EMG_CUDA(cudaGetLastError());
-        const unsigned g = grid_for(p.n_groups, dfk::kOwnWarps, 152u * 16u);
-        dfk::k_fill_st<false><<<g, 32 * dfk::kOwnWarps, dfk::kStSmem, s>>>(
-            p.st, p.ipos, reinterpret_cast<const int2*>(p.groups), p.n_groups,
-            reinterpret_cast<const dfk::EntDesc*>(p.edesc), p.inc_c, p.tscale, p.mu_flag,
+    if (p.n_groups > 0 && p.canon && p.n_pos <= dfk::kSmallPos) {
+        dfk::k_fill_small<<<grid_for(p.n_pos, dfk::kFillThreads), dfk::kFillThreads, 0, s>>>(
+            p.st, p.n_pos, p.pdesc, p.prows, p.n_pos, p.own_u, p.own_stride, p.tscale, p.mu_flag,
             reinterpret_cast<double2*>(E), reinterpret_cast<double2*>(B));
         EMG_CUDA(cudaGetLastError());
-        dfk::k_fill_st<true><<<g, 32 * dfk::kOwnWarps, dfk::kStSmem, s>>>(
-            p.st, p.ipos, reinterpret_cast<const int2*>(p.groups), p.n_groups,
-            reinterpret_cast<const dfk::EntDesc*>(p.edesc), p.inc_c, p.tscale, p.mu_flag,
-            reinterpret_cast<double2*>(E), reinterpret_cast<double2*>(B));
+    } else if (p.n_groups > 0 && p.canon) {
+        const unsigned g = grid_for(p.n_pos, dfk::kFillThreads), go = grid_for(p.n_own, dfk::kFillThreads);
+        auto* E2 = reinterpret_cast<double2*>(E);
+        auto* B2 = reinterpret_cast<double2*>(B);
+        // one of the two instantiations returns at once: which one is only known on the device
+        if (p.n_own > 0) {
+            dfk::k_fill_own<false><<<go, dfk::kFillThreads, 0, s>>>(p.st, p.n_own, p.own_stride, p.own_u, p.tscale,
+                                                                   p.mu_flag, p.own_r);
+            dfk::k_fill_own<true><<<go, dfk::kFillThreads, 0, s>>>(p.st, p.n_own, p.own_stride, p.own_u, p.tscale,
+                                                                  p.mu_flag, p.own_r);
+        }
+        dfk::k_fill_st<false><<<g, dfk::kFillThreads, 0, s>>>(p.st, p.n_pos, p.pdesc, p.prows, p.n_pos, p.own_r, p.tscale,
+                                                             p.mu_flag, E2, B2);
+        dfk::k_fill_st<true><<<g, dfk::kFillThreads, 0, s>>>(p.st, p.n_pos, p.pdesc, p.prows, p.n_pos, p.own_r, p.tscale,
+                                                            p.mu_flag, E2, B2);
         EMG_CUDA(cudaGetLastError());
     } else if (p.n_groups > 0) {
         const unsigned g = grid_for(p.n_groups, dfk::kWarps, 152u * 32u);
