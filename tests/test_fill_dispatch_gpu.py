@@ -83,3 +83,25 @@ def test_fan(torch_cuda, ring, complex_mu):
     E, B = tet_mass_stiffness_matrices(field, er, ur)
     Eo, Bo = oracle.tet_mass_stiffness_matrices(field, er, ur)
     assert rel_to_rowmax(E, Eo) <= TOL and rel_to_rowmax(B, Bo) <= TOL
+
+
+@pytest.mark.parametrize("ring", [3, 6, 7, 12, 13])
+def test_tensor_fan(torch_cuda, ring):
+    """Full tensors around one edge: two edges or one to a group (six, seven tets), the largest
+    group (twelve), and the FP64 fill next to the groups (thirteen)."""
+    from emerge_gb300.assembly import tet_mass_stiffness_matrices
+    from emerge_gb300.mesh import Nedelec2Basis, TetMesh
+    ang = 2 * np.pi * np.arange(ring) / ring
+    pts = np.stack([np.cos(ang), np.sin(ang), 0.5 + 0.1 * np.sin(3 * ang)])
+    nodes = np.concatenate([np.array([[0, 0], [0, 0], [0, 1.0]]), pts], axis=1)
+    k = np.arange(ring)
+    m = TetMesh(nodes, np.stack([0 * k, 0 * k + 1, 2 + k, 2 + (k + 1) % ring]))
+    field = Nedelec2Basis(m)
+    rng = np.random.default_rng(ring)
+    er, ur = (rng.uniform(-0.3, 0.3, (3, 3, ring)) + 1j * rng.uniform(-0.03, 0.03, (3, 3, ring)) for _ in range(2))
+    er[range(3), range(3)] += 4.0
+    ur[range(3), range(3)] += 1.5
+    E, B = tet_mass_stiffness_matrices(field, er, ur)
+    Eo, Bo = oracle.tet_mass_stiffness_matrices(field, er, ur)
+    assert np.array_equal(E.indptr, Eo.indptr) and np.array_equal(E.indices, Eo.indices)
+    assert rel_to_rowmax(E, Eo) <= TOL and rel_to_rowmax(B, Bo) <= TOL
