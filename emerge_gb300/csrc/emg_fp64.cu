@@ -135,10 +135,9 @@ __device__ __forceinline__ double combine(const float (&S)[kDig], int E) {
 // Modes of a Gauss-Jordan step k on the w x w matrix M (row-major), P = inverse of tile (k, k):
 //   kRow:  rows[r][c] = sum_k P[r][k] M[k0 + k][c] for the columns outside tile k, and P itself
 //          inside (rows: 64 x w); extra CTAs keep the column panel: cols[r][k] = M[r][k0 + k].
-//   kLook: M[r][c] -= sum_k cols[r][k] rows[k][c] on tile (la, la) alone.
-//   kRest: the same everywhere else; columns of tile k take 0 - sum (rows holds P there), rows of
-//          tile k take rows.
-constexpr int kRow = 0, kLook = 1, kRest = 2;
+//   kRest: M[r][c] -= sum_k cols[r][k] rows[k][c] but for tile (la, la) (k_look64); columns of
+//          tile k take 0 - sum (rows holds P there), rows of tile k take rows.
+constexpr int kRow = 0, kRest = 1;
 
 template <int MODE>
 __global__ void __maxnreg__(200)   // 256 threads leave room on the SM for a CTA of the pivot tile's cluster
@@ -181,12 +180,6 @@ __global__ void __maxnreg__(200)   // 256 threads leave room on the SM for a CTA
             const int r = (int)r0 + i / kTile, c = i % kTile;
             if (r < tb && c < tb && k0 + c >= c0 && k0 + c < c0 + kM) rows[(int64_t)r * w + k0 + c] = P[r * kTile + c];
         }
-    } else if (MODE == kLook) {
-        c0 = (int64_t)la * kTile;
-        cend = min(w, c0 + kTile);
-        r0 = c0 + (int64_t)bx * kN;
-        rend = cend;
-        if (r0 >= rend) return;
     } else {
         c0 = (int64_t)(bx % nct) * kM;
         cend = w;
@@ -418,6 +411,69 @@ __global__ void __maxnreg__(200)   // 256 threads leave room on the SM for a CTA
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(kTmemCols) : "memory");
 }
 
+// The lookahead of step k on the FP64 pipe: tile (la, la) is all that the next pivot tile waits for.
+//   part 0: rows[r][c] = sum_k P[r][k] M[k0 + k][c] in the columns of tile la
+//   part 1: M[r][c] -= sum_k M[r][k0 + k] rows[k][c] on tile (la, la)
+// 128 CTAs of 8 x 4 outputs, a quarter of K per warp: 4096 cycles of an SM's FP64 pipe each.  On the
+// tensor cores one 64 x 64 tile is one or two CTAs that take as long as a full wave, 35 us for
+// the whole row panel before it and 33 for the tile, all on the chain of the pivot tiles; these
+// two launches take 4.7 us each, and the row panel runs beside the next pivot tile (a 26-slab point
+// of 311 tiles: 75 -> 55 ms).
+constexpr int kLookCtas = 128, kLookRows = 8, kLookCols = 4, kTileThreads = 128;
+
+__device__ __forceinline__ void cmadd(double2& s, double2 a, double2 b) {   // s += a b
+    s.x = fma(a.x, b.x, s.x);
+    s.y = fma(a.x, b.y, s.y);
+    s.x = fma(-a.y, b.y, s.x);
+    s.y = fma(a.y, b.x, s.y);
+}
+
+__global__ void __launch_bounds__(kTileThreads) k_look64(int part, int64_t w, int k, int la, double2* __restrict__ Sinv,
+                                                         int64_t totD, int64_t offD, const double2* __restrict__ pinv,
+                                                         double2* __restrict__ rows_, int64_t sbuf) {
+    __shared__ double2 As[kLookRows][kTile + 1], Bs[kTile][kLookCols + 1], red[kTileThreads / 32][32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int r0 = ((int)blockIdx.x / (kTile / kLookCols)) * kLookRows, c0 = ((int)blockIdx.x % (kTile / kLookCols)) * kLookCols;
+    const int64_t f = blockIdx.z, k0 = (int64_t)k * kTile, l0 = (int64_t)la * kTile;
+    double2* M = Sinv + f * totD + offD;
+    double2* rows = rows_ + f * sbuf;
+    const int nv = (int)min((int64_t)kTile, w - l0);   // tile k is a full one: la comes after it
+    const double2 z2 = make_double2(0.0, 0.0);
+#pragma unroll
+    for (int q = 0; q < kLookRows * kTile / kTileThreads; ++q) {
+        const int i = tid + q * kTileThreads, r = i / kTile, kk = i % kTile;
+        As[r][kk] = part == 0          ? pinv[f * kTile * kTile + (r0 + r) * kTile + kk]
+                    : r0 + r < nv ? M[(l0 + r0 + r) * w + k0 + kk]
+                                       : z2;
+    }
+#pragma unroll
+    for (int q = 0; q < kLookCols * kTile / kTileThreads; ++q) {
+        const int i = tid + q * kTileThreads, kk = i / kLookCols, c = i % kLookCols;
+        const double2* src = part == 0 ? M + k0 * w : rows;
+        Bs[kk][c] = c0 + c < nv ? src[(int64_t)kk * w + l0 + c0 + c] : z2;
+    }
+    __syncthreads();
+    const int r = lane / kLookCols, c = lane % kLookCols;
+    double2 s = z2;
+#pragma unroll
+    for (int kk = 0; kk < kTile / 4; ++kk) cmadd(s, As[r][warp * (kTile / 4) + kk], Bs[warp * (kTile / 4) + kk][c]);
+    red[warp][lane] = s;
+    __syncthreads();
+    if (warp == 0 && c0 + c < nv) {
+#pragma unroll
+        for (int q = 1; q < kTileThreads / 32; ++q) {
+            s.x += red[q][lane].x;
+            s.y += red[q][lane].y;
+        }
+        if (part == 0) {
+            rows[(int64_t)(r0 + r) * w + l0 + c0 + c] = s;
+        } else if (r0 + r < nv) {
+            double2& m = M[(l0 + r0 + r) * w + l0 + c0 + c];
+            m = make_double2(m.x - s.x, m.y - s.y);
+        }
+    }
+}
+
 // FP64 inverse of pivot tile k by a cluster of 16 CTAs of 128 threads: in-place Gauss-Jordan exchange
 // steps with implicit pivoting (see emg_gj.cuh for the FP32 form), four columns per CTA, thread
 // (row t / 2, columns 2 (t % 2), + 1).  CTA J runs the four steps of its own panel, the others
@@ -425,8 +481,8 @@ __global__ void __maxnreg__(200)   // 256 threads leave room on the SM for a CTA
 // them to their columns as a rank-4 product, so the 1 M FMAs of a tile are spread over 16 SMs'
 // FP64 pipes.  Pivots compare max(|re|, |im|) (14 bits of it, the lowest row on ties); a pivot of
 // |a|^2 at or below rel_thr^2 max|a|^2 is replaced by that threshold and counted.  One CTA took
-// 600 us a tile (85 % of its FP64 pipe), this 129.
-constexpr int kRanks = 16, kTileThreads = 128, kPc = 4;
+// 600 us a tile (85 % of its FP64 pipe), this 115 (124 while products run beside it).
+constexpr int kRanks = 16, kPc = 4;
 
 __device__ __forceinline__ double2 remote(const double2* p, int rank) {
     uint32_t a;
@@ -439,13 +495,6 @@ __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-__device__ __forceinline__ void cmadd(double2& s, double2 a, double2 b) {   // s += a b
-    s.x = fma(a.x, b.x, s.x);
-    s.y = fma(a.x, b.y, s.y);
-    s.x = fma(-a.y, b.y, s.x);
-    s.y = fma(a.y, b.x, s.y);
-}
-
 __global__ void __launch_bounds__(kTileThreads) k_tile64(int64_t w, int k, double2* __restrict__ Sinv, int64_t totD,
                                                          int64_t offD, double2* __restrict__ pinv, double rel_thr,
                                                          int32_t* __restrict__ perturbed) {
@@ -521,7 +570,9 @@ __global__ void __launch_bounds__(kTileThreads) k_tile64(int64_t w, int k, doubl
                 const double2 pr0 = sh.row[buf][pw][2 * h], pr1 = sh.row[buf][pw][2 * h + 1];
                 double2 g = sh.row[buf][pw][q];
                 double d = g.x * g.x + g.y * g.y;
-                const bool small = !(d > thr2);   // also catches a zero pivot
+                // !(d > thr2) on the bits, off the FP64 pipe; also a zero pivot or a NaN
+                const long long db = __double_as_longlong(d);
+                const bool small = db <= __double_as_longlong(thr2) || db > 0x7ff0000000000000ll;
                 if (small) {
                     g = make_double2(thr2 > 0.0 ? sqrt(thr2) : 1.0, 0.0);
                     d = g.x * g.x;
@@ -535,7 +586,7 @@ __global__ void __launch_bounds__(kTileThreads) k_tile64(int64_t w, int k, doubl
                 const bool own = r == p;
                 used |= own;
                 const double mx_ = own ? -1.0 : m.x, my_ = own ? 0.0 : m.y;
-                const double t = h ? fma(my_, g.x, -mx_ * g.y) : fma(mx_, g.x, my_ * g.y);
+                const double t = fma(h ? my_ : mx_, g.x, (h ? -mx_ : my_) * g.y);
                 y = fma(y, fma(er, er, er), y);
                 const double fp = t * y, fo = __shfl_xor_sync(0xffffffffu, fp, 1);
                 const double2 fn = h ? make_double2(-fo, -fp) : make_double2(-fp, -fo);
@@ -642,7 +693,6 @@ int fp64_step(int stage, int64_t w, int k, int la, int64_t F, double2* Sinv, int
     static bool attr = false;
     if (!attr) {
         EMG_CUDA(cudaFuncSetAttribute(f64::k_prod64<f64::kRow>, cudaFuncAttributeMaxDynamicSharedMemorySize, f64::kSmem + 1024));
-        EMG_CUDA(cudaFuncSetAttribute(f64::k_prod64<f64::kLook>, cudaFuncAttributeMaxDynamicSharedMemorySize, f64::kSmem + 1024));
         EMG_CUDA(cudaFuncSetAttribute(f64::k_prod64<f64::kRest>, cudaFuncAttributeMaxDynamicSharedMemorySize, f64::kSmem + 1024));
         attr = true;
     }
@@ -650,10 +700,11 @@ int fp64_step(int stage, int64_t w, int k, int la, int64_t F, double2* Sinv, int
     const unsigned nt = (unsigned)((w + f64::kTile - 1) / f64::kTile);
     constexpr int sm = f64::kSmem + 1024;
     if (stage == 0)
-        f64::k_prod64<f64::kRow><<<dim3(2 * nct + nt, 1, (unsigned)F), f64::kThreads, sm, st>>>(
-            w, k, la, Sinv, totD, offD, pinv, rows, cols, sbuf, status);
+        for (int part = 0; part < 2; ++part)
+            f64::k_look64<<<dim3(f64::kLookCtas, 1, (unsigned)F), f64::kTileThreads, 0, st>>>(part, w, k, la, Sinv, totD, offD,
+                                                                                            pinv, rows, sbuf);
     else if (stage == 1)
-        f64::k_prod64<f64::kLook><<<dim3(f64::kTile / f64::kN, 1, (unsigned)F), f64::kThreads, sm, st>>>(
+        f64::k_prod64<f64::kRow><<<dim3(2 * nct + nt, 1, (unsigned)F), f64::kThreads, sm, st>>>(
             w, k, la, Sinv, totD, offD, pinv, rows, cols, sbuf, status);
     else
         f64::k_prod64<f64::kRest><<<dim3(nct * nrt, 1, (unsigned)F), f64::kThreads, sm, st>>>(

@@ -1178,17 +1178,17 @@ int slab_factor_t(emg_slab* s, int64_t F, const int32_t* amat_h, int64_t Bm, con
                 if (nt == 1) break;
                 const T* P = pset(k);
                 const int la = k + 1 < nt ? k + 1 : -1;
-                // stage 0: row panel, 1: tile (la, la), 2: the rest
+                // stage 0: tile (la, la), 1: row panel, 2: the rest (the CUDA-core lookahead reads the panel)
                 auto stage = [&](int q) -> int {
                     if constexpr (sizeof(R) == 8) {
                         if (tc_update)
                             return emg::fp64_step(q, w, k, la, F, Sinv, s->totD, s->offD[i], P, rowbuf, colbuf,
                                                   s->maxw * kTile, s->tc_status, st);
                     }
-                    if (q == 0)
+                    if (q == 1)
                         k_gj_panel<R><<<dim3(nt, 1, (unsigned)F), kThreads, 0, st>>>(0, w, k, Sinv, s->totD, s->offD[i], P,
                                                                                      -1);
-                    else if (q == 1)
+                    else if (q == 0)
                         k_gj_panel<R><<<dim3(1, 1, (unsigned)F), kThreads, 0, st>>>(3, w, k, Sinv, s->totD, s->offD[i], P,
                                                                                     la);
                     else {
@@ -1199,14 +1199,15 @@ int slab_factor_t(emg_slab* s, int64_t F, const int32_t* amat_h, int64_t Bm, con
                     }
                     return EMG_OK;
                 };
-                rc = stage(0);
+                rc = tc_update ? EMG_OK : stage(1);
                 if (!rc && la >= 0) {
-                    rc = stage(1);
+                    rc = stage(0);
                     EMG_CUDA(cudaEventRecord(side.tile_ready, st));
                     EMG_CUDA(cudaStreamWaitEvent(side.st, side.tile_ready, 0));
                     if (!rc) rc = tile(la, side.st);
                     EMG_CUDA(cudaEventRecord(side.diag_done, side.st));
                 }
+                if (!rc && tc_update) rc = stage(1);
                 if (!rc) rc = stage(2);
                 if (rc) {
                     cudaDeviceSynchronize();   // the side stream and the buffers go away
