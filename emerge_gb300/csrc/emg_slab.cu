@@ -285,48 +285,107 @@ __global__ void __launch_bounds__(kThreads) k_gj_panel(int mode, int64_t w, int 
         }
 }
 
-// First half of step k for the tensor-core update: CTAs x < nt form the row panel M[k, c] = Pinv
-// M[k, c] (c != k), CTAs nt + r keep the column tiles M[r, k] in colbuf (rows of 64, zero
-// beyond the tile), so that the second half may overwrite them.  Grid: 2 nt x 1 x F.
-template <typename R>
-__global__ void __launch_bounds__(kThreads) k_gj_row(int64_t w, int k, int nt, typename C2<R>::T* __restrict__ Sinv,
-                                                     int64_t totD, int64_t offD, const typename C2<R>::T* __restrict__ pinv,
-                                                     typename C2<R>::T* __restrict__ colbuf, int64_t scol) {
-    using T = typename C2<R>::T;
-    __shared__ Tile<R> sm;
+// First half of step k for the tensor-core update.  CTAs x < strips form 16 columns of the row
+// panel each, M[k, c] = Pinv M[k, c] (c != k); those of tile la go on to the next pivot tile,
+// M[la, la] -= M[la, k] (Pinv M[k, la]), so that the update's first CTA only has to invert it.  CTA
+// strips + r keeps column tile M[r, k] in colbuf (rows of 64, zero beyond the tile), so that the
+// second half may overwrite it.  A CTA of 256 threads, four outputs each, reads two K of both operands
+// at a time from shared memory.  The pivot chain is what bounds a factorization: 64-column tiles
+// took 10 us, then the next pivot tile's product 13 us of the update's first CTA (an update of 42 us
+// and its 29 us inverse at up to 1400 wide).  With this and the launches chained (launch_pdl), a
+// point of 145 slabs up to 2768 wide went from 396 to 340 ms, a sweep of 219-slab factors up to
+// 1400 wide, with its solves, from 599 to 491.
+// Grid: strips + nt x 1 x F.
+constexpr int kStrip = 16, kPairs = kTile / 2, kLdP = kPairs + 1;
+__device__ __forceinline__ void strip_mac(float2 (&acc)[4], const float4 (*As)[kLdP], const float4* b, int r0) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) acc[i] = make_float2(0.f, 0.f);
+#pragma unroll 8
+    for (int q = 0; q < kPairs; ++q) {
+        const float4 y = b[q];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float4 x = As[r0 + 16 * i][q];
+            cfma(acc[i], make_float2(x.x, x.y), make_float2(y.x, y.y));
+            cfma(acc[i], make_float2(x.z, x.w), make_float2(y.z, y.w));
+        }
+    }
+}
+__global__ void __launch_bounds__(kThreads) k_gj_row(int64_t w, int k, int la, int strips, float2* Sinv, int64_t totD,
+                                                     int64_t offD, const float2* pinv, float2* colbuf, int64_t scol) {
+    __shared__ float4 As[kTile][kLdP], Bs[kStrip][kLdP];
     const int64_t f = blockIdx.z, k0 = (int64_t)k * kTile;
-    T* M = Sinv + f * totD + offD;
+    float2* M = Sinv + f * totD + offD;
     const int tb = (int)min((int64_t)kTile, w - k0);
-    const int tid = threadIdx.x;
-    const int bx = (int)blockIdx.x;
-    if (bx >= nt) {
-        const int64_t r0 = (int64_t)(bx - nt) * kTile;
-        T* out = colbuf + f * scol + r0 * kTile;
+    const int tid = threadIdx.x, bx = (int)blockIdx.x;
+    const float2 z2 = make_float2(0.f, 0.f);
+    pdl_wait();
+    pdl_trigger();
+    if (bx >= strips) {
+        const int64_t r0 = (int64_t)(bx - strips) * kTile;
+        float2* out = colbuf + f * scol + r0 * kTile;
 #pragma unroll
         for (int q = 0; q < kTile * kTile / kThreads; ++q) {
             const int i = tid + q * kThreads, r = i / kTile, c = i % kTile;
-            if (r0 + r < w) out[i] = c < tb ? M[(r0 + r) * w + k0 + c] : czero<T>();
+            if (r0 + r < w) out[i] = c < tb ? M[(r0 + r) * w + k0 + c] : z2;
         }
         return;
     }
-    if (bx == k) return;
-    const int ty = tid >> 4, tx = tid & 15;
-    const int64_t c0 = (int64_t)bx * kTile;
-    const int nc = (int)min((int64_t)kTile, w - c0);
-    T* out = M + k0 * w + c0;
-    T acc[4][4];
+    const int64_t c0 = (int64_t)bx * kStrip, l0 = (int64_t)la * kTile;
+    if (c0 / kTile == k) return;
+    const bool ahead = la >= 0 && c0 / kTile == la;
+    const int nc = (int)min((int64_t)kStrip, w - c0), lt = (int)min((int64_t)kTile, w - l0);
+    const int c = tid % kStrip, r0 = tid / kStrip;
+    {
+        const float4* P = reinterpret_cast<const float4*>(pinv + f * kTile * kTile);
+        float4 pv[kTile * kPairs / kThreads];
+        float2 bv[kTile * kStrip / kThreads];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+        for (int q = 0; q < kTile * kStrip / kThreads; ++q)
+            bv[q] = (r0 + 16 * q < tb && c < nc) ? M[(k0 + r0 + 16 * q) * w + c0 + c] : z2;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = czero<T>();
-    tile_mac<R>(acc, pinv + f * kTile * kTile, kTile, out, w, tb, nc, tb, sm);
+        for (int q = 0; q < kTile * kPairs / kThreads; ++q) pv[q] = P[tid + q * kThreads];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+        for (int q = 0; q < kTile * kStrip / kThreads; ++q) reinterpret_cast<float2*>(&Bs[c][0])[r0 + 16 * q] = bv[q];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int r = ty + 16 * i, c = tx + 16 * j;
-            if (r < tb && c < nc) out[(int64_t)r * w + c] = acc[i][j];
+        for (int q = 0; q < kTile * kPairs / kThreads; ++q) {
+            const int r = (tid + q * kThreads) / kPairs, p = tid % kPairs;
+            float4 v = pv[q];
+            if (r >= tb || 2 * p >= tb) v.x = v.y = 0.f;        // nothing is kept beyond the tile
+            if (r >= tb || 2 * p + 1 >= tb) v.z = v.w = 0.f;
+            As[r][p] = v;
         }
+    }
+    float2 cv[kTile * kTile / kThreads], m[4];
+    if (ahead) {   // uniform: the lookahead's operands are in flight under the strip's product
+#pragma unroll
+        for (int q = 0; q < kTile * kTile / kThreads; ++q) {
+            const int i = tid + q * kThreads, r = i / kTile;
+            cv[q] = r < lt ? M[(l0 + r) * w + k0 + i % kTile] : z2;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) m[i] = (r0 + 16 * i < lt && c < nc) ? M[(l0 + r0 + 16 * i) * w + c0 + c] : z2;
+    }
+    __syncthreads();
+    float2 acc[4];
+    strip_mac(acc, As, Bs[c], r0);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        if (r0 + 16 * i < tb && c < nc) M[(k0 + r0 + 16 * i) * w + c0 + c] = acc[i];
+    if (!ahead) return;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) reinterpret_cast<float2*>(&Bs[c][0])[r0 + 16 * i] = acc[i];
+#pragma unroll
+    for (int q = 0; q < kTile * kTile / kThreads; ++q) {
+        const int i = tid + q * kThreads;
+        reinterpret_cast<float2*>(&As[i / kTile][0])[i % kTile] = cv[q];
+    }
+    __syncthreads();
+    strip_mac(acc, As, Bs[c], r0);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        if (r0 + 16 * i < lt && c < nc) M[(l0 + r0 + 16 * i) * w + c0 + c] = make_float2(m[i].x - acc[i].x, m[i].y - acc[i].y);
 }
 
 // C = alpha A B + diag I for F batched w x w row-major blocks (batch stride
@@ -430,35 +489,59 @@ __global__ void k_scatter(int64_t n, int64_t Bc, const int32_t* __restrict__ per
 
 // mode 0: Y[row] -= sum C[row,k] Z[prev0 + cidx[k]]    (forward coupling)
 // mode 1: Y[row]  = sum U[row,k] Z[next0 + uidx[k]]    (backward coupling)
-// A row has some 20 entries: four of them in flight per thread, two of its columns apart.
+// A row has some 20 entries: kCoupleIn of them in flight per thread, their indices and values
+// (which no solve writes) read before the wait for the product that writes Z.  The launches of
+// a solve are a chain of 8 to 20 us each (launch_pdl); see k_gj_row for a sweep's time.
+constexpr int kCoupleIn = 8;
 template <typename R>
-__global__ void k_couple(int mode, int64_t w, int64_t row0, int64_t nb0, int64_t Bc, const int32_t* __restrict__ colfac,
-                         const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx,
-                         const typename C2<R>::T* __restrict__ val, int64_t nval, const typename C2<R>::T* __restrict__ Z,
-                         typename C2<R>::T* __restrict__ Y) {
+__global__ void __launch_bounds__(256) k_couple(int mode, int64_t w, int64_t row0, int64_t nb0, int64_t Bc,
+                                                const int32_t* __restrict__ colfac, const int64_t* __restrict__ ptr,
+                                                const int32_t* __restrict__ idx, const typename C2<R>::T* __restrict__ val,
+                                                int64_t nval, const typename C2<R>::T* Z, typename C2<R>::T* Y) {
     using T = typename C2<R>::T;
     const int64_t total = w * Bc;
+    bool waited = false;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
         const int64_t row = row0 + t / Bc, c = t % Bc;
         const T* v = val + (int64_t)colfac[c] * nval;
         const T* z = Z + nb0 * Bc + c;
         const int64_t k1 = ptr[row + 1];
         int64_t k = ptr[row];
-        T s0 = czero<T>(), s1 = czero<T>();
-        for (; k + 4 <= k1; k += 4) {
-            const int32_t i0 = idx[k], i1 = idx[k + 1], i2 = idx[k + 2], i3 = idx[k + 3];
-            const T a0 = v[k], a1 = v[k + 1], a2 = v[k + 2], a3 = v[k + 3];
-            const T z0 = z[i0 * Bc], z1 = z[i1 * Bc], z2 = z[i2 * Bc], z3 = z[i3 * Bc];
-            cfma(s0, a0, z0);
-            cfma(s1, a1, z1);
-            cfma(s0, a2, z2);
-            cfma(s1, a3, z3);
+        T a[kCoupleIn], s0 = czero<T>(), s1 = czero<T>();
+        int32_t id[kCoupleIn];
+        auto fetch = [&]() {
+#pragma unroll
+            for (int u = 0; u < kCoupleIn; ++u) {
+                id[u] = k + u < k1 ? idx[k + u] : -1;
+                a[u] = k + u < k1 ? v[k + u] : czero<T>();
+            }
+        };
+        fetch();
+        if (!waited) {
+            pdl_wait();
+            pdl_trigger();
+            waited = true;
         }
-        for (; k < k1; ++k) cfma(s0, v[k], z[idx[k] * Bc]);
         T& y = Y[row * Bc + c];
+        T y0 = czero<T>();
+        if (mode == 0) y0 = y;
+        while (k < k1) {
+            T x[kCoupleIn], b[kCoupleIn];
+#pragma unroll
+            for (int u = 0; u < kCoupleIn; ++u) {
+                x[u] = id[u] >= 0 ? z[id[u] * Bc] : czero<T>();
+                b[u] = a[u];
+            }
+            k += kCoupleIn;
+            fetch();
+#pragma unroll
+            for (int u = 0; u < kCoupleIn; u += 2) {
+                cfma(s0, b[u], x[u]);
+                cfma(s1, b[u + 1], x[u + 1]);
+            }
+        }
         const T s = mk(s0.x + s1.x, s0.y + s1.y);
-        if (mode == 0) { y.x -= s.x; y.y -= s.y; }
-        else y = s;
+        y = mode == 0 ? mk(y0.x - s.x, y0.y - s.y) : s;
     }
 }
 
@@ -477,7 +560,7 @@ __global__ void k_narrow(int64_t nv, const double2* __restrict__ in, float2* __r
 // lane sums are folded so that each shuffle halves the values a lane carries (9 adds for four
 // complex columns, 40 one by one): in FP64 the pipe bounds the kernel, and the run-time column
 // count of up to 16 issued its unused products too (4 columns, 1250 wide: 268 -> 45
-// us); in FP32 it is bound by reading S_i^-1 (2 columns, 1812 wide: 37.7 -> 12 us).
+// us); in FP32 it is bound by reading S_i^-1 (2 columns, up to 2768 wide: 37.7 -> 15.9 us).
 // Grid: row blocks x groups.
 constexpr int kRowRows = 2, kRowWarps = kThreads / 32 / kRowRows;
 template <int NV, typename R>
@@ -504,8 +587,8 @@ __device__ __forceinline__ R lane_sum(R (&v)[NV]) {   // lane l: the sum of valu
 template <typename R, int NC>
 __global__ void __launch_bounds__(kThreads) k_rowmv(int64_t w, int64_t row0, int64_t Bc, const Group* __restrict__ groups,
                                                     const typename C2<R>::T* __restrict__ Sinv, int64_t totD, int64_t offD,
-                                                    const typename C2<R>::T* __restrict__ Y, R alpha, int beta,
-                                                    typename C2<R>::T* __restrict__ Out) {
+                                                    const typename C2<R>::T* Y, R alpha, int beta,
+                                                    typename C2<R>::T* Out) {
     using T = typename C2<R>::T;
     constexpr int NV = 2 * NC;                     // values of a lane: re and im of NC columns
     __shared__ R part[kRowRows][kRowWarps][NV];
@@ -514,34 +597,42 @@ __global__ void __launch_bounds__(kThreads) k_rowmv(int64_t w, int64_t row0, int
     const Group g = groups[blockIdx.y];
     const T* S = Sinv + (int64_t)g.fac * totD + offD + r * w;
     const T* Yb = Y + row0 * Bc + g.col0;
+    constexpr int kStep = kRowWarps * 32, kIn = 4;
+    T a[kIn];                                      // loads of the row in flight
+    auto fetch = [&](int64_t k) {
+#pragma unroll
+        for (int u = 0; u < kIn; ++u) a[u] = (r < w && k + u * kStep < w) ? S[k + u * kStep] : czero<T>();
+    };
+    fetch(kw * 32 + lane);
+    pdl_wait();
+    pdl_trigger();
     for (int c0 = 0; c0 < g.ncol; c0 += NC) {
         const int nc = min(NC, g.ncol - c0);
         R v[NV];
 #pragma unroll
         for (int j = 0; j < NV; ++j) v[j] = 0;
         if (r < w) {
-            auto mac = [&](T s, int64_t k) {
-                const T* y = Yb + k * Bc + c0;
+            if (c0 > 0) fetch(kw * 32 + lane);
+            for (int64_t k = kw * 32 + lane; k < w; k += kIn * kStep) {
+                T s[kIn];
 #pragma unroll
-                for (int j = 0; j < NC; ++j) {
-                    if (NC > 1 && j >= nc) break;   // uniform
-                    const T x = y[j];
-                    v[2 * j] = fma(s.x, x.x, v[2 * j]);
-                    v[2 * j] = fma(-s.y, x.y, v[2 * j]);
-                    v[2 * j + 1] = fma(s.x, x.y, v[2 * j + 1]);
-                    v[2 * j + 1] = fma(s.y, x.x, v[2 * j + 1]);
+                for (int u = 0; u < kIn; ++u) s[u] = a[u];
+                fetch(k + kIn * kStep);
+#pragma unroll
+                for (int u = 0; u < kIn; ++u) {
+                    if (k + u * kStep >= w) break;
+                    const T* y = Yb + (k + u * kStep) * Bc + c0;
+#pragma unroll
+                    for (int j = 0; j < NC; ++j) {
+                        if (NC > 1 && j >= nc) break;   // uniform
+                        const T x = y[j];
+                        v[2 * j] = fma(s[u].x, x.x, v[2 * j]);
+                        v[2 * j] = fma(-s[u].y, x.y, v[2 * j]);
+                        v[2 * j + 1] = fma(s[u].x, x.y, v[2 * j + 1]);
+                        v[2 * j + 1] = fma(s[u].y, x.x, v[2 * j + 1]);
+                    }
                 }
-            };
-            int64_t k = kw * 32 + lane;
-            constexpr int kStep = kRowWarps * 32;
-            for (; k + 3 * kStep < w; k += 4 * kStep) {
-                const T s0 = S[k], s1 = S[k + kStep], s2 = S[k + 2 * kStep], s3 = S[k + 3 * kStep];
-                mac(s0, k);
-                mac(s1, k + kStep);
-                mac(s2, k + 2 * kStep);
-                mac(s3, k + 3 * kStep);
             }
-            for (; k < w; k += kStep) mac(S[k], k);
         }
         const R sum = lane_sum<NV>(v);
         constexpr int kPer = 32 / NV;              // lanes holding the same value
@@ -1160,12 +1251,13 @@ int slab_factor_t(emg_slab* s, int64_t F, const int32_t* amat_h, int64_t Bm, con
         rc = tile(0, st);
         if (rc) return rc;
         if (tc_update && sizeof(R) == 4) {
-            // FP32: two launches a step on one stream; the second one's first CTA is the lookahead
+            // FP32: two launches a step on one stream; the second one's first CTA inverts the next tile
             for (int k = 0; k < nt && nt > 1; ++k) {
                 if constexpr (sizeof(R) == 4) {
-                    k_gj_row<R><<<dim3(2 * nt, 1, (unsigned)F), kThreads, 0, st>>>(w, k, nt, Sinv, s->totD, s->offD[i],
-                                                                                   pset(k), colbuf, s->maxw * kTile);
-                    rc = emg::tc_gj_update(w, k, k + 1 < nt ? k + 1 : -1, F, Sinv, s->totD, s->offD[i], colbuf,
+                    const int strips = (int)((w + kStrip - 1) / kStrip), la = k + 1 < nt ? k + 1 : -1;
+                    EMG_CUDA(launch_pdl(k_gj_row, dim3(strips + nt, 1, (unsigned)F), dim3(kThreads), 0, st, 0, w, k, la,
+                                        strips, Sinv, s->totD, s->offD[i], pset(k), colbuf, s->maxw * kTile));
+                    rc = emg::tc_gj_update(w, k, la, F, Sinv, s->totD, s->offD[i], colbuf,
                                            s->maxw * kTile, pset(k), pset(k + 1), rel_thr, s->perturbed, s->tc_status,
                                            st);
                     if (rc) return rc;
@@ -1414,21 +1506,26 @@ struct SlabPrecond : emg::Precond {
             const dim3 g((unsigned)((w + kRowRows - 1) / kRowRows), G);
             auto rowmv = maxcol <= 1 ? k_rowmv<R, 1> : maxcol <= 2 ? k_rowmv<R, 2> : maxcol <= 4 ? k_rowmv<R, 4>
                                                                                               : k_rowmv<R, 8>;
-            rowmv<<<g, kThreads, 0, st>>>(w, s->off[i], Bc, s->groups, Sinv, s->totD, s->offD[i], Y, alpha, beta, Z);
+            const cudaError_t e = launch_pdl(rowmv, g, dim3(kThreads), 0, st, 0, w, s->off[i], Bc, s->groups, Sinv, s->totD,
+                                             s->offD[i], Y, alpha, beta, Z);
+            if (e != cudaSuccess && !rc) rc = cuda_status(e, "slab row product");
         };
         k_gather<R, TI><<<grid_for(s->n * Bc, 256), 256, 0, st>>>(s->n, Bc, s->perm, in, Y);
-        for (int i = 0; i < s->m; ++i) {
+        auto couple = [&](int mode, int64_t i, int64_t nb) {
             const int64_t w = s->off[i + 1] - s->off[i];
-            if (i > 0)
-                k_couple<R><<<grid_for(w * Bc, 256), 256, 0, st>>>(0, w, s->off[i], s->off[i - 1], Bc, s->colfac, s->cptr,
-                                                                   s->cidx, Cv, s->nC, Z, Y);
-            dense(w, i, (R)1, 0);
+            const cudaError_t e =
+                launch_pdl(k_couple<R>, dim3(grid_for(w * Bc, 256)), dim3(256), 0, st, 0, mode, w, s->off[i], s->off[nb], Bc,
+                           s->colfac, mode == 0 ? s->cptr : s->uptr, mode == 0 ? s->cidx : s->uidx, mode == 0 ? Cv : Uv,
+                           mode == 0 ? s->nC : s->nU, Z, Y);
+            if (e != cudaSuccess && !rc) rc = cuda_status(e, "slab coupling");
+        };
+        for (int i = 0; i < s->m; ++i) {
+            if (i > 0) couple(0, i, i - 1);
+            dense(s->off[i + 1] - s->off[i], i, (R)1, 0);
         }
         for (int i = s->m - 2; i >= 0; --i) {
-            const int64_t w = s->off[i + 1] - s->off[i];
-            k_couple<R><<<grid_for(w * Bc, 256), 256, 0, st>>>(1, w, s->off[i], s->off[i + 1], Bc, s->colfac, s->uptr,
-                                                               s->uidx, Uv, s->nU, Z, Y);
-            dense(w, i, (R)-1, 1);
+            couple(1, i, i + 1);
+            dense(s->off[i + 1] - s->off[i], i, (R)-1, 1);
         }
         k_scatter<R, TI><<<grid_for(s->n * Bc, 256), 256, 0, st>>>(s->n, Bc, s->perm, Z, out);
         EMG_CUDA(cudaGetLastError());

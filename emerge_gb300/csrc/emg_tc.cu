@@ -383,12 +383,13 @@ __device__ __forceinline__ float tf32_rn(float x) {
 __global__ void __launch_bounds__(kSpThreads, 1) k_slab_split(int64_t w, int64_t row0, int64_t Bc,
                                                               const TcGroup* __restrict__ groups, int G,
                                                               const float2* __restrict__ Sinv, int64_t totD, int64_t offD,
-                                                              const float2* __restrict__ Y, float alpha, int beta,
-                                                              float2* __restrict__ Out, int32_t* __restrict__ status) {
+                                                              const float2* Y, float alpha, int beta, float2* Out,
+                                                              int32_t* status) {
     extern __shared__ __align__(1024) unsigned char dsm[];
     char* base = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(dsm) + 1023) & ~(uintptr_t)1023);
     __shared__ __align__(8) uint64_t mbar[2];
     __shared__ uint32_t tmem_base;
+    pdl_trigger();
     const TcGroup g = groups[blockIdx.z % G];
     const int64_t c0 = (int64_t)(blockIdx.z / G) * kN, r0 = (int64_t)blockIdx.y * kM;
     if (c0 >= g.ncol) return;          // uniform per cluster, before any TMEM allocation or cluster barrier
@@ -418,7 +419,7 @@ __global__ void __launch_bounds__(kSpThreads, 1) k_slab_split(int64_t w, int64_t
     const int bp = ((lane & 3) << 1) + ((lane >> 4) << 3), bk = (lane >> 2) & 3;
     const float2 z2 = make_float2(0.f, 0.f);
     float2 va[8][2], vb[4][2];
-    auto load = [&](int ch) {
+    auto load_s = [&](int ch) {
         const int64_t k0 = ks0 + (int64_t)ch * kK;
 #pragma unroll
         for (int it = 0; it < 8; ++it) {
@@ -428,6 +429,9 @@ __global__ void __launch_bounds__(kSpThreads, 1) k_slab_split(int64_t w, int64_t
             va[it][0] = (gr < w && gk < ks1) ? src[0] : z2;
             va[it][1] = (gr < w && gk + 1 < ks1) ? src[1] : z2;
         }
+    };
+    auto load_y = [&](int ch) {
+        const int64_t k0 = ks0 + (int64_t)ch * kK;
 #pragma unroll
         for (int it = 0; it < 4; ++it) {
             if (it >= n16) break;
@@ -468,7 +472,9 @@ __global__ void __launch_bounds__(kSpThreads, 1) k_slab_split(int64_t w, int64_t
             }
         }
     };
-    if (nk > 0) load(0);
+    if (nk > 0) load_s(0);
+    pdl_wait();                        // S is of the factorization; Y is written by the launch before
+    if (nk > 0) load_y(0);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -530,7 +536,10 @@ __global__ void __launch_bounds__(kSpThreads, 1) k_slab_split(int64_t w, int64_t
                              smem_u32(&mbar[buf]))
                          : "memory");
         }
-        if (ch + 1 < nk) load(ch + 1);
+        if (ch + 1 < nk) {
+            load_s(ch + 1);
+            load_y(ch + 1);
+        }
     }
     // the last two chunks' MMAs (one more bounded wait each after a time-out, before the TMEM goes)
     for (int ch = max(0, nk - 2); ch < nk; ++ch)
@@ -774,10 +783,11 @@ __global__ void __launch_bounds__(kThreads) k_gemm_bf16_tc(int M, int N, int K, 
 //   4. the accumulators go TMEM -> shared memory, and the output block is written
 //      back minus the product.
 // Rows of tile k, and tile (la, la) when la >= 0, keep their values.  The first CTA of each
-// factor (la >= 0) is the lookahead: it forms tile (la, la) in FP32 and inverts it, so the
-// serial pivot chain runs under the update and a step is two launches on one stream (with
-// the lookahead on a side stream, its events and three more launches a step took 113 us on
-// average at widths up to 2768 and 61 + 15 at up to 1358; this takes 72 and 55).  Grid: 1 + column tiles x row blocks of 128, x F.
+// factor (la >= 0) is the lookahead: it inverts tile (la, la), which k_gj_row has updated, so the
+// serial pivot chain runs under the update and a step is two launches on one stream (with the
+// lookahead on a side stream, its events and three more launches a step took 113 us on average
+// at widths up to 2768 and 76 at up to 1358; with the tile's product in the first CTA too
+// and plain launches 72 and 55).  Grid: 1 + column tiles x row blocks of 128, x F.
 constexpr int kUpdM = 128, kUpdN = 64, kUpdTile = 64, kUpdThreads = 256;
 constexpr int kUpdATile = kUpdM * kK * 4;                  // one 128 x 32 FP32 tile: 16 KB
 constexpr int kUpdBTile = kUpdN * kK * 4;                  // one 64 x 32 FP32 tile: 8 KB
@@ -785,58 +795,26 @@ constexpr int kUpdChunk = 4 * kUpdATile + 4 * kUpdBTile;   // one K chunk: 96 KB
 constexpr int kUpdSmem = 2 * kUpdChunk;                    // the epilogue reuses 66.5 KB of it
 constexpr int kUpdLd = kUpdN + 1;                          // row stride of the staged product (float2)
 
-// The lookahead CTA: T = M[la, la] - C[la] M[k, la] in FP32, inverted into M[la, la] and pout.
-// buf: 3 x 64 x 65 complex in shared memory.
-__device__ __forceinline__ void gj_lookahead(int64_t w, int k, int la, int tb, float2* __restrict__ M,
-                                             const float2* __restrict__ C, float2* __restrict__ pout, float rel_thr,
-                                             int32_t* __restrict__ pert, float2* buf) {
+// The lookahead CTA: tile (la, la), which the row panel's launch updated, inverted into M[la, la]
+// and pout.  Ts: 64 x 65 complex in shared memory.
+__device__ __forceinline__ void gj_lookahead(int64_t w, int la, float2* M, float2* pout, float rel_thr, int32_t* pert,
+                                             float2* Ts) {
     __shared__ gj::PivotShared sh;
-    constexpr int kLd = gj::kLd;
-    float2 *Ts = buf, *As = buf + kUpdTile * kLd, *Bs = As + kUpdTile * kLd;
-    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-    const int64_t l0 = (int64_t)la * kUpdTile, k0 = (int64_t)k * kUpdTile;
+    const int64_t l0 = (int64_t)la * kUpdTile;
     const int lt = (int)min((int64_t)kUpdTile, w - l0);
+    float2* T = M + l0 * w + l0;
 #pragma unroll
     for (int q = 0; q < kUpdTile * kUpdTile / kUpdThreads; ++q) {
-        const int r = (tid + q * kUpdThreads) / kUpdTile, c = tid % kUpdTile;
-        As[r * kLd + c] = r < lt ? C[(l0 + r) * kUpdTile + c] : make_float2(0.f, 0.f);
-        Bs[r * kLd + c] = (r < tb && c < lt) ? M[(k0 + r) * w + l0 + c] : make_float2(0.f, 0.f);
+        const int r = ((int)threadIdx.x + q * kUpdThreads) / kUpdTile, c = (int)threadIdx.x % kUpdTile;
+        Ts[r * gj::kLd + c] = (r < lt && c < lt) ? T[r * w + c] : make_float2(r == c ? 1.f : 0.f, 0.f);
     }
-    float2 acc[4][4], m[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int r = ty + 16 * i, c = tx + 16 * j;
-            m[i][j] = (r < lt && c < lt) ? M[(l0 + r) * w + l0 + c] : make_float2(r == c ? 1.f : 0.f, 0.f);
-            acc[i][j] = make_float2(0.f, 0.f);
-        }
     __syncthreads();
-#pragma unroll 8
-    for (int kk = 0; kk < kUpdTile; ++kk) {
-        float2 av[4], bv[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) av[i] = As[(ty + 16 * i) * kLd + kk];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) bv[j] = Bs[kk * kLd + tx + 16 * j];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) gj::cmadd(acc[i][j], av[i], bv[j]);
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-            Ts[(ty + 16 * i) * kLd + tx + 16 * j] = make_float2(m[i][j].x - acc[i][j].x, m[i][j].y - acc[i][j].y);
-    __syncthreads();
-    gj::invert_tile(Ts, lt, rel_thr, sh, pert, M + l0 * w + l0, w, pout);
+    gj::invert_tile(Ts, lt, rel_thr, sh, pert, T, w, pout);
 }
 
 __global__ void __launch_bounds__(kUpdThreads, 1) k_gj_update_tc(
-    int64_t w, int k, int la, float2* __restrict__ Sinv, int64_t totD, int64_t offD, const float2* __restrict__ colbuf,
-    int64_t scol, const float2* __restrict__ pinv, float2* __restrict__ pinv_next, float rel_thr,
-    int32_t* __restrict__ perturbed, int32_t* __restrict__ status) {
+    int64_t w, int k, int la, float2* Sinv, int64_t totD, int64_t offD, const float2* colbuf, int64_t scol,
+    const float2* pinv, float2* pinv_next, float rel_thr, int32_t* perturbed, int32_t* status) {
     extern __shared__ __align__(1024) unsigned char dsm[];
     char* base = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(dsm) + 1023) & ~(uintptr_t)1023);
     __shared__ __align__(8) uint64_t mbar;
@@ -849,8 +827,10 @@ __global__ void __launch_bounds__(kUpdThreads, 1) k_gj_update_tc(
     const int64_t k0 = (int64_t)k * kUpdTile;
     const int tb = (int)min((int64_t)kUpdTile, w - k0);
     const float2 z2 = make_float2(0.f, 0.f);
+    pdl_trigger();
     if (blockIdx.x == 0) {             // uniform per CTA, before any TMEM allocation
-        if (la >= 0) gj_lookahead(w, k, la, tb, M, C, pinv_next + (int64_t)blockIdx.z * kUpdTile * kUpdTile, rel_thr,
+        pdl_wait();
+        if (la >= 0) gj_lookahead(w, la, M, pinv_next + (int64_t)blockIdx.z * kUpdTile * kUpdTile, rel_thr,
                                   perturbed + blockIdx.z, reinterpret_cast<float2*>(base));
         return;
     }
@@ -871,6 +851,7 @@ __global__ void __launch_bounds__(kUpdThreads, 1) k_gj_update_tc(
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    pdl_wait();
     // 1. operand loads.  A: warp item wi = warp + 8 it (it < 16) is row block wi / 8 and
     //    8-wide K block wi % 8; lane -> row (lane & 15) >> 1, K pair 2 (lane & 1) + 4 (lane >> 4).
     //    B: item wi = warp + 8 it (it < 8) is 16-wide column block wi / 16 and 4-deep K
@@ -1100,20 +1081,9 @@ int tc_slab_split(int64_t w, int64_t row0, int64_t Bc, const void* groups, int G
     int ranks = 1;
     while (ranks < 8 && 2 * ranks <= max_splits && (int64_t)ct * rt * G * 2 * ranks <= 152 && w >= 2 * ranks * 2 * tc::kK)
         ranks *= 2;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)ranks, (unsigned)rt, (unsigned)(G * ct));
-    cfg.blockDim = dim3(tc::kSpThreads);
-    cfg.dynamicSmemBytes = tc::kSpSmem + 1024;
-    cfg.stream = st;
-    cudaLaunchAttribute la[1];
-    la[0].id = cudaLaunchAttributeClusterDimension;
-    la[0].val.clusterDim.x = (unsigned)ranks;
-    la[0].val.clusterDim.y = 1;
-    la[0].val.clusterDim.z = 1;
-    cfg.attrs = la;
-    cfg.numAttrs = 1;
-    EMG_CUDA(cudaLaunchKernelEx(&cfg, tc::k_slab_split, w, row0, Bc, static_cast<const tc::TcGroup*>(groups), G, Sinv, totD,
-                                offD, Y, alpha, beta, Out, status));
+    EMG_CUDA(launch_pdl(tc::k_slab_split, dim3((unsigned)ranks, (unsigned)rt, (unsigned)(G * ct)), dim3(tc::kSpThreads),
+                        tc::kSpSmem + 1024, st, ranks, w, row0, Bc, static_cast<const tc::TcGroup*>(groups), G, Sinv, totD,
+                        offD, Y, alpha, beta, Out, status));
     return EMG_OK;
 }
 }  // namespace emg
@@ -1141,9 +1111,9 @@ int tc_gj_update(int64_t w, int k, int la, int64_t F, float2* Sinv, int64_t totD
         attr = true;
     }
     const int64_t tiles = ((w + tc::kUpdN - 1) / tc::kUpdN) * ((w + tc::kUpdM - 1) / tc::kUpdM);
-    tc::k_gj_update_tc<<<dim3((unsigned)(1 + tiles), 1, (unsigned)F), tc::kUpdThreads, tc::kUpdSmem + 1024, st>>>(
-        w, k, la, Sinv, totD, offD, colbuf, scol, pinv, pinv_next, rel_thr, perturbed, status);
-    EMG_CUDA(cudaGetLastError());
+    EMG_CUDA(launch_pdl(tc::k_gj_update_tc, dim3((unsigned)(1 + tiles), 1, (unsigned)F), dim3(tc::kUpdThreads),
+                        tc::kUpdSmem + 1024, st, 0, w, k, la, Sinv, totD, offD, colbuf, scol, pinv, pinv_next, rel_thr,
+                        perturbed, status));
     return EMG_OK;
 }
 }  // namespace emg

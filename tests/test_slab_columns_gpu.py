@@ -71,3 +71,20 @@ def test_split_settings_agree(system):
         errs.append(float(torch.linalg.norm(y - x) / torch.linalg.norm(x)))
     slab.set_max_splits(8)
     assert max(errs) <= 2 * min(errs)
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+@pytest.mark.parametrize("cols", [2, 24])
+def test_replayed_cycles(system, precision, cols):
+    """Cycles of one step replay a captured graph of the chained solve launches."""
+    torch, sysr, A, slab = system
+    slab.factor(A, [0], precision)
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    b = torch.view_as_complex(torch.randn((sysr.n, cols, 2), generator=gen, device="cuda", dtype=torch.float64))
+    cm = torch.ones(cols, dtype=torch.int32, device="cuda")          # the other frequency's matrix: several cycles
+    x, its, res = slab.gmres(A, b, cm, [0] * cols, tol=1e-3, restart=1, max_iter=12)
+    y, its_y, res_y = slab.gmres(A, b, cm, [0] * cols, tol=1e-3, restart=1, max_iter=12)
+    assert its.min() > 1 and np.array_equal(its, its_y)
+    assert torch.equal(torch.view_as_real(x), torch.view_as_real(y))
+    true = (torch.linalg.norm(b - sysr.spmv(A, x, cm), dim=0) / torch.linalg.norm(b, dim=0)).cpu().numpy()
+    assert np.all(np.abs(true - res) <= 1e-9)                        # the reported residual is that of x
