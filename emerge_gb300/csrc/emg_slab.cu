@@ -62,8 +62,8 @@ __device__ __forceinline__ double2 to_d(double2 v) { return v; }
 
 constexpr int kTile = 64;          // Gauss-Jordan tile and GEMM output tile
 constexpr int kThreads = 256;
-constexpr int kMaxRows = 16;       // rows per CTA in the Schur-complement kernel
-constexpr int kSchurSmem = 200 * 1024;
+constexpr int kSchurSmem = 200 * 1024;            // column block of the Schur-complement kernel
+constexpr int64_t kSchurScratch = 64ll << 20;     // C_i S_{i-1}^-1, rows of a part
 constexpr int64_t kMaxWidth = 12288;
 
 template <typename R> struct Tile {
@@ -156,52 +156,82 @@ __global__ void k_offvals(int64_t nn, int64_t Bm, int64_t F, const int32_t* __re
     }
 }
 
-// S_i -= (C_i S_{i-1}^-1) U_{i-1} for rows [a0, a0+nr) of slab i (grid: row blocks x 1 x F).
-template <typename R>
-__global__ void __launch_bounds__(kThreads) k_schur(int64_t wp, int64_t w, int64_t row0, int rb,
-                                                    const int64_t* __restrict__ cptr, const int32_t* __restrict__ cidx,
-                                                    const typename C2<R>::T* __restrict__ Cval, int64_t nC,
-                                                    const int64_t* __restrict__ ucptr, const int32_t* __restrict__ ucrow,
-                                                    const typename C2<R>::T* __restrict__ UCval, int64_t nU,
-                                                    typename C2<R>::T* __restrict__ Sinv, int64_t totD, int64_t offPrev,
-                                                    int64_t offCur) {
+// Out[x][j] (-)= sum_k val(j, k) In[idx(j, k)][x]: rows of a sparse matrix (some 20 entries each)
+// times a dense one, transposed.  Run twice it forms S_i -= (C_i S_{i-1}^-1) U_{i-1}: first the rows
+// of C_i with In = S_{i-1}^-1, then the columns of U_{i-1} with In = the first result.  A CTA keeps XB
+// columns of all of In in shared memory, so every entry of In is read once from memory and the
+// combinations, 20 reads for each, come from there; a thread has one or two of the columns and every
+// kSpThreads / (XB / 2)-th row, four entries in flight.  Rows of the dense operand straight from L2,
+// then combined in shared memory by thread per column, took 303 us (FP32, 1812 wide on average) and
+// 207 (FP64, 737 wide, where the pipe needs 150), the two launches of this 123 and 180.  Grid: column blocks x 1 x F.
+constexpr int kSpThreads = 512, kSpIn = 4;
+template <typename R, int XB>
+__global__ void __launch_bounds__(kSpThreads) k_sparse_rows(
+    int64_t nr, int64_t nx, int64_t nj, int64_t j0, const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx,
+    const typename C2<R>::T* __restrict__ val, int64_t sval, const typename C2<R>::T* __restrict__ In, int64_t ldi,
+    int64_t sIn, typename C2<R>::T* __restrict__ Out, int64_t ldo, int64_t sOut, int subtract) {
     using T = typename C2<R>::T;
+    constexpr int CT = XB >= 2 ? 2 : 1, LX = XB / CT;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    T* Rs = reinterpret_cast<T*>(smem_raw);
-    const int64_t f = blockIdx.z;
-    const int64_t a0 = (int64_t)blockIdx.x * rb;
-    const int nr = (int)min((int64_t)rb, w - a0);
-    const T* Sp = Sinv + f * totD + offPrev;
-    T* Sc = Sinv + f * totD + offCur;
-    const T* Cv = Cval + f * nC;
-    const T* Uv = UCval + f * nU;
-    for (int64_t idx = threadIdx.x; idx < (int64_t)nr * wp; idx += blockDim.x) {
-        const int64_t a = idx / wp, col = idx % wp;
-        const int64_t row = row0 + a0 + a;
-        T acc = czero<T>();
-        for (int64_t k = cptr[row]; k < cptr[row + 1]; ++k) cfma(acc, Cv[k], Sp[(int64_t)cidx[k] * wp + col]);
-        Rs[idx] = acc;
+    T* buf = reinterpret_cast<T*>(smem_raw);
+    const int64_t f = blockIdx.z, x0 = (int64_t)blockIdx.x * XB;
+    In += f * sIn + x0;
+    Out += f * sOut;
+    val += f * sval;
+    const int nxb = (int)min((int64_t)XB, nx - x0);
+#pragma unroll 4
+    for (int64_t i = threadIdx.x; i < nr * XB; i += kSpThreads) {
+        const int64_t r = i / XB;
+        const int x = (int)(i % XB);
+        buf[i] = x < nxb ? In[r * ldi + x] : czero<T>();
     }
     __syncthreads();
-    for (int64_t j = threadIdx.x; j < w; j += blockDim.x) {
-        T acc[kMaxRows];
+    const int xl = (threadIdx.x % LX) * CT;
+    for (int64_t j = threadIdx.x / LX; j < nj; j += kSpThreads / LX) {
+        T acc[CT];
 #pragma unroll
-        for (int a = 0; a < kMaxRows; ++a) acc[a] = czero<T>();
-        for (int64_t k = ucptr[row0 + j]; k < ucptr[row0 + j + 1]; ++k) {
-            const int64_t r = ucrow[k];
-            const T u = Uv[k];
+        for (int c = 0; c < CT; ++c) acc[c] = czero<T>();
+        const int64_t k1 = ptr[j0 + j + 1];
+        for (int64_t k = ptr[j0 + j]; k < k1; k += kSpIn) {
+            int32_t id[kSpIn];
+            T v[kSpIn];
 #pragma unroll
-            for (int a = 0; a < kMaxRows; ++a)
-                if (a < nr) cfma(acc[a], Rs[a * wp + r], u);
+            for (int u = 0; u < kSpIn; ++u) {
+                id[u] = k + u < k1 ? idx[k + u] : -1;
+                v[u] = k + u < k1 ? val[k + u] : czero<T>();
+            }
+#pragma unroll
+            for (int u = 0; u < kSpIn; ++u) {
+                if (id[u] < 0) break;
+#pragma unroll
+                for (int c = 0; c < CT; ++c) cfma(acc[c], v[u], buf[id[u] * XB + xl + c]);
+            }
         }
 #pragma unroll
-        for (int a = 0; a < kMaxRows; ++a)
-            if (a < nr) {
-                T& s = Sc[(a0 + a) * w + j];
-                s.x -= acc[a].x;
-                s.y -= acc[a].y;
+        for (int c = 0; c < CT; ++c)
+            if (xl + c < nxb) {
+                T& o = Out[(x0 + xl + c) * ldo + j];
+                o = subtract ? mk(o.x - acc[c].x, o.y - acc[c].y) : acc[c];
             }
     }
+}
+
+// Its launch: the widest column block that fits in shared memory and gives two CTAs per SM.
+template <typename R>
+cudaError_t sparse_rows(int64_t nr, int64_t nx, int64_t nj, int64_t j0, const int64_t* ptr, const int32_t* idx,
+                        const typename C2<R>::T* val, int64_t sval, const typename C2<R>::T* In, int64_t ldi, int64_t sIn,
+                        typename C2<R>::T* Out, int64_t ldo, int64_t sOut, int subtract, int64_t F, cudaStream_t st) {
+    int xb = 8;
+    while (xb > 1 && (nr * xb * (int64_t)sizeof(typename C2<R>::T) > kSchurSmem || (xb > 2 && (nx + xb - 1) / xb * F < 2 * 152)))
+        xb /= 2;
+    auto kern = xb == 8 ? k_sparse_rows<R, 8> : xb == 4 ? k_sparse_rows<R, 4> : xb == 2 ? k_sparse_rows<R, 2>
+                                                                                      : k_sparse_rows<R, 1>;
+    const size_t smem = (size_t)nr * xb * sizeof(typename C2<R>::T);
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSchurSmem);
+    if (e != cudaSuccess) return e;
+    kern<<<dim3((unsigned)((nx + xb - 1) / xb), 1, (unsigned)F), kSpThreads, smem, st>>>(
+        nr, nx, nj, j0, ptr, idx, val, sval, In, ldi, sIn, Out, ldo, sOut, subtract);
+    return cudaGetLastError();
 }
 
 // The FP32 pivot tile k by itself (emg_gj.cuh): M[k, k] and pinv receive its inverse.  Grid 1 x 1 x F.
@@ -1170,6 +1200,14 @@ int slab_factor_t(emg_slab* s, int64_t F, const int32_t* amat_h, int64_t Bm, con
         if (rc) { dfree(colbuf); slab_free_factors(s); return rc; }
     }
     struct TmpC { T *a, *b; ~TmpC() { if (a) cudaFree(a); if (b) cudaFree(b); } } tmpc{colbuf, rowbuf};
+    // C_i S_{i-1}^-1, transposed, ``part`` rows of slab i at a time
+    const int64_t part = std::min<int64_t>(s->maxw, std::max<int64_t>(64, kSchurScratch / (F * s->maxw * (int64_t)sizeof(T))));
+    T* Rt = nullptr;
+    if (s->m > 1) {
+        rc = dalloc(&Rt, F * part * s->maxw, "slab Schur rows");
+        if (rc) { slab_free_factors(s); return rc; }
+    }
+    struct TmpR { T* a; ~TmpR() { if (a) cudaFree(a); } } tmpr{Rt};
     // Newton-Schulz scratch: a copy of S_i and the factor 2I - S_i X (F blocks of maxw^2)
     T *Scopy = nullptr, *Rbuf = nullptr;
     double* npart = nullptr;
@@ -1196,7 +1234,6 @@ int slab_factor_t(emg_slab* s, int64_t F, const int32_t* amat_h, int64_t Bm, con
         k_offvals<R><<<grid_for(s->nU * F, 256), 256, 0, st>>>(s->nU, Bm, F, amat, A, s->ucsrc, static_cast<T*>(s->UCval));
     }
     EMG_CUDA(cudaGetLastError());
-    EMG_CUDA(cudaFuncSetAttribute(k_schur<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSchurSmem));
     const R rel_thr = sizeof(R) == 4 ? (R)1e-6 : (R)1e-13;
     // the side stream of the pivot-tile lookahead and its two events
     struct Side {
@@ -1223,14 +1260,13 @@ int slab_factor_t(emg_slab* s, int64_t F, const int32_t* amat_h, int64_t Bm, con
         const int64_t w = s->off[i + 1] - s->off[i];
         if (i > 0) {
             const int64_t wp = s->off[i] - s->off[i - 1];
-            // rows per CTA: enough CTAs for two per SM, at most kMaxRows, within shared memory
-            const int64_t rb_grid = std::max<int64_t>(1, (w * F) / (2 * 152));
-            const int rb = (int)std::max<int64_t>(
-                1, std::min<int64_t>({(int64_t)kMaxRows, kSchurSmem / (wp * (int64_t)sizeof(T)), rb_grid}));
-            const dim3 g((unsigned)((w + rb - 1) / rb), 1, (unsigned)F);
-            k_schur<R><<<g, kThreads, (size_t)rb * wp * sizeof(T), st>>>(
-                wp, w, s->off[i], rb, s->cptr, s->cidx, static_cast<const T*>(s->Cval), s->nC, s->ucptr, s->ucrow,
-                static_cast<const T*>(s->UCval), s->nU, Sinv, s->totD, s->offD[i - 1], s->offD[i]);
+            for (int64_t a0 = 0; a0 < w; a0 += part) {
+                const int64_t na = std::min(part, w - a0);
+                EMG_CUDA(sparse_rows<R>(wp, wp, na, s->off[i] + a0, s->cptr, s->cidx, static_cast<const T*>(s->Cval), s->nC,
+                                        Sinv + s->offD[i - 1], wp, s->totD, Rt, na, part * s->maxw, 0, F, st));
+                EMG_CUDA(sparse_rows<R>(wp, na, w, s->off[i], s->ucptr, s->ucrow, static_cast<const T*>(s->UCval), s->nU, Rt,
+                                        na, part * s->maxw, Sinv + s->offD[i] + a0 * w, w, s->totD, 1, F, st));
+            }
         }
         const int nt = (int)((w + kTile - 1) / kTile);
         if (refine > 0)   // keep S_i for the refinement

@@ -88,3 +88,18 @@ def test_replayed_cycles(system, precision, cols):
     assert torch.equal(torch.view_as_real(x), torch.view_as_real(y))
     true = (torch.linalg.norm(b - sysr.spmv(A, x, cm), dim=0) / torch.linalg.norm(b, dim=0)).cpu().numpy()
     assert np.all(np.abs(true - res) <= 1e-9)                        # the reported residual is that of x
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_factor_counts(system, precision):
+    """The Schur products take 2, 4 or 8 columns a block with the number of factors, and with a
+    hundred the rows in parts; no sum changes its order."""
+    torch, sysr, A, slab = system
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    b = torch.view_as_complex(torch.randn((sysr.n, 2, 2), generator=gen, device="cuda", dtype=torch.float64))
+    slab.factor(A, [0, 1], precision)
+    ref = torch.view_as_real(slab.apply(b, [0, 1]))
+    for F in (3, 6, 12, 30, 100):
+        slab.factor(A, [0, 1] + [0] * (F - 3) + [1], precision)
+        for fac in ([0, 1], [0, F - 1], [F - 2 if F > 3 else 0, 1]):
+            assert torch.equal(torch.view_as_real(slab.apply(b, fac)), ref), F
