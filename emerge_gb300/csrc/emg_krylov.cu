@@ -306,6 +306,9 @@ __global__ void k_spmv_fam(int64_t n, int64_t nnz, int64_t Bc, int nfam, const d
 // memory in a fixed order.  Bound by the FP64 pipe (4 DFMA per product).  A thread per
 // column walking 1024 rows left 97 blocks with one load in flight each (48 columns, 98k
 // rows, 13 vectors on average: 3553 -> 276 us a call).
+// FUN: part[blk][j][c] = sum_{rows in blk} V[r][j] W[r,c] for the nj columns of V (rows of vstride),
+// not conjugated: a few functionals of every column (the library's long-K product has one CTA
+// for them: 2590 us for 2282 unknowns and 20 columns, this below 30).
 constexpr int kDotThreads = 256, kDotJ = 4;
 constexpr int kMaxRestart = 256;
 __device__ __forceinline__ void dot_acc(double2& s, double2 v, double2 w) { cfmac(s, v, w); }
@@ -315,7 +318,7 @@ __device__ __forceinline__ void dot_acc(float2& s, float2 v, float2 w) {
     s.x = fmaf(v.y, w.y, s.x);
     s.y = fmaf(-v.y, w.x, s.y);
 }
-template <typename T>
+template <typename T, bool FUN>
 __global__ void __launch_bounds__(kDotThreads) k_dots_partial(int64_t n, int Bc, int cw, int nj, int64_t rows,
                                                               const T* __restrict__ V, int64_t vstride,
                                                               const T* __restrict__ W, double2* __restrict__ part) {
@@ -327,14 +330,18 @@ __global__ void __launch_bounds__(kDotThreads) k_dots_partial(int64_t n, int Bc,
 #pragma unroll
     for (int j = 0; j < kDotJ; ++j) acc[j].x = acc[j].y = 0;
     if (g < groups && c < Bc) {
-        const T* Vb = V + j0 * vstride;
+        const T* Vb = FUN ? V + j0 : V + j0 * vstride;
+        auto acc1 = [&](int j, int64_t r, int64_t t, T w) {
+            if constexpr (FUN) cfma(acc[j], Vb[r * vstride + j], w);
+            else dot_acc(acc[j], Vb[j * vstride + t], w);
+        };
         if (jn == kDotJ) {
 #pragma unroll 2
             for (int64_t r = r0 + g; r < r1; r += groups) {
                 const int64_t t = r * Bc + c;
                 const T w = W[t];
 #pragma unroll
-                for (int j = 0; j < kDotJ; ++j) dot_acc(acc[j], Vb[j * vstride + t], w);
+                for (int j = 0; j < kDotJ; ++j) acc1(j, r, t, w);
             }
         } else {
             for (int64_t r = r0 + g; r < r1; r += groups) {
@@ -342,7 +349,7 @@ __global__ void __launch_bounds__(kDotThreads) k_dots_partial(int64_t n, int Bc,
                 const T w = W[t];
 #pragma unroll
                 for (int j = 0; j < kDotJ - 1; ++j)
-                    if (j < jn) dot_acc(acc[j], Vb[j * vstride + t], w);
+                    if (j < jn) acc1(j, r, t, w);
             }
         }
     }
@@ -926,13 +933,13 @@ void spmv(const emg_rplan* p, int64_t Bc, const int32_t* cmat, int64_t Bm, const
 // for each (fewer spend more on the reduction than on the products).
 int64_t dot_rows(int64_t n) { return std::max<int64_t>(64, (n + 2 * 152 - 1) / (2 * 152)); }
 
-template <typename T>
+template <typename T, bool FUN = false>
 void dots(int64_t n, int64_t Bc, int nj, const T* V, int64_t vstride, const T* W, double2* part, double2* out,
           cudaStream_t s) {
     const int64_t rows = dot_rows(n), nblk = (n + rows - 1) / rows;
     const int ct = (int)((Bc + 127) / 128), cw = (int)((Bc + ct - 1) / ct);
     const dim3 g((unsigned)nblk, (unsigned)ct, (unsigned)((nj + kry::kDotJ - 1) / kry::kDotJ));
-    kry::k_dots_partial<T><<<g, kry::kDotThreads, 0, s>>>(n, (int)Bc, cw, nj, rows, V, vstride, W, part);
+    kry::k_dots_partial<T, FUN><<<g, kry::kDotThreads, 0, s>>>(n, (int)Bc, cw, nj, rows, V, vstride, W, part);
     kry::k_dots_final<<<(unsigned)(((int64_t)nj * Bc * 32 + 127) / 128), 128, 0, s>>>(nblk, Bc, nj, part, out);
 }
 }  // namespace
@@ -1368,6 +1375,22 @@ struct IluPrecond : emg::Precond {
     }
 };
 }  // namespace
+
+extern "C" int64_t emg_functionals_work(int64_t n, int np, int64_t Bc) {
+    if (n <= 0 || np <= 0 || Bc <= 0) return 0;
+    return (n + dot_rows(n) - 1) / dot_rows(n) * np * Bc;
+}
+
+extern "C" int emg_functionals(int64_t n, int np, int64_t Bc, const double* U, const double* X, double* work, double* G,
+                               void* stream) {
+    using namespace emg;
+    EMG_CHECK_ARG(n > 0 && np > 0 && np <= 65535 && Bc > 0 && Bc < (1ll << 31) && U && X && work && G,
+                  "emg_functionals: bad argument");
+    dots<double2, true>(n, Bc, np, reinterpret_cast<const double2*>(U), np, reinterpret_cast<const double2*>(X),
+                        reinterpret_cast<double2*>(work), reinterpret_cast<double2*>(G), (cudaStream_t)stream);
+    EMG_CUDA(cudaGetLastError());
+    return EMG_OK;
+}
 
 extern "C" int emg_gmres(const emg_rplan* pc, int64_t Bc, const int32_t* cmat, int64_t Bm, const double* A_,
                          const double* LU_, const double* rhs_, double* x_, int restart, int max_iter, double tol,

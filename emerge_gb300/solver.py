@@ -33,6 +33,19 @@ def _stream() -> ctypes.c_void_p:
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
+def functionals(U: torch.Tensor, X: torch.Tensor) -> torch.Tensor:
+    """U.T @ X (np, C) of a few functionals U (n, np) of the columns of X (n, C), complex128."""
+    n, npo = U.shape
+    C = int(X.shape[1])
+    if n == 0 or npo == 0 or C == 0 or not X.is_cuda:
+        return U.T @ X
+    U, X = U.contiguous(), X.contiguous()
+    G = torch.empty((npo, C), dtype=X.dtype, device=X.device)
+    work = torch.empty(_lib.load().emg_functionals_work(n, npo, C), dtype=X.dtype, device=X.device)
+    _lib.call("emg_functionals", n, npo, C, _vp(U), _vp(X), _vp(work), _vp(G), _stream())
+    return G
+
+
 class RestrictedSystem:
     """PEC-restricted CSR pattern + ILU(0) structure (emg_rplan)."""
 
@@ -564,7 +577,7 @@ class FrequencySweep:
         Lumped ports (emfreq3d.py:752-766): V = line voltage, pfield = sqrt((V - [i = j] V0)^2
         / (2 Z0)), pmode = sqrt(V0^2 / (2 Z0)), principal square roots as the reference."""
         npo = len(self.ports)
-        G = -(self.u_w.T @ X).cpu().numpy()                                                      # (np, nf*np)
+        G = -functionals(self.u_w, X).cpu().numpy()                                              # (np, nf*np)
         V = {i: (w[:, None] * X[r]).sum(dim=0).cpu().numpy() for i, (r, w) in self._vfun.items()}
         S = np.zeros((nf, npo, npo), dtype=np.complex128)
         for f in range(nf):

@@ -190,6 +190,12 @@ int emg_spmv(const emg_rplan* plan, int64_t Bc, const int32_t* cmat, int64_t Bm,
 int emg_spmv_family(const emg_rplan* plan, int64_t Bc, int nfam, const double* fam, const double* coef,
                     const double* X, const double* Bv, double* Y, void* stream);
 
+/* G [np][Bc] = U^T X (no conjugate) for a few functionals U [n][np] of the columns of X [n][Bc],
+ * complex, DEVICE; work: emg_functionals_work(n, np, Bc) complex entries.  Sums in a fixed order. */
+int64_t emg_functionals_work(int64_t n, int np, int64_t Bc);
+int emg_functionals(int64_t n, int np, int64_t Bc, const double* U, const double* X, double* work, double* G,
+                    void* stream);
+
 /* out[i][c] = full[c][solve_ids[i]] (full: Bc vectors of N) and the inverse
  * scatter (zeros on removed DOFs). */
 int emg_rplan_gather(const emg_rplan* plan, int64_t Bc, const double* full, double* out, void* stream);
