@@ -687,6 +687,110 @@ __global__ void __launch_bounds__(kThreads) k_rowmv(int64_t w, int64_t row0, int
     }
 }
 
+// The FP32 product for groups of up to 64 columns on narrow slabs: a CTA has kR8 rows and all
+// columns, K split over its 16 warps; lane -> rows lane / 8 and lane / 8 + 4, columns lane % 8 + 8 j.
+// The rows of S_i^-1 come to shared memory under the launch before (they are of the
+// factorization), so after the wait only Y is read, each value once per CTA and for two rows of
+// a lane; the warps' sums are added in warp order.  Bound by latency on narrow slabs, by the
+// FMAs of the SMs in use on wide ones.  A tensor-core tile has 10 us of set-up, cluster barriers and
+// reduction that this has not: product and coupling of 48 columns take 23 us instead of 32 on
+// slabs of 941 (rms), 20 columns 8.5 instead of 17 on slabs of 156.
+// Grid: row blocks x groups.
+constexpr int kR8 = 8, kR8Warps = 16, kR8Threads = 32 * kR8Warps;
+__host__ __device__ inline int rows8_ld(int64_t w) { return (int)((w + 3) / 4 * 4) + 2 + (int)((16 - ((w + 3) / 4 * 4) % 16) % 16); }
+template <int NC>
+__global__ void __launch_bounds__(kR8Threads, 1) k_rows8(int64_t w, int64_t row0, int64_t Bc, const Group* __restrict__ groups,
+                                                         const float2* __restrict__ Sinv, int64_t totD, int64_t offD,
+                                                         const float2* Y, float alpha, int beta, float2* Out) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    float2* sm = reinterpret_cast<float2*>(smem_raw);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rg = lane >> 3, cg = lane & 7;
+    const int ld = rows8_ld(w), wi = (int)w;
+    const int64_t r0 = (int64_t)blockIdx.x * kR8;
+    const Group g = groups[blockIdx.y];
+    pdl_trigger();
+    {
+        const int r = warp & (kR8 - 1);
+        const float2* src = Sinv + (int64_t)g.fac * totD + offD + (r0 + r) * w;
+        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(sm + r * ld);
+        const bool in = r0 + r < w;
+        for (int k = (warp / kR8) * 32 + lane; k < (wi + 3) / 4 * 4; k += 64) {
+            if (in && k < wi) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + 8u * k), "l"(src + k) : "memory");
+            else sm[r * ld + k] = make_float2(0.f, 0.f);
+        }
+    }
+    const int kper = ((wi + kR8Warps - 1) / kR8Warps + 3) & ~3, ka = min(wi, warp * kper), kb = min(wi, ka + kper);
+    const float2* Yb = Y + row0 * Bc + g.col0 + cg;
+    float2 acc[2][NC];
+#pragma unroll
+    for (int j = 0; j < NC; ++j) acc[0][j] = acc[1][j] = make_float2(0.f, 0.f);
+    pdl_wait();
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    for (int k = ka; k < kb; k += 4) {
+        float2 y[4][NC];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int j = 0; j < NC; ++j)
+                y[u][j] = (k + u < kb && cg + 8 * j < g.ncol) ? Yb[(int64_t)(k + u) * Bc + 8 * j] : make_float2(0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const float4* sp = reinterpret_cast<const float4*>(sm + (rg + 4 * i) * ld + k);
+            const float4 a = sp[0], b = sp[1];
+            const float2 sv[4] = {make_float2(a.x, a.y), make_float2(a.z, a.w), make_float2(b.x, b.y), make_float2(b.z, b.w)};
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int j = 0; j < NC; ++j) cfma(acc[i][j], sv[u], y[u][j]);
+        }
+    }
+    __syncthreads();                   // the rows of S_i^-1 make room for the warps' sums
+    constexpr int kC = 8 * NC;
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < NC; ++j) sm[(warp * kR8 + rg + 4 * i) * kC + cg + 8 * j] = acc[i][j];
+    __syncthreads();
+    for (int e = tid; e < kR8 * kC; e += kR8Threads) {
+        const int r = e / kC, c = e % kC;
+        if (r0 + r >= w || c >= g.ncol) continue;
+        float2 v = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int q = 0; q < kR8Warps; ++q) {
+            const float2 x = sm[(q * kR8) * kC + e];
+            v.x += x.x;
+            v.y += x.y;
+        }
+        float2& o = Out[(row0 + r0 + r) * Bc + g.col0 + c];
+        if (beta) { o.x += alpha * v.x; o.y += alpha * v.y; }
+        else o = make_float2(alpha * v.x, alpha * v.y);
+    }
+}
+
+// Where it is the faster one: up to 64 columns while the row blocks of all groups are one round of
+// the SMs, and beyond that while rounds x width x columns stays below 45,000 (us a product and
+// coupling, here / tensor cores: 941 wide, one group of 64 columns 27 / 35, two of 24 27 / 30, three of
+// 16 26 / 29, three of 32 41 / 32; 735 wide, three of 32 30 / 28).
+inline bool rows8_wins(int64_t w, int G, int maxcol) {
+    const int64_t rounds = ((w + kR8 - 1) / kR8 * G + 151) / 152;
+    return maxcol <= 64 && sizeof(float2) * (size_t)(kR8 * rows8_ld(w)) <= (size_t)kSchurSmem &&
+           (rounds == 1 || rounds * w * ((maxcol + 7) / 8 * 8) <= 45000);
+}
+
+inline cudaError_t rows8(int64_t w, int64_t row0, int64_t Bc, const Group* groups, int G, int maxcol, const float2* Sinv,
+                         int64_t totD, int64_t offD, const float2* Y, float alpha, int beta, float2* Out, cudaStream_t st) {
+    const int nc = (maxcol + 7) / 8;
+    auto kern = nc <= 1 ? k_rows8<1> : nc <= 2 ? k_rows8<2> : nc <= 3 ? k_rows8<3> : nc <= 4 ? k_rows8<4> : nc <= 6 ? k_rows8<6>
+                                                                                                          : k_rows8<8>;
+    const int ncw = nc <= 4 ? nc : nc <= 6 ? 6 : 8;
+    const size_t smem = sizeof(float2) * (size_t)std::max(kR8 * rows8_ld(w), kR8Warps * kR8 * 8 * ncw);
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSchurSmem);
+    if (e != cudaSuccess) return e;
+    return launch_pdl(kern, dim3((unsigned)((w + kR8 - 1) / kR8), (unsigned)G), dim3(kR8Threads), smem, st, 0, w, row0, Bc,
+                      groups, Sinv, totD, offD, Y, alpha, beta, Out);
+}
+
 // The same product for wide groups: 64 x 64 output tiles through tile_mac, with
 // the K range split over ``splits`` CTAs when the tiles alone would not fill the
 // GPU.  A split writes its partial tile to ``part``; the last split of a tile to
@@ -1503,14 +1607,22 @@ struct SlabPrecond : emg::Precond {
             }
         }
         // dense slab product: rows of few columns for groups narrower than s->wide; wider FP32
-        // groups on the tensor cores (TF32 products if asked for, else split ones), FP64 groups
-        // as 128 x 16 tiles up to 16 columns and 64 x 64 tiles above
+        // groups by row blocks or on the tensor cores (TF32 products if asked for, else split
+        // ones), FP64 groups as 128 x 16 tiles up to 16 columns and 64 x 64 tiles above
         int rc = EMG_OK;
         auto dense = [&](int64_t w, int64_t i, R alpha, int beta) {
             if constexpr (sizeof(R) == 4) {
-                if (maxcol >= s->wide) {
+                // (several groups of four or more columns go there too: 4 columns of two factors on
+                // slabs of 941 take 24 us by rows, 17 by row blocks)
+                if (maxcol >= s->wide || (maxcol >= 4 && !s->use_tc && (int64_t)maxcol * G >= s->wide)) {
                     const auto* Sf = reinterpret_cast<const float2*>(Sinv);
                     const auto* Yf = reinterpret_cast<const float2*>(Y);
+                    if (!s->use_tc && rows8_wins(w, (int)G, maxcol)) {
+                        const cudaError_t e = rows8(w, s->off[i], Bc, s->groups, (int)G, maxcol, Sf, s->totD, s->offD[i], Yf,
+                                                    (float)alpha, beta, reinterpret_cast<float2*>(Z), st);
+                        if (e != cudaSuccess && !rc) rc = cuda_status(e, "slab row-block product");
+                        return;
+                    }
                     const int e = s->use_tc ? emg::tc_slab_product(w, s->off[i], Bc, s->groups, (int)G, maxcol, Sf, s->totD,
                                                                    s->offD[i], Yf, (float)alpha, beta,
                                                                    reinterpret_cast<float2*>(Z), s->tc_status, st)

@@ -103,3 +103,42 @@ def test_factor_counts(system, precision):
         slab.factor(A, [0, 1] + [0] * (F - 3) + [1], precision)
         for fac in ([0, 1], [0, F - 1], [F - 2 if F > 3 else 0, 1]):
             assert torch.equal(torch.view_as_real(slab.apply(b, fac)), ref), F
+
+
+def test_split_settings_agree_on_tiles(system):
+    """The same with more columns than the row blocks take: the tensor-core tiles' K split."""
+    torch, sysr, A, slab = system
+    slab.factor(A, [0], "fp32")
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    x = torch.view_as_complex(torch.randn((sysr.n, 70, 2), generator=gen, device="cuda", dtype=torch.float64))
+    b = sysr.spmv(A, x, torch.zeros(70, dtype=torch.int32, device="cuda"))
+    errs = []
+    for splits in (1, 2, 4, 8, 16):
+        slab.set_max_splits(splits)
+        y = slab.apply(b, [0] * 70)
+        assert torch.equal(torch.view_as_real(y), torch.view_as_real(slab.apply(b, [0] * 70)))
+        errs.append(float(torch.linalg.norm(y - x) / torch.linalg.norm(x)))
+    slab.set_max_splits(8)
+    assert max(errs) <= 2 * min(errs)
+
+
+@pytest.mark.parametrize("n", [1, 3, 7, 8, 9, 63, 129, 515, 1217])
+def test_row_blocks(system, n):
+    """Row blocks on one slab of a known inverse: widths and column counts around their tiles."""
+    torch = system[0]
+    from emerge_gb300.solver import RestrictedSystem, SlabFactor
+    ip = torch.arange(0, n * n + 1, n, dtype=torch.int64, device="cuda")
+    ix = torch.arange(n, dtype=torch.int32, device="cuda").repeat(n)
+    slab = SlabFactor(RestrictedSystem(ip, ix, n * n, np.arange(n)), np.arange(n))
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    rnd = lambda *s: torch.view_as_complex(torch.randn((*s, 2), generator=gen, device="cuda", dtype=torch.float64))  # noqa: E731
+    A = [rnd(n, n) / (2 * n) ** 0.5 + 3.0 * torch.eye(n, device="cuda") for _ in range(3)]
+    slab.factor(torch.stack([a.reshape(-1) for a in A], dim=1).contiguous(), [0, 1, 2], "fp32")
+    for cols in (1, 4, 8, 9, 16, 17, 24, 31, 32, 33, 48, 49, 64):
+        for G in (1, 2, 3):
+            b = rnd(n, cols * G)
+            y = slab.apply(b, sum(([g] * cols for g in range(G)), []))
+            for g in range(G):
+                r = A[g] @ y[:, g * cols:(g + 1) * cols] - b[:, g * cols:(g + 1) * cols]
+                # inverse and product: relative errors of a few n eps, condition below 100
+                assert float(torch.linalg.norm(r)) <= 200 * n * 2.0 ** -23 * float(torch.linalg.norm(b))
