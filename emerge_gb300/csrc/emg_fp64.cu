@@ -25,6 +25,7 @@
 // chunks of N = 32 MMAs one after the other); the same tiles take 250 on the FP64 pipe.
 #include <algorithm>
 
+#include "emg_gj.cuh"
 #include "emg_krylov.cuh"
 
 namespace emg {
@@ -412,13 +413,13 @@ __global__ void __maxnreg__(200)   // 256 threads leave room on the SM for a CTA
 }
 
 // The lookahead of step k on the FP64 pipe: tile (la, la) is all that the next pivot tile waits for.
-//   part 0: rows[r][c] = sum_k P[r][k] M[k0 + k][c] in the columns of tile la
+//   part 0: rows[r][c] = sum_k P[r][k] M[k0 + k][c] in the columns of tile la (rows: work space)
 //   part 1: M[r][c] -= sum_k M[r][k0 + k] rows[k][c] on tile (la, la)
 // 128 CTAs of 8 x 4 outputs, a quarter of K per warp: 4096 cycles of an SM's FP64 pipe each.  On the
 // tensor cores one 64 x 64 tile is one or two CTAs that take as long as a full wave, 35 us for
 // the whole row panel before it and 33 for the tile, all on the chain of the pivot tiles; these
-// two launches take 4.7 us each, and the row panel runs beside the next pivot tile (a 26-slab point
-// of 311 tiles: 75 -> 55 ms).
+// two launches take 4.6 us each on the pivot tiles' stream (a 26-slab point of 311 tiles: 75 -> 55 ms
+// with the row panel after them on one stream, see fp64_step's caller for both beside each other).
 constexpr int kLookCtas = 128, kLookRows = 8, kLookCols = 4, kTileThreads = 128;
 
 __device__ __forceinline__ void cmadd(double2& s, double2 a, double2 b) {   // s += a b
@@ -428,48 +429,179 @@ __device__ __forceinline__ void cmadd(double2& s, double2 a, double2 b) {   // s
     s.y = fma(a.y, b.x, s.y);
 }
 
-__global__ void __launch_bounds__(kTileThreads) k_look64(int part, int64_t w, int k, int la, double2* __restrict__ Sinv,
-                                                         int64_t totD, int64_t offD, const double2* __restrict__ pinv,
-                                                         double2* __restrict__ rows_, int64_t sbuf) {
-    __shared__ double2 As[kLookRows][kTile + 1], Bs[kTile][kLookCols + 1], red[kTileThreads / 32][32];
+constexpr int kNewton = 3;
+constexpr float kNewtonDone = 1e-8f;
+struct NewtonWork {                    // per factor; R also holds the lookahead's row tile
+    double2 X[2][kTile * kTile], R[kTile * kTile];
+    float2 seed[kTile * kTile];
+    unsigned rmax[kNewton];            // largest |entry| of R of each step, as float bits
+    int32_t replaced;
+    unsigned pad[4];                     // a multiple of 16 bytes with the above
+};
+
+// The CTA's 8 x 4 outputs of a 64 x 64 x 64 product: a(r, kk), b(kk, c) give the operands, the sum for
+// output (lane / 4, lane % 4) is returned to warp 0.
+struct Look {
+    double2 As[kLookRows][kTile + 1], Bs[kTile][kLookCols + 1], red[kTileThreads / 32][32];
+};
+template <class FA, class FB>
+__device__ __forceinline__ double2 look_block(Look& sm, FA a, FB b) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int r0 = ((int)blockIdx.x / (kTile / kLookCols)) * kLookRows, c0 = ((int)blockIdx.x % (kTile / kLookCols)) * kLookCols;
-    const int64_t f = blockIdx.z, k0 = (int64_t)k * kTile, l0 = (int64_t)la * kTile;
-    double2* M = Sinv + f * totD + offD;
-    double2* rows = rows_ + f * sbuf;
-    const int nv = (int)min((int64_t)kTile, w - l0);   // tile k is a full one: la comes after it
-    const double2 z2 = make_double2(0.0, 0.0);
 #pragma unroll
     for (int q = 0; q < kLookRows * kTile / kTileThreads; ++q) {
-        const int i = tid + q * kTileThreads, r = i / kTile, kk = i % kTile;
-        As[r][kk] = part == 0          ? pinv[f * kTile * kTile + (r0 + r) * kTile + kk]
-                    : r0 + r < nv ? M[(l0 + r0 + r) * w + k0 + kk]
-                                       : z2;
+        const int i = tid + q * kTileThreads;
+        sm.As[i / kTile][i % kTile] = a(i / kTile, i % kTile);
     }
 #pragma unroll
     for (int q = 0; q < kLookCols * kTile / kTileThreads; ++q) {
-        const int i = tid + q * kTileThreads, kk = i / kLookCols, c = i % kLookCols;
-        const double2* src = part == 0 ? M + k0 * w : rows;
-        Bs[kk][c] = c0 + c < nv ? src[(int64_t)kk * w + l0 + c0 + c] : z2;
+        const int i = tid + q * kTileThreads;
+        sm.Bs[i / kLookCols][i % kLookCols] = b(i / kLookCols, i % kLookCols);
     }
     __syncthreads();
     const int r = lane / kLookCols, c = lane % kLookCols;
-    double2 s = z2;
+    double2 s = make_double2(0.0, 0.0);
 #pragma unroll
-    for (int kk = 0; kk < kTile / 4; ++kk) cmadd(s, As[r][warp * (kTile / 4) + kk], Bs[warp * (kTile / 4) + kk][c]);
-    red[warp][lane] = s;
+    for (int kk = 0; kk < kTile / 4; ++kk) cmadd(s, sm.As[r][warp * (kTile / 4) + kk], sm.Bs[warp * (kTile / 4) + kk][c]);
+    sm.red[warp][lane] = s;
     __syncthreads();
-    if (warp == 0 && c0 + c < nv) {
+    if (warp == 0) {
 #pragma unroll
         for (int q = 1; q < kTileThreads / 32; ++q) {
-            s.x += red[q][lane].x;
-            s.y += red[q][lane].y;
+            s.x += sm.red[q][lane].x;
+            s.y += sm.red[q][lane].y;
         }
-        if (part == 0) {
-            rows[(int64_t)(r0 + r) * w + l0 + c0 + c] = s;
-        } else if (r0 + r < nv) {
-            double2& m = M[(l0 + r0 + r) * w + l0 + c0 + c];
-            m = make_double2(m.x - s.x, m.y - s.y);
+    }
+    return s;
+}
+
+__global__ void __launch_bounds__(kTileThreads) k_look64(int part, int64_t w, int k, int la, double2* Sinv, int64_t totD,
+                                                         int64_t offD, const double2* pinv, NewtonWork* work) {
+    __shared__ Look sm;
+    const int r0 = ((int)blockIdx.x / (kTile / kLookCols)) * kLookRows, c0 = ((int)blockIdx.x % (kTile / kLookCols)) * kLookCols;
+    const int64_t f = blockIdx.z, k0 = (int64_t)k * kTile, l0 = (int64_t)la * kTile;
+    double2* M = Sinv + f * totD + offD;
+    double2* rows = work[f].R;
+    const double2* P = pinv + f * kTile * kTile;
+    const int nv = (int)min((int64_t)kTile, w - l0);   // tile k is a full one: la comes after it
+    const double2 z2 = make_double2(0.0, 0.0);
+    const double2* src = part == 0 ? M + k0 * w + l0 : rows;
+    const int64_t ld = part == 0 ? w : kTile;
+    const double2 s = look_block(
+        sm,
+        [&](int r, int kk) {
+            return part == 0 ? P[(r0 + r) * kTile + kk] : r0 + r < nv ? M[(l0 + r0 + r) * w + k0 + kk] : z2;
+        },
+        [&](int kk, int c) { return c0 + c < nv ? src[(int64_t)kk * ld + c0 + c] : z2; });
+    const int r = r0 + (int)threadIdx.x / kLookCols, c = c0 + (int)threadIdx.x % kLookCols;
+    if (threadIdx.x >= 32 || c >= nv) return;
+    if (part == 0) {
+        rows[r * kTile + c] = s;
+    } else if (r < nv) {
+        double2& m = M[(l0 + r) * w + l0 + c];
+        m = make_double2(m.x - s.x, m.y - s.y);
+    }
+}
+
+// The FP64 inverse of a pivot tile from an FP32 one.  k_seed64 inverts the tile T, scaled by a power of
+// two, in FP32 (emg_gj.cuh); then up to three Newton steps R = I - T X, X <- X + X R in FP64, 128 CTAs
+// each, square the residual: the step that meets a residual of at most 1e-8 ends with one of 1e-16,
+// the rounding of the FP64 products, which the exchange steps of k_tile64 have too, and stores the
+// result.  A tile that does not get there (a condition beyond some 1e5, a pivot to be replaced, values
+// beyond FP32, NaN) is left as it was and k_tile64 inverts it; else that returns at once.
+// A tile took 124 us in k_tile64 beside the products; the seed takes 36, a step two launches of 5.
+// The solve's error against 64 bits: geometric means over 8 to 24 frequencies of seven systems 0.43
+// to 1.2 times those of FP64 exchange steps with FMAs.
+// step ``it`` met the bound of the residual's norm (64 times its largest entry), or is too far from it
+__device__ __forceinline__ bool newton_met(const NewtonWork& nw, int it) {
+    return 64.f * __uint_as_float(nw.rmax[it]) <= kNewtonDone;
+}
+
+__device__ __forceinline__ bool newton_lost(const NewtonWork& nw, int it) {
+    return __uint_as_float(nw.rmax[it]) > (it == 0 ? 0.1f : 1e-3f);
+}
+
+__global__ void __launch_bounds__(gj::kThreads, 1) k_seed64(int64_t w, int k, const double2* Sinv, int64_t totD, int64_t offD,
+                                                            NewtonWork* work) {
+    __shared__ float2 Ts[kTile * gj::kLd];
+    __shared__ gj::PivotShared sh;
+    __shared__ int s_e;
+    const int64_t f = blockIdx.z, k0 = (int64_t)k * kTile;
+    const double2* M = Sinv + f * totD + offD + k0 * w + k0;
+    NewtonWork& nw = work[f];
+    const int tb = (int)min((int64_t)kTile, w - k0), tid = threadIdx.x;
+    constexpr int kPer = kTile * kTile / gj::kThreads;
+    if (tid == 0) s_e = 0;
+    if (tid < kNewton) nw.rmax[tid] = 0u;
+    if (tid == 0) nw.replaced = 0;
+    double2 v[kPer];
+    int e = 0;
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+        const int r = (tid + q * gj::kThreads) / kTile, c = tid % kTile;
+        v[q] = (r < tb && c < tb) ? M[(int64_t)r * w + c] : make_double2(0.0, 0.0);
+        e = max(e, max(((unsigned)__double2hiint(v[q].x) >> 20) & 0x7ffu, ((unsigned)__double2hiint(v[q].y) >> 20) & 0x7ffu));
+    }
+    e = __reduce_max_sync(0xffffffffu, e);
+    __syncthreads();
+    if ((tid & 31) == 0) atomicMax(&s_e, e);
+    __syncthreads();
+    // 2^-(s_e - 1023): entries below 2; out of a double's normal range k_tile64 takes the tile
+    const double scale = (s_e > 0 && s_e < 2045) ? __hiloint2double((2046 - s_e) << 20, 0) : 1.0;
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+        const int r = (tid + q * gj::kThreads) / kTile, c = tid % kTile;
+        Ts[r * gj::kLd + c] = (r < tb && c < tb) ? make_float2((float)(v[q].x * scale), (float)(v[q].y * scale))
+                                                 : make_float2(r == c ? 1.f : 0.f, 0.f);
+    }
+    __syncthreads();
+    gj::invert_tile(Ts, tb, 1e-6f, sh, &nw.replaced, nw.seed, kTile, nw.seed);
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+        const int i = tid + q * gj::kThreads, r = i / kTile, c = i % kTile;
+        const float2 x = nw.seed[i];
+        nw.X[0][i] = (r < tb && c < tb) ? make_double2(x.x * scale, x.y * scale) : make_double2(r == c ? 1.0 : 0.0, 0.0);
+    }
+}
+
+// Newton step ``it``: part 0 forms R, part 1 the next X (the result if R met the bound).
+__global__ void __launch_bounds__(kTileThreads) k_newton64(int part, int it, int64_t w, int k, double2* Sinv, int64_t totD,
+                                                           int64_t offD, double2* pinv, NewtonWork* work) {
+    __shared__ Look sm;
+    const int r0 = ((int)blockIdx.x / (kTile / kLookCols)) * kLookRows, c0 = ((int)blockIdx.x % (kTile / kLookCols)) * kLookCols;
+    const int64_t f = blockIdx.z, k0 = (int64_t)k * kTile;
+    double2* T = Sinv + f * totD + offD + k0 * w + k0;
+    NewtonWork& nw = work[f];
+    const int tb = (int)min((int64_t)kTile, w - k0);
+    pdl_wait();
+    pdl_trigger();                       // only now: waiting CTAs take shared memory from the products
+    for (int i = 0; i < it; ++i)
+        if (newton_met(nw, i) || newton_lost(nw, i)) return;   // done, or k_tile64's, since an earlier step
+    const double2* X = nw.X[it & 1];
+    const double2 s = look_block(
+        sm,
+        [&](int r, int kk) {
+            r += r0;
+            if (part == 1) return X[r * kTile + kk];
+            return r < tb && kk < tb ? T[(int64_t)r * w + kk] : make_double2(r == kk ? 1.0 : 0.0, 0.0);
+        },
+        [&](int kk, int c) { return (part == 0 ? X : nw.R)[kk * kTile + c0 + c]; });
+    if (threadIdx.x >= 32) return;
+    const int r = r0 + (int)threadIdx.x / kLookCols, c = c0 + (int)threadIdx.x % kLookCols;
+    if (part == 0) {
+        const double2 v = make_double2((r == c ? 1.0 : 0.0) - s.x, -s.y);
+        nw.R[r * kTile + c] = v;
+        const double m = fmax(fabs(v.x), fabs(v.y));
+        const float mf = (m <= 3e38 && v.x == v.x && v.y == v.y) ? __double2float_ru(m) : __int_as_float(0x7f800000);
+        const unsigned best = __reduce_max_sync(0xffffffffu, __float_as_uint(mf));
+        if (threadIdx.x == 0) atomicMax(&nw.rmax[it], best);
+    } else {
+        const double2 x = X[r * kTile + c], v = make_double2(x.x + s.x, x.y + s.y);
+        if (!newton_met(nw, it)) {
+            nw.X[(it + 1) & 1][r * kTile + c] = v;
+        } else if (r < tb && c < tb) {
+            T[(int64_t)r * w + c] = v;
+            pinv[(f * kTile + r) * kTile + c] = v;
         }
     }
 }
@@ -481,7 +613,8 @@ __global__ void __launch_bounds__(kTileThreads) k_look64(int part, int64_t w, in
 // them to their columns as a rank-4 product, so the 1 M FMAs of a tile are spread over 16 SMs'
 // FP64 pipes.  Pivots compare max(|re|, |im|) (14 bits of it, the lowest row on ties); a pivot of
 // |a|^2 at or below rel_thr^2 max|a|^2 is replaced by that threshold and counted.  One CTA took
-// 600 us a tile (85 % of its FP64 pipe), this 115 (124 while products run beside it).
+// 600 us a tile (85 % of its FP64 pipe), this 115 (124 while products run beside it).  It takes the
+// tiles that the Newton steps leave.
 constexpr int kRanks = 16, kPc = 4;
 
 __device__ __forceinline__ double2 remote(const double2* p, int rank) {
@@ -497,7 +630,7 @@ __device__ __forceinline__ void cluster_sync() {
 }
 __global__ void __launch_bounds__(kTileThreads) k_tile64(int64_t w, int k, double2* __restrict__ Sinv, int64_t totD,
                                                          int64_t offD, double2* __restrict__ pinv, double rel_thr,
-                                                         int32_t* __restrict__ perturbed) {
+                                                         int32_t* __restrict__ perturbed, const NewtonWork* __restrict__ work) {
     struct __align__(16) Shared {
         double2 V[kTile][kPc];                 // multipliers of this CTA's panel
         double2 row[2][kTileThreads / 32][kPc];   // candidate row of each warp
@@ -512,6 +645,10 @@ __global__ void __launch_bounds__(kTileThreads) k_tile64(int64_t w, int k, doubl
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, r = tid >> 1, h = tid & 1;
     const int rank = (int)blockIdx.x;
     const int64_t f = blockIdx.z, k0 = (int64_t)k * kTile;
+    for (int i = 0; i < kNewton; ++i) {     // uniform over the cluster
+        if (newton_lost(work[f], i)) break;
+        if (newton_met(work[f], i)) return;   // the inverse is there
+    }
     double2* M = Sinv + f * totD + offD + k0 * w + k0;
     const int tb = (int)min((int64_t)kTile, w - k0);
     double2 a[2];
@@ -666,13 +803,29 @@ __global__ void __launch_bounds__(kTileThreads) k_tile64(int64_t w, int k, doubl
 }  // namespace f64
 
 // Launch hooks (declared in emg_krylov.cuh).
+int64_t fp64_tile_work() { return sizeof(f64::NewtonWork); }
+
 int fp64_tile(int64_t w, int k, int64_t F, double2* Sinv, int64_t totD, int64_t offD, double2* pinv, double rel_thr,
-              int32_t* perturbed, cudaStream_t st) {
+              int32_t* perturbed, void* work, cudaStream_t st) {
     static bool attr = false;
     if (!attr) {
         EMG_CUDA(cudaFuncSetAttribute(f64::k_tile64, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        // they run beside k_prod64, which needs most of an SM's shared memory: another split of it would make
+        // the SM drain first
+        constexpr auto kCarve = cudaFuncAttributePreferredSharedMemoryCarveout;
+        EMG_CUDA(cudaFuncSetAttribute(f64::k_tile64, kCarve, cudaSharedmemCarveoutMaxShared));
+        EMG_CUDA(cudaFuncSetAttribute(f64::k_seed64, kCarve, cudaSharedmemCarveoutMaxShared));
+        EMG_CUDA(cudaFuncSetAttribute(f64::k_newton64, kCarve, cudaSharedmemCarveoutMaxShared));
+        EMG_CUDA(cudaFuncSetAttribute(f64::k_look64, kCarve, cudaSharedmemCarveoutMaxShared));
         attr = true;
     }
+    auto* nw = static_cast<f64::NewtonWork*>(work);
+    f64::k_seed64<<<dim3(1, 1, (unsigned)F), gj::kThreads, 0, st>>>(w, k, Sinv, totD, offD, nw);
+    EMG_CUDA(cudaGetLastError());
+    for (int it = 0; it < f64::kNewton; ++it)
+        for (int part = 0; part < 2; ++part)
+            EMG_CUDA(launch_pdl(f64::k_newton64, dim3(f64::kLookCtas, 1, (unsigned)F), dim3(f64::kTileThreads), 0, st, 0, part,
+                                it, w, k, Sinv, totD, offD, pinv, nw));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(f64::kRanks, 1, (unsigned)F);
     cfg.blockDim = dim3(f64::kTileThreads);
@@ -684,16 +837,20 @@ int fp64_tile(int64_t w, int k, int64_t F, double2* Sinv, int64_t totD, int64_t 
     la[0].val.clusterDim.z = 1;
     cfg.attrs = la;
     cfg.numAttrs = 1;
-    EMG_CUDA(cudaLaunchKernelEx(&cfg, f64::k_tile64, w, k, Sinv, totD, offD, pinv, rel_thr, perturbed));
+    EMG_CUDA(cudaLaunchKernelEx(&cfg, f64::k_tile64, w, k, Sinv, totD, offD, pinv, rel_thr, perturbed,
+                                static_cast<const f64::NewtonWork*>(nw)));
     return EMG_OK;
 }
 
 int fp64_step(int stage, int64_t w, int k, int la, int64_t F, double2* Sinv, int64_t totD, int64_t offD, const double2* pinv,
-              double2* rows, double2* cols, int64_t sbuf, int32_t* status, cudaStream_t st) {
+              double2* rows, double2* cols, int64_t sbuf, void* work, int32_t* status, cudaStream_t st) {
     static bool attr = false;
     if (!attr) {
         EMG_CUDA(cudaFuncSetAttribute(f64::k_prod64<f64::kRow>, cudaFuncAttributeMaxDynamicSharedMemorySize, f64::kSmem + 1024));
         EMG_CUDA(cudaFuncSetAttribute(f64::k_prod64<f64::kRest>, cudaFuncAttributeMaxDynamicSharedMemorySize, f64::kSmem + 1024));
+        constexpr auto kCarve = cudaFuncAttributePreferredSharedMemoryCarveout;
+        EMG_CUDA(cudaFuncSetAttribute(f64::k_prod64<f64::kRow>, kCarve, cudaSharedmemCarveoutMaxShared));
+        EMG_CUDA(cudaFuncSetAttribute(f64::k_prod64<f64::kRest>, kCarve, cudaSharedmemCarveoutMaxShared));
         attr = true;
     }
     const unsigned nct = (unsigned)((w + f64::kM - 1) / f64::kM), nrt = (unsigned)((w + f64::kN - 1) / f64::kN);
@@ -702,7 +859,8 @@ int fp64_step(int stage, int64_t w, int k, int la, int64_t F, double2* Sinv, int
     if (stage == 0)
         for (int part = 0; part < 2; ++part)
             f64::k_look64<<<dim3(f64::kLookCtas, 1, (unsigned)F), f64::kTileThreads, 0, st>>>(part, w, k, la, Sinv, totD, offD,
-                                                                                            pinv, rows, sbuf);
+                                                                                            pinv,
+                                                                                            static_cast<f64::NewtonWork*>(work));
     else if (stage == 1)
         f64::k_prod64<f64::kRow><<<dim3(2 * nct + nt, 1, (unsigned)F), f64::kThreads, sm, st>>>(
             w, k, la, Sinv, totD, offD, pinv, rows, cols, sbuf, status);

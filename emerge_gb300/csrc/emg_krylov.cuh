@@ -89,13 +89,14 @@ int tc_gj_update(int64_t w, int k, int la, int64_t F, float2* Sinv, int64_t totD
 
 // FP64 block Gauss-Jordan on the tensor cores (emg_fp64.cu).  fp64_tile: inverse of pivot tile
 // (k, k) of the F complex128 w x w blocks Sinv + f totD + offD, into M and pinv (64 x 64 per
-// factor).  fp64_step: stage 0 updates tile (la, la) by itself, stage 1 forms the row panel (``rows``,
+// factor); work: fp64_tile_work() bytes per factor.  fp64_step: stage 0 updates tile (la, la) by itself, stage 1 forms the row panel (``rows``,
 // 64 x w) and keeps the column panel (``cols``, w x 64), stage 2 updates everything else; rows and
-// cols have sbuf entries per factor.  status (device) is set to 1 if a bounded wait ran out.
+// cols have sbuf entries per factor, work as above.  status (device) is set to 1 if a bounded wait ran out.
+int64_t fp64_tile_work();
 int fp64_tile(int64_t w, int k, int64_t F, double2* Sinv, int64_t totD, int64_t offD, double2* pinv, double rel_thr,
-              int32_t* perturbed, cudaStream_t st);
+              int32_t* perturbed, void* work, cudaStream_t st);
 int fp64_step(int stage, int64_t w, int k, int la, int64_t F, double2* Sinv, int64_t totD, int64_t offD, const double2* pinv,
-              double2* rows, double2* cols, int64_t sbuf, int32_t* status, cudaStream_t st);
+              double2* rows, double2* cols, int64_t sbuf, void* work, int32_t* status, cudaStream_t st);
 
 // Preconditioner on FP32 vectors (the inner solves of the mixed-precision refinement).
 struct Precond32 {

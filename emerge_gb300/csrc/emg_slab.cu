@@ -1304,6 +1304,12 @@ int slab_factor_t(emg_slab* s, int64_t F, const int32_t* amat_h, int64_t Bm, con
         if (rc) { dfree(colbuf); slab_free_factors(s); return rc; }
     }
     struct TmpC { T *a, *b; ~TmpC() { if (a) cudaFree(a); if (b) cudaFree(b); } } tmpc{colbuf, rowbuf};
+    char* tile_work = nullptr;         // FP64 pivot tiles
+    if (sizeof(R) == 8) {
+        rc = dalloc(&tile_work, F * emg::fp64_tile_work(), "slab pivot work");
+        if (rc) { slab_free_factors(s); return rc; }
+    }
+    struct TmpW { char* a; ~TmpW() { if (a) cudaFree(a); } } tmpw{tile_work};
     // C_i S_{i-1}^-1, transposed, ``part`` rows of slab i at a time
     const int64_t part = std::min<int64_t>(s->maxw, std::max<int64_t>(64, kSchurScratch / (F * s->maxw * (int64_t)sizeof(T))));
     T* Rt = nullptr;
@@ -1342,10 +1348,11 @@ int slab_factor_t(emg_slab* s, int64_t F, const int32_t* amat_h, int64_t Bm, con
     // the side stream of the pivot-tile lookahead and its two events
     struct Side {
         cudaStream_t st = nullptr;
-        cudaEvent_t tile_ready = nullptr, diag_done = nullptr;
+        cudaEvent_t tile_ready = nullptr, diag_done = nullptr, update_done = nullptr;
         ~Side() {
             if (tile_ready) cudaEventDestroy(tile_ready);
             if (diag_done) cudaEventDestroy(diag_done);
+            if (update_done) cudaEventDestroy(update_done);
             if (st) cudaStreamDestroy(st);
         }
     } side;
@@ -1360,6 +1367,7 @@ int slab_factor_t(emg_slab* s, int64_t F, const int32_t* amat_h, int64_t Bm, con
     }
     EMG_CUDA(cudaEventCreateWithFlags(&side.tile_ready, cudaEventDisableTiming));
     EMG_CUDA(cudaEventCreateWithFlags(&side.diag_done, cudaEventDisableTiming));
+    EMG_CUDA(cudaEventCreateWithFlags(&side.update_done, cudaEventDisableTiming));
     for (int i = 0; i < s->m; ++i) {
         const int64_t w = s->off[i + 1] - s->off[i];
         if (i > 0) {
@@ -1385,7 +1393,7 @@ int slab_factor_t(emg_slab* s, int64_t F, const int32_t* amat_h, int64_t Bm, con
                 k_gj_tile32<<<dim3(1, 1, (unsigned)F), gj::kThreads, 0, ts>>>(w, k, Sinv, s->totD, s->offD[i], pset(k),
                                                                              rel_thr, s->perturbed);
             else
-                return emg::fp64_tile(w, k, F, Sinv, s->totD, s->offD[i], pset(k), rel_thr, s->perturbed, ts);
+                return emg::fp64_tile(w, k, F, Sinv, s->totD, s->offD[i], pset(k), rel_thr, s->perturbed, tile_work, ts);
             return EMG_OK;
         };
         rc = tile(0, st);
@@ -1403,49 +1411,56 @@ int slab_factor_t(emg_slab* s, int64_t F, const int32_t* amat_h, int64_t Bm, con
                     if (rc) return rc;
                 }
             }
-        } else {
-            // the lookahead tile on the side stream; step k + 1 waits for it
-            for (int k = 0; k < nt; ++k) {
-                if (k > 0) EMG_CUDA(cudaStreamWaitEvent(st, side.diag_done, 0));
-                if (nt == 1) break;
-                const T* P = pset(k);
-                const int la = k + 1 < nt ? k + 1 : -1;
-                // stage 0: tile (la, la), 1: row panel, 2: the rest (the CUDA-core lookahead reads the panel)
-                auto stage = [&](int q) -> int {
-                    if constexpr (sizeof(R) == 8) {
-                        if (tc_update)
-                            return emg::fp64_step(q, w, k, la, F, Sinv, s->totD, s->offD[i], P, rowbuf, colbuf,
-                                                  s->maxw * kTile, s->tc_status, st);
-                    }
-                    if (q == 1)
-                        k_gj_panel<R><<<dim3(nt, 1, (unsigned)F), kThreads, 0, st>>>(0, w, k, Sinv, s->totD, s->offD[i], P,
-                                                                                     -1);
-                    else if (q == 0)
-                        k_gj_panel<R><<<dim3(1, 1, (unsigned)F), kThreads, 0, st>>>(3, w, k, Sinv, s->totD, s->offD[i], P,
-                                                                                    la);
-                    else {
-                        k_gj_panel<R><<<dim3(nt, nt, (unsigned)F), kThreads, 0, st>>>(2, w, k, Sinv, s->totD, s->offD[i],
-                                                                                      P, la);
-                        k_gj_panel<R><<<dim3(nt, 1, (unsigned)F), kThreads, 0, st>>>(1, w, k, Sinv, s->totD, s->offD[i], P,
-                                                                                     -1);
-                    }
-                    return EMG_OK;
+        } else if (tc_update && nt > 1) {
+            // FP64: the pivot tiles have the side stream, row panel and update the caller's.  Tile k + 1
+            // needs tile k and the update of step k - 1; the row panel of step k needs tile k, its
+            // update overwrites what the lookahead reads.  A step is the longer of the two chains:
+            // row panel 36 us and update 37 (480 wide) to 115 (1250), or lookahead 10, seed 36 and
+            // Newton steps 25 (311 tiles of 737 on average: 42.8 ms a solve, 46.5 with the lookahead
+            // before the row panel on one stream).
+            if constexpr (sizeof(R) == 8) {
+                auto step = [&](int q, int k, int la, cudaStream_t ts) {
+                    return emg::fp64_step(q, w, k, la, F, Sinv, s->totD, s->offD[i], pset(k), rowbuf, colbuf, s->maxw * kTile,
+                                          tile_work, s->tc_status, ts);
                 };
-                rc = tc_update ? EMG_OK : stage(1);
-                if (!rc && la >= 0) {
-                    rc = stage(0);
-                    EMG_CUDA(cudaEventRecord(side.tile_ready, st));
-                    EMG_CUDA(cudaStreamWaitEvent(side.st, side.tile_ready, 0));
-                    if (!rc) rc = tile(la, side.st);
-                    EMG_CUDA(cudaEventRecord(side.diag_done, side.st));
-                }
-                if (!rc && tc_update) rc = stage(1);
-                if (!rc) rc = stage(2);
-                if (rc) {
-                    cudaDeviceSynchronize();   // the side stream and the buffers go away
-                    return rc;
+                EMG_CUDA(cudaEventRecord(side.update_done, st));
+                for (int k = 0; k < nt && !rc; ++k) {
+                    const int la = k + 1 < nt ? k + 1 : -1;
+                    if (k > 0) EMG_CUDA(cudaStreamWaitEvent(st, side.diag_done, 0));
+                    if (la >= 0) {
+                        EMG_CUDA(cudaStreamWaitEvent(side.st, side.update_done, 0));
+                        rc = step(0, k, la, side.st);
+                        EMG_CUDA(cudaEventRecord(side.tile_ready, side.st));
+                        if (!rc) rc = tile(la, side.st);
+                        EMG_CUDA(cudaEventRecord(side.diag_done, side.st));
+                    }
+                    if (!rc) rc = step(1, k, la, st);
+                    if (la >= 0) EMG_CUDA(cudaStreamWaitEvent(st, side.tile_ready, 0));
+                    if (!rc) rc = step(2, k, la, st);
+                    EMG_CUDA(cudaEventRecord(side.update_done, st));
                 }
             }
+        } else {
+            // CUDA cores: the lookahead tile on the side stream; step k + 1 waits for it
+            for (int k = 0; k < nt && nt > 1 && !rc; ++k) {
+                if (k > 0) EMG_CUDA(cudaStreamWaitEvent(st, side.diag_done, 0));
+                const T* P = pset(k);
+                const int la = k + 1 < nt ? k + 1 : -1;
+                k_gj_panel<R><<<dim3(nt, 1, (unsigned)F), kThreads, 0, st>>>(0, w, k, Sinv, s->totD, s->offD[i], P, -1);
+                if (la >= 0) {
+                    k_gj_panel<R><<<dim3(1, 1, (unsigned)F), kThreads, 0, st>>>(3, w, k, Sinv, s->totD, s->offD[i], P, la);
+                    EMG_CUDA(cudaEventRecord(side.tile_ready, st));
+                    EMG_CUDA(cudaStreamWaitEvent(side.st, side.tile_ready, 0));
+                    rc = tile(la, side.st);
+                    EMG_CUDA(cudaEventRecord(side.diag_done, side.st));
+                }
+                k_gj_panel<R><<<dim3(nt, nt, (unsigned)F), kThreads, 0, st>>>(2, w, k, Sinv, s->totD, s->offD[i], P, la);
+                k_gj_panel<R><<<dim3(nt, 1, (unsigned)F), kThreads, 0, st>>>(1, w, k, Sinv, s->totD, s->offD[i], P, -1);
+            }
+        }
+        if (rc) {
+            cudaDeviceSynchronize();   // the side stream and the buffers go away
+            return rc;
         }
         // X <- X (2I - S X): squares the residual I - S X of the inverse.  S_i's copy
         // is free once 2I - S X is formed and receives the new X.

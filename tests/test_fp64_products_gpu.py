@@ -89,3 +89,34 @@ def test_non_finite_entries_stay_visible(torch_cuda):
     slab.factor(A.reshape(-1, 1).contiguous(), [0], "fp64")
     X = slab.apply(torch.ones((n, 1), dtype=torch.complex128, device="cuda"), [0])
     assert not bool(torch.isfinite(torch.view_as_real(X)).all())
+
+
+@pytest.mark.parametrize("n", [40, 64, 130])
+@pytest.mark.parametrize("cond", [1e2, 1e4, 1e7, 1e11])
+def test_ill_conditioned_tiles(torch_cuda, n, cond):
+    """Tiles that the Newton steps from an FP32 inverse take, and those left to the exchange steps."""
+    torch = torch_cuda
+    sysr, slab = _dense_system(torch, n)
+    U, V = (torch.linalg.qr(_matrix(torch, n, s) - 3.0 * torch.eye(n, device="cuda"))[0] for s in (21, 22))
+    d = torch.logspace(0, -np.log10(cond), n, dtype=torch.float64, device="cuda")
+    A = (U * d) @ V
+    slab.factor(A.reshape(-1, 1).contiguous(), [0], "fp64")
+    X = slab.apply(torch.eye(n, dtype=torch.complex128, device="cuda"), [0] * n)
+    R = A @ X - torch.eye(n, device="cuda")
+    # pivots of a tile may be smaller than those of the whole matrix: a factor of its growth
+    assert float(torch.linalg.norm(R, ord=2)) <= 1000 * n * cond * EPS
+    assert slab.info()["perturbed_pivots"] == 0
+
+
+@pytest.mark.parametrize("n", [10, 64, 100])
+def test_zero_pivot_is_replaced(torch_cuda, n):
+    torch = torch_cuda
+    sysr, slab = _dense_system(torch, n)
+    d = torch.full((n,), 3.0 + 1.0j, dtype=torch.complex128, device="cuda")
+    d[5] = 0.0
+    slab.factor(torch.diag(d).reshape(-1, 1).contiguous(), [0], "fp64")
+    X = slab.apply(torch.eye(n, dtype=torch.complex128, device="cuda"), [0] * n)
+    assert slab.info()["perturbed_pivots"] == 1
+    keep = [i for i in range(n) if i != 5]
+    assert torch.allclose(torch.diag(X)[keep], 1.0 / d[keep], rtol=1e-14, atol=0.0)
+    assert bool(torch.isfinite(torch.view_as_real(X)).all())
