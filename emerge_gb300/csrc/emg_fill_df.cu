@@ -228,17 +228,21 @@ __global__ void k_prep2(const double* __restrict__ nodes, int64_t nN, const int3
 
 // Per fill (FP64, thread per tet): complex scales sE = mu_inv * gscale.x and
 // sB = eps * gscale.y, stored as float-float (re.h, re.l, im.h, im.l).
-// *complex_mu (when given) becomes 1 if any tet's mu^-1 has a nonzero imaginary part.
+// *complex_mu (when given) becomes 1 if any tet's mu^-1 has a nonzero imaginary part.  Runs beside
+// the last blocks of k_elem, which resets the flag.
 __global__ void k_scales(const double2* __restrict__ gscale, const double2* __restrict__ eps,
-                         const double2* __restrict__ mu_inv, int64_t nT, float4* __restrict__ tscale,
-                         int* __restrict__ complex_mu) {
+                         const double2* __restrict__ mu_inv, int64_t nT, float4* __restrict__ tscale, int* complex_mu) {
+    bool any = false;
+    pdl_trigger();
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nT; t += (int64_t)gridDim.x * blockDim.x) {
         const double2 g = gscale[t], m = mu_inv[t], e = eps[t];
         const df a = split(m.x * g.x), b = split(m.y * g.x), c = split(e.x * g.y), d = split(e.y * g.y);
         tscale[2 * t] = make_float4(a.h, a.l, b.h, b.l);
         tscale[2 * t + 1] = make_float4(c.h, c.l, d.h, d.l);
-        if (complex_mu && (b.h != 0.f || b.l != 0.f)) atomicOr(complex_mu, 1);
+        any |= b.h != 0.f || b.l != 0.f;
     }
+    pdl_wait();
+    if (complex_mu && any) atomicOr(complex_mu, 1);
 }
 
 // ------------------------------------------------------------- the blocks ---
@@ -782,6 +786,7 @@ __global__ void __launch_bounds__(kElemThreads) k_elem(const float2* __restrict_
     __shared__ float2 sinv[kInv * kElemThreads];
     __shared__ float vt[625];
     const int tid = threadIdx.x;
+    pdl_trigger();
     if (blockIdx.x == 0 && blockIdx.y == 0 && tid == 0) *complex_mu = 0;   // k_scales, launched after this, sets it
     for (int i = tid; i < 625; i += kElemThreads) vt[i] = c_vint[i];
     for (int64_t t0 = (int64_t)blockIdx.x * kElemThreads; t0 < nT; t0 += (int64_t)gridDim.x * kElemThreads) {
@@ -1081,26 +1086,27 @@ __global__ void __launch_bounds__(kFillThreads) k_fill_st(const float4* __restri
 
 // The whole owner pass of a small mesh in one launch, thread per position: up to kSmallPos positions a
 // launch costs as much as its work (360 tets: five launches 74 us a fill, three and sliced
-// element blocks 31).
+// element blocks 31, the three overlapped 27).
 constexpr int64_t kSmallPos = 152 * 4 * kFillThreads;
-__global__ void __launch_bounds__(kFillThreads) k_fill_small(const float4* __restrict__ st, int64_t n_pos,
+__global__ void __launch_bounds__(kFillThreads) k_fill_small(const float4* st, int64_t n_pos,
                                                              const uint2* __restrict__ pdesc,
                                                              const longlong2* __restrict__ rows, int64_t half,
                                                              const uint32_t* __restrict__ own_u, int64_t stride,
-                                                             const float4* __restrict__ tscale,
-                                                             const int* __restrict__ complex_mu, double2* __restrict__ E,
-                                                             double2* __restrict__ B) {
+                                                             const float4* tscale, const int* complex_mu, double2* E,
+                                                             double2* B) {
     const int64_t i = blockIdx.x * (int64_t)kFillThreads + threadIdx.x;
     if (i >= n_pos) return;
-    double2 r[4];
-    if (*complex_mu) fill_position<4, true>(st, tscale, pdesc[i], own_u, stride, nullptr, r);
-    else fill_position<3, true>(st, tscale, pdesc[i], own_u, stride, nullptr, r);
+    const uint2 d = pdesc[i];
     int64_t o1 = i, o2 = i + half;
     if (rows) {
         const longlong2 o = rows[i];
         o1 = o.x;
         o2 = o.y;
     }
+    pdl_wait();
+    double2 r[4];
+    if (*complex_mu) fill_position<4, true>(st, tscale, d, own_u, stride, nullptr, r);
+    else fill_position<3, true>(st, tscale, d, own_u, stride, nullptr, r);
     B[o1] = r[0];
     B[o2] = r[2];
     E[o1] = r[1];
@@ -1390,16 +1396,20 @@ int df_fill(const DfPlan& p, int64_t nT, const int32_t* partner, const int64_t* 
         dfk::k_elem<<<dim3(ge, gy), dfk::kElemThreads, 0, s>>>(p.inv, nT, p.st, p.mu_flag);
     }
     if (nT > 0) {
-        dfk::k_scales<<<grid_for(nT, 256), 256, 0, s>>>(p.gscale, reinterpret_cast<const double2*>(eps),
-                                                         reinterpret_cast<const double2*>(mu_inv), nT, p.tscale,
-                                                         p.mu_flag);
+        // after k_elem it may start early (what it reads was there before k_elem was launched)
+        const auto* e2 = reinterpret_cast<const double2*>(eps);
+        const auto* m2 = reinterpret_cast<const double2*>(mu_inv);
+        if (p.n_groups > 0 && p.canon)
+            EMG_CUDA(launch_pdl(dfk::k_scales, dim3(grid_for(nT, 256)), dim3(256), 0, s, 0, p.gscale, e2, m2, nT, p.tscale,
+                                p.mu_flag));
+        else
+            dfk::k_scales<<<grid_for(nT, 256), 256, 0, s>>>(p.gscale, e2, m2, nT, p.tscale, p.mu_flag);
         EMG_CUDA(cudaGetLastError());
     }
     if (p.n_groups > 0 && p.canon && p.n_pos <= dfk::kSmallPos) {
-        dfk::k_fill_small<<<grid_for(p.n_pos, dfk::kFillThreads), dfk::kFillThreads, 0, s>>>(
-            p.st, p.n_pos, p.pdesc, p.prows, p.n_pos, p.own_u, p.own_stride, p.tscale, p.mu_flag,
-            reinterpret_cast<double2*>(E), reinterpret_cast<double2*>(B));
-        EMG_CUDA(cudaGetLastError());
+        EMG_CUDA(launch_pdl(dfk::k_fill_small, dim3(grid_for(p.n_pos, dfk::kFillThreads)), dim3(dfk::kFillThreads), 0, s, 0,
+                            p.st, p.n_pos, p.pdesc, p.prows, p.n_pos, p.own_u, p.own_stride, p.tscale, p.mu_flag,
+                            reinterpret_cast<double2*>(E), reinterpret_cast<double2*>(B)));
     } else if (p.n_groups > 0 && p.canon) {
         const unsigned g = grid_for(p.n_pos, dfk::kFillThreads), go = grid_for(p.n_own, dfk::kFillThreads);
         auto* E2 = reinterpret_cast<double2*>(E);
