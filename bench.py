@@ -296,7 +296,8 @@ def run_gpu(args, rank, world):
         "parity": parity,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "peak_source": peak_kind,
-                     "kernel": "one assembly step: k_scales + k_elem + k_fill_st (+ its Im E pass, empty for real mu)",
+                     "kernel": "one assembly step: k_elem + k_scales + k_fill_own + k_fill_st (each of the last two also "
+                               "launched for complex mu, where it returns at once)",
                      "algorithmic_bytes_per_launch": int(alg_bytes), "traffic": traffic_per_launch(n),
                      # the float-float arithmetic runs on the FP32/integer pipes: its bound is the
                      # warp-instruction issue rate at the sampled SM clock
@@ -304,7 +305,7 @@ def run_gpu(args, rank, world):
                                  "floor_ms": issue_floor_ms(FILL_WARP_INST_PER_TET * nT, clk.summary()),
                                  "frac": issue_floor_ms(FILL_WARP_INST_PER_TET * nT, clk.summary())
                                  / statistics.median(launch_ms)}},
-        "gpu_launches": 4 * args.steps,
+        "gpu_launches": 6 * args.steps,   # k_elem, k_scales, k_fill_own and k_fill_st for real and for complex mu
         "clocks": clk.summary(),
     }
     if rank == 0:

@@ -18,18 +18,16 @@
 // one dense matrix x block-of-vectors product forward, the same backward:
 //     z_i = S_i^-1 (b_i - C_i z_{i-1}),   x_i = z_i - S_i^-1 U_i x_{i+1}.
 //
-// Kernels.  S_i - C_i S_{i-1}^-1 U_{i-1} is one launch per slab: a CTA owns a few
-// rows, builds R = C S^-1 for them in shared memory from coalesced rows of S^-1,
-// then multiplies by the sparse U columns.  S_i^-1 is computed in place by blocked
-// Gauss-Jordan with 64 x 64 tiles: the pivot tile is inverted by one CTA with
-// partial pivoting inside the tile (a pivot below a relative threshold is replaced
-// by the threshold and counted), the pivot row panel is multiplied by it, every
-// other tile gets a rank-64 update (the bulk of the flops: for FP32 factors on the
-// tcgen05 tensor cores with split-TF32 products, emg_tc.cu; for FP64 a tiled complex
-// GEMM on the FP64 pipes), and the pivot column panel is multiplied by minus it.  The
-// next pivot tile is updated first and inverted on a side stream while the rest of
-// the step runs (one-step lookahead).  Several factorizations (anchor frequencies) run
-// in the same launches (grid z), each with its own values.
+// Kernels.  S_i - C_i S_{i-1}^-1 U_{i-1} is two launches of k_sparse_rows.  S_i^-1 is
+// computed in place by blocked Gauss-Jordan with 64 x 64 tiles: the pivot tile is
+// inverted with partial pivoting inside the tile (a pivot below a relative threshold is
+// replaced by the threshold and counted), the pivot row panel is multiplied by it, every
+// other tile gets a rank-64 update (the bulk of the flops, on the tcgen05 tensor cores:
+// split-TF32 products in emg_tc.cu, exact FP16-digit products for FP64 in emg_fp64.cu),
+// and the pivot column panel is multiplied by minus it.  The next pivot tile is updated
+// first and inverted while the rest of the step runs (one-step lookahead).  Several
+// factorizations (anchor frequencies) run in the same launches (grid z), each with its
+// own values.
 #include <algorithm>
 #include <cmath>
 #include <vector>

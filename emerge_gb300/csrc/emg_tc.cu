@@ -1,6 +1,7 @@
 // 5th-generation tensor-core (tcgen05) kernels: a TF32 GEMM tile, the complex slab
-// product of the slab solve (TF32), and the rank-64 Gauss-Jordan update of FP32 slab
-// factorizations in split-TF32 (FP32-equivalent) precision (k_gj_update_tc, below).
+// product of the slab solve in TF32 and in split-TF32 (FP32-equivalent) precision
+// (k_slab_split), and the rank-64 Gauss-Jordan update of FP32 slab factorizations in
+// split-TF32 (k_gj_update_tc).
 //
 // GEMM tile: D[M x N] = A[M x K] B[N x K]^T (row-major FP32 in and out, TF32 products, FP32
 // accumulation in tensor memory).  One CTA of 128 threads owns a 128 x 64 tile of D:

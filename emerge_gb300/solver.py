@@ -232,13 +232,14 @@ class SlabFactor:
         _lib.call("emg_slab_set_tensor_cores", self._h, int(bool(on)))
 
     def set_factor_tensor_cores(self, on: bool = True) -> None:
-        """Run the rank-64 updates of FP32 factorizations on the tcgen05 tensor cores
-        with split-TF32 products (FP32-equivalent rounding; the default), or on the
-        CUDA cores in FP32."""
+        """Run the rank-64 products of factorizations on the tcgen05 tensor cores (the
+        default): split-TF32 in FP32 (FP32-equivalent rounding), exact FP16 digits in
+        FP64; or on the CUDA cores."""
         _lib.call("emg_slab_set_factor_tensor_cores", self._h, int(bool(on)))
 
     def set_wide_group(self, min_columns: int) -> None:
-        """Column groups of at least ``min_columns`` use the tiled dense products."""
+        """Column groups of at least ``min_columns`` use the products that share rows of
+        the inverse between columns, narrower ones rows of few columns."""
         _lib.call("emg_slab_set_wide_group", self._h, int(min_columns))
         self._wide = int(min_columns)
 
