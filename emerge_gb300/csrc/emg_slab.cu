@@ -163,11 +163,11 @@ __global__ void k_offvals(int64_t nn, int64_t Bm, int64_t F, const int32_t* __re
 // then combined in shared memory by thread per column, took 303 us (FP32, 1812 wide on average) and
 // 207 (FP64, 737 wide, where the pipe needs 150), the two launches of this 123 and 180.  Grid: column blocks x 1 x F.
 constexpr int kSpThreads = 512, kSpIn = 4;
-template <typename R, int XB>
+template <typename R, int XB, bool SUB>
 __global__ void __launch_bounds__(kSpThreads) k_sparse_rows(
     int64_t nr, int64_t nx, int64_t nj, int64_t j0, const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx,
     const typename C2<R>::T* __restrict__ val, int64_t sval, const typename C2<R>::T* __restrict__ In, int64_t ldi,
-    int64_t sIn, typename C2<R>::T* __restrict__ Out, int64_t ldo, int64_t sOut, int subtract) {
+    int64_t sIn, typename C2<R>::T* __restrict__ Out, int64_t ldo, int64_t sOut) {
     using T = typename C2<R>::T;
     constexpr int CT = XB >= 2 ? 2 : 1, LX = XB / CT;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -202,33 +202,39 @@ __global__ void __launch_bounds__(kSpThreads) k_sparse_rows(
             for (int u = 0; u < kSpIn; ++u) {
                 if (id[u] < 0) break;
 #pragma unroll
-                for (int c = 0; c < CT; ++c) cfma(acc[c], v[u], buf[id[u] * XB + xl + c]);
+                for (int c = 0; c < CT; ++c) {
+                    const T b = buf[id[u] * XB + xl + c];
+                    if (SUB) cfma(acc[c], b, v[u]);   // the factors in the order (C S^-1) U
+                    else cfma(acc[c], v[u], b);
+                }
             }
         }
 #pragma unroll
         for (int c = 0; c < CT; ++c)
             if (xl + c < nxb) {
                 T& o = Out[(x0 + xl + c) * ldo + j];
-                o = subtract ? mk(o.x - acc[c].x, o.y - acc[c].y) : acc[c];
+                o = SUB ? mk(o.x - acc[c].x, o.y - acc[c].y) : acc[c];
             }
     }
 }
 
 // Its launch: the widest column block that fits in shared memory and gives two CTAs per SM.
-template <typename R>
+template <typename R, bool SUB>
 cudaError_t sparse_rows(int64_t nr, int64_t nx, int64_t nj, int64_t j0, const int64_t* ptr, const int32_t* idx,
                         const typename C2<R>::T* val, int64_t sval, const typename C2<R>::T* In, int64_t ldi, int64_t sIn,
-                        typename C2<R>::T* Out, int64_t ldo, int64_t sOut, int subtract, int64_t F, cudaStream_t st) {
+                        typename C2<R>::T* Out, int64_t ldo, int64_t sOut, int64_t F, cudaStream_t st) {
     int xb = 8;
     while (xb > 1 && (nr * xb * (int64_t)sizeof(typename C2<R>::T) > kSchurSmem || (xb > 2 && (nx + xb - 1) / xb * F < 2 * 152)))
         xb /= 2;
-    auto kern = xb == 8 ? k_sparse_rows<R, 8> : xb == 4 ? k_sparse_rows<R, 4> : xb == 2 ? k_sparse_rows<R, 2>
-                                                                                      : k_sparse_rows<R, 1>;
+    auto kern = xb == 8   ? k_sparse_rows<R, 8, SUB>
+                : xb == 4 ? k_sparse_rows<R, 4, SUB>
+                : xb == 2 ? k_sparse_rows<R, 2, SUB>
+                          : k_sparse_rows<R, 1, SUB>;
     const size_t smem = (size_t)nr * xb * sizeof(typename C2<R>::T);
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSchurSmem);
     if (e != cudaSuccess) return e;
     kern<<<dim3((unsigned)((nx + xb - 1) / xb), 1, (unsigned)F), kSpThreads, smem, st>>>(
-        nr, nx, nj, j0, ptr, idx, val, sval, In, ldi, sIn, Out, ldo, sOut, subtract);
+        nr, nx, nj, j0, ptr, idx, val, sval, In, ldi, sIn, Out, ldo, sOut);
     return cudaGetLastError();
 }
 
@@ -1372,10 +1378,10 @@ int slab_factor_t(emg_slab* s, int64_t F, const int32_t* amat_h, int64_t Bm, con
             const int64_t wp = s->off[i] - s->off[i - 1];
             for (int64_t a0 = 0; a0 < w; a0 += part) {
                 const int64_t na = std::min(part, w - a0);
-                EMG_CUDA(sparse_rows<R>(wp, wp, na, s->off[i] + a0, s->cptr, s->cidx, static_cast<const T*>(s->Cval), s->nC,
-                                        Sinv + s->offD[i - 1], wp, s->totD, Rt, na, part * s->maxw, 0, F, st));
-                EMG_CUDA(sparse_rows<R>(wp, na, w, s->off[i], s->ucptr, s->ucrow, static_cast<const T*>(s->UCval), s->nU, Rt,
-                                        na, part * s->maxw, Sinv + s->offD[i] + a0 * w, w, s->totD, 1, F, st));
+                EMG_CUDA((sparse_rows<R, false>)(wp, wp, na, s->off[i] + a0, s->cptr, s->cidx, static_cast<const T*>(s->Cval), s->nC,
+                                        Sinv + s->offD[i - 1], wp, s->totD, Rt, na, part * s->maxw, F, st));
+                EMG_CUDA((sparse_rows<R, true>)(wp, na, w, s->off[i], s->ucptr, s->ucrow, static_cast<const T*>(s->UCval), s->nU, Rt,
+                                        na, part * s->maxw, Sinv + s->offD[i] + a0 * w, w, s->totD, F, st));
             }
         }
         const int nt = (int)((w + kTile - 1) / kTile);
