@@ -67,7 +67,9 @@ SIGNATURES = {
     "emg_rplan_pattern": (ctypes.c_int, [c_vp, c_vp, c_vp]),
     "emg_spmv_family": (ctypes.c_int, [c_vp, c_i64, ctypes.c_int, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp]),
     "emg_functionals_work": (c_i64, [c_i64, ctypes.c_int, c_i64]),
-    "emg_functionals": (ctypes.c_int, [c_i64, ctypes.c_int, c_i64, c_vp, c_vp, c_vp, c_vp, c_vp]),
+    "emg_functionals": (ctypes.c_int, [c_i64, ctypes.c_int, c_i64, c_vp, c_i64, ctypes.c_int, c_vp, c_vp, c_vp, c_vp]),
+    "emg_column_dots": (ctypes.c_int, [c_i64, c_i64, c_vp, c_vp, c_vp, c_vp, c_vp]),
+    "emg_sub_product": (ctypes.c_int, [c_i64, ctypes.c_int, c_i64, c_vp, c_i64, c_vp, c_vp, c_vp, c_vp]),
     "emg_gmres_slab_family": (ctypes.c_int, [c_vp, c_vp, c_i64, ctypes.c_int, c_vp, c_vp, c_vp, c_vp, c_vp,
                                              ctypes.c_int, ctypes.c_int, ctypes.c_double, c_vp, c_vp, c_vp]),
     "emg_gmres_slab_mixed": (ctypes.c_int, [c_vp, c_vp, c_i64, c_vp, c_i64, c_vp, c_vp, c_vp, c_vp, ctypes.c_int,

@@ -307,8 +307,8 @@ __global__ void k_spmv_fam(int64_t n, int64_t nnz, int64_t Bc, int nfam, const d
 // column walking 1024 rows left 97 blocks with one load in flight each (48 columns, 98k
 // rows, 13 vectors on average: 3553 -> 276 us a call).
 // FUN: part[blk][j][c] = sum_{rows in blk} V[r][j] W[r,c] for the nj columns of V (rows of vstride),
-// not conjugated: a few functionals of every column (the library's long-K product has one CTA
-// for them: 2590 us for 2282 unknowns and 20 columns, this below 30).
+// conjugated (2) or not (1): a few functionals of every column (the library's long-K product has one
+// CTA for them: 2590 us for 2282 unknowns and 20 columns, this below 30).
 constexpr int kDotThreads = 256, kDotJ = 4;
 constexpr int kMaxRestart = 256;
 __device__ __forceinline__ void dot_acc(double2& s, double2 v, double2 w) { cfmac(s, v, w); }
@@ -318,7 +318,7 @@ __device__ __forceinline__ void dot_acc(float2& s, float2 v, float2 w) {
     s.x = fmaf(v.y, w.y, s.x);
     s.y = fmaf(-v.y, w.x, s.y);
 }
-template <typename T, bool FUN>
+template <typename T, int FUN>
 __global__ void __launch_bounds__(kDotThreads) k_dots_partial(int64_t n, int Bc, int cw, int nj, int64_t rows,
                                                               const T* __restrict__ V, int64_t vstride,
                                                               const T* __restrict__ W, double2* __restrict__ part) {
@@ -332,7 +332,8 @@ __global__ void __launch_bounds__(kDotThreads) k_dots_partial(int64_t n, int Bc,
     if (g < groups && c < Bc) {
         const T* Vb = FUN ? V + j0 : V + j0 * vstride;
         auto acc1 = [&](int j, int64_t r, int64_t t, T w) {
-            if constexpr (FUN) cfma(acc[j], Vb[r * vstride + j], w);
+            if constexpr (FUN == 1) cfma(acc[j], Vb[r * vstride + j], w);
+            else if constexpr (FUN == 2) dot_acc(acc[j], Vb[r * vstride + j], w);
             else dot_acc(acc[j], Vb[j * vstride + t], w);
         };
         if (jn == kDotJ) {
@@ -367,6 +368,32 @@ __global__ void __launch_bounds__(kDotThreads) k_dots_partial(int64_t n, int Bc,
     __syncthreads();
     if (g == 0 && c < Bc)
         for (int j = 0; j < jn; ++j) part[((int64_t)blockIdx.x * nj + j0 + j) * Bc + c] = red[j][tid];
+}
+
+// out[r, c] = W[r, c] - sum_j V[r][j] C[j][c] (rows of V: ldv), thread per (row, column), C in shared
+// memory kSubC entries at a time.  For a basis of 40 vectors and a block of 4 the library's two
+// products took 180 us each, the dots before it and this some 60 together.
+constexpr int kSubC = 2048;
+__global__ void __launch_bounds__(256) k_sub_product(int64_t n, int nj, int Bc, const double2* __restrict__ V, int64_t ldv,
+                                                     const double2* __restrict__ C, const double2* W, double2* out) {
+    __shared__ double2 sc[kSubC];
+    const int jc = kSubC / Bc;                      // vectors a round (Bc <= kSubC)
+    const int64_t total = n * Bc, step = (int64_t)gridDim.x * blockDim.x;
+    for (int j0 = 0; j0 < nj; j0 += jc) {
+        const int jn = min(jc, nj - j0);
+        __syncthreads();
+        for (int i = threadIdx.x; i < jn * Bc; i += blockDim.x) sc[i] = C[(int64_t)j0 * Bc + i];
+        __syncthreads();
+        for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += step) {
+            const int64_t r = t / Bc;
+            const int c = (int)(t - r * Bc);
+            const double2* v = V + r * ldv + j0;
+            double2 s = j0 ? out[t] : W[t];
+#pragma unroll 4
+            for (int j = 0; j < jn; ++j) cfms(s, v[j], sc[j * Bc + c]);
+            out[t] = s;
+        }
+    }
 }
 
 // out[j][c] = sum of the nblk partials: a warp per (j, c), lanes over the blocks
@@ -933,7 +960,7 @@ void spmv(const emg_rplan* p, int64_t Bc, const int32_t* cmat, int64_t Bm, const
 // for each (fewer spend more on the reduction than on the products).
 int64_t dot_rows(int64_t n) { return std::max<int64_t>(64, (n + 2 * 152 - 1) / (2 * 152)); }
 
-template <typename T, bool FUN = false>
+template <typename T, int FUN = 0>
 void dots(int64_t n, int64_t Bc, int nj, const T* V, int64_t vstride, const T* W, double2* part, double2* out,
           cudaStream_t s) {
     const int64_t rows = dot_rows(n), nblk = (n + rows - 1) / rows;
@@ -1381,13 +1408,36 @@ extern "C" int64_t emg_functionals_work(int64_t n, int np, int64_t Bc) {
     return (n + dot_rows(n) - 1) / dot_rows(n) * np * Bc;
 }
 
-extern "C" int emg_functionals(int64_t n, int np, int64_t Bc, const double* U, const double* X, double* work, double* G,
+extern "C" int emg_functionals(int64_t n, int np, int64_t Bc, const double* U, int64_t ldu, int conj, const double* X,
+                               double* work, double* G, void* stream) {
+    using namespace emg;
+    EMG_CHECK_ARG(n > 0 && np > 0 && np <= 65535 && Bc > 0 && Bc < (1ll << 31) && ldu >= np && U && X && work && G,
+                  "emg_functionals: bad argument");
+    auto run = conj ? dots<double2, 2> : dots<double2, 1>;
+    run(n, Bc, np, reinterpret_cast<const double2*>(U), ldu, reinterpret_cast<const double2*>(X),
+        reinterpret_cast<double2*>(work), reinterpret_cast<double2*>(G), (cudaStream_t)stream);
+    EMG_CUDA(cudaGetLastError());
+    return EMG_OK;
+}
+
+extern "C" int emg_column_dots(int64_t n, int64_t Bc, const double* X, const double* Y, double* work, double* G,
                                void* stream) {
     using namespace emg;
-    EMG_CHECK_ARG(n > 0 && np > 0 && np <= 65535 && Bc > 0 && Bc < (1ll << 31) && U && X && work && G,
-                  "emg_functionals: bad argument");
-    dots<double2, true>(n, Bc, np, reinterpret_cast<const double2*>(U), np, reinterpret_cast<const double2*>(X),
-                        reinterpret_cast<double2*>(work), reinterpret_cast<double2*>(G), (cudaStream_t)stream);
+    EMG_CHECK_ARG(n > 0 && Bc > 0 && Bc < (1ll << 31) && X && Y && work && G, "emg_column_dots: bad argument");
+    dots<double2>(n, Bc, 1, reinterpret_cast<const double2*>(X), 0, reinterpret_cast<const double2*>(Y),
+                  reinterpret_cast<double2*>(work), reinterpret_cast<double2*>(G), (cudaStream_t)stream);
+    EMG_CUDA(cudaGetLastError());
+    return EMG_OK;
+}
+
+extern "C" int emg_sub_product(int64_t n, int nj, int64_t Bc, const double* V, int64_t ldv, const double* C, const double* W,
+                               double* out, void* stream) {
+    using namespace emg;
+    EMG_CHECK_ARG(n > 0 && nj > 0 && Bc > 0 && Bc <= kry::kSubC && ldv >= nj && V && C && W && out,
+                  "emg_sub_product: bad argument");
+    kry::k_sub_product<<<grid_for(n * Bc, 256), 256, 0, (cudaStream_t)stream>>>(
+        n, nj, (int)Bc, reinterpret_cast<const double2*>(V), ldv, reinterpret_cast<const double2*>(C),
+        reinterpret_cast<const double2*>(W), reinterpret_cast<double2*>(out));
     EMG_CUDA(cudaGetLastError());
     return EMG_OK;
 }

@@ -33,17 +33,44 @@ def _stream() -> ctypes.c_void_p:
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
-def functionals(U: torch.Tensor, X: torch.Tensor) -> torch.Tensor:
-    """U.T @ X (np, C) of a few functionals U (n, np) of the columns of X (n, C), complex128."""
+def _rows(V: torch.Tensor):
+    """V with contiguous rows, and their stride."""
+    if V.stride(1) != 1 or V.stride(0) < V.shape[1]:
+        V = V.contiguous()
+    return V, int(V.stride(0))
+
+
+def functionals(U: torch.Tensor, X: torch.Tensor, conj: bool = False) -> torch.Tensor:
+    """U.T @ X (U.conj().T @ X with ``conj``) (np, C) of a few functionals U (n, np) of the
+    columns of X (n, C), complex128."""
     n, npo = U.shape
     C = int(X.shape[1])
     if n == 0 or npo == 0 or C == 0 or not X.is_cuda:
-        return U.T @ X
-    U, X = U.contiguous(), X.contiguous()
+        return (U.conj() if conj else U).T @ X
+    (U, ldu), X = _rows(U), X.contiguous()
     G = torch.empty((npo, C), dtype=X.dtype, device=X.device)
     work = torch.empty(_lib.load().emg_functionals_work(n, npo, C), dtype=X.dtype, device=X.device)
-    _lib.call("emg_functionals", n, npo, C, _vp(U), _vp(X), _vp(work), _vp(G), _stream())
+    _lib.call("emg_functionals", n, npo, C, _vp(U), ldu, int(conj), _vp(X), _vp(work), _vp(G), _stream())
     return G
+
+
+def column_dots(X: torch.Tensor, Y: torch.Tensor) -> torch.Tensor:
+    """(C,) column-wise conj(X) . Y of complex128 CUDA tensors (n, C)."""
+    n, C = (int(v) for v in X.shape)
+    X, Y = X.contiguous(), Y.contiguous()
+    G = torch.empty(C, dtype=X.dtype, device=X.device)
+    work = torch.empty(_lib.load().emg_functionals_work(n, 1, C), dtype=X.dtype, device=X.device)
+    _lib.call("emg_column_dots", n, C, _vp(X), _vp(Y), _vp(work), _vp(G), _stream())
+    return G
+
+
+def sub_product(W: torch.Tensor, V: torch.Tensor, C: torch.Tensor) -> torch.Tensor:
+    """W - V @ C for V (n, m) and a block W (n, c) of complex128 CUDA tensors."""
+    (V, ldv), C, W = _rows(V), C.contiguous(), W.contiguous()
+    out = torch.empty_like(W)
+    _lib.call("emg_sub_product", int(V.shape[0]), int(V.shape[1]), int(W.shape[1]), _vp(V), ldv, _vp(C), _vp(W), _vp(out),
+              _stream())
+    return out
 
 
 class RestrictedSystem:

@@ -190,11 +190,16 @@ int emg_spmv(const emg_rplan* plan, int64_t Bc, const int32_t* cmat, int64_t Bm,
 int emg_spmv_family(const emg_rplan* plan, int64_t Bc, int nfam, const double* fam, const double* coef,
                     const double* X, const double* Bv, double* Y, void* stream);
 
-/* G [np][Bc] = U^T X (no conjugate) for a few functionals U [n][np] of the columns of X [n][Bc],
- * complex, DEVICE; work: emg_functionals_work(n, np, Bc) complex entries.  Sums in a fixed order. */
+/* G [np][Bc] = U^T X, or U^H X with conj != 0, for a few functionals U [n][np] (rows of ldu) of the
+ * columns of X [n][Bc]; G [Bc] = the column-wise conj(X) . Y; out = W - V C for V [n][nj] (rows of ldv),
+ * C [nj][Bc], W and out [n][Bc] (may be the same), Bc <= 2048.  Complex, DEVICE; work:
+ * emg_functionals_work(n, np, Bc) complex entries (np = 1 for the dots).  Sums in a fixed order. */
 int64_t emg_functionals_work(int64_t n, int np, int64_t Bc);
-int emg_functionals(int64_t n, int np, int64_t Bc, const double* U, const double* X, double* work, double* G,
-                    void* stream);
+int emg_functionals(int64_t n, int np, int64_t Bc, const double* U, int64_t ldu, int conj, const double* X,
+                    double* work, double* G, void* stream);
+int emg_column_dots(int64_t n, int64_t Bc, const double* X, const double* Y, double* work, double* G, void* stream);
+int emg_sub_product(int64_t n, int nj, int64_t Bc, const double* V, int64_t ldv, const double* C, const double* W,
+                    double* out, void* stream);
 
 /* out[i][c] = full[c][solve_ids[i]] (full: Bc vectors of N) and the inverse
  * scatter (zeros on removed DOFs). */
