@@ -55,8 +55,10 @@ def functionals(U: torch.Tensor, X: torch.Tensor, conj: bool = False) -> torch.T
 
 
 def column_dots(X: torch.Tensor, Y: torch.Tensor) -> torch.Tensor:
-    """(C,) column-wise conj(X) . Y of complex128 CUDA tensors (n, C)."""
+    """(C,) column-wise conj(X) . Y of complex128 blocks (n, C)."""
     n, C = (int(v) for v in X.shape)
+    if n == 0 or C == 0 or not X.is_cuda:
+        return (X.conj() * Y).sum(dim=0)
     X, Y = X.contiguous(), Y.contiguous()
     G = torch.empty(C, dtype=X.dtype, device=X.device)
     work = torch.empty(_lib.load().emg_functionals_work(n, 1, C), dtype=X.dtype, device=X.device)
@@ -65,7 +67,9 @@ def column_dots(X: torch.Tensor, Y: torch.Tensor) -> torch.Tensor:
 
 
 def sub_product(W: torch.Tensor, V: torch.Tensor, C: torch.Tensor) -> torch.Tensor:
-    """W - V @ C for V (n, m) and a block W (n, c) of complex128 CUDA tensors."""
+    """W - V @ C for V (n, m) and a block W (n, c), complex128."""
+    if 0 in V.shape or W.shape[1] == 0 or not W.is_cuda:
+        return W - V @ C
     (V, ldv), C, W = _rows(V), C.contiguous(), W.contiguous()
     out = torch.empty_like(W)
     _lib.call("emg_sub_product", int(V.shape[0]), int(V.shape[1]), int(W.shape[1]), _vp(V), ldv, _vp(C), _vp(W), _vp(out),
