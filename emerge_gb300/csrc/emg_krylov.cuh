@@ -81,17 +81,18 @@ int tc_slab_split(int64_t w, int64_t row0, int64_t Bc, const void* groups, int G
 // precision (split-TF32 products, FP32 accumulation; emg_tc.cu), for the F complex64 w x w
 // blocks Sinv + f totD + offD: M[r, c] -= C[r] M[k, c] and M[r, k] = -C[r] pinv with the old
 // column panel C (colbuf + f scol, rows of 64) and the row panel already formed; rows of tile
-// k keep their values.  With la >= 0 the launch's first CTA per factor forms tile (la, la)
-// and inverts it into M and pinv_next.  status (device) set to 1 if a bounded wait ran out.
+// k keep their values.  With la >= 0 the launch's first CTA per factor inverts tile (la, la)
+// (which the row panel's launch has updated) into M and pinv_next.  status (device) set to 1 if a bounded wait ran out.
 int tc_gj_update(int64_t w, int k, int la, int64_t F, float2* Sinv, int64_t totD, int64_t offD, const float2* colbuf,
                  int64_t scol, const float2* pinv, float2* pinv_next, float rel_thr, int32_t* perturbed,
                  int32_t* status, cudaStream_t st);
 
 // FP64 block Gauss-Jordan on the tensor cores (emg_fp64.cu).  fp64_tile: inverse of pivot tile
 // (k, k) of the F complex128 w x w blocks Sinv + f totD + offD, into M and pinv (64 x 64 per
-// factor); work: fp64_tile_work() bytes per factor.  fp64_step: stage 0 updates tile (la, la) by itself, stage 1 forms the row panel (``rows``,
-// 64 x w) and keeps the column panel (``cols``, w x 64), stage 2 updates everything else; rows and
-// cols have sbuf entries per factor, work as above.  status (device) is set to 1 if a bounded wait ran out.
+// factor); work: fp64_tile_work() bytes per factor.  fp64_step: stage 0 updates tile (la, la) by
+// itself, stage 1 forms the row panel (``rows``, 64 x w) and keeps the column panel (``cols``,
+// w x 64), stage 2 updates everything else; rows and cols have sbuf entries per factor, work as
+// above.  status (device) is set to 1 if a bounded wait ran out.
 int64_t fp64_tile_work();
 int fp64_tile(int64_t w, int k, int64_t F, double2* Sinv, int64_t totD, int64_t offD, double2* pinv, double rel_thr,
               int32_t* perturbed, void* work, cudaStream_t st);
