@@ -807,8 +807,10 @@ int64_t fp64_tile_work() { return sizeof(f64::NewtonWork); }
 
 int fp64_tile(int64_t w, int k, int64_t F, double2* Sinv, int64_t totD, int64_t offD, double2* pinv, double rel_thr,
               int32_t* perturbed, void* work, cudaStream_t st) {
-    static bool attr = false;
-    if (!attr) {
+    static bool attr[64] = {false};   // per device
+    int dev = 0;
+    EMG_CUDA(cudaGetDevice(&dev));
+    if (dev >= 64 || !attr[dev]) {
         EMG_CUDA(cudaFuncSetAttribute(f64::k_tile64, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         // they run beside k_prod64, which needs most of an SM's shared memory: another split of it would make
         // the SM drain first
@@ -817,7 +819,7 @@ int fp64_tile(int64_t w, int k, int64_t F, double2* Sinv, int64_t totD, int64_t 
         EMG_CUDA(cudaFuncSetAttribute(f64::k_seed64, kCarve, cudaSharedmemCarveoutMaxShared));
         EMG_CUDA(cudaFuncSetAttribute(f64::k_newton64, kCarve, cudaSharedmemCarveoutMaxShared));
         EMG_CUDA(cudaFuncSetAttribute(f64::k_look64, kCarve, cudaSharedmemCarveoutMaxShared));
-        attr = true;
+        if (dev < 64) attr[dev] = true;
     }
     auto* nw = static_cast<f64::NewtonWork*>(work);
     f64::k_seed64<<<dim3(1, 1, (unsigned)F), gj::kThreads, 0, st>>>(w, k, Sinv, totD, offD, nw);
@@ -844,14 +846,16 @@ int fp64_tile(int64_t w, int k, int64_t F, double2* Sinv, int64_t totD, int64_t 
 
 int fp64_step(int stage, int64_t w, int k, int la, int64_t F, double2* Sinv, int64_t totD, int64_t offD, const double2* pinv,
               double2* rows, double2* cols, int64_t sbuf, void* work, int32_t* status, cudaStream_t st) {
-    static bool attr = false;
-    if (!attr) {
+    static bool attr[64] = {false};   // per device
+    int dev = 0;
+    EMG_CUDA(cudaGetDevice(&dev));
+    if (dev >= 64 || !attr[dev]) {
         EMG_CUDA(cudaFuncSetAttribute(f64::k_prod64<f64::kRow>, cudaFuncAttributeMaxDynamicSharedMemorySize, f64::kSmem + 1024));
         EMG_CUDA(cudaFuncSetAttribute(f64::k_prod64<f64::kRest>, cudaFuncAttributeMaxDynamicSharedMemorySize, f64::kSmem + 1024));
         constexpr auto kCarve = cudaFuncAttributePreferredSharedMemoryCarveout;
         EMG_CUDA(cudaFuncSetAttribute(f64::k_prod64<f64::kRow>, kCarve, cudaSharedmemCarveoutMaxShared));
         EMG_CUDA(cudaFuncSetAttribute(f64::k_prod64<f64::kRest>, kCarve, cudaSharedmemCarveoutMaxShared));
-        attr = true;
+        if (dev < 64) attr[dev] = true;
     }
     const unsigned nct = (unsigned)((w + f64::kM - 1) / f64::kM), nrt = (unsigned)((w + f64::kN - 1) / f64::kN);
     const unsigned nt = (unsigned)((w + f64::kTile - 1) / f64::kTile);

@@ -1054,10 +1054,12 @@ namespace emg {
 int tc_slab_product(int64_t w, int64_t row0, int64_t Bc, const void* groups, int G, int maxcol, const float2* Sinv,
                     int64_t totD, int64_t offD, const float2* Y, float alpha, int beta, float2* Out, int32_t* status,
                     cudaStream_t st) {
-    static bool attr = false;
-    if (!attr) {
+    static bool attr[64] = {false};   // per device
+    int dev = 0;
+    EMG_CUDA(cudaGetDevice(&dev));
+    if (dev >= 64 || !attr[dev]) {
         EMG_CUDA(cudaFuncSetAttribute(tc::k_cgemm_tf32, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::kCxSmem + 1024));
-        attr = true;
+        if (dev < 64) attr[dev] = true;
     }
     const dim3 grid((unsigned)((maxcol + tc::kN - 1) / tc::kN), (unsigned)((w + tc::kM - 1) / tc::kM), (unsigned)G);
     tc::k_cgemm_tf32<<<grid, tc::kThreads, tc::kCxSmem + 1024, st>>>(
@@ -1072,10 +1074,12 @@ namespace emg {
 int tc_slab_split(int64_t w, int64_t row0, int64_t Bc, const void* groups, int G, int maxcol, int max_splits,
                   const float2* Sinv, int64_t totD, int64_t offD, const float2* Y, float alpha, int beta, float2* Out,
                   int32_t* status, cudaStream_t st) {
-    static bool attr = false;
-    if (!attr) {
+    static bool attr[64] = {false};   // per device
+    int dev = 0;
+    EMG_CUDA(cudaGetDevice(&dev));
+    if (dev >= 64 || !attr[dev]) {
         EMG_CUDA(cudaFuncSetAttribute(tc::k_slab_split, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::kSpSmem + 1024));
-        attr = true;
+        if (dev < 64) attr[dev] = true;
     }
     const int ct = (maxcol + tc::kN - 1) / tc::kN, rt = (int)((w + tc::kM - 1) / tc::kM);
     // K split: double it while the CTAs fit one wave and each keeps two chunks
@@ -1105,11 +1109,13 @@ namespace emg {
 int tc_gj_update(int64_t w, int k, int la, int64_t F, float2* Sinv, int64_t totD, int64_t offD, const float2* colbuf,
                  int64_t scol, const float2* pinv, float2* pinv_next, float rel_thr, int32_t* perturbed,
                  int32_t* status, cudaStream_t st) {
-    static bool attr = false;
-    if (!attr) {
+    static bool attr[64] = {false};   // per device
+    int dev = 0;
+    EMG_CUDA(cudaGetDevice(&dev));
+    if (dev >= 64 || !attr[dev]) {
         EMG_CUDA(cudaFuncSetAttribute(tc::k_gj_update_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       tc::kUpdSmem + 1024));
-        attr = true;
+        if (dev < 64) attr[dev] = true;
     }
     const int64_t tiles = ((w + tc::kUpdN - 1) / tc::kUpdN) * ((w + tc::kUpdM - 1) / tc::kUpdM);
     EMG_CUDA(launch_pdl(tc::k_gj_update_tc, dim3((unsigned)(1 + tiles), 1, (unsigned)F), dim3(tc::kUpdThreads),
