@@ -187,10 +187,10 @@ def run_reference(args, rank, world):
 # material scaling and accumulation (36 ee x 40 + 48 ef/fe x 73 + 16 ff x 129 + 100 x 36)
 FP64_TFLOPS = 1.18         # GB300 FP64 FMA throughput measured by a probe kernel (DFMA chain)
 FP32_TFLOPS = 74.8         # GB300 FP32 FMA throughput measured by a probe kernel
-# warp instructions per tet of one fill (k_elem 1274 + k_fill_st 3570), from the ncu
-# capture summarised in profiles/k_elem_k_fill_st_cube40.md; the fill runs on the FP32 and
+# warp instructions per tet of one fill (k_elem 1280 + k_fill_own 50 + k_fill_st 1387), from the
+# ncu capture summarised in profiles/fill_cube40.md; the fill runs on the FP32 and
 # integer pipes, so its compute bound is the issue rate of 152 SMs x 4 schedulers
-FILL_WARP_INST_PER_TET = 4844
+FILL_WARP_INST_PER_TET = 2717
 
 
 def run_gpu(args, rank, world):
