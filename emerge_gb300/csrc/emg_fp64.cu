@@ -4,25 +4,31 @@
 // GB300's FP64 pipe does two FMAs per SM and clock: one 64 x 64 x 64 complex product takes
 // 253 us of one SM, and a factorization spends all its time there.
 //
-// Products (k_prod64).  Both operands are first scaled along K by powers of two that bring the
-// largest entry of the tile's rows to one at every K, so that a badly scaled unknown costs no
-// digits; then every operand row is scaled by the power of two above its largest entry and its
-// entries are written as seven balanced radix-512 digits, 62 bits below that power (an FP64
-// significand has 53): x = 2^E sum_i d_i 2^-(8 + 9 i), |d_i| <= 256.  Digits are exact in FP16,
-// a digit product and its sum over K = 64 are integers below 2^24, and the FP32 accumulators of
-// tcgen05.mma kind::f16 hold them exactly.  The 28 digit pairs with i + j <= 6 go to seven
-// accumulators by weight (the dropped ones are below 2^-60 of the row maxima's product), which
-// the epilogue adds as one 64-bit integer and rounds once to FP64: the product is
-// closer to exact than a chain of 64 FP64 FMAs.  A row that holds a non-finite value gives NaN.
+// Products (k_prod64), from integer digit slices on a matrix unit (the scheme of Ozaki, Ogita, Oishi
+// and Rump, "Error-free transformations of matrix multiplication", 2012).  Both operands are first
+// scaled along K by powers of two that bring the largest entry of the tile's rows to one at every K, so
+// that a badly scaled unknown costs no digits; then every operand row is scaled by the power of two
+// above its largest entry and its entries are written as eight balanced radix-256 digits, 62 bits
+// below that power: x = 2^E sum_i d_i 2^-(6 + 8 i), |d_0| <= 64, |d_i| <= 128.  Digits are
+// exact in FP16.  The 36 digit pairs with i + j <= 7 go to eight accumulators by weight.  Over K = 64 and
+// both parts of a complex operand a pair sums to at most 128 2^14 = 2^21 (half of it with one d_0), so
+// accumulator s holds integers up to 2^21 max(s, 1/4) <= 7 2^21 < 2^24, exact in FP32 for every
+// operand (seven radix-512 digits pass 2^24 for rows of nearly equal values).  The epilogue adds them as one
+// 64-bit integer and rounds once to FP64.  What is left out, relative to the product of the scaled
+// row maxima: the pairs with i + j >= 8, below 2^-52.1 at worst (2^-58 for random digits), the bits of the operands
+// beyond their 62, below 2^-54, and those of the sum beyond 2^-55.  The bound is normwise: a product of
+// small entries of rows with large ones keeps fewer bits than an FP64 chain of its own; normwise the product
+// is closer to exact than a chain of 64 FP64 FMAs (1.0 against 3.4 half-eps for random operands, 2.0 against
+// 3.8 for entries spread over six decades).  A row that holds a non-finite value gives NaN.
 //
 // One CTA forms a 128 (matrix columns, MMA rows) x 32 (matrix rows) tile, so that the lanes of a
 // warp read and write consecutive entries of a matrix row.  Four 16-deep K chunks through two
-// shared buffers (84 KB each, canonical K-major layout): all threads split the next chunk of
+// shared buffers (96 KB each, canonical K-major layout): all threads split the next chunk of
 // both operands while the MMAs of the last run.  The 32 rows enter as N = 64, [Re | Im] for the
 // real plane of the columns and [-Im | Re] for the imaginary one, so that one MMA (M = 128, N = 64,
-// K = 16) serves both parts of the result: 56 per chunk, 448 of 512 TMEM columns.  A launch of one
-// wave takes 36 us, bound by the integer work of the split and the epilogue (46 with two 32-deep
-// chunks of N = 32 MMAs one after the other); the same tiles take 250 on the FP64 pipe.
+// K = 16) serves both parts of the result: 72 per chunk, all 512 TMEM columns.  A launch of one
+// wave takes 37 us, bound by the integer work of the split and the epilogue (36 with seven digits in 84
+// KB, 46 with two 32-deep chunks of N = 32 MMAs one after the other); the same tiles take 250 on the FP64 pipe.
 #include <algorithm>
 
 #include "emg_gj.cuh"
@@ -31,9 +37,9 @@
 namespace emg {
 namespace f64 {
 
-constexpr int kM = 128, kN = 32, kKc = 16, kTile = 64, kThreads = 256, kDig = 7;
+constexpr int kM = 128, kN = 32, kKc = 16, kTile = 64, kThreads = 256, kDig = 8;
 constexpr int kAPlane = kM * kKc * 2, kBPlane = 2 * kN * kKc * 2;   // one digit of one plane: 4 KB / 2 KB
-constexpr int kBuf = 2 * kDig * (kAPlane + kBPlane);                // a chunk: 84 KB
+constexpr int kBuf = 2 * kDig * (kAPlane + kBPlane);                // a chunk: 96 KB
 constexpr int kSmem = 2 * kBuf;
 constexpr uint32_t kTmemCols = 512;
 constexpr int kNone = -(1 << 16);                                   // exponent of a zero row
@@ -72,27 +78,25 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t phase) {
 __device__ __forceinline__ int expo(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }   // biased exponent
 
 // x = t 2^(e - 1022) with |t| < 1 for biased exponents up to e (no entry is above its row's e): t 2^62 plus the bias that makes
-// every digit non-negative (256 in each of the seven 9-bit fields).
+// every digit non-negative (128 in each of the eight bytes; the sum lies between 2^62 and 2^63 + 2^63).
 __device__ __forceinline__ uint64_t fixed62(double x, int e) {
-    constexpr uint64_t kBias = 256ull * ((1ull << 0) + (1ull << 9) + (1ull << 18) + (1ull << 27) + (1ull << 36) + (1ull << 45) +
-                                         (1ull << 54));
+    constexpr uint64_t kBias = 0x8080808080808080ull;
     const int hi = __double2hiint(x), ex = (hi >> 20) & 0x7ff;
     uint64_t m = ((uint64_t)((hi & 0xfffff) | 0x100000) << 32) | (uint32_t)__double2loint(x);
     const int sh = 9 - (e - ex);
     m = ex == 0 || sh <= -53 ? 0ull : sh >= 0 ? m << sh : m >> -sh;
     return kBias + (hi < 0 ? 0ull - m : m);
 }
-// digit i of two such values as a pair of FP16: the field u in 1024 + u, minus 1280
+// digit i of two such values as a pair of FP16: byte u of 1024 + u, minus 1152
 template <int I>
 __device__ __forceinline__ uint32_t digit2(uint64_t a, uint64_t b) {
-    constexpr int s = 9 * (6 - I);
-    const uint32_t ua = I == 0 ? (uint32_t)(a >> s) : (uint32_t)(a >> s) & 511u;
-    const uint32_t ub = I == 0 ? (uint32_t)(b >> s) : (uint32_t)(b >> s) & 511u;
+    constexpr uint32_t n = 3 - (I & 3), sel = n | n << 4 | (n + 4) << 8 | (n + 4) << 12;
+    const uint32_t u = __byte_perm((uint32_t)(a >> (I < 4 ? 32 : 0)), (uint32_t)(b >> (I < 4 ? 32 : 0)), sel);
     uint32_t r;
-    asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"((ua | (ub << 16)) + 0x64006400u), "r"(0x65006500u));
+    asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"((u & 0x00ff00ffu) | 0x64006400u), "r"(0x64806480u));
     return r;
 }
-// the seven digits of eight K-adjacent values (K entry j relative to exponent e + sgn es[j]): one
+// the eight digits of eight K-adjacent values (K entry j relative to exponent e + sgn es[j]): one
 // core-matrix row (16 bytes) per digit plane, and its negative or itself in a second place
 template <bool TWO>
 __device__ __forceinline__ void put_digits(const double (&v)[8], int e, const int* es, int sgn, char* dst, int plane,
@@ -108,18 +112,17 @@ __device__ __forceinline__ void put_digits(const double (&v)[8], int e, const in
         if (TWO)                                                                                                  \
             *reinterpret_cast<uint4*>(dst2 + (I) * plane) = make_uint4(x.x ^ flip, x.y ^ flip, x.z ^ flip, x.w ^ flip); \
     }
-    EMG_PUT(0) EMG_PUT(1) EMG_PUT(2) EMG_PUT(3) EMG_PUT(4) EMG_PUT(5) EMG_PUT(6)
+    EMG_PUT(0) EMG_PUT(1) EMG_PUT(2) EMG_PUT(3) EMG_PUT(4) EMG_PUT(5) EMG_PUT(6) EMG_PUT(7)
 #undef EMG_PUT
 }
 
-// sum_s S_s 2^-(16 + 9 s) times 2^E, rounded once.  The S_s are integers of magnitude up to 2^25.
+// sum_s S_s 2^-(12 + 8 s) times 2^E, rounded once.  The S_s are integers, |S_s| <= 2^21 max(s, 1/4).
 __device__ __forceinline__ double combine(const float (&S)[kDig], int E) {
     const int i0 = __float2int_rn(S[0]), i1 = __float2int_rn(S[1]), i2 = __float2int_rn(S[2]), i3 = __float2int_rn(S[3]);
-    const int i4 = __float2int_rn(S[4]), i5 = __float2int_rn(fmaf(S[6], 0x1p-15f, S[5] * 0x1p-6f));
-    long long T = ((long long)i0 * 512 + i1) << 30;   // units of 2^-55
-    T += (long long)i2 * (1 << 21);
-    T += (long long)i3 * (1 << 12);
-    T += (long long)i4 * 8 + i5;
+    const int i4 = __float2int_rn(S[4]), i5 = __float2int_rn(S[5]), lo = __float2int_rn(fmaf(S[7], 0x1p-13f, S[6] * 0x1p-5f));
+    long long T = (long long)(i0 * 256 + i1) << 35;   // units of 2^-55
+    T += (long long)(i2 * 256 + i3) << 19;
+    T += (long long)i4 * 2048 + (i5 * 8 + lo);
     unsigned long long a = T < 0 ? 0ull - (unsigned long long)T : (unsigned long long)T;
     if (a == 0 || E < -4000) return 0.0;   // (a zero row)
     const int lz = __clzll((long long)a);

@@ -23,7 +23,7 @@
 // inverted with partial pivoting inside the tile (a pivot below a relative threshold is
 // replaced by the threshold and counted), the pivot row panel is multiplied by it, every
 // other tile gets a rank-64 update (the bulk of the flops, on the tcgen05 tensor cores:
-// split-TF32 products in emg_tc.cu, exact FP16-digit products for FP64 in emg_fp64.cu),
+// split-TF32 products in emg_tc.cu, FP16-digit products for FP64 in emg_fp64.cu),
 // and the pivot column panel is multiplied by minus it.  The next pivot tile is updated
 // first and inverted while the rest of the step runs (one-step lookahead).  Several
 // factorizations (anchor frequencies) run in the same launches (grid z), each with its

@@ -264,8 +264,8 @@ class SlabFactor:
 
     def set_factor_tensor_cores(self, on: bool = True) -> None:
         """Run the rank-64 products of factorizations on the tcgen05 tensor cores (the
-        default): split-TF32 in FP32 (FP32-equivalent rounding), exact FP16 digits in
-        FP64; or on the CUDA cores."""
+        default): split-TF32 in FP32 (FP32-equivalent rounding), FP16 digits with exact
+        sums in FP64 (normwise as accurate as FP64 chains); or on the CUDA cores."""
         _lib.call("emg_slab_set_factor_tensor_cores", self._h, int(bool(on)))
 
     def set_wide_group(self, min_columns: int) -> None:

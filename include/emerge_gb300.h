@@ -287,7 +287,8 @@ int emg_slab_set_tensor_cores(emg_slab* slab, int on);
 /* on != 0 (default): the rank-64 products of factorizations (emg_slab_factor) run on
  * the tcgen05 tensor cores: precision 1 with split-TF32 products (all four terms of
  * x = hi + lo) and FP32 accumulation, i.e. FP32-equivalent rounding, precision 2 with
- * exact FP16-digit products rounded once to FP64; off: CUDA cores.  A tensor-core
+ * FP16-digit products with exact sums, rounded once to FP64 (as close to the product as FP64
+ * chains normwise, i.e. against the scaled row maxima); off: CUDA cores.  A tensor-core
  * tile whose bounded wait runs out makes emg_slab_factor return EMG_ERR_CUDA with the
  * factors released.  (Replaces nothing in the reference: part of the GPU solver
  * behind fem/solver.py's solve slot.) */

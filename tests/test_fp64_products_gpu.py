@@ -120,3 +120,31 @@ def test_zero_pivot_is_replaced(torch_cuda, n):
     keep = [i for i in range(n) if i != 5]
     assert torch.allclose(torch.diag(X)[keep], 1.0 / d[keep], rtol=1e-14, atol=0.0)
     assert bool(torch.isfinite(torch.view_as_real(X)).all())
+
+
+def _product_of(torch, B, C, tensor_cores):
+    """B C by a factorization: the inverse of [[1, B, 0], [0, 1, C], [0, 0, 1]] holds it."""
+    n = 192
+    M = torch.eye(n, dtype=torch.complex128)
+    M[:64, 64:128], M[64:128, 128:] = torch.as_tensor(B), torch.as_tensor(C)
+    _, slab = _dense_system(torch, n)
+    slab.set_factor_tensor_cores(tensor_cores)
+    slab.factor(M.cuda().reshape(-1, 1).contiguous(), [0], "fp64")
+    return slab.apply(torch.eye(n, dtype=torch.complex128, device="cuda"), [0] * n).cpu().numpy()[:64, 128:]
+
+
+@pytest.mark.parametrize("tensor_cores", [True, False])
+@pytest.mark.parametrize("spread", [0.0, 2.0 ** -40, 2.0 ** -30, 2.0 ** -21, 2.0 ** -12])
+def test_repeated_values(torch_cuda, tensor_cores, spread):
+    """Products of rows and columns of one value each, or of values that differ in their low digits
+    only: no digit sum may leave the integers that an accumulator holds."""
+    torch = torch_cuda
+    rng = np.random.default_rng(3)
+    c = np.r_[0.92371687, 1.0 - 2.0 ** -30, rng.uniform(0.5, 1.0, 62)]
+    vary = lambda: 1.0 + spread * rng.uniform(-1.0, 1.0, (64, 64))  # noqa: E731
+    B = c[:, None] * vary() + 1j * c[:, None] * vary()
+    C = c[None, :] * vary() + 1j * c[None, :] * vary()
+    X = _product_of(torch, B, C, tensor_cores)
+    wide = lambda a: a.astype(np.clongdouble)  # noqa: E731
+    # a chain of 64 complex products of four roundings: at most 130 of half an eps each (and one for the result)
+    assert np.all(np.abs(X - wide(B) @ wide(C)) <= 131 * EPS / 2 * (np.abs(B) @ np.abs(C)))
