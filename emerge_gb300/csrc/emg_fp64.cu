@@ -717,18 +717,12 @@ __global__ void __launch_bounds__(kTileThreads) k_tile64(int64_t w, int k, doubl
                     g = make_double2(thr2 > 0.0 ? sqrt(thr2) : 1.0, 0.0);
                     d = g.x * g.x;
                 }
-                // 1 / d: the approximate reciprocal and one cubic step, e <- 1 - d y, y (1 + e + e^2)
-                double y;
-                asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-                const double er = fma(-d, y, 1.0);
-                // the multiplier f = a_rc / g = a_rc conj(g) / |g|^2, -1 / g in the pivot row: one part per
-                // thread of the row; a_rc conj(g) does not wait for the reciprocal
+                // the multiplier f = a_rc / g, -1 / g in the pivot row: one part per thread of the row
+                const double y = __drcp_rn(d), ix = g.x * y, iy = -g.y * y;
                 const bool own = r == p;
                 used |= own;
                 const double mx_ = own ? -1.0 : m.x, my_ = own ? 0.0 : m.y;
-                const double t = fma(h ? my_ : mx_, g.x, (h ? -mx_ : my_) * g.y);
-                y = fma(y, fma(er, er, er), y);
-                const double fp = t * y, fo = __shfl_xor_sync(0xffffffffu, fp, 1);
+                const double fp = fma(h ? my_ : mx_, ix, (h ? mx_ : -my_) * iy), fo = __shfl_xor_sync(0xffffffffu, fp, 1);
                 const double2 fn = h ? make_double2(-fo, -fp) : make_double2(-fp, -fo);
                 double2 b0 = own ? make_double2(0.0, 0.0) : a[0], b1 = own ? make_double2(0.0, 0.0) : a[1];
                 cmadd(b0, fn, pr0);

@@ -148,3 +148,28 @@ def test_repeated_values(torch_cuda, tensor_cores, spread):
     wide = lambda a: a.astype(np.clongdouble)  # noqa: E731
     # a chain of 64 complex products of four roundings: at most 130 of half an eps each (and one for the result)
     assert np.all(np.abs(X - wide(B) @ wide(C)) <= 131 * EPS / 2 * (np.abs(B) @ np.abs(C)))
+
+
+@pytest.mark.parametrize("scale", [9e-155, 1.0, 1.2e154])
+def test_pivots_at_the_ends_of_the_range(torch_cuda, scale):
+    """Tiles for the exchange steps (one zero pivot, one pair that is singular in FP32) whose squared
+    pivots are subnormal or have a subnormal reciprocal."""
+    torch = torch_cuda
+    n = 40
+    sysr, slab = _dense_system(torch, n)
+    A = np.eye(n) + 0.01 * np.random.default_rng(4).uniform(-1, 1, (n, n))
+    A[5], A[:, 5] = 0.0, 0.0
+    keep = np.delete(np.arange(n), 5)
+    if scale >= 1.0:
+        A[[7, 8]], A[:, [7, 8]] = 0.0, 0.0
+        A[7:9, 7:9] = [[1.0, 1.0], [1.0, 1.0 + 2.0 ** -24]]
+    slab.factor(torch.as_tensor(scale * A + 0j, device="cuda").reshape(-1, 1).contiguous(), [0], "fp64")
+    X = slab.apply(torch.eye(n, dtype=torch.complex128, device="cuda"), [0] * n).cpu().numpy()
+    assert slab.info()["perturbed_pivots"] == 1
+    K = A[np.ix_(keep, keep)]
+    Y, apart = scale * X[np.ix_(keep, keep)], np.isin(keep, (7, 8)) & (scale >= 1.0)
+    ref = np.linalg.inv(K)
+    # without the pair, whose rows and columns are apart: condition below 3, a subnormal |pivot|^2 has 50 bits
+    assert np.all(np.abs(Y - ref)[~apart] <= 64 * n * EPS * np.max(np.abs(ref), axis=1)[~apart, None])
+    # the pair, condition 2^26: the residual of each entry against the magnitudes of its products
+    assert np.all(np.abs(K @ Y - np.eye(n - 1)) <= 64 * n * EPS * (np.abs(K) @ np.abs(Y)) + 64 * n * EPS)
