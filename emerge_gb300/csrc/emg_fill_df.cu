@@ -996,13 +996,23 @@ __device__ __forceinline__ double sum_double(float s, float e) {
     return __longlong_as_double((long long)((v + (unsigned long long)(long long)t) | ((unsigned long long)(hb & 0x80000000u) << 32)));
 }
 
+// How the owner pass loads the staging buffer and the scales: read-only where the launches that write
+// them are complete before it starts, ordinary loads, which stay behind pdl_wait, where it starts under them.
+struct ReadOnly {
+    const float4* p;
+    __device__ __forceinline__ float4 operator[](int64_t i) const { return __ldg(p + i); }
+};
+struct Plain {
+    const float4* p;
+    __device__ __forceinline__ float4 operator[](int64_t i) const { return p[i]; }
+};
+
 // the products of staged unit u with its tet's scales: Re B, Im B, Re E and (IM) Im E of both rows
-template <int NC>
-__device__ __forceinline__ void unit_products(const float4* __restrict__ st, const float4* __restrict__ tscale, uint32_t u,
-                                              acc2 (&r)[NC]) {
+template <int NC, class L>
+__device__ __forceinline__ void unit_products(L st, L tscale, uint32_t u, acc2 (&r)[NC]) {
     const int64_t t = (int64_t)(u / (200u * kStBlk)) * kStBlk + u % kStBlk;
-    const float4 d = __ldg(st + 2 * (int64_t)u), f = __ldg(st + 2 * (int64_t)u + 1);
-    const float4 ce = __ldg(tscale + 2 * t), cb = __ldg(tscale + 2 * t + 1);
+    const float4 d = st[2 * (int64_t)u], f = st[2 * (int64_t)u + 1];
+    const float4 ce = tscale[2 * t], cb = tscale[2 * t + 1];
     const unsigned long long dh = pk(d.x, d.y), dl = pk(d.z, d.w), fh = pk(f.x, f.y), fl = pk(f.z, f.w);
     r[0] = prod2(cb.x, cb.y, fh, fl);
     r[1] = prod2(cb.z, cb.w, fh, fl);
@@ -1025,25 +1035,24 @@ __device__ __forceinline__ void to_rows(const acc2 (&a)[NC], double2 (&r)[4]) { 
 
 constexpr int kFillThreads = 256;
 // both rows of position i: its one or two units, or (own column) the sum of k_fill_own
-template <int NC, bool INLINE>
-__device__ __forceinline__ void fill_position(const float4* __restrict__ st, const float4* __restrict__ tscale, uint2 u,
-                                              const uint32_t* __restrict__ own_u, int64_t stride,
-                                              const double2* __restrict__ own_r, double2 (&r)[4]) {
+template <int NC, bool INLINE, class L>
+__device__ __forceinline__ void fill_position(L st, L tscale, uint2 u, const uint32_t* own_u, int64_t stride,
+                                              const double2* own_r, double2 (&r)[4]) {
     acc2 a[NC], b[NC];
     if (u.x != kNoUnit) {
-        unit_products<NC>(st, tscale, u.x, a);
+        unit_products(st, tscale, u.x, a);
         if (u.y != kNoUnit) {
-            unit_products<NC>(st, tscale, u.y, b);
+            unit_products(st, tscale, u.y, b);
 #pragma unroll
             for (int c = 0; c < NC; ++c) add_to(a[c], b[c]);
         }
         to_rows<NC>(a, r);
     } else if (INLINE) {
-        unit_products<NC>(st, tscale, own_u[u.y], a);
+        unit_products(st, tscale, own_u[u.y], a);
         for (int q = 1; q < kKmax; ++q) {
             const uint32_t v = own_u[q * stride + u.y];
             if (v == kNoUnit) break;
-            unit_products<NC>(st, tscale, v, b);
+            unit_products(st, tscale, v, b);
 #pragma unroll
             for (int c = 0; c < NC; ++c) add_to(a[c], b[c]);
         }
@@ -1070,7 +1079,7 @@ __global__ void __launch_bounds__(kFillThreads) k_fill_st(const float4* __restri
         const uint2 u = next;
         if (i + step < n_pos) next = pdesc[i + step];
         double2 r[4];
-        fill_position<IM ? 4 : 3, false>(st, tscale, u, nullptr, 0, own_r, r);
+        fill_position<IM ? 4 : 3, false>(ReadOnly{st}, ReadOnly{tscale}, u, nullptr, 0, own_r, r);
         int64_t o1 = i, o2 = i + half;
         if (rows) {
             const longlong2 o = rows[i];
@@ -1105,8 +1114,8 @@ __global__ void __launch_bounds__(kFillThreads) k_fill_small(const float4* st, i
     }
     pdl_wait();
     double2 r[4];
-    if (*complex_mu) fill_position<4, true>(st, tscale, d, own_u, stride, nullptr, r);
-    else fill_position<3, true>(st, tscale, d, own_u, stride, nullptr, r);
+    if (*complex_mu) fill_position<4, true>(Plain{st}, Plain{tscale}, d, own_u, stride, nullptr, r);
+    else fill_position<3, true>(Plain{st}, Plain{tscale}, d, own_u, stride, nullptr, r);
     B[o1] = r[0];
     B[o2] = r[2];
     E[o1] = r[1];
@@ -1127,12 +1136,12 @@ __global__ void __launch_bounds__(kFillThreads) k_fill_own(const float4* __restr
 #pragma unroll
         for (int q = 0; q < kKmax; ++q) u[q] = own_u[q * stride + i];
         acc2 a[NC];
-        unit_products<NC>(st, tscale, u[0], a);
+        unit_products(ReadOnly{st}, ReadOnly{tscale}, u[0], a);
 #pragma unroll
         for (int q = 1; q < kKmax; ++q) {
             if (u[q] == kNoUnit) break;
             acc2 b[NC];
-            unit_products<NC>(st, tscale, u[q], b);
+            unit_products(ReadOnly{st}, ReadOnly{tscale}, u[q], b);
 #pragma unroll
             for (int c = 0; c < NC; ++c) add_to(a[c], b[c]);
         }
