@@ -362,8 +362,10 @@ __global__ void __launch_bounds__(kThreads) k_cgemm_tf32(int64_t w, int64_t row0
 // slab is a few hundred to a few thousand wide, so the row tiles alone leave most SMs idle and
 // the product is bound by latency.  Per CTA, 32-wide K chunks through two shared buffers: the
 // loads of the next chunk (registers) and the split run under the MMAs of the last.  An accumulator
-// rounds toward zero at every MMA, so chunk ch goes to accumulator pair ch % 4 (512 TMEM columns,
-// small terms first), summed in FP32.  The partial tiles meet in distributed shared memory,
+// rounds toward zero at every MMA, so each chunk has an accumulator pair to itself (pair ch % 4 of
+// 512 TMEM columns, small terms first), read out and added in FP32 registers, in chunk order, before chunk
+// ch + 4 takes it over: 0.3 to 0.5 of the error of FP32 FMA chains at 941 to 2768 wide (chunks sharing a pair
+// had up to 7 times it, and took as long).  The partial tiles meet in distributed shared memory,
 // each CTA adding the ranks of its share of the rows in rank order.
 // The 64 x 64 CUDA-core tiles with a K split through global partials took 53 us for 48
 // columns of a 950-wide slab on average (45 CTAs) and 29 us for 16 columns, this 19 and 12 to 22
@@ -481,6 +483,39 @@ __global__ void __launch_bounds__(kSpThreads, 1) k_slab_split(int64_t w, int64_t
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t taddr = tmem_base;
     const uint32_t id = idesc_tf32(kM, 16 * n16), idneg = id | (1u << 13);
+    // this warp's part of the sums: TMEM lanes 32 (w % 4) .. + 31 (rows), column blocks w / 4, w / 4 + 2
+    const uint32_t lane_addr = taddr + ((uint32_t)((warp & 3) * 32) << 16);
+    float2 sum[2][16];
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int c = 0; c < 16; ++c) sum[j][c] = z2;
+    auto add_set = [&](int q) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int b = (warp >> 2) + 2 * j;
+            if (b >= n16) break;       // uniform per warp
+            uint32_t vr[16], vi[16];
+            asm volatile(
+                "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
+                "%14, %15}, [%16];"
+                : "=r"(vr[0]), "=r"(vr[1]), "=r"(vr[2]), "=r"(vr[3]), "=r"(vr[4]), "=r"(vr[5]), "=r"(vr[6]), "=r"(vr[7]), "=r"(vr[8]), "=r"(vr[9]), "=r"(vr[10]), "=r"(vr[11]), "=r"(vr[12]), "=r"(vr[13]), "=r"(vr[14]), "=r"(vr[15])
+                : "r"(lane_addr + (uint32_t)(2 * q * kTmemCols + 16 * b))
+                : "memory");
+            asm volatile(
+                "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
+                "%14, %15}, [%16];"
+                : "=r"(vi[0]), "=r"(vi[1]), "=r"(vi[2]), "=r"(vi[3]), "=r"(vi[4]), "=r"(vi[5]), "=r"(vi[6]), "=r"(vi[7]), "=r"(vi[8]), "=r"(vi[9]), "=r"(vi[10]), "=r"(vi[11]), "=r"(vi[12]), "=r"(vi[13]), "=r"(vi[14]), "=r"(vi[15])
+                : "r"(lane_addr + (uint32_t)((2 * q + 1) * kTmemCols + 16 * b))
+                : "memory");
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int c = 0; c < 16; ++c) {
+                sum[j][c].x += __uint_as_float(vr[c]);
+                sum[j][c].y += __uint_as_float(vi[c]);
+            }
+        }
+    };
     bool ok = true;
     for (int ch = 0; ch < nk; ++ch) {
         const int buf = ch & 1;
@@ -488,6 +523,10 @@ __global__ void __launch_bounds__(kSpThreads, 1) k_slab_split(int64_t w, int64_t
         // the MMAs that read this buffer two chunks ago are done
         if (ch >= 2 && ok && !mbar_wait(smem_u32(&mbar[buf]), (uint32_t)(((ch >> 1) - 1) & 1))) ok = false;
         if (ok) split(cb);
+        if (ch >= 4 && __all_sync(0xffffffffu, ok)) {   // chunk ch - 4's MMAs were committed before those
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            add_set(ch & 3);
+        }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         ok = !__syncthreads_or(!ok);   // uniform
@@ -515,7 +554,7 @@ __global__ void __launch_bounds__(kSpThreads, 1) k_slab_split(int64_t w, int64_t
                     const uint64_t brl = make_desc(b0 + 1 * kSpBTile + off, 128, 1024);
                     const uint64_t bih = make_desc(b0 + 2 * kSpBTile + off, 128, 1024);
                     const uint64_t bil = make_desc(b0 + 3 * kSpBTile + off, 128, 1024);
-                    const uint32_t first = (ch < 4 && ks == 0) ? 0u : 1u;
+                    const uint32_t first = ks == 0 ? 0u : 1u;
                     if (term == 0) {
                         EMG_UMMA(dre, arh, brl, id, first);
                         EMG_UMMA(dre, arl, brh, id, 1u);
@@ -550,36 +589,14 @@ __global__ void __launch_bounds__(kSpThreads, 1) k_slab_split(int64_t w, int64_t
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     float2* P = reinterpret_cast<float2*>(base);
     {
-        // warp w reads TMEM lanes 32 (w % 4) .. + 31 (rows), column blocks w / 4, w / 4 + 2
-        const int row = (warp & 3) * 32 + lane, sets = min(nk, 4);
-        const uint32_t lane_addr = taddr + ((uint32_t)((warp & 3) * 32) << 16);
-        for (int b = warp >> 2; b < n16; b += 2) {
-            float2 sum[16];
+        for (int ch = max(0, nk - 4); ch < nk; ++ch) add_set(ch & 3);
+        const int row = (warp & 3) * 32 + lane;
 #pragma unroll
-            for (int c = 0; c < 16; ++c) sum[c] = z2;
-            for (int q = 0; q < sets; ++q) {
-                uint32_t vr[16], vi[16];
-                asm volatile(
-                    "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
-                    "%14, %15}, [%16];"
-                    : "=r"(vr[0]), "=r"(vr[1]), "=r"(vr[2]), "=r"(vr[3]), "=r"(vr[4]), "=r"(vr[5]), "=r"(vr[6]), "=r"(vr[7]), "=r"(vr[8]), "=r"(vr[9]), "=r"(vr[10]), "=r"(vr[11]), "=r"(vr[12]), "=r"(vr[13]), "=r"(vr[14]), "=r"(vr[15])
-                    : "r"(lane_addr + (uint32_t)(2 * q * kTmemCols + 16 * b))
-                    : "memory");
-                asm volatile(
-                    "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
-                    "%14, %15}, [%16];"
-                    : "=r"(vi[0]), "=r"(vi[1]), "=r"(vi[2]), "=r"(vi[3]), "=r"(vi[4]), "=r"(vi[5]), "=r"(vi[6]), "=r"(vi[7]), "=r"(vi[8]), "=r"(vi[9]), "=r"(vi[10]), "=r"(vi[11]), "=r"(vi[12]), "=r"(vi[13]), "=r"(vi[14]), "=r"(vi[15])
-                    : "r"(lane_addr + (uint32_t)((2 * q + 1) * kTmemCols + 16 * b))
-                    : "memory");
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        for (int j = 0; j < 2; ++j) {
+            const int b = (warp >> 2) + 2 * j;
+            if (b >= n16) break;
 #pragma unroll
-                for (int c = 0; c < 16; ++c) {
-                    sum[c].x += __uint_as_float(vr[c]);
-                    sum[c].y += __uint_as_float(vi[c]);
-                }
-            }
-#pragma unroll
-            for (int c = 0; c < 16; ++c) P[row * kSpLd + 16 * b + c] = sum[c];
+            for (int c = 0; c < 16; ++c) P[row * kSpLd + 16 * b + c] = sum[j][c];
         }
     }
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
