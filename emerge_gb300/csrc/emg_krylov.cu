@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "emg_krylov.cuh"
+#include "emg_rules.cuh"
 
 namespace emg {
 namespace kry {
@@ -309,7 +310,7 @@ __global__ void k_spmv_fam(int64_t n, int64_t nnz, int64_t Bc, int nfam, const d
 // FUN: part[blk][j][c] = sum_{rows in blk} V[r][j] W[r,c] for the nj columns of V (rows of vstride),
 // conjugated (2) or not (1): a few functionals of every column (the library's long-K product has one
 // CTA for them: 2590 us for 2282 unknowns and 20 columns, this below 30).
-constexpr int kDotThreads = 256, kDotJ = 4;
+constexpr int kDotThreads = rules::kDotThreads, kDotJ = 4;
 constexpr int kMaxRestart = 256;
 __device__ __forceinline__ void dot_acc(double2& s, double2 v, double2 w) { cfmac(s, v, w); }
 __device__ __forceinline__ void dot_acc(float2& s, float2 v, float2 w) {
@@ -956,15 +957,12 @@ void spmv(const emg_rplan* p, int64_t Bc, const int32_t* cmat, int64_t Bm, const
         kry::k_spmv<<<grid_for(n * Bc, 256), 256, 0, s>>>(n, Bc, cmat, Bm, p->rptr, p->rind, A, X, Bv, Y);
 }
 
-// Rows of a block of the partial dots: two blocks per SM where there are at least 64 rows
-// for each (fewer spend more on the reduction than on the products).
-int64_t dot_rows(int64_t n) { return std::max<int64_t>(64, (n + 2 * 152 - 1) / (2 * 152)); }
-
 template <typename T, int FUN = 0>
 void dots(int64_t n, int64_t Bc, int nj, const T* V, int64_t vstride, const T* W, double2* part, double2* out,
           cudaStream_t s) {
-    const int64_t rows = dot_rows(n), nblk = (n + rows - 1) / rows;
-    const int ct = (int)((Bc + 127) / 128), cw = (int)((Bc + ct - 1) / ct);
+    constexpr bool fp32 = sizeof(T) == sizeof(float2);
+    const int64_t rows = rules::dot_rows(n, Bc, fp32), nblk = rules::dot_blocks(n, Bc, fp32);
+    const int ct = (int)((Bc + 127) / 128), cw = rules::dot_tile(Bc);
     const dim3 g((unsigned)nblk, (unsigned)ct, (unsigned)((nj + kry::kDotJ - 1) / kry::kDotJ));
     kry::k_dots_partial<T, FUN><<<g, kry::kDotThreads, 0, s>>>(n, (int)Bc, cw, nj, rows, V, vstride, W, part);
     kry::k_dots_final<<<(unsigned)(((int64_t)nj * Bc * 32 + 127) / 128), 128, 0, s>>>(nblk, Bc, nj, part, out);
@@ -996,7 +994,7 @@ int gmres_run(emg_rplan* p, int64_t Bc, const MatArg& A, const double2* rhs, dou
     cudaStream_t s = p->gs;
     const int m = restart;
     const int64_t vec = n * Bc;
-    const int64_t nblk = (n + dot_rows(n) - 1) / dot_rows(n);
+    const int64_t nblk = rules::dot_blocks(n, Bc, false);
     // workspace layout
     size_t off = 0;
     auto take = [&](size_t bytes) { size_t o = off; off = (off + bytes + 255) & ~(size_t)255; return o; };
@@ -1286,7 +1284,7 @@ int ir_run(emg_rplan* p, int64_t Bc, const MatArg& A, const float2* A32, const d
     EMG_CUDA(cudaStreamWaitEvent(p->gs, p->ev_in, 0));
     cudaStream_t s = p->gs;
     const int m = restart, T = 256;
-    const int64_t vec = n * Bc, nblk = (n + dot_rows(n) - 1) / dot_rows(n);
+    const int64_t vec = n * Bc, nblk = rules::dot_blocks(n, Bc, true);   // at least the FP64 dots' blocks
     size_t off = 0;
     auto take = [&](size_t bytes) { size_t o = off; off = (off + bytes + 255) & ~(size_t)255; return o; };
     const size_t oR64 = take(sizeof(double2) * vec), oR32 = take(sizeof(float2) * vec), oD32 = take(sizeof(float2) * vec);
@@ -1405,7 +1403,7 @@ struct IluPrecond : emg::Precond {
 
 extern "C" int64_t emg_functionals_work(int64_t n, int np, int64_t Bc) {
     if (n <= 0 || np <= 0 || Bc <= 0) return 0;
-    return (n + dot_rows(n) - 1) / dot_rows(n) * np * Bc;
+    return rules::dot_blocks(n, Bc, false) * np * Bc;
 }
 
 extern "C" int emg_functionals(int64_t n, int np, int64_t Bc, const double* U, int64_t ldu, int conj, const double* X,
