@@ -33,6 +33,17 @@ def _stream() -> ctypes.c_void_p:
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
+def _kernel_blocks(*blocks: torch.Tensor):
+    """The blocks as the kernels below read them, or None where the torch expression is to compute or
+    to refuse them: they take complex128 matrices of the current device, without a gradient to record."""
+    for t in blocks:
+        if (type(t) is not torch.Tensor or not t.is_cuda or t.dtype != torch.complex128 or t.dim() != 2 or t.numel() == 0
+                or t.device.index != torch.cuda.current_device() or (t.requires_grad and torch.is_grad_enabled())):
+            return None
+    # a lazily conjugated (negated) view keeps its bit through contiguous()
+    return [t.resolve_conj().resolve_neg() for t in blocks]
+
+
 def _rows(V: torch.Tensor):
     """V with contiguous rows, and their stride."""
     if V.stride(1) != 1 or V.stride(0) < V.shape[1]:
@@ -43,11 +54,11 @@ def _rows(V: torch.Tensor):
 def functionals(U: torch.Tensor, X: torch.Tensor, conj: bool = False) -> torch.Tensor:
     """U.T @ X (U.conj().T @ X with ``conj``) (np, C) of a few functionals U (n, np) of the
     columns of X (n, C), complex128."""
-    n, npo = U.shape
-    C = int(X.shape[1])
-    if n == 0 or npo == 0 or C == 0 or not X.is_cuda:
+    ok = _kernel_blocks(U, X)
+    if ok is None or U.shape[0] != X.shape[0]:
         return (U.conj() if conj else U).T @ X
-    (U, ldu), X = _rows(U), X.contiguous()
+    (n, npo), C = U.shape, int(X.shape[1])
+    (U, ldu), X = _rows(ok[0]), ok[1].contiguous()
     G = torch.empty((npo, C), dtype=X.dtype, device=X.device)
     work = torch.empty(_lib.load().emg_functionals_work(n, npo, C), dtype=X.dtype, device=X.device)
     _lib.call("emg_functionals", n, npo, C, _vp(U), ldu, int(conj), _vp(X), _vp(work), _vp(G), _stream())
@@ -56,10 +67,11 @@ def functionals(U: torch.Tensor, X: torch.Tensor, conj: bool = False) -> torch.T
 
 def column_dots(X: torch.Tensor, Y: torch.Tensor) -> torch.Tensor:
     """(C,) column-wise conj(X) . Y of complex128 blocks (n, C)."""
-    n, C = (int(v) for v in X.shape)
-    if n == 0 or C == 0 or not X.is_cuda:
+    ok = _kernel_blocks(X, Y)
+    if ok is None or X.shape != Y.shape:
         return (X.conj() * Y).sum(dim=0)
-    X, Y = X.contiguous(), Y.contiguous()
+    X, Y = (t.contiguous() for t in ok)
+    n, C = (int(v) for v in X.shape)
     G = torch.empty(C, dtype=X.dtype, device=X.device)
     work = torch.empty(_lib.load().emg_functionals_work(n, 1, C), dtype=X.dtype, device=X.device)
     _lib.call("emg_column_dots", n, C, _vp(X), _vp(Y), _vp(work), _vp(G), _stream())
@@ -68,9 +80,10 @@ def column_dots(X: torch.Tensor, Y: torch.Tensor) -> torch.Tensor:
 
 def sub_product(W: torch.Tensor, V: torch.Tensor, C: torch.Tensor) -> torch.Tensor:
     """W - V @ C for V (n, m) and a block W (n, c), complex128."""
-    if 0 in V.shape or W.shape[1] == 0 or not W.is_cuda:
+    ok = _kernel_blocks(W, V, C)
+    if ok is None or W.shape[0] != V.shape[0] or tuple(C.shape) != (V.shape[1], W.shape[1]):
         return W - V @ C
-    (V, ldv), C, W = _rows(V), C.contiguous(), W.contiguous()
+    W, (V, ldv), C = ok[0].contiguous(), _rows(ok[1]), ok[2].contiguous()
     out = torch.empty_like(W)
     _lib.call("emg_sub_product", int(V.shape[0]), int(V.shape[1]), int(W.shape[1]), _vp(V), ldv, _vp(C), _vp(W), _vp(out),
               _stream())

@@ -50,3 +50,47 @@ def test_projection_pieces(n, m, cols):
     assert np.all(np.abs(got - (wide(W) - wide(V) @ wide(C))) <= (m + 8) * 2.0 ** -52 * (np.abs(W) + np.abs(V) @ np.abs(C)))
     got = column_dots(Wd, Wd).cpu().numpy()
     assert np.all(np.abs(got - (wide(W).conj() * wide(W)).sum(axis=0)) <= (n + 8) * 2.0 ** -52 * (np.abs(W) ** 2).sum(axis=0))
+
+
+def _block(torch, *shape, seed=0, device="cuda"):
+    gen = torch.Generator(device="cpu").manual_seed(seed)
+    return torch.view_as_complex(torch.randn((*shape, 2), generator=gen, dtype=torch.float64)).to(device)
+
+
+def test_lazily_conjugated_blocks():
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from emerge_gb300.solver import column_dots, functionals, sub_product
+    V, W, C = _block(torch, 65, 3), _block(torch, 65, 4, seed=1), _block(torch, 3, 4, seed=2)
+    near = lambda a, b: bool(((a - b).abs() <= 80 * 2.0 ** -52 * 100).all())  # noqa: E731
+    for view in (torch.conj, torch._neg_view, lambda t: torch._neg_view(t.conj())):
+        v, w, c = view(V), view(W), view(C)
+        vr, wr, cr = (t.resolve_conj().resolve_neg().clone() for t in (v, w, c))
+        assert near(functionals(v, W), vr.T @ W) and near(functionals(V, w), V.T @ wr)
+        assert near(functionals(v, w, conj=True), vr.conj().T @ wr)
+        assert near(column_dots(w, W), (wr.conj() * W).sum(dim=0)) and near(column_dots(W, w), (W.conj() * wr).sum(dim=0))
+        assert near(sub_product(w, v, c), wr - vr @ cr)
+
+
+def test_what_torch_refuses_stays_refused():
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from emerge_gb300.solver import column_dots, functionals, sub_product
+    V, W, C = _block(torch, 65, 3), _block(torch, 65, 4, seed=1), _block(torch, 3, 4, seed=2)
+    for call in (lambda: functionals(V, W[:60]), lambda: functionals(V[:60], W), lambda: functionals(V, W.to(torch.complex64)),
+                 lambda: functionals(V.cpu(), W), lambda: column_dots(W, W[:60]), lambda: column_dots(W, W.cpu()),
+                 lambda: sub_product(W, V, C[:2]), lambda: sub_product(W, V, C[:, :3]), lambda: sub_product(W[:60], V, C),
+                 lambda: sub_product(W, V.to(torch.complex64), C), lambda: sub_product(W, V, C.cpu())):
+        with pytest.raises(RuntimeError):
+            call()
+    # and what it computes is computed
+    V4, W4, C4 = (t.to(torch.complex64) for t in (V, W, C))
+    assert torch.allclose(functionals(V4, W4), V4.T @ W4) and torch.allclose(sub_product(W4, V4, C4), W4 - V4 @ C4)
+    assert torch.allclose(column_dots(W4, W), (W4.conj() * W).sum(dim=0))
+    assert torch.allclose(column_dots(W, W[:1]), (W.conj() * W[:1]).sum(dim=0))
+    assert torch.allclose(functionals(V.real, W.real), V.real.T @ W.real)
+    g = W.clone().requires_grad_()
+    column_dots(g, g).real.sum().backward()
+    assert torch.allclose(g.grad, 2 * W)
