@@ -55,7 +55,7 @@ def functionals(U: torch.Tensor, X: torch.Tensor, conj: bool = False) -> torch.T
     """U.T @ X (U.conj().T @ X with ``conj``) (np, C) of a few functionals U (n, np) of the
     columns of X (n, C), complex128."""
     ok = _kernel_blocks(U, X)
-    if ok is None or U.shape[0] != X.shape[0]:
+    if ok is None or U.shape[0] != X.shape[0] or U.shape[1] > 65535:
         return (U.conj() if conj else U).T @ X
     (n, npo), C = U.shape, int(X.shape[1])
     (U, ldu), X = _rows(ok[0]), ok[1].contiguous()
@@ -81,7 +81,8 @@ def column_dots(X: torch.Tensor, Y: torch.Tensor) -> torch.Tensor:
 def sub_product(W: torch.Tensor, V: torch.Tensor, C: torch.Tensor) -> torch.Tensor:
     """W - V @ C for V (n, m) and a block W (n, c), complex128."""
     ok = _kernel_blocks(W, V, C)
-    if ok is None or W.shape[0] != V.shape[0] or tuple(C.shape) != (V.shape[1], W.shape[1]):
+    if (ok is None or W.shape[0] != V.shape[0] or tuple(C.shape) != (V.shape[1], W.shape[1])
+            or W.shape[1] > 2048):               # the kernel keeps a row of C in shared memory
         return W - V @ C
     W, (V, ldv), C = ok[0].contiguous(), _rows(ok[1]), ok[2].contiguous()
     out = torch.empty_like(W)

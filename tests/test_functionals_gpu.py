@@ -73,6 +73,15 @@ def test_lazily_conjugated_blocks():
         assert near(sub_product(w, v, c), wr - vr @ cr)
 
 
+def test_more_columns_than_the_kernel_takes():
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from emerge_gb300.solver import sub_product
+    V, W, C = _block(torch, 17, 3), _block(torch, 17, 2049, seed=1), _block(torch, 3, 2049, seed=2)
+    assert torch.allclose(sub_product(W, V, C), W - V @ C, rtol=0.0, atol=1e-13)
+
+
 def test_what_torch_refuses_stays_refused():
     import torch
     if not torch.cuda.is_available():
