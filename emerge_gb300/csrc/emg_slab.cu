@@ -1485,7 +1485,7 @@ int slab_factor_t(emg_slab* s, int64_t F, const int32_t* amat_h, int64_t Bm, con
     if (tc_update) EMG_CUDA(cudaMemcpyAsync(&tcs, s->tc_status, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
     EMG_CUDA(cudaStreamSynchronize(st));
     if (tcs) {   // a tensor-core tile gave up waiting: the factors are not usable
-        EMG_CUDA(cudaMemset(s->tc_status, 0, sizeof(int32_t)));
+        EMG_CUDA(cudaMemsetAsync(s->tc_status, 0, sizeof(int32_t), st));
         slab_free_factors(s);
         set_error("slab factor: a tensor-core update tile timed out waiting for its MMAs");
         return EMG_ERR_CUDA;
@@ -1520,20 +1520,23 @@ int tc_check(emg_slab* s, cudaStream_t st) {
     EMG_CUDA(cudaMemcpyAsync(&h, s->tc_status, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
     EMG_CUDA(cudaStreamSynchronize(st));
     if (h) {
-        EMG_CUDA(cudaMemset(s->tc_status, 0, sizeof(int32_t)));
+        EMG_CUDA(cudaMemsetAsync(s->tc_status, 0, sizeof(int32_t), st));
         set_error("slab solve: a tensor-core tile timed out waiting for its MMAs");
         return EMG_ERR_CUDA;
     }
     return EMG_OK;
 }
 
-// The slab solve as a GMRES preconditioner: column c uses factor cfac[c].
+// The slab solve as a GMRES preconditioner: column c uses factor cfac[c].  prepare() orders its copies
+// and fills on the caller's stream ``in``: a solve before them on it may still read the same arrays.
 struct SlabPrecond : emg::Precond {
     emg_slab* s;
+    cudaStream_t in;
     std::vector<int32_t> cfac;
     std::vector<emg::slab::Group> groups;
     int64_t Bc = 0;
-    SlabPrecond(emg_slab* s_, int64_t Bc_, const int32_t* cfac_) : s(s_), cfac(cfac_, cfac_ + Bc_), Bc(Bc_) {
+    SlabPrecond(emg_slab* s_, int64_t Bc_, const int32_t* cfac_, cudaStream_t in_)
+        : s(s_), in(in_), cfac(cfac_, cfac_ + Bc_), Bc(Bc_) {
         for (int64_t c = 0; c < Bc; ++c) {
             if (!groups.empty() && groups.back().fac == cfac[c] && groups.back().col0 + groups.back().ncol == c)
                 groups.back().ncol++;
@@ -1586,14 +1589,14 @@ struct SlabPrecond : emg::Precond {
                 s->kcnt_n = 0;
                 int rc = dalloc(&s->kcnt, tiles_max, "slab split-K counters");
                 if (rc) return rc;
-                EMG_CUDA(cudaMemset(s->kcnt, 0, sizeof(int32_t) * tiles_max));
+                EMG_CUDA(cudaMemsetAsync(s->kcnt, 0, sizeof(int32_t) * tiles_max, in));
                 s->kcnt_n = tiles_max;
             }
         }
         if (!s->tc_status) {
             int rc = dalloc(&s->tc_status, 1, "slab tensor-core status");
             if (rc) return rc;
-            EMG_CUDA(cudaMemset(s->tc_status, 0, sizeof(int32_t)));
+            EMG_CUDA(cudaMemsetAsync(s->tc_status, 0, sizeof(int32_t), in));
         }
         if ((int64_t)groups.size() > s->ngroups_cap) {
             dfree(s->groups);
@@ -1601,8 +1604,8 @@ struct SlabPrecond : emg::Precond {
             if (rc) return rc;
             s->ngroups_cap = (int64_t)groups.size();
         }
-        EMG_CUDA(cudaMemcpy(s->colfac, cfac.data(), sizeof(int32_t) * bc, cudaMemcpyHostToDevice));
-        EMG_CUDA(cudaMemcpy(s->groups, groups.data(), sizeof(emg::slab::Group) * groups.size(), cudaMemcpyHostToDevice));
+        EMG_CUDA(cudaMemcpyAsync(s->colfac, cfac.data(), sizeof(int32_t) * bc, cudaMemcpyHostToDevice, in));
+        EMG_CUDA(cudaMemcpyAsync(s->groups, groups.data(), sizeof(emg::slab::Group) * groups.size(), cudaMemcpyHostToDevice, in));
         return EMG_OK;
     }
     template <typename R, typename TI>
@@ -1707,7 +1710,7 @@ struct SlabPrecond : emg::Precond {
 // the mixed-precision refinement.
 struct SlabPrecond32 : emg::Precond32 {
     SlabPrecond base;
-    SlabPrecond32(emg_slab* s_, int64_t Bc_, const int32_t* cfac_) : base(s_, Bc_, cfac_) {}
+    SlabPrecond32(emg_slab* s_, int64_t Bc_, const int32_t* cfac_, cudaStream_t in) : base(s_, Bc_, cfac_, in) {}
     int prepare(int64_t bc) override { return base.prepare(bc); }
     int apply(const float2* in, float2* out, cudaStream_t st) override { return base.run<float, float2>(in, out, st); }
 };
@@ -1720,7 +1723,7 @@ extern "C" int emg_slab_apply(emg_slab* s, int64_t Bc, const int32_t* cfac, cons
     EMG_CHECK_ARG(s->F > 0, "emg_slab_apply: no factorization");
     for (int64_t c = 0; c < Bc; ++c) EMG_CHECK_ARG(cfac[c] >= 0 && cfac[c] < s->F, "emg_slab_apply: cfac out of range");
     if (s->n == 0) return EMG_OK;
-    SlabPrecond M(s, Bc, cfac);
+    SlabPrecond M(s, Bc, cfac, (cudaStream_t)stream);
     int rc = M.prepare(Bc);
     if (rc) return rc;
     rc = M.apply(reinterpret_cast<const double2*>(X_in), reinterpret_cast<double2*>(X_out), (cudaStream_t)stream);
@@ -1738,7 +1741,7 @@ extern "C" int emg_gmres_slab(const emg_rplan* pc, emg_slab* s, int64_t Bc, cons
     EMG_CHECK_ARG(restart >= 1 && restart <= 256 && max_iter >= 1 && tol > 0, "emg_gmres_slab: restart must be in [1, 256]");
     EMG_CHECK_ARG(s->F > 0, "emg_gmres_slab: no factorization");
     for (int64_t c = 0; c < Bc; ++c) EMG_CHECK_ARG(cfac[c] >= 0 && cfac[c] < s->F, "emg_gmres_slab: cfac out of range");
-    SlabPrecond M(s, Bc, cfac);
+    SlabPrecond M(s, Bc, cfac, (cudaStream_t)stream);
     MatArg Am;
     Am.A = reinterpret_cast<const double2*>(A);
     Am.Bm = Bm;
@@ -1786,7 +1789,7 @@ extern "C" int emg_gmres_slab_family(const emg_rplan* pc, emg_slab* s, int64_t B
     EMG_CHECK_ARG(s->F > 0, "emg_gmres_slab_family: no factorization");
     for (int64_t c = 0; c < Bc; ++c)
         EMG_CHECK_ARG(cfac[c] >= 0 && cfac[c] < s->F, "emg_gmres_slab_family: cfac out of range");
-    SlabPrecond M(s, Bc, cfac);
+    SlabPrecond M(s, Bc, cfac, (cudaStream_t)stream);
     MatArg Am;
     Am.nfam = nfam;
     Am.fam = reinterpret_cast<const double2*>(fam);
@@ -1818,7 +1821,7 @@ extern "C" int emg_gmres_slab_mixed(const emg_rplan* pc, emg_slab* s, int64_t Bc
     cudaStream_t st = (cudaStream_t)stream;
     slab::k_narrow<<<grid_for(p->nnz * Bm, 256), 256, 0, st>>>(p->nnz * Bm, reinterpret_cast<const double2*>(A), A32);
     EMG_CUDA(cudaGetLastError());
-    SlabPrecond32 M(s, Bc, cfac);
+    SlabPrecond32 M(s, Bc, cfac, st);
     MatArg Am;
     Am.A = reinterpret_cast<const double2*>(A);
     Am.Bm = Bm;

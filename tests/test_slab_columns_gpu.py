@@ -142,3 +142,26 @@ def test_row_blocks(system, n):
                 r = A[g] @ y[:, g * cols:(g + 1) * cols] - b[:, g * cols:(g + 1) * cols]
                 # inverse and product: relative errors of a few n eps, condition below 100
                 assert float(torch.linalg.norm(r)) <= 200 * n * 2.0 ** -23 * float(torch.linalg.norm(b))
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+@pytest.mark.parametrize("cols", [2, 24])
+def test_solves_in_a_row_on_another_stream(system, precision, cols):
+    """Solves with other columns' factors follow each other on a stream without a wait: each works with
+    its own column tables."""
+    torch, sysr, A, slab = system
+    slab.factor(A, [0, 1], precision)
+    gen = torch.Generator(device="cuda").manual_seed(8)
+    b = torch.view_as_complex(torch.randn((sysr.n, cols, 2), generator=gen, device="cuda", dtype=torch.float64))
+    facs = [[0] * cols, [1] * cols, [0] + [1] * (cols - 1), [c % 2 for c in range(cols)]]
+    refs = []
+    for fac in facs:
+        refs.append(torch.view_as_real(slab.apply(b, fac)))
+        torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        got = [slab.apply(b, facs[i % 4]) for i in range(12)]
+    side.synchronize()
+    for i, y in enumerate(got):
+        assert torch.equal(torch.view_as_real(y), refs[i % 4]), i
