@@ -1513,9 +1513,10 @@ extern "C" int emg_slab_factor(emg_slab* s, int precision, int64_t F, const int3
 }
 
 namespace {
-// EMG_ERR_CUDA if a tensor-core tile of the last solve gave up waiting (and reset).
-int tc_check(emg_slab* s, cudaStream_t st) {
-    if (!s->tc_status || s->prec != 1) return EMG_OK;
+// EMG_ERR_CUDA if a tensor-core tile of the last solve gave up waiting (and reset).  Waits for the
+// stream, so only where the solve launched such tiles.
+int tc_check(emg_slab* s, bool launched, cudaStream_t st) {
+    if (!launched) return EMG_OK;
     int32_t h = 0;
     EMG_CUDA(cudaMemcpyAsync(&h, s->tc_status, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
     EMG_CUDA(cudaStreamSynchronize(st));
@@ -1535,6 +1536,7 @@ struct SlabPrecond : emg::Precond {
     std::vector<int32_t> cfac;
     std::vector<emg::slab::Group> groups;
     int64_t Bc = 0;
+    bool tc_tiles = false;             // the solve launched tensor-core tiles, which may set tc_status
     SlabPrecond(emg_slab* s_, int64_t Bc_, const int32_t* cfac_, cudaStream_t in_)
         : s(s_), in(in_), cfac(cfac_, cfac_ + Bc_), Bc(Bc_) {
         for (int64_t c = 0; c < Bc; ++c) {
@@ -1645,6 +1647,7 @@ struct SlabPrecond : emg::Precond {
                         if (e != cudaSuccess && !rc) rc = cuda_status(e, "slab row-block product");
                         return;
                     }
+                    tc_tiles = true;
                     const int e = s->use_tc ? emg::tc_slab_product(w, s->off[i], Bc, s->groups, (int)G, maxcol, Sf, s->totD,
                                                                    s->offD[i], Yf, (float)alpha, beta,
                                                                    reinterpret_cast<float2*>(Z), s->tc_status, st)
@@ -1728,7 +1731,7 @@ extern "C" int emg_slab_apply(emg_slab* s, int64_t Bc, const int32_t* cfac, cons
     if (rc) return rc;
     rc = M.apply(reinterpret_cast<const double2*>(X_in), reinterpret_cast<double2*>(X_out), (cudaStream_t)stream);
     if (rc) return rc;
-    return tc_check(s, (cudaStream_t)stream);
+    return tc_check(s, M.tc_tiles, (cudaStream_t)stream);
 }
 
 extern "C" int emg_gmres_slab(const emg_rplan* pc, emg_slab* s, int64_t Bc, const int32_t* cmat, int64_t Bm,
@@ -1748,7 +1751,7 @@ extern "C" int emg_gmres_slab(const emg_rplan* pc, emg_slab* s, int64_t Bc, cons
     Am.cmat = cmat;
     const int rc = gmres_run(p, Bc, Am, reinterpret_cast<const double2*>(rhs), reinterpret_cast<double2*>(x), restart,
                              max_iter, tol, iters_out, resid_out, (cudaStream_t)stream, M, true);
-    return rc ? rc : tc_check(s, (cudaStream_t)stream);
+    return rc ? rc : tc_check(s, M.tc_tiles, (cudaStream_t)stream);
 }
 
 extern "C" int emg_slab_set_factor_tensor_cores(emg_slab* s, int on) {
@@ -1796,7 +1799,7 @@ extern "C" int emg_gmres_slab_family(const emg_rplan* pc, emg_slab* s, int64_t B
     Am.coef = reinterpret_cast<const double2*>(coef);
     const int rc = gmres_run(p, Bc, Am, reinterpret_cast<const double2*>(rhs), reinterpret_cast<double2*>(x), restart,
                              max_iter, tol, iters_out, resid_out, (cudaStream_t)stream, M, true);
-    return rc ? rc : tc_check(s, (cudaStream_t)stream);
+    return rc ? rc : tc_check(s, M.tc_tiles, (cudaStream_t)stream);
 }
 
 extern "C" int emg_gmres_slab_mixed(const emg_rplan* pc, emg_slab* s, int64_t Bc, const int32_t* cmat, int64_t Bm,
@@ -1829,5 +1832,5 @@ extern "C" int emg_gmres_slab_mixed(const emg_rplan* pc, emg_slab* s, int64_t Bc
     rc = ir_run(p, Bc, Am, A32, reinterpret_cast<const double2*>(rhs), reinterpret_cast<double2*>(x), restart, max_iter,
                 tol, inner_tol, iters_out, resid_out, steps_out, st, M);
     EMG_CUDA(cudaStreamSynchronize(st));   // A32 is freed on return
-    return rc ? rc : tc_check(s, st);
+    return rc ? rc : tc_check(s, M.base.tc_tiles, st);
 }

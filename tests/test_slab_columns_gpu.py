@@ -165,3 +165,21 @@ def test_solves_in_a_row_on_another_stream(system, precision, cols):
     side.synchronize()
     for i, y in enumerate(got):
         assert torch.equal(torch.view_as_real(y), refs[i % 4]), i
+
+
+@pytest.mark.parametrize("precision,cols", [("fp32", 1), ("fp32", 20), ("fp64", 20)])
+def test_a_solve_does_not_wait_for_the_gpu(system, precision, cols):
+    """A product by rows or row blocks has no status to read: the call returns while earlier work runs."""
+    torch, sysr, A, slab = system
+    slab.factor(A, [0], precision)
+    b = torch.ones((sysr.n, cols), dtype=torch.complex128, device="cuda")
+    ref = slab.apply(b, [0] * cols)                # work space and kernels are there
+    x = torch.ones((8192, 8192), device="cuda")
+    torch.cuda.synchronize()
+    done = torch.cuda.Event()
+    for _ in range(100):                           # over 100 ms of FP32 products
+        x = x @ x * 0.0
+    done.record()
+    y = slab.apply(b, [0] * cols)
+    assert not done.query()
+    assert torch.equal(torch.view_as_real(y), torch.view_as_real(ref))
