@@ -1623,11 +1623,13 @@ struct SlabPrecond : emg::Precond {
         int maxcol = 0;
         for (const auto& g : groups) maxcol = std::max(maxcol, (int)g.ncol);
         if constexpr (sizeof(R) == 8) {
-            static bool narrow_attr = false;   // the 128 x 16 tiles need 74 KB
-            if (!narrow_attr) {
+            static bool narrow_attr[64] = {false};   // per device; the 128 x 16 tiles need 74 KB
+            int dev = 0;
+            EMG_CUDA(cudaGetDevice(&dev));
+            if (dev >= 64 || !narrow_attr[dev]) {
                 EMG_CUDA(cudaFuncSetAttribute(k_slab_gemm16<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                               (int)sizeof(NarrowTile<R>)));
-                narrow_attr = true;
+                if (dev < 64) narrow_attr[dev] = true;
             }
         }
         // dense slab product: rows of few columns for groups narrower than s->wide; wider FP32
