@@ -873,17 +873,28 @@ __global__ void k_pair_check(const int32_t* __restrict__ ent_list, int64_t n_ent
         if (ent_list[i] != i || partner[i] != i + n_ent || over[i]) atomicOr(ragged, 1);
 }
 
+// *n_own += two own columns for every edge with more than two tets (k_pos_desc lists their units).
+__global__ void k_own_count(const int32_t* __restrict__ ents, int64_t n, const int64_t* __restrict__ inc_ptr,
+                            const int64_t* __restrict__ inc_c, unsigned long long* __restrict__ n_own) {
+    unsigned mine = 0;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t i0 = inc_ptr[ents[i]], k = inc_ptr[ents[i] + 1] - i0;
+        if (k > 2 && (inc_c[i0] & 15) < 6) mine += 2;
+    }
+    mine = __reduce_add_sync(0xffffffffu, mine);
+    if ((threadIdx.x & 31) == 0 && mine) atomicAdd(n_own, (unsigned long long)mine);
+}
+
 // Plan time, warp per fast-fill entity: per CSR position of its first row the one or two staged
 // units summed there, in tet order (kNoUnit: none), and (rows given) the position in both rows.  An
 // own column of an edge with more than two tets has (kNoUnit, i) instead, and its units in
-// column i of ``own_u``: kKmax arrays of 2 n_e, kNoUnit beyond the edge's tets.
+// column i of ``own_u``: kKmax arrays of ``stride``, kNoUnit beyond the edge's tets.
 constexpr uint32_t kNoUnit = 0xffffffffu;
 __global__ void k_pos_desc(const int32_t* __restrict__ ents, int64_t n_e, const int32_t* __restrict__ partner,
                            const int64_t* __restrict__ inc_ptr, const int64_t* __restrict__ inc_c,
                            const int64_t* __restrict__ indptr, const uint8_t* __restrict__ ipos,
                            const int64_t* __restrict__ pofs, uint2* __restrict__ pdesc, longlong2* __restrict__ rows,
-                           uint32_t* __restrict__ own_u,
-                           unsigned long long* __restrict__ n_own) {
+                           uint32_t* __restrict__ own_u, int64_t stride, unsigned long long* __restrict__ n_own) {
     __shared__ uint2 con[8][kNmax];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int64_t i = blockIdx.x * 8ll + w; i < n_e; i += gridDim.x * 8ll) {
@@ -914,7 +925,7 @@ __global__ void k_pos_desc(const int32_t* __restrict__ ents, int64_t n_e, const 
             for (int64_t q = 0; q < kKmax; ++q) {
                 const int64_t code = q < k ? inc_c[i0 + q] : 0;
                 const int slot = (int)(code & 15);
-                own_u[q * 2 * n_e + (int64_t)at] =
+                own_u[q * stride + (int64_t)at] =
                     q < k ? (uint32_t)st_unit(code >> 4, slot, slot + (lane < 10 ? 0 : 10)) : kNoUnit;
             }
         }
@@ -1124,7 +1135,7 @@ __global__ void __launch_bounds__(kFillThreads) k_fill_small(const float4* st, i
 
 // The own columns of edges with more than two tets, thread per (edge, column), tets in order.
 template <bool IM>
-__global__ void __launch_bounds__(kFillThreads) k_fill_own(const float4* __restrict__ st, int64_t n_own, int64_t stride,
+__global__ void __launch_bounds__(kFillThreads) k_fill_own(const float4* __restrict__ st, int64_t n_own,
                                                            const uint32_t* __restrict__ own_u,
                                                            const float4* __restrict__ tscale,
                                                            const int* __restrict__ complex_mu,
@@ -1134,7 +1145,7 @@ __global__ void __launch_bounds__(kFillThreads) k_fill_own(const float4* __restr
     for (int64_t i = blockIdx.x * (int64_t)kFillThreads + threadIdx.x; i < n_own; i += (int64_t)gridDim.x * kFillThreads) {
         uint32_t u[kKmax];
 #pragma unroll
-        for (int q = 0; q < kKmax; ++q) u[q] = own_u[q * stride + i];
+        for (int q = 0; q < kKmax; ++q) u[q] = own_u[q * n_own + i];
         acc2 a[NC];
         unit_products(ReadOnly{st}, ReadOnly{tscale}, u[0], a);
 #pragma unroll
@@ -1234,8 +1245,6 @@ int upload_vint() {
 void df_plan_free(DfPlan* p) {
     dfree(p->recs);
     dfree(p->inv);
-    dfree(p->dofc);
-    dfree(p->inc_c);
     dfree(p->pdesc);
     dfree(p->prows);
     dfree(p->own_u);
@@ -1263,8 +1272,11 @@ int df_plan_build(const double* nodes, int64_t nN, const int32_t* tets, int64_t 
     int64_t *flags = nullptr, *scans = nullptr, *tmp = nullptr;
     uint64_t* cslot = nullptr;
     uint8_t *ipos = nullptr, *over = nullptr;   // CSR positions of the incidences' 20 columns; see k_pos_check
+    int32_t* dofc = nullptr;                    // DOF ids in canonical slot order (nT x 20)
+    int64_t* inc_c = nullptr;                   // incidences with canonical slots
     auto cleanup = [&]() {
-        dfree(d_err); dfree(flags); dfree(scans); dfree(tmp); dfree(cslot); dfree(ipos); dfree(over);
+        dfree(d_err); dfree(flags); dfree(scans); dfree(tmp); dfree(cslot); dfree(ipos); dfree(over); dfree(dofc);
+        dfree(inc_c);
     };
 #define TRY(x) do { int _r = (x); if (_r) { cleanup(); df_plan_free(p); return _r; } } while (0)
 #define TRYC(x) do { cudaError_t _e = (x); if (_e != cudaSuccess) { cleanup(); df_plan_free(p); return cuda_status(_e, #x); } } while (0)
@@ -1278,27 +1290,27 @@ int df_plan_build(const double* nodes, int64_t nN, const int32_t* tets, int64_t 
     int h_flags[2] = {0, 0};
     if (nT > 0) {
         TRY(dalloc(&p->inv, (int64_t)dfk::kInv * nT, "df canonical invariants"));
-        TRY(dalloc(&p->dofc, 20 * nT, "df canonical DOF ids"));
+        TRY(dalloc(&dofc, 20 * nT, "df canonical DOF ids"));
         TRY(dalloc(&cslot, nT, "df canonical slots"));
         dfk::k_prep3<<<grid_for(nT, T), T, 0, s>>>(nodes, nN, tets, nT, edges, nE, tris, nTri, t2f, t2e, edge_len,
-                                                   p->inv, p->dofc, cslot, p->gscale, d_err, d_err + 1);
+                                                   p->inv, dofc, cslot, p->gscale, d_err, d_err + 1);
         TRYC(cudaGetLastError());
         TRYC(cudaMemcpyAsync(h_flags, d_err, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
         TRYC(cudaStreamSynchronize(s));
     }
     p->canon = nT > 0 && h_flags[0] == 0 && h_flags[1] == 0;
     if (p->canon) {
-        TRY(dalloc(&p->inc_c, n_inc, "df canonical incidences"));
+        TRY(dalloc(&inc_c, n_inc, "df canonical incidences"));
         if (n_inc > 0) {
-            dfk::k_inc_canon<<<grid_for(n_inc, T), T, 0, s>>>(inc, n_inc, cslot, p->inc_c);
+            dfk::k_inc_canon<<<grid_for(n_inc, T), T, 0, s>>>(inc, n_inc, cslot, inc_c);
             TRYC(cudaGetLastError());
         }
         TRY(dalloc(&ipos, 20 * n_inc, "df CSR positions of the incidences"));
         TRY(dalloc(&over, n_ent, "df position check"));
         if (n_ent > 0) {
-            dfk::k_inc_pos<<<grid_for(n_ent * 32, T, 152u * 64u), T, 0, s>>>(ent_list, n_ent, inc_ptr, p->inc_c, p->dofc,
+            dfk::k_inc_pos<<<grid_for(n_ent * 32, T, 152u * 64u), T, 0, s>>>(ent_list, n_ent, inc_ptr, inc_c, dofc,
                                                                             indptr, indices, ipos);
-            dfk::k_pos_check<<<grid_for(n_ent * 32, T, 152u * 64u), T, 0, s>>>(ent_list, n_ent, inc_ptr, p->inc_c, indptr,
+            dfk::k_pos_check<<<grid_for(n_ent * 32, T, 152u * 64u), T, 0, s>>>(ent_list, n_ent, inc_ptr, inc_c, indptr,
                                                                               ipos, over);
             TRYC(cudaGetLastError());
         }
@@ -1307,7 +1319,7 @@ int df_plan_build(const double* nodes, int64_t nN, const int32_t* tets, int64_t 
         TRY(dalloc(&p->mu_flag, 1, "df complex-mu flag"));
     } else {
         dfree(p->inv);
-        dfree(p->dofc);
+        dfree(dofc);
         TRY(dalloc(reinterpret_cast<dfk::Rec2**>(&p->recs), nT, "df records"));
         TRYC(cudaMemsetAsync(d_err, 0, 2 * sizeof(int), s));
         if (nT > 0) {
@@ -1368,15 +1380,16 @@ int df_plan_build(const double* nodes, int64_t nN, const int32_t* tets, int64_t 
             }
             TRY(dalloc(&p->pdesc, p->n_pos, "df position descriptors"));
             if (ragged) TRY(dalloc(&p->prows, p->n_pos, "df position rows"));
-            TRY(dalloc(&p->own_u, 2 * ng * dfk::kKmax, "df own column units"));
-            p->own_stride = 2 * ng;
             unsigned long long* n_own = reinterpret_cast<unsigned long long*>(flags);
-            TRYC(cudaMemsetAsync(n_own, 0, sizeof(unsigned long long), s));
-            dfk::k_pos_desc<<<grid_for(ng * 32, T, 152u * 64u), T, 0, s>>>(
-                ents, ng, partner, inc_ptr, p->inc_c, indptr, ipos, scans, p->pdesc, p->prows, p->own_u, n_own);
+            TRYC(cudaMemsetAsync(n_own, 0, 2 * sizeof(unsigned long long), s));
+            dfk::k_own_count<<<grid_for(ng, T), T, 0, s>>>(ents, ng, inc_ptr, inc_c, n_own);
             TRYC(cudaGetLastError());
             TRYC(cudaMemcpyAsync(&p->n_own, n_own, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
             TRYC(cudaStreamSynchronize(s));
+            TRY(dalloc(&p->own_u, p->n_own * dfk::kKmax, "df own column units"));
+            dfk::k_pos_desc<<<grid_for(ng * 32, T, 152u * 64u), T, 0, s>>>(
+                ents, ng, partner, inc_ptr, inc_c, indptr, ipos, scans, p->pdesc, p->prows, p->own_u, p->n_own, n_own + 1);
+            TRYC(cudaGetLastError());
             TRY(dalloc(&p->own_r, 4 * p->n_own, "df own column sums"));
         }
     }
@@ -1417,7 +1430,7 @@ int df_fill(const DfPlan& p, int64_t nT, const int32_t* partner, const int64_t* 
     }
     if (p.n_groups > 0 && p.canon && p.n_pos <= dfk::kSmallPos) {
         EMG_CUDA(launch_pdl(dfk::k_fill_small, dim3(grid_for(p.n_pos, dfk::kFillThreads)), dim3(dfk::kFillThreads), 0, s, 0,
-                            p.st, p.n_pos, p.pdesc, p.prows, p.n_pos, p.own_u, p.own_stride, p.tscale, p.mu_flag,
+                            p.st, p.n_pos, p.pdesc, p.prows, p.n_pos, p.own_u, p.n_own, p.tscale, p.mu_flag,
                             reinterpret_cast<double2*>(E), reinterpret_cast<double2*>(B)));
     } else if (p.n_groups > 0 && p.canon) {
         const unsigned g = grid_for(p.n_pos, dfk::kFillThreads), go = grid_for(p.n_own, dfk::kFillThreads);
@@ -1425,9 +1438,9 @@ int df_fill(const DfPlan& p, int64_t nT, const int32_t* partner, const int64_t* 
         auto* B2 = reinterpret_cast<double2*>(B);
         // one of the two instantiations returns at once: which one is only known on the device
         if (p.n_own > 0) {
-            dfk::k_fill_own<false><<<go, dfk::kFillThreads, 0, s>>>(p.st, p.n_own, p.own_stride, p.own_u, p.tscale,
+            dfk::k_fill_own<false><<<go, dfk::kFillThreads, 0, s>>>(p.st, p.n_own, p.own_u, p.tscale,
                                                                    p.mu_flag, p.own_r);
-            dfk::k_fill_own<true><<<go, dfk::kFillThreads, 0, s>>>(p.st, p.n_own, p.own_stride, p.own_u, p.tscale,
+            dfk::k_fill_own<true><<<go, dfk::kFillThreads, 0, s>>>(p.st, p.n_own, p.own_u, p.tscale,
                                                                   p.mu_flag, p.own_r);
         }
         dfk::k_fill_st<false><<<g, dfk::kFillThreads, 0, s>>>(p.st, p.n_pos, p.pdesc, p.prows, p.n_pos, p.own_r, p.tscale,

@@ -15,19 +15,16 @@ struct DfPlan {
     double2* gscale = nullptr;   // per-tet FP64 scales of the curl-curl and mass blocks
     float4* tscale = nullptr;    // per-tet complex material scales (written by each fill)
     // canonical-frame fill (every tet's orientations follow one vertex order): per-tet
-    // invariants (43 x nT float pairs), DOF ids in canonical slot order (nT x 20),
-    // incidences with canonical slots, position descriptors, and the staging
-    // buffer of the element blocks
+    // invariants (43 x nT float pairs), position descriptors, and the staging buffer of the
+    // element blocks
     bool canon = false;
     float2* inv = nullptr;
-    int32_t* dofc = nullptr;
-    int64_t* inc_c = nullptr;
     uint2* pdesc = nullptr;      // per CSR position of the entities' first rows: the staged units summed there
     longlong2* prows = nullptr;    // and its positions in both rows (NULL: i and i + n_pos)
     int64_t n_pos = 0;
-    uint32_t* own_u = nullptr;   // own columns of edges with more than two tets: staged units, kDfMaxInc arrays
+    uint32_t* own_u = nullptr;   // own columns of edges with more than two tets: kDfMaxInc arrays of n_own staged units
     double2* own_r = nullptr;    // and their sums in a fill
-    int64_t n_own = 0, own_stride = 0;
+    int64_t n_own = 0;
     float4* st = nullptr;        // staged element blocks: 32 B per (tet, row pair, column), tets interleaved by 8
     int* mu_flag = nullptr;      // set by a fill whose mu^-1 has an imaginary part
     int2* groups = nullptr;      // warp work units: (first index into gents, entity count)

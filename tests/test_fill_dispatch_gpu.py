@@ -105,3 +105,24 @@ def test_tensor_fan(torch_cuda, ring):
     Eo, Bo = oracle.tet_mass_stiffness_matrices(field, er, ur)
     assert np.array_equal(E.indptr, Eo.indptr) and np.array_equal(E.indices, Eo.indices)
     assert rel_to_rowmax(E, Eo) <= TOL and rel_to_rowmax(B, Bo) <= TOL
+
+
+def test_memory_of_a_plan(torch_cuda):
+    """A plan keeps per tet its staged blocks (6400 B), invariants, scales, record and incidences, per matrix
+    entry a column and half a descriptor, and own-column tables for edges alone."""
+    torch = torch_cuda
+    from emerge_gb300.assembly import AssemblyPlan
+    from emerge_gb300.mesh import Nedelec2Basis, unit_cube
+    m = unit_cube(40)
+    field = Nedelec2Basis(m)
+    AssemblyPlan(Nedelec2Basis(unit_cube(2)))      # the library and its tables are loaded
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    used = lambda: -torch.cuda.mem_get_info()[0] - torch.cuda.memory_reserved()  # noqa: E731
+    before = used()
+    plan = AssemblyPlan(field)
+    torch.cuda.synchronize()
+    N, nnz = int(field.n_field), int(plan.nnz)
+    per_tet = 6400 + 344 + 32 + 16 + 544 + 80
+    bound = per_tet * m.n_tets + 28 * N + (4 + 4) * nnz + 2 * m.n_edges * (12 * 4 + 4 * 16)
+    assert used() - before <= bound + (64 << 20)   # 2 MB pages of some 25 arrays
