@@ -33,6 +33,7 @@
 
 #include "emg_gj.cuh"
 #include "emg_krylov.cuh"
+#include "emg_rules.cuh"
 
 namespace emg {
 namespace f64 {
@@ -285,11 +286,13 @@ __global__ void __maxnreg__(200)   // 256 threads leave room on the SM for a CTA
     const uint32_t taddr = tmem_base;
     constexpr int kChunks = kTile / kKc;
     bool ok = true;
+    int committed = 0;                 // chunks whose MMAs were issued (uniform)
 #pragma unroll 1
     for (int ch = 0; ch < kChunks; ++ch) {
         char* abase = base + (ch & 1) * kBuf;
         char* bbase = abase + 2 * kDig * kAPlane;
-        if (ch >= 2) ok = mbar_wait(smem_u32(&mbar[ch & 1]), 0u);   // the MMAs that read this buffer are done
+        // the MMAs that read this buffer are done
+        if (ch >= 2) ok = mbar_wait(smem_u32(&mbar[rules::chunk_buffer(ch - 2)]), rules::chunk_parity(ch - 2));
         {
             double v[8];
             char* dst = abase + (am >> 3) * 256 + akb * 128 + (am & 7) * 16;
@@ -343,6 +346,7 @@ __global__ void __maxnreg__(200)   // 256 threads leave room on the SM for a CTA
                              smem_u32(&mbar[ch & 1]))
                          : "memory");
         }
+        ++committed;
         if (ch + 1 < kChunks) load(ch + 1);
     }
     // this thread's outputs: column c0 + 32 (warp % 4) + lane, rows r0 + 16 (warp / 4) + n, four at a
@@ -359,9 +363,9 @@ __global__ void __maxnreg__(200)   // 256 threads leave room on the SM for a CTA
         }
     };
     if (MODE != kRow) fetch(0);
-    // chunk 3 is the second of its buffer, chunk 2 of the other (after a time-out: one more bounded wait)
-    if (!mbar_wait(smem_u32(&mbar[0]), ok ? 1u : 0u)) ok = false;
-    if (!mbar_wait(smem_u32(&mbar[1]), ok ? 1u : 0u)) ok = false;
+    // the last two chunks, also after a time-out (one more bounded wait each before the TMEM goes)
+    for (int c = rules::pending_from(committed); c < committed; ++c)
+        if (!mbar_wait(smem_u32(&mbar[rules::chunk_buffer(c)]), rules::chunk_parity(c))) ok = false;
     ok = !__syncthreads_or(!ok);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (ok) {

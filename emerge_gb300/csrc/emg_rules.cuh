@@ -26,5 +26,13 @@ constexpr int64_t dot_blocks(int64_t n, int64_t Bc, bool fp32) {
     return (n + dot_rows(n, Bc, fp32) - 1) / dot_rows(n, Bc, fp32);
 }
 
+// K chunks of a tile through two shared buffers (emg_tc.cu, emg_fp64.cu): the MMAs of chunk c arrive at the
+// mbarrier of its buffer, and a wait for them names the parity of that barrier's phase.  Of
+// ``committed`` chunks those from pending_from on may still run: a tile that ends, also early after a
+// time-out, waits for these before its tensor memory goes.
+constexpr int chunk_buffer(int c) { return c & 1; }
+constexpr unsigned chunk_parity(int c) { return (unsigned)(c >> 1) & 1u; }
+constexpr int pending_from(int committed) { return committed > 2 ? committed - 2 : 0; }
+
 }  // namespace rules
 }  // namespace emg

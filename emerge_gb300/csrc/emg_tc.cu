@@ -21,6 +21,7 @@
 
 #include "emg_gj.cuh"
 #include "emg_krylov.cuh"
+#include "emg_rules.cuh"
 
 namespace emg {
 namespace tc {
@@ -517,11 +518,12 @@ __global__ void __launch_bounds__(kSpThreads, 1) k_slab_split(int64_t w, int64_t
         }
     };
     bool ok = true;
+    int committed = 0;                 // chunks whose MMAs were issued (uniform)
     for (int ch = 0; ch < nk; ++ch) {
-        const int buf = ch & 1;
+        const int buf = rules::chunk_buffer(ch);
         char* cb = base + buf * kSpChunk;
         // the MMAs that read this buffer two chunks ago are done
-        if (ch >= 2 && ok && !mbar_wait(smem_u32(&mbar[buf]), (uint32_t)(((ch >> 1) - 1) & 1))) ok = false;
+        if (ch >= 2 && !mbar_wait(smem_u32(&mbar[buf]), rules::chunk_parity(ch - 2))) ok = false;
         if (ok) split(cb);
         if (ch >= 4 && __all_sync(0xffffffffu, ok)) {   // chunk ch - 4's MMAs were committed before those
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -576,14 +578,15 @@ __global__ void __launch_bounds__(kSpThreads, 1) k_slab_split(int64_t w, int64_t
                              smem_u32(&mbar[buf]))
                          : "memory");
         }
+        ++committed;
         if (ch + 1 < nk) {
             load_s(ch + 1);
             load_y(ch + 1);
         }
     }
-    // the last two chunks' MMAs (one more bounded wait each after a time-out, before the TMEM goes)
-    for (int ch = max(0, nk - 2); ch < nk; ++ch)
-        if (!mbar_wait(smem_u32(&mbar[ch & 1]), (uint32_t)((ch >> 1) & 1))) ok = false;
+    // the last two chunks, also after a time-out (one more bounded wait each before the TMEM goes)
+    for (int c = rules::pending_from(committed); c < committed; ++c)
+        if (!mbar_wait(smem_u32(&mbar[rules::chunk_buffer(c)]), rules::chunk_parity(c))) ok = false;
     if (!ok) atomicExch(status, 1);
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");

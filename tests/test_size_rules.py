@@ -31,3 +31,37 @@ for (long long n : {1ll, 63ll, 64ll, 65ll, 2282ll, 20000ll, 98304ll, 265000ll, 6
         if (dot_groups(Bc) < 1 || dot_tile(Bc) > 128) { std::printf("tile %lld\n", Bc); return 1; }
     }
 """)
+
+
+def test_waits_for_chunks(tmp_path):
+    """The waits of the two-buffer pipelines against a model of the barriers: a wait of a parity returns when the
+    barrier's current phase has the other one.  The waits after the loop, also when it ends early, cover every
+    chunk that is committed and may still run, and none of them outlasts its chunk."""
+    _run(tmp_path, r"""
+for (int committed = 0; committed <= 40; ++committed)
+    for (int done = std::max(0, committed - 2); done <= committed; ++done) {   // chunks 0 .. done - 1 have arrived
+        int arrivals[2] = {0, 0};
+        for (int c = 0; c < done; ++c) ++arrivals[chunk_buffer(c)];
+        auto returns = [&](int c) { return (unsigned)(arrivals[chunk_buffer(c)] & 1) != chunk_parity(c); };
+        if (pending_from(committed) < 0 || (committed >= 2 && pending_from(committed) > committed - 2)) return 1;
+        for (int c = pending_from(committed); c < committed; ++c)
+            if (returns(c) != (c < done)) { std::printf("committed %d done %d chunk %d\n", committed, done, c); return 1; }
+    }
+for (int ch = 2; ch < 40; ++ch)                    // the wait before a buffer is written again
+    for (int done = ch - 2; done <= ch; ++done) {
+        int arrivals[2] = {0, 0};
+        for (int c = 0; c < done; ++c) ++arrivals[chunk_buffer(c)];
+        if (chunk_buffer(ch - 2) != chunk_buffer(ch)) return 1;
+        if (((unsigned)(arrivals[chunk_buffer(ch)] & 1) != chunk_parity(ch - 2)) != (done >= ch - 1)) return 1;
+    }
+""")
+
+
+def test_pipelines_follow_the_rules():
+    """Both two-buffer kernels name their barriers and parities by these rules only."""
+    import re
+    for name in ("emg_tc.cu", "emg_fp64.cu"):
+        text = open(os.path.join(ROOT, "emerge_gb300", "csrc", name)).read()
+        waits = re.findall(r"mbar_wait\(smem_u32\(&mbar\[(.*?)\]\), (.*?)\)\)?[; ]", text)
+        assert len(waits) == 2 and all("rules::chunk_parity(" in p for _, p in waits), waits
+        assert "for (int c = rules::pending_from(committed); c < committed; ++c)" in text
