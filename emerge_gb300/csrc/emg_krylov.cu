@@ -971,7 +971,11 @@ void spmv(const emg_rplan* p, int64_t Bc, const int32_t* cmat, int64_t Bm, const
           const double2* Bv, double2* Y, cudaStream_t s) {
     const int64_t n = p->ns;
     const unsigned g = (unsigned)((n * kry::kSpmvLanes + 127) / 128);
-    if (Bc <= 2)
+    // (one column in the kernel for two was slower than a thread per row from 76k rows on: 138k rows 116 us, a
+    // thread per row 101, a kernel of its own 70)
+    if (Bc == 1)
+        kry::k_spmv_w<1><<<g, 128, 0, s>>>(n, (int)Bc, cmat, Bm, p->rptr, p->rind, A, X, Bv, Y);
+    else if (Bc == 2)
         kry::k_spmv_w<2><<<g, 128, 0, s>>>(n, (int)Bc, cmat, Bm, p->rptr, p->rind, A, X, Bv, Y);
     else if (Bc <= 4)
         kry::k_spmv_w<4><<<g, 128, 0, s>>>(n, (int)Bc, cmat, Bm, p->rptr, p->rind, A, X, Bv, Y);
