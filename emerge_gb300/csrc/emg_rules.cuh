@@ -34,5 +34,41 @@ constexpr int chunk_buffer(int c) { return c & 1; }
 constexpr unsigned chunk_parity(int c) { return (unsigned)(c >> 1) & 1u; }
 constexpr int pending_from(int committed) { return committed > 2 ? committed - 2 : 0; }
 
+// K splits of a tiled slab product: two CTAs per SM, at least 256 of K and at most max_splits each.
+constexpr int gemm_splits(int64_t tiles, int64_t w, int max_splits) {
+    int64_t sp = (2 * 152 + tiles - 1) / (tiles > 1 ? tiles : 1);
+    const int64_t most = w / 256 > 1 ? w / 256 : 1;
+    if (sp > most) sp = most;
+    if (sp > max_splits) sp = max_splits;
+    return sp > 1 ? (int)sp : 1;
+}
+// CTAs of a cluster of the split-TF32 product (``col_tiles`` column tiles in all groups together): doubled while the CTAs
+// fit one wave and each keeps two chunks of 32.
+constexpr int split_ranks(int64_t w, int64_t col_tiles, int max_splits) {
+    const int64_t tiles = (w + 127) / 128 * col_tiles;
+    int ranks = 1;
+    while (ranks < 8 && 2 * ranks <= max_splits && tiles * 2 * ranks <= 152 && w >= 2 * ranks * 64) ranks *= 2;
+    return ranks;
+}
+// FP32 groups of up to 16 columns on wide slabs: 128 x 16 CUDA-core tiles (k_slab_gemm16) where they are
+// faster than what the slab takes else, row blocks (rows8) or split-TF32 tiles.  Estimates in us.  The
+// tiles take 0.1 per K of a split, two thirds of it more for every CTA that an SM has beyond the first,
+// and 4 at the launch, which the others hide under the one before; row blocks 0.0075 per K and CTA of an
+// SM; the split tiles 2.4 per 32 of K of a cluster's CTA, twice where clusters of eight do not all fit.
+// Measured (tiles / else): 2000 wide, one group 31 / 47, two 50 / 44, three 70 / 88; 2500, two 73 / 99;
+// 1500, four 52 / 61; 1000, two 33 / 17 (row blocks).  Over 700 to 2500 wide and one to four groups of 8 and
+// 16 columns the choice is within 4 % of the faster one, launches counted.
+constexpr bool narrow_tiles_win(int64_t w, int G, int maxcol, int max_splits, bool rows8) {
+    const int64_t tiles = (w + 127) / 128 * G;
+    const int sp = gemm_splits(tiles, w, max_splits), ranks = split_ranks(w, G, max_splits);
+    const int64_t rounds = (tiles * sp + 151) / 152;
+    const double kper = (double)((w + sp - 1) / sp);
+    const double narrow = 0.1 * kper * (0.35 + 0.65 * rounds) + 6;
+    const double rows = 0.0075 * w * ((double)((w + 7) / 8 * G) / 152) * (maxcol <= 8 ? 1.0 : 1.2) + 4;
+    const double chunks = (double)(((w + ranks - 1) / ranks + 31) / 32);
+    const double split = 2.4 * chunks * (ranks == 8 && tiles > 14 ? 2 : 1) + 5;
+    return maxcol <= 16 && narrow < (rows8 ? rows : split);
+}
+
 }  // namespace rules
 }  // namespace emg

@@ -34,6 +34,7 @@
 
 #include "emg_gj.cuh"
 #include "emg_krylov.cuh"
+#include "emg_rules.cuh"
 
 namespace emg {
 namespace slab {
@@ -1007,14 +1008,6 @@ __global__ void __launch_bounds__(kThreads) k_slab_gemm16(int64_t w, int64_t row
         }
 }
 
-// K splits of a wide-group product: enough CTAs for two per SM, at least 256
-// columns of K per split, at most max_splits (8 unless tuned).
-inline int gemm_splits(int64_t tiles, int64_t w, int max_splits = 8) {
-    int64_t sp = (2 * 152 + tiles - 1) / std::max<int64_t>(tiles, 1);
-    sp = std::min<int64_t>(sp, std::max<int64_t>(1, w / 256));
-    return (int)std::max<int64_t>(1, std::min<int64_t>(sp, std::max(1, max_splits)));
-}
-
 }  // namespace slab
 }  // namespace emg
 
@@ -1546,6 +1539,11 @@ struct SlabPrecond : emg::Precond {
                 groups.push_back({cfac[c], (int32_t)c, 1, 0});
         }
     }
+    // FP32 groups that share rows of the inverse between columns: wide ones, and several of four or
+    // more columns (4 columns of two factors on slabs of 941 take 24 us by rows, 17 by row blocks)
+    bool wide32(int maxcol) const {
+        return maxcol >= s->wide || (maxcol >= 4 && !s->use_tc && (int64_t)maxcol * (int64_t)groups.size() >= s->wide);
+    }
     int prepare(int64_t bc) override {
         using namespace emg;
         const size_t bytes = (s->prec == 1 ? sizeof(float2) : sizeof(double2)) * (size_t)s->n * (size_t)bc;
@@ -1563,7 +1561,7 @@ struct SlabPrecond : emg::Precond {
         // split-K scratch for the wide-group products (largest need over the slabs)
         int maxcol = 0;
         for (const auto& g : groups) maxcol = std::max(maxcol, (int)g.ncol);
-        if (s->prec == 2 && maxcol >= s->wide) {
+        if (s->prec == 2 ? maxcol >= s->wide : maxcol <= emg::slab::kNarrowN && wide32(maxcol)) {
             const int64_t ct = (maxcol + emg::slab::kTile - 1) / emg::slab::kTile, G = (int64_t)groups.size();
             size_t need = 0;
             int64_t tiles_max = 0;
@@ -1574,10 +1572,10 @@ struct SlabPrecond : emg::Precond {
             for (int i = 0; i < s->m; ++i) {
                 const int64_t w = s->off[i + 1] - s->off[i];
                 const int64_t tiles = (narrow ? 1 : ct) * ((w + tm - 1) / tm) * G;
-                const int sp = emg::slab::gemm_splits(tiles, w, s->max_splits);
+                const int sp = emg::rules::gemm_splits(tiles, w, s->max_splits);
                 tiles_max = std::max(tiles_max, tiles);
                 if (sp > 1)
-                    need = std::max(need, (size_t)tiles * sp * (size_t)slot * sizeof(double2));
+                    need = std::max(need, (size_t)tiles * sp * (size_t)slot * (s->prec == 2 ? sizeof(double2) : sizeof(float2)));
             }
             if (need > s->kpart_bytes) {
                 if (s->kpart) cudaFree(s->kpart);
@@ -1622,7 +1620,7 @@ struct SlabPrecond : emg::Precond {
         const unsigned G = (unsigned)groups.size();
         int maxcol = 0;
         for (const auto& g : groups) maxcol = std::max(maxcol, (int)g.ncol);
-        if constexpr (sizeof(R) == 8) {
+        {
             static bool narrow_attr[64] = {false};   // per device; the 128 x 16 tiles need 74 KB
             int dev = 0;
             EMG_CUDA(cudaGetDevice(&dev));
@@ -1633,17 +1631,28 @@ struct SlabPrecond : emg::Precond {
             }
         }
         // dense slab product: rows of few columns for groups narrower than s->wide; wider FP32
-        // groups by row blocks or on the tensor cores (TF32 products if asked for, else split
-        // ones), FP64 groups as 128 x 16 tiles up to 16 columns and 64 x 64 tiles above
+        // groups by row blocks, as 128 x 16 tiles (up to 16 columns, rules::narrow_tiles_win) or on the
+        // tensor cores (TF32 products if asked for, else split ones), FP64 groups as 128 x 16
+        // tiles up to 16 columns and 64 x 64 tiles above
         int rc = EMG_OK;
+        auto narrow = [&](int64_t w, int64_t i, R alpha, int beta) {
+            const int64_t rt = (w + kNarrowM - 1) / kNarrowM;
+            const int sp = rules::gemm_splits(rt * G, w, s->max_splits);
+            k_slab_gemm16<R><<<dim3(1u, (unsigned)(rt * sp), G), kThreads, sizeof(NarrowTile<R>), st>>>(
+                w, s->off[i], Bc, s->groups, Sinv, s->totD, s->offD[i], Y, alpha, beta, Z, sp,
+                static_cast<T*>(s->kpart), s->kcnt);
+        };
         auto dense = [&](int64_t w, int64_t i, R alpha, int beta) {
             if constexpr (sizeof(R) == 4) {
-                // (several groups of four or more columns go there too: 4 columns of two factors on
-                // slabs of 941 take 24 us by rows, 17 by row blocks)
-                if (maxcol >= s->wide || (maxcol >= 4 && !s->use_tc && (int64_t)maxcol * G >= s->wide)) {
+                if (wide32(maxcol)) {
                     const auto* Sf = reinterpret_cast<const float2*>(Sinv);
                     const auto* Yf = reinterpret_cast<const float2*>(Y);
-                    if (!s->use_tc && rows8_wins(w, (int)G, maxcol)) {
+                    const bool by_rows = !s->use_tc && rows8_wins(w, (int)G, maxcol);
+                    if (!s->use_tc && rules::narrow_tiles_win(w, (int)G, maxcol, s->max_splits, by_rows)) {
+                        narrow(w, i, alpha, beta);
+                        return;
+                    }
+                    if (by_rows) {
                         const cudaError_t e = rows8(w, s->off[i], Bc, s->groups, (int)G, maxcol, Sf, s->totD, s->offD[i], Yf,
                                                     (float)alpha, beta, reinterpret_cast<float2*>(Z), st);
                         if (e != cudaSuccess && !rc) rc = cuda_status(e, "slab row-block product");
@@ -1662,16 +1671,12 @@ struct SlabPrecond : emg::Precond {
             }
             if constexpr (sizeof(R) == 8) {
                 if (maxcol >= s->wide && maxcol <= kNarrowN) {
-                    const int64_t rt = (w + kNarrowM - 1) / kNarrowM;
-                    const int sp = gemm_splits(rt * G, w, s->max_splits);
-                    k_slab_gemm16<R><<<dim3(1u, (unsigned)(rt * sp), G), kThreads, sizeof(NarrowTile<R>), st>>>(
-                        w, s->off[i], Bc, s->groups, Sinv, s->totD, s->offD[i], Y, alpha, beta, Z, sp,
-                        static_cast<T*>(s->kpart), s->kcnt);
+                    narrow(w, i, alpha, beta);
                     return;
                 }
                 if (maxcol >= s->wide) {
                     const int64_t ct = (maxcol + kTile - 1) / kTile, rt = (w + kTile - 1) / kTile;
-                    const int sp = gemm_splits(ct * rt * G, w, s->max_splits);
+                    const int sp = rules::gemm_splits(ct * rt * G, w, s->max_splits);
                     k_slab_gemm<R><<<dim3((unsigned)ct, (unsigned)(rt * sp), G), kThreads, 0, st>>>(
                         w, s->off[i], Bc, s->groups, Sinv, s->totD, s->offD[i], Y, alpha, beta, Z, sp,
                         static_cast<T*>(s->kpart), s->kcnt);

@@ -1102,10 +1102,7 @@ int tc_slab_split(int64_t w, int64_t row0, int64_t Bc, const void* groups, int G
         if (dev < 64) attr[dev] = true;
     }
     const int ct = (maxcol + tc::kN - 1) / tc::kN, rt = (int)((w + tc::kM - 1) / tc::kM);
-    // K split: double it while the CTAs fit one wave and each keeps two chunks
-    int ranks = 1;
-    while (ranks < 8 && 2 * ranks <= max_splits && (int64_t)ct * rt * G * 2 * ranks <= 152 && w >= 2 * ranks * 2 * tc::kK)
-        ranks *= 2;
+    const int ranks = rules::split_ranks(w, (int64_t)ct * G, max_splits);
     EMG_CUDA(launch_pdl(tc::k_slab_split, dim3((unsigned)ranks, (unsigned)rt, (unsigned)(G * ct)), dim3(tc::kSpThreads),
                         tc::kSpSmem + 1024, st, ranks, w, row0, Bc, static_cast<const tc::TcGroup*>(groups), G, Sinv, totD,
                         offD, Y, alpha, beta, Out, status));

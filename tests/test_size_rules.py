@@ -65,3 +65,35 @@ def test_pipelines_follow_the_rules():
         waits = re.findall(r"mbar_wait\(smem_u32\(&mbar\[(.*?)\]\), (.*?)\)\)?[; ]", text)
         assert len(waits) == 2 and all("rules::chunk_parity(" in p for _, p in waits), waits
         assert "for (int c = rules::pending_from(committed); c < committed; ++c)" in text
+
+
+def test_narrow_tiles(tmp_path):
+    """The choice between 128 x 16 tiles and row blocks or split tiles against measured times (width, groups, columns,
+    us of the latter, us of the tiles, whose launch takes 4 more): within 4 % of the faster one."""
+    _run(tmp_path, r"""
+const struct { int w, G, c; double other, tiles; } t[] = {
+{700, 1, 8, 8.5, 32.2}, {700, 1, 16, 8.6, 32.7}, {700, 2, 8, 10.2, 32.3}, {700, 2, 16, 12.8, 32.6}, {700, 3,
+8, 10.3, 32.5}, {700, 3, 16, 13.0, 33.0}, {700, 4, 8, 14.4, 32.7}, {700, 4, 16, 18.1, 33.0}, {1000, 1, 8,
+11.0, 32.4}, {1000, 1, 16, 11.5, 32.7}, {1000, 2, 8, 13.6, 32.8}, {1000, 2, 16, 17.4, 33.1}, {1000, 3, 8,
+19.4, 32.7}, {1000, 3, 16, 24.9, 33.3}, {1000, 4, 8, 23.4, 33.0}, {1000, 4, 16, 24.7, 33.3}, {1250, 1, 8,
+15.5, 29.8}, {1250, 1, 16, 20.6, 30.6}, {1250, 2, 8, 23.0, 30.3}, {1250, 2, 16, 29.0, 30.6}, {1250, 3, 8,
+29.2, 30.6}, {1250, 3, 16, 29.2, 30.9}, {1250, 4, 8, 51.3, 49.9}, {1250, 4, 16, 52.1, 50.2}, {1500, 1, 8,
+18.6, 31.2}, {1500, 1, 16, 20.1, 31.8}, {1500, 2, 8, 26.9, 31.6}, {1500, 2, 16, 33.5, 31.9}, {1500, 3, 8,
+33.4, 51.3}, {1500, 3, 16, 33.6, 52.2}, {1500, 4, 8, 59.9, 51.9}, {1500, 4, 16, 60.9, 51.8}, {1750, 1, 8,
+21.7, 32.7}, {1750, 1, 16, 22.4, 33.0}, {1750, 2, 8, 31.2, 53.2}, {1750, 2, 16, 38.2, 53.5}, {1750, 3, 8,
+70.0, 53.2}, {1750, 3, 16, 70.3, 54.0}, {1750, 4, 8, 72.2, 74.9}, {1750, 4, 16, 73.2, 75.1}, {2000, 1, 8,
+30.7, 31.2}, {2000, 1, 16, 47.0, 31.5}, {2000, 2, 8, 44.0, 49.9}, {2000, 2, 16, 44.7, 50.6}, {2000, 3, 8,
+87.5, 69.6}, {2000, 3, 16, 88.7, 70.1}, {2000, 4, 8, 88.6, 92.0}, {2000, 4, 16, 90.1, 91.8}, {2250, 1, 8,
+35.4, 29.0}, {2250, 1, 16, 51.3, 29.7}, {2250, 2, 8, 46.6, 48.7}, {2250, 2, 16, 47.7, 48.9}, {2250, 3, 8,
+91.3, 87.7}, {2250, 3, 16, 92.7, 88.3}, {2250, 4, 8, 92.7, 104.5}, {2250, 4, 16, 93.8, 105.2}, {2500, 1, 8,
+50.8, 51.2}, {2500, 1, 16, 51.5, 51.1}, {2500, 2, 8, 98.6, 73.4}, {2500, 2, 16, 98.8, 73.4}, {2500, 3, 8,
+99.4, 99.8}, {2500, 3, 16, 101.3, 100.5}, {2500, 4, 8, 192.6, 133.5}, {2500, 4, 16, 194.7, 133.0}};
+auto ld = [](long long w) { return (w + 3) / 4 * 4 + 2 + (16 - (w + 3) / 4 * 4 % 16) % 16; };
+for (const auto& m : t) {
+    const long long rounds = ((m.w + 7) / 8 * m.G + 151) / 152;            // rows8_wins
+    const bool rows8 = 64 * ld(m.w) <= 200 * 1024 && (rounds == 1 || rounds * m.w * ((m.c + 7) / 8 * 8) <= 45000);
+    const double got = narrow_tiles_win(m.w, m.G, m.c, 8, rows8) ? m.tiles + 4 : m.other;
+    if (got > 1.04 * std::min(m.tiles + 4, m.other)) { std::printf("%d %d %d: %g\\n", m.w, m.G, m.c, got); return 1; }
+}
+if (narrow_tiles_win(2000, 1, 17, 8, false)) return 1;
+""")

@@ -183,3 +183,26 @@ def test_a_solve_does_not_wait_for_the_gpu(system, precision, cols):
     y = slab.apply(b, [0] * cols)
     assert not done.query()
     assert torch.equal(torch.view_as_real(y), torch.view_as_real(ref))
+
+
+@pytest.mark.parametrize("n", [1473, 1505])
+def test_narrow_tiles_of_wide_slabs(system, n):
+    """Four groups of up to 16 columns on slabs so wide that the 128 x 16 tiles serve them."""
+    torch = system[0]
+    from emerge_gb300.solver import RestrictedSystem, SlabFactor
+    ip = torch.arange(0, n * n + 1, n, dtype=torch.int64, device="cuda")
+    ix = torch.arange(n, dtype=torch.int32, device="cuda").repeat(n)
+    slab = SlabFactor(RestrictedSystem(ip, ix, n * n, np.arange(n)), np.arange(n))
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    rnd = lambda *s: torch.view_as_complex(torch.randn((*s, 2), generator=gen, device="cuda", dtype=torch.float64))  # noqa: E731
+    A = [rnd(n, n) / (2 * n) ** 0.5 + 3.0 * torch.eye(n, device="cuda") for _ in range(4)]
+    slab.factor(torch.stack([a.reshape(-1) for a in A], dim=1).contiguous(), [0, 1, 2, 3], "fp32")
+    for sizes in ([4] * 4, [8] * 4, [9, 4, 1, 16], [16] * 4):
+        b = rnd(n, sum(sizes))
+        y = slab.apply(b, sum(([g] * c for g, c in enumerate(sizes)), []))
+        assert torch.equal(torch.view_as_real(y), torch.view_as_real(slab.apply(b, sum(([g] * c for g, c in enumerate(sizes)), []))))
+        for g, c in enumerate(sizes):
+            col = sum(sizes[:g])
+            r = A[g] @ y[:, col:col + c] - b[:, col:col + c]
+            # inverse and product: relative errors of a few n eps, condition below 100
+            assert float(torch.linalg.norm(r)) <= 200 * n * 2.0 ** -23 * float(torch.linalg.norm(b[:, col:col + c]))
