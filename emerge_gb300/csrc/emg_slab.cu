@@ -1733,6 +1733,13 @@ extern "C" int emg_slab_apply(emg_slab* s, int64_t Bc, const int32_t* cfac, cons
     EMG_CHECK_ARG(s->F > 0, "emg_slab_apply: no factorization");
     for (int64_t c = 0; c < Bc; ++c) EMG_CHECK_ARG(cfac[c] >= 0 && cfac[c] < s->F, "emg_slab_apply: cfac out of range");
     if (s->n == 0) return EMG_OK;
+    // the column tables come from this call's host arrays, which a graph would read again after they are gone
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    EMG_CUDA(cudaStreamIsCapturing((cudaStream_t)stream, &capture));
+    if (capture != cudaStreamCaptureStatusNone) {
+        set_error("emg_slab_apply: cannot be captured in a graph");
+        return EMG_ERR_CUDA;
+    }
     SlabPrecond M(s, Bc, cfac, (cudaStream_t)stream);
     int rc = M.prepare(Bc);
     if (rc) return rc;

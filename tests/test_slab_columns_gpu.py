@@ -206,3 +206,18 @@ def test_narrow_tiles_of_wide_slabs(system, n):
             r = A[g] @ y[:, col:col + c] - b[:, col:col + c]
             # inverse and product: relative errors of a few n eps, condition below 100
             assert float(torch.linalg.norm(r)) <= 200 * n * 2.0 ** -23 * float(torch.linalg.norm(b[:, col:col + c]))
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_a_solve_cannot_be_captured(system, precision):
+    """A captured solve would read the caller's column tables at every replay: refused, and the handle stays usable."""
+    torch, sysr, A, slab = system
+    from emerge_gb300._lib import EmgError
+    slab.factor(A, [0], precision)
+    b = torch.ones((sysr.n, 2), dtype=torch.complex128, device="cuda")
+    ref = slab.apply(b, [0, 0])
+    torch.cuda.synchronize()
+    with pytest.raises(EmgError):
+        with torch.cuda.graph(torch.cuda.CUDAGraph()):
+            slab.apply(b, [0, 0])
+    assert torch.equal(torch.view_as_real(slab.apply(b, [0, 0])), torch.view_as_real(ref))
