@@ -9,7 +9,12 @@
 // converts to FP64 with integer instructions when storing.  FP64 is used only
 // once per tet: for the geometry (plan) and the material scales (per fill).
 //
-// Work decomposition (entity-owner, as in emg_assembly.cu):
+// Meshes in which every tet's orientations follow one vertex order (the usual case) take the
+// canonical-frame fill in the second half of this file: element blocks per tet into a staging buffer
+// (k_elem), then an owner pass with a thread per CSR position (k_fill_st, k_fill_own, or k_fill_small
+// in one launch).  Other meshes take the per-lane fill k_fill_df of the first half.
+//
+// Work decomposition of the per-lane fill (entity-owner, as in emg_assembly.cu):
 //  * a warp owns one edge entity, or two face entities (rows r1/r2 each);
 //  * phase A computes the 2x2 blocks (row entity x edge column) of every
 //    incident tet, phase B the blocks with face columns; all lanes of a phase

@@ -1043,9 +1043,9 @@ struct emg_slab {
     size_t kpart_bytes = 0;
     int32_t* kcnt = nullptr;          // per-tile arrival counters (zero between launches)
     int64_t kcnt_n = 0;
-    int use_tc = 0;                   // wide-group products of FP32 factors on the tcgen05 tensor cores
-    int tc_factor = 1;                // rank-64 updates of FP32 factorizations on the tcgen05 tensor cores
-    int wide = 8;                     // column groups at least this wide use the tiled products
+    int use_tc = 0;                   // wide-group products of FP32 factors in plain TF32
+    int tc_factor = 1;                // rank-64 products of factorizations on the tcgen05 tensor cores
+    int wide = 8;                     // column groups at least this wide share rows of the inverse between columns
     int max_splits = 8;               // split-K cap of the tiled products
     int32_t* tc_status = nullptr;     // set by a tensor-core tile whose bounded wait ran out
 };
@@ -1412,8 +1412,8 @@ int slab_factor_t(emg_slab* s, int64_t F, const int32_t* amat_h, int64_t Bm, con
             // FP64: the pivot tiles have the side stream, row panel and update the caller's.  Tile k + 1
             // needs tile k and the update of step k - 1; the row panel of step k needs tile k, its
             // update overwrites what the lookahead reads.  A step is the longer of the two chains:
-            // row panel 36 us and update 37 (480 wide) to 115 (1250), or lookahead 10, seed 36 and
-            // Newton steps 25 (311 tiles of 737 on average: 42.8 ms a solve, 46.5 with the lookahead
+            // row panel 37 us and update 37 (480 wide) to 105 (1250), or lookahead 10, seed 36 and
+            // Newton steps 25 (311 tiles of 737 on average: 43.4 ms a solve; at 42.8 it took 46.5 with the lookahead
             // before the row panel on one stream).
             if constexpr (sizeof(R) == 8) {
                 auto step = [&](int q, int k, int la, cudaStream_t ts) {

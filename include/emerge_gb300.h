@@ -277,7 +277,8 @@ int emg_slab_levels(const emg_slab* slab, int64_t* off_out, int32_t* perm_out);
 int emg_slab_factor(emg_slab* slab, int precision, int64_t F, const int32_t* amat, int64_t Bm, const double* A,
                     int refine, void* stream);
 /* X_out = A_f^-1 X_in column by column, f = cfac[c] (HOST int32, Bc); X_in and
- * X_out are distinct DEVICE [n_solve][Bc] complex arrays. */
+ * X_out are distinct DEVICE [n_solve][Bc] complex arrays.  Ordered on ``stream``; waits for it only
+ * where tensor-core tiles ran, to read their status.  A capturing stream is refused. */
 int emg_slab_apply(emg_slab* slab, int64_t Bc, const int32_t* cfac, const double* X_in, double* X_out, void* stream);
 /* on != 0: the dense products of FP32-factor solves over wide column groups (see
  * emg_slab_set_wide_group) run on the tcgen05 tensor cores (TF32 products, FP32 accumulation);
@@ -294,12 +295,12 @@ int emg_slab_set_tensor_cores(emg_slab* slab, int on);
  * behind fem/solver.py's solve slot.) */
 int emg_slab_set_factor_tensor_cores(emg_slab* slab, int on);
 /* Column groups of at least min_columns use products that share rows between columns
- * (FP32: row blocks or split-TF32 tensor-core tiles, whichever is faster at the slab's
- * width; FP64: 128 x 16 or 64 x 64 tiles), narrower ones rows of few columns.  FP32 groups of four
+ * (FP32: row blocks, 128 x 16 tiles or split-TF32 tensor-core tiles, whichever is faster at the
+ * slab's width; FP64: 128 x 16 or 64 x 64 tiles), narrower ones rows of few columns.  FP32 groups of four
  * or more columns count together.  Default 8. */
 int emg_slab_set_wide_group(emg_slab* slab, int min_columns);
 /* Cap on the K splits of the tiled products (1..16; default 8): clusters of up to 8
- * CTAs per FP32 tile, for FP64 two CTAs per SM with at least 256 K columns each. */
+ * CTAs per split-TF32 tile, else two CTAs per SM with at least 256 K columns each. */
 int emg_slab_set_max_splits(emg_slab* slab, int max_splits);
 
 /* Flexible GMRES (FGMRES, restart <= 256) right-preconditioned by the slab
