@@ -436,28 +436,34 @@ __device__ __forceinline__ void cmadd(double2& s, double2 a, double2 b) {   // s
     s.y = fma(a.y, b.x, s.y);
 }
 
-constexpr int kNewton = 3;
-constexpr float kNewtonDone = 1e-8f;
-struct NewtonWork {                    // per factor; R also holds the lookahead's row tile
-    double2 X[2][kTile * kTile], R[kTile * kTile];
+constexpr int kPowers = 4;
+struct TileWork {                      // per factor; R also holds the lookahead's row tile
+    double2 X[kTile * kTile], R[kTile * kTile], P[kTile * kTile], A[kTile * kTile], Q[kTile * kTile];
     float2 seed[kTile * kTile];
-    unsigned rmax[kNewton];            // largest |entry| of R of each step, as float bits
+    int32_t rexp[kTile];               // biased exponent of the largest entry of each row of the tile
+    unsigned rmax[kPowers];            // largest |entry| of R, R^2, R^4, R^8, as float bits
     int32_t replaced;
-    unsigned pad[4];                     // a multiple of 16 bytes with the above
+    unsigned pad[3];                   // a multiple of 16 bytes with the above
 };
 
-// The CTA's 8 x 4 outputs of a 64 x 64 x 64 product: a(r, kk), b(kk, c) give the operands, the sum for
-// output (lane / 4, lane % 4) is returned to warp 0.
+// The CTA's 8 x 4 outputs of up to NA 64 x 64 x 64 products of one right operand (the second one if ``two``):
+// a(r, kk, v) gives the entries of the left operands, b(kk, c) that of the right one; the sums for output
+// (lane / 4, lane % 4) are returned to warp 0.
+template <int NA>
 struct Look {
-    double2 As[kLookRows][kTile + 1], Bs[kTile][kLookCols + 1], red[kTileThreads / 32][32];
+    double2 As[NA][kLookRows][kTile + 1], Bs[kTile][kLookCols + 1], red[NA][kTileThreads / 32][32];
 };
-template <class FA, class FB>
-__device__ __forceinline__ double2 look_block(Look& sm, FA a, FB b) {
+template <int NA, class FA, class FB>
+__device__ __forceinline__ void look_block(Look<NA>& sm, bool two, FA a, FB b, double2 (&s)[NA]) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 #pragma unroll
     for (int q = 0; q < kLookRows * kTile / kTileThreads; ++q) {
         const int i = tid + q * kTileThreads;
-        sm.As[i / kTile][i % kTile] = a(i / kTile, i % kTile);
+        double2 v[NA];
+        a(i / kTile, i % kTile, v);
+#pragma unroll
+        for (int m = 0; m < NA; ++m)
+            if (m == 0 || two) sm.As[m][i / kTile][i % kTile] = v[m];
     }
 #pragma unroll
     for (int q = 0; q < kLookCols * kTile / kTileThreads; ++q) {
@@ -466,24 +472,36 @@ __device__ __forceinline__ double2 look_block(Look& sm, FA a, FB b) {
     }
     __syncthreads();
     const int r = lane / kLookCols, c = lane % kLookCols;
-    double2 s = make_double2(0.0, 0.0);
 #pragma unroll
-    for (int kk = 0; kk < kTile / 4; ++kk) cmadd(s, sm.As[r][warp * (kTile / 4) + kk], sm.Bs[warp * (kTile / 4) + kk][c]);
-    sm.red[warp][lane] = s;
+    for (int m = 0; m < NA; ++m) s[m] = make_double2(0.0, 0.0);
+    if (NA == 1 || !two) {
+#pragma unroll
+        for (int kk = 0; kk < kTile / 4; ++kk) cmadd(s[0], sm.As[0][r][warp * (kTile / 4) + kk], sm.Bs[warp * (kTile / 4) + kk][c]);
+    } else {
+#pragma unroll
+        for (int kk = 0; kk < kTile / 4; ++kk) {
+            const double2 y = sm.Bs[warp * (kTile / 4) + kk][c];
+#pragma unroll
+            for (int m = 0; m < NA; ++m) cmadd(s[m], sm.As[m][r][warp * (kTile / 4) + kk], y);
+        }
+    }
+#pragma unroll
+    for (int m = 0; m < NA; ++m) sm.red[m][warp][lane] = s[m];
     __syncthreads();
     if (warp == 0) {
 #pragma unroll
-        for (int q = 1; q < kTileThreads / 32; ++q) {
-            s.x += sm.red[q][lane].x;
-            s.y += sm.red[q][lane].y;
-        }
+        for (int m = 0; m < NA; ++m)
+#pragma unroll
+            for (int q = 1; q < kTileThreads / 32; ++q) {
+                s[m].x += sm.red[m][q][lane].x;
+                s[m].y += sm.red[m][q][lane].y;
+            }
     }
-    return s;
 }
 
 __global__ void __launch_bounds__(kTileThreads) k_look64(int part, int64_t w, int k, int la, double2* Sinv, int64_t totD,
-                                                         int64_t offD, const double2* pinv, NewtonWork* work) {
-    __shared__ Look sm;
+                                                         int64_t offD, const double2* pinv, TileWork* work) {
+    __shared__ Look<1> sm;
     const int r0 = ((int)blockIdx.x / (kTile / kLookCols)) * kLookRows, c0 = ((int)blockIdx.x % (kTile / kLookCols)) * kLookCols;
     const int64_t f = blockIdx.z, k0 = (int64_t)k * kTile, l0 = (int64_t)la * kTile;
     double2* M = Sinv + f * totD + offD;
@@ -493,12 +511,14 @@ __global__ void __launch_bounds__(kTileThreads) k_look64(int part, int64_t w, in
     const double2 z2 = make_double2(0.0, 0.0);
     const double2* src = part == 0 ? M + k0 * w + l0 : rows;
     const int64_t ld = part == 0 ? w : kTile;
-    const double2 s = look_block(
-        sm,
-        [&](int r, int kk) {
-            return part == 0 ? P[(r0 + r) * kTile + kk] : r0 + r < nv ? M[(l0 + r0 + r) * w + k0 + kk] : z2;
+    double2 sums[1];
+    look_block<1>(
+        sm, false,
+        [&](int r, int kk, double2 (&v)[1]) {
+            v[0] = part == 0 ? P[(r0 + r) * kTile + kk] : r0 + r < nv ? M[(l0 + r0 + r) * w + k0 + kk] : z2;
         },
-        [&](int kk, int c) { return c0 + c < nv ? src[(int64_t)kk * ld + c0 + c] : z2; });
+        [&](int kk, int c) { return c0 + c < nv ? src[(int64_t)kk * ld + c0 + c] : z2; }, sums);
+    const double2 s = sums[0];
     const int r = r0 + (int)threadIdx.x / kLookCols, c = c0 + (int)threadIdx.x % kLookCols;
     if (threadIdx.x >= 32 || c >= nv) return;
     if (part == 0) {
@@ -510,46 +530,55 @@ __global__ void __launch_bounds__(kTileThreads) k_look64(int part, int64_t w, in
 }
 
 // The FP64 inverse of a pivot tile from an FP32 one.  k_seed64 inverts the tile T, scaled by a power of
-// two, in FP32 (emg_gj.cuh); then up to three Newton steps R = I - T X, X <- X + X R in FP64, 128 CTAs
-// each, square the residual: the step that meets a residual of at most 1e-8 ends with one of 1e-16,
-// the rounding of the FP64 products, which the exchange steps of k_tile64 have too, and stores the
-// result.  A tile that does not get there (a condition beyond some 1e5, a pivot to be replaced, values
-// beyond FP32, NaN) is left as it was and k_tile64 inverts it; else that returns at once.
-// A tile took 124 us in k_tile64 beside the products; the seed takes 36, a step two launches of 5.
-// One application's error against 64 bits, with the products above: geometric means over 12 frequencies of
-// six guides and filters 0.58 to 1.08 times (0.84 over all) those of FP64 exchange steps with FMAs.
-// step ``it`` met the bound of the residual's norm (64 times its largest entry), or is too far from it
-__device__ __forceinline__ bool newton_met(const NewtonWork& nw, int it) {
-    return 64.f * __uint_as_float(nw.rmax[it]) <= kNewtonDone;
-}
-
-__device__ __forceinline__ bool newton_lost(const NewtonWork& nw, int it) {
-    return __uint_as_float(nw.rmax[it]) > (it == 0 ? 0.1f : 1e-3f);
-}
+// two, in FP32 (emg_gj.cuh) and rounds it to 22 bits below each column's largest entry, X.  Then T^-1 =
+// X (1 + R + R^2 + ...), R = 1 - T X, in FP64, 128 CTAs a launch (k_series64).  R is formed once, and nearly
+// exactly: T = T1 + T2 with the 20 bits of T1 below its rows' largest entries, so that every
+// product and sum of T1 X is a multiple of one power of two and below 2^49 of it, exact in FP64, and
+// the rounding of T2 X is 2^-20 of that of T X.  The series is summed by doubling, with the powers of R beside it,
+//   X <- X + X R,  X <- X + X R^2,  X <- X + X R^4,  X <- X + X R^8,
+// until the norm of the power (64 times its largest entry) is 3e-9 and the rest, its square, 1e-17; what is added is
+// small beside X, and so is its rounding.  (Newton steps X <- X + X (1 - T X), which round 1 - T X of a final X, take
+// some 25 us where this takes 31.  Against FP64 exchange steps, the error of one application with
+// CUDA-core products, geometric means over 16 to 24 frequencies of two guides and two filters: theirs 1.05 to
+// 1.23 times, this 0.60 to 0.87; with the products above 0.38 to 0.59 on six.)  A tile that is not near
+// enough (a condition beyond some 1e5, a pivot to be replaced, values beyond FP32, NaN) is left as it was
+// and k_tile64 inverts it; else that returns at once.
+// A tile took 124 us in k_tile64 beside the products; the seed takes 37, a launch of the series 6 to 9.
+// R^(2^i) ends the series after its launch i + 1, or is too large for it to converge soon (also a NaN)
+__device__ __forceinline__ bool series_met(const TileWork& nw, int i) { return 64.f * __uint_as_float(nw.rmax[i]) <= 3e-9f; }
+__device__ __forceinline__ bool series_lost(const TileWork& nw, int i) { return !(__uint_as_float(nw.rmax[i]) <= 0.1f); }
 
 __global__ void __launch_bounds__(gj::kThreads, 1) k_seed64(int64_t w, int k, const double2* Sinv, int64_t totD, int64_t offD,
-                                                            NewtonWork* work) {
+                                                            TileWork* work) {
     __shared__ float2 Ts[kTile * gj::kLd];
     __shared__ gj::PivotShared sh;
-    __shared__ int s_e;
+    __shared__ int s_e, rexp[kTile];
+    __shared__ unsigned cmax[kTile];
     const int64_t f = blockIdx.z, k0 = (int64_t)k * kTile;
     const double2* M = Sinv + f * totD + offD + k0 * w + k0;
-    NewtonWork& nw = work[f];
+    TileWork& nw = work[f];
     const int tb = (int)min((int64_t)kTile, w - k0), tid = threadIdx.x;
     constexpr int kPer = kTile * kTile / gj::kThreads;
     if (tid == 0) s_e = 0;
-    if (tid < kNewton) nw.rmax[tid] = 0u;
+    if (tid < kPowers) nw.rmax[tid] = 0u;
     if (tid == 0) nw.replaced = 0;
+    if (tid < kTile) rexp[tid] = 0;
+    if (tid < kTile) cmax[tid] = 0u;
+    __syncthreads();
     double2 v[kPer];
     int e = 0;
 #pragma unroll
     for (int q = 0; q < kPer; ++q) {
         const int r = (tid + q * gj::kThreads) / kTile, c = tid % kTile;
         v[q] = (r < tb && c < tb) ? M[(int64_t)r * w + c] : make_double2(0.0, 0.0);
-        e = max(e, max(((unsigned)__double2hiint(v[q].x) >> 20) & 0x7ffu, ((unsigned)__double2hiint(v[q].y) >> 20) & 0x7ffu));
     }
-    e = __reduce_max_sync(0xffffffffu, e);
-    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {   // a warp's values are of one row
+        const int r = (tid + q * gj::kThreads) / kTile;
+        const int er = __reduce_max_sync(0xffffffffu, max(expo(v[q].x), expo(v[q].y)));
+        if ((tid & 31) == 0) atomicMax(&rexp[r], er);
+        e = max(e, er);
+    }
     if ((tid & 31) == 0) atomicMax(&s_e, e);
     __syncthreads();
     // 2^-(s_e - 1023): entries below 2; out of a double's normal range k_tile64 takes the tile
@@ -562,55 +591,100 @@ __global__ void __launch_bounds__(gj::kThreads, 1) k_seed64(int64_t w, int k, co
     }
     __syncthreads();
     gj::invert_tile(Ts, tb, 1e-6f, sh, &nw.replaced, nw.seed, kTile, nw.seed);
+    if (tid < kTile) nw.rexp[tid] = tid < tb ? rexp[tid] : 1023;
     __syncthreads();
+    // 22 bits below the column's largest entry: multiples of the last bit of 3 2^ec, |x| < 2^ec
+    float2 x[kPer];
+    unsigned top = 0u;
 #pragma unroll
     for (int q = 0; q < kPer; ++q) {
         const int i = tid + q * gj::kThreads, r = i / kTile, c = i % kTile;
-        const float2 x = nw.seed[i];
-        nw.X[0][i] = (r < tb && c < tb) ? make_double2(x.x * scale, x.y * scale) : make_double2(r == c ? 1.0 : 0.0, 0.0);
+        x[q] = (r < tb && c < tb) ? nw.seed[i] : make_float2(r == c ? 1.f : 0.f, 0.f);
+        top = max(top, max(__float_as_uint(x[q].x) & 0x7fffffffu, __float_as_uint(x[q].y) & 0x7fffffffu));
+    }
+    atomicMax(&cmax[tid % kTile], top);            // a thread's entries are of one column
+    __syncthreads();
+    const unsigned ec = (cmax[tid % kTile] >> 23) + 1u;   // biased; beyond FP32 the residual shows it
+    const float grid = ec < 253u ? 3.f * __uint_as_float(ec << 23) : 0.f;
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+        const int i = tid + q * gj::kThreads, r = i / kTile, c = i % kTile;
+        const float xr = __fsub_rn(__fadd_rn(x[q].x, grid), grid), xi = __fsub_rn(__fadd_rn(x[q].y, grid), grid);
+        const double sc = (r < tb && c < tb) ? scale : 1.0;
+        nw.X[i] = make_double2(xr * sc, xi * sc);
     }
 }
 
-// Newton step ``it``: part 0 forms R, part 1 the next X (the result if R met the bound).
-__global__ void __launch_bounds__(kTileThreads) k_newton64(int part, int it, int64_t w, int k, double2* Sinv, int64_t totD,
-                                                           int64_t offD, double2* pinv, NewtonWork* work) {
-    __shared__ Look sm;
+// Entry a of a row whose largest has biased exponent e: its bits down to 2^-20 of 2^(e - 1022) (the rest is a - this).
+__device__ __forceinline__ double top_bits(double a, int e) {
+    const int drop = e - expo(a) + 33;             // low bits of the 53
+    const long long b = __double_as_longlong(a);
+    return drop >= 53 ? 0.0 : __longlong_as_double(b & ~((1ll << drop) - 1));
+}
+
+// Launches 0 to 4 of a tile: R; X + X R and R^2; with R^2, and R^4; with R^4, and R^8; with R^8.  The one that ends the
+// series stores the inverse, the later ones return at once.  A buffer is written again when its last reader is
+// done: X and R; A and P; X and Q; A and R.
+template <int STAGE>
+__global__ void __launch_bounds__(kTileThreads) k_series64(int64_t w, int k, double2* Sinv, int64_t totD, int64_t offD,
+                                                           double2* pinv, TileWork* work) {
+    constexpr int NA = STAGE == 4 ? 1 : 2;
+    __shared__ Look<NA> sm;
     const int r0 = ((int)blockIdx.x / (kTile / kLookCols)) * kLookRows, c0 = ((int)blockIdx.x % (kTile / kLookCols)) * kLookCols;
     const int64_t f = blockIdx.z, k0 = (int64_t)k * kTile;
     double2* T = Sinv + f * totD + offD + k0 * w + k0;
-    NewtonWork& nw = work[f];
+    TileWork& nw = work[f];
     const int tb = (int)min((int64_t)kTile, w - k0);
     pdl_wait();
     pdl_trigger();                       // only now: waiting CTAs take shared memory from the products
-    for (int i = 0; i < it; ++i)
-        if (newton_met(nw, i) || newton_lost(nw, i)) return;   // done, or k_tile64's, since an earlier step
-    const double2* X = nw.X[it & 1];
-    const double2 s = look_block(
-        sm,
-        [&](int r, int kk) {
+    bool last = false;
+    if constexpr (STAGE > 0) {
+#pragma unroll
+        for (int i = 0; i < STAGE; ++i)
+            if (series_lost(nw, i) || (i + 1 < STAGE && series_met(nw, i))) return;   // k_tile64's, or done
+        last = series_met(nw, STAGE - 1);
+        if (STAGE == kPowers && !last) return;
+    }
+    const double2* left = STAGE == 2 || STAGE == 4 ? nw.A : nw.X;         // the sum so far
+    const double2* right = STAGE == 0 ? nw.X : STAGE == 2 ? nw.P : STAGE == 3 ? nw.Q : nw.R;   // the power of R
+    double2 s[NA];
+    look_block<NA>(
+        sm, NA == 2 && !last,
+        [&](int r, int kk, double2 (&v)[NA]) {
             r += r0;
-            if (part == 1) return X[r * kTile + kk];
-            return r < tb && kk < tb ? T[(int64_t)r * w + kk] : make_double2(r == kk ? 1.0 : 0.0, 0.0);
+            if constexpr (STAGE == 0) {
+                const double2 a = r < tb && kk < tb ? T[(int64_t)r * w + kk] : make_double2(r == kk ? 1.0 : 0.0, 0.0);
+                const int e = nw.rexp[r];
+                v[0] = make_double2(top_bits(a.x, e), top_bits(a.y, e));
+                v[1] = make_double2(a.x - v[0].x, a.y - v[0].y);
+            } else {
+                v[0] = left[r * kTile + kk];
+                if constexpr (NA == 2) v[1] = last ? make_double2(0.0, 0.0) : right[r * kTile + kk];
+            }
         },
-        [&](int kk, int c) { return (part == 0 ? X : nw.R)[kk * kTile + c0 + c]; });
+        [&](int kk, int c) { return right[kk * kTile + c0 + c]; }, s);
     if (threadIdx.x >= 32) return;
-    const int r = r0 + (int)threadIdx.x / kLookCols, c = c0 + (int)threadIdx.x % kLookCols;
-    if (part == 0) {
-        const double2 v = make_double2((r == c ? 1.0 : 0.0) - s.x, -s.y);
-        nw.R[r * kTile + c] = v;
-        const double m = fmax(fabs(v.x), fabs(v.y));
-        const float mf = (m <= 3e38 && v.x == v.x && v.y == v.y) ? __double2float_ru(m) : __int_as_float(0x7f800000);
-        const unsigned best = __reduce_max_sync(0xffffffffu, __float_as_uint(mf));
-        if (threadIdx.x == 0) atomicMax(&nw.rmax[it], best);
+    const int r = r0 + (int)threadIdx.x / kLookCols, c = c0 + (int)threadIdx.x % kLookCols, o = r * kTile + c;
+    double2 p = s[NA - 1];               // the next power, or R
+    if constexpr (STAGE == 0) {
+        p = make_double2((r == c ? 1.0 : 0.0) - s[0].x - s[1].x, -s[0].y - s[1].y);
     } else {
-        const double2 x = X[r * kTile + c], v = make_double2(x.x + s.x, x.y + s.y);
-        if (!newton_met(nw, it)) {
-            nw.X[(it + 1) & 1][r * kTile + c] = v;
-        } else if (r < tb && c < tb) {
-            T[(int64_t)r * w + c] = v;
-            pinv[(f * kTile + r) * kTile + c] = v;
+        const double2 x = left[o], v = make_double2(x.x + s[0].x, x.y + s[0].y);
+        if (!last) {
+            (STAGE == 2 ? nw.X : nw.A)[o] = v;
+        } else {
+            if (r < tb && c < tb) {
+                T[(int64_t)r * w + c] = v;
+                pinv[(f * kTile + r) * kTile + c] = v;
+            }
+            return;
         }
     }
+    (STAGE == 1 ? nw.P : STAGE == 2 ? nw.Q : nw.R)[o] = p;
+    const double m = fmax(fabs(p.x), fabs(p.y));
+    const float mf = (m <= 3e38 && p.x == p.x && p.y == p.y) ? __double2float_ru(m) : __int_as_float(0x7f800000);
+    const unsigned best = __reduce_max_sync(0xffffffffu, __float_as_uint(mf));
+    if (threadIdx.x == 0) atomicMax(&nw.rmax[min(STAGE, kPowers - 1)], best);
 }
 
 // FP64 inverse of pivot tile k by a cluster of 16 CTAs of 128 threads: in-place Gauss-Jordan exchange
@@ -621,7 +695,7 @@ __global__ void __launch_bounds__(kTileThreads) k_newton64(int part, int it, int
 // FP64 pipes.  Pivots compare max(|re|, |im|) (14 bits of it, the lowest row on ties); a pivot of
 // |a|^2 at or below rel_thr^2 max|a|^2 is replaced by that threshold and counted.  One CTA took
 // 600 us a tile (85 % of its FP64 pipe), this 115 (124 while products run beside it).  It takes the
-// tiles that the Newton steps leave.
+// tiles that the series leaves.
 constexpr int kRanks = 16, kPc = 4;
 
 __device__ __forceinline__ double2 remote(const double2* p, int rank) {
@@ -637,7 +711,7 @@ __device__ __forceinline__ void cluster_sync() {
 }
 __global__ void __launch_bounds__(kTileThreads) k_tile64(int64_t w, int k, double2* __restrict__ Sinv, int64_t totD,
                                                          int64_t offD, double2* __restrict__ pinv, double rel_thr,
-                                                         int32_t* __restrict__ perturbed, const NewtonWork* __restrict__ work) {
+                                                         int32_t* __restrict__ perturbed, const TileWork* __restrict__ work) {
     struct __align__(16) Shared {
         double2 V[kTile][kPc];                 // multipliers of this CTA's panel
         double2 row[2][kTileThreads / 32][kPc];   // candidate row of each warp
@@ -652,9 +726,9 @@ __global__ void __launch_bounds__(kTileThreads) k_tile64(int64_t w, int k, doubl
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, r = tid >> 1, h = tid & 1;
     const int rank = (int)blockIdx.x;
     const int64_t f = blockIdx.z, k0 = (int64_t)k * kTile;
-    for (int i = 0; i < kNewton; ++i) {     // uniform over the cluster
-        if (newton_lost(work[f], i)) break;
-        if (newton_met(work[f], i)) return;   // the inverse is there
+    for (int i = 0; i < kPowers; ++i) {     // uniform over the cluster
+        if (series_lost(work[f], i)) break;
+        if (series_met(work[f], i)) return;   // the inverse is there
     }
     double2* M = Sinv + f * totD + offD + k0 * w + k0;
     const int tb = (int)min((int64_t)kTile, w - k0);
@@ -804,7 +878,7 @@ __global__ void __launch_bounds__(kTileThreads) k_tile64(int64_t w, int k, doubl
 }  // namespace f64
 
 // Launch hooks (declared in emg_krylov.cuh).
-int64_t fp64_tile_work() { return sizeof(f64::NewtonWork); }
+int64_t fp64_tile_work() { return sizeof(f64::TileWork); }
 
 int fp64_tile(int64_t w, int k, int64_t F, double2* Sinv, int64_t totD, int64_t offD, double2* pinv, double rel_thr,
               int32_t* perturbed, void* work, cudaStream_t st) {
@@ -818,17 +892,26 @@ int fp64_tile(int64_t w, int k, int64_t F, double2* Sinv, int64_t totD, int64_t 
         constexpr auto kCarve = cudaFuncAttributePreferredSharedMemoryCarveout;
         EMG_CUDA(cudaFuncSetAttribute(f64::k_tile64, kCarve, cudaSharedmemCarveoutMaxShared));
         EMG_CUDA(cudaFuncSetAttribute(f64::k_seed64, kCarve, cudaSharedmemCarveoutMaxShared));
-        EMG_CUDA(cudaFuncSetAttribute(f64::k_newton64, kCarve, cudaSharedmemCarveoutMaxShared));
+        EMG_CUDA(cudaFuncSetAttribute(f64::k_series64<0>, kCarve, cudaSharedmemCarveoutMaxShared));
+        EMG_CUDA(cudaFuncSetAttribute(f64::k_series64<1>, kCarve, cudaSharedmemCarveoutMaxShared));
+        EMG_CUDA(cudaFuncSetAttribute(f64::k_series64<2>, kCarve, cudaSharedmemCarveoutMaxShared));
+        EMG_CUDA(cudaFuncSetAttribute(f64::k_series64<3>, kCarve, cudaSharedmemCarveoutMaxShared));
+        EMG_CUDA(cudaFuncSetAttribute(f64::k_series64<4>, kCarve, cudaSharedmemCarveoutMaxShared));
         EMG_CUDA(cudaFuncSetAttribute(f64::k_look64, kCarve, cudaSharedmemCarveoutMaxShared));
         if (dev < 64) attr[dev] = true;
     }
-    auto* nw = static_cast<f64::NewtonWork*>(work);
+    auto* nw = static_cast<f64::TileWork*>(work);
     f64::k_seed64<<<dim3(1, 1, (unsigned)F), gj::kThreads, 0, st>>>(w, k, Sinv, totD, offD, nw);
     EMG_CUDA(cudaGetLastError());
-    for (int it = 0; it < f64::kNewton; ++it)
-        for (int part = 0; part < 2; ++part)
-            EMG_CUDA(launch_pdl(f64::k_newton64, dim3(f64::kLookCtas, 1, (unsigned)F), dim3(f64::kTileThreads), 0, st, 0, part,
-                                it, w, k, Sinv, totD, offD, pinv, nw));
+    for (int i = 0; i < 5; ++i) {
+        auto stage = i == 0   ? f64::k_series64<0>
+                     : i == 1 ? f64::k_series64<1>
+                     : i == 2 ? f64::k_series64<2>
+                     : i == 3 ? f64::k_series64<3>
+                              : f64::k_series64<4>;
+        EMG_CUDA(launch_pdl(stage, dim3(f64::kLookCtas, 1, (unsigned)F), dim3(f64::kTileThreads), 0, st, 0, w, k, Sinv, totD, offD,
+                            pinv, nw));
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(f64::kRanks, 1, (unsigned)F);
     cfg.blockDim = dim3(f64::kTileThreads);
@@ -841,7 +924,7 @@ int fp64_tile(int64_t w, int k, int64_t F, double2* Sinv, int64_t totD, int64_t 
     cfg.attrs = la;
     cfg.numAttrs = 1;
     EMG_CUDA(cudaLaunchKernelEx(&cfg, f64::k_tile64, w, k, Sinv, totD, offD, pinv, rel_thr, perturbed,
-                                static_cast<const f64::NewtonWork*>(nw)));
+                                static_cast<const f64::TileWork*>(nw)));
     return EMG_OK;
 }
 
@@ -865,7 +948,7 @@ int fp64_step(int stage, int64_t w, int k, int la, int64_t F, double2* Sinv, int
         for (int part = 0; part < 2; ++part)
             f64::k_look64<<<dim3(f64::kLookCtas, 1, (unsigned)F), f64::kTileThreads, 0, st>>>(part, w, k, la, Sinv, totD, offD,
                                                                                             pinv,
-                                                                                            static_cast<f64::NewtonWork*>(work));
+                                                                                            static_cast<f64::TileWork*>(work));
     else if (stage == 1)
         f64::k_prod64<f64::kRow><<<dim3(2 * nct + nt, 1, (unsigned)F), f64::kThreads, sm, st>>>(
             w, k, la, Sinv, totD, offD, pinv, rows, cols, sbuf, status);

@@ -1412,9 +1412,9 @@ int slab_factor_t(emg_slab* s, int64_t F, const int32_t* amat_h, int64_t Bm, con
             // FP64: the pivot tiles have the side stream, row panel and update the caller's.  Tile k + 1
             // needs tile k and the update of step k - 1; the row panel of step k needs tile k, its
             // update overwrites what the lookahead reads.  A step is the longer of the two chains:
-            // row panel 37 us and update 37 (480 wide) to 105 (1250), or lookahead 10, seed 36 and
-            // Newton steps 25 (311 tiles of 737 on average: 43.4 ms a solve; at 42.8 it took 46.5 with the lookahead
-            // before the row panel on one stream).
+            // row panel 37 us and update 37 (480 wide) to 105 (1250), or lookahead 10, seed 37 and
+            // series 31 (311 tiles of 737 on average: 44.6 ms a solve; with the lookahead before the row
+            // panel on one stream 9 % more).
             if constexpr (sizeof(R) == 8) {
                 auto step = [&](int q, int k, int la, cudaStream_t ts) {
                     return emg::fp64_step(q, w, k, la, F, Sinv, s->totD, s->offD[i], pset(k), rowbuf, colbuf, s->maxw * kTile,

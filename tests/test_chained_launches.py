@@ -47,7 +47,7 @@ def _chained():
 
 def test_loads_after_the_wait():
     funcs, kernels = _functions(), _chained()
-    assert {"k_scales", "k_fill_small", "k_newton64", "k_gj_row", "k_couple", "k_rowmv", "k_rows8", "k_slab_split",
+    assert {"k_scales", "k_fill_small", "k_series64", "k_gj_row", "k_couple", "k_rowmv", "k_rows8", "k_slab_split",
             "k_gj_update_tc"} <= kernels <= set(funcs)
     bad = []
     for kernel in sorted(kernels):

@@ -173,3 +173,22 @@ def test_pivots_at_the_ends_of_the_range(torch_cuda, scale):
     assert np.all(np.abs(Y - ref)[~apart] <= 64 * n * EPS * np.max(np.abs(ref), axis=1)[~apart, None])
     # the pair, condition 2^26: the residual of each entry against the magnitudes of its products
     assert np.all(np.abs(K @ Y - np.eye(n - 1)) <= 64 * n * EPS * (np.abs(K) @ np.abs(Y)) + 64 * n * EPS)
+
+
+@pytest.mark.parametrize("n", [1, 17, 40, 64])
+@pytest.mark.parametrize("cond", [1e1, 1e2, 1e3, 1e4])
+def test_tile_inverse_is_near_its_rounding(torch_cuda, n, cond):
+    """One pivot tile from its FP32 inverse: the residual is formed nearly exactly, so the error is the
+    rounding of the result, not that times the condition."""
+    torch = torch_cuda
+    sysr, slab = _dense_system(torch, n)
+    U, V = (torch.linalg.qr(_matrix(torch, n, s) - 3.0 * torch.eye(n, device="cuda"))[0] for s in (31, 32))
+    A = (U * torch.logspace(0, -np.log10(cond), n, dtype=torch.float64, device="cuda")) @ V
+    slab.factor(A.reshape(-1, 1).contiguous(), [0], "fp64")
+    X = slab.apply(torch.eye(n, dtype=torch.complex128, device="cuda"), [0] * n).cpu().numpy()
+    T = A.cpu().numpy().astype(np.clongdouble)
+    ref = np.linalg.inv(A.cpu().numpy()).astype(np.clongdouble)
+    for _ in range(3):
+        ref = ref + ref @ (np.eye(n) - T @ ref)
+    # three or four sums of half an eps of the largest entry and products with a residual below 0.1
+    assert np.max(np.abs(X - ref)) <= 8 * EPS * np.max(np.abs(ref))
